@@ -338,8 +338,9 @@ def _total(case):
 
 def _slot(case):
     """Bytes per planted match."""
-    return {"host": 4 * KIB, "stream": 16 * KIB, "literals": 16 * KIB, "regex": 16 * KIB, "anchored": 4 * KIB,
-            "unbounded": 16 * KIB, "batch": 16 * KIB, "dna": MIB}[case["kind"]]
+    if case["kind"] in ("literals", "regex", "anchored", "unbounded"):
+        return 16 * KIB if case["bytes"] > 256 * MIB else 64 * KIB if case["bytes"] > 4 * MIB else 4 * KIB
+    return {"host": 4 * KIB, "stream": 16 * KIB, "batch": 16 * KIB, "dna": MIB}[case["kind"]]
 
 
 def _input(case, seed, texts, dev):
@@ -366,8 +367,8 @@ def prepare(case, seed):
     if kind == "stream":
         return {"kind": kind, "pipeline": ws.StreamPipeline.new(matcher), "data": data.cpu().numpy(),
                 "piece": case["piece"]}
-    # room for twice the matches that are expected
-    cap = 1 << max(12, int(2 * (n // _slot(case) + n // (64 * KIB) + n * chance + 512)).bit_length())
+    # room for half as many matches again as are expected
+    cap = 1 << int(1.5 * (n // _slot(case) + n // (4 * MIB) + n * chance + 256)).bit_length()
     state = {"kind": kind, "matcher": matcher, "data": data, "bytes": n, "cap": cap,
              "count": torch.zeros(1, dtype=torch.int64, device=dev), "place": torch.arange(cap, device=dev),
              "last": torch.full((1,), LAST, device=dev)}
