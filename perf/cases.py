@@ -362,13 +362,14 @@ def prepare(case, seed):
     matcher, texts, chance = _matcher_of(case)
     dev, kind, n = "cuda:0", case["kind"], _total(case)
     data = _input(case, seed, texts, dev)
-    if kind == "host":
-        return {"kind": kind, "matcher": matcher, "data": data.cpu().numpy().tobytes()}
-    if kind == "stream":
-        return {"kind": kind, "pipeline": ws.StreamPipeline.new(matcher), "data": data.cpu().numpy(),
-                "piece": case["piece"]}
     # room for half as many matches again as are expected
     cap = 1 << int(1.5 * (n // _slot(case) + n // (4 * MIB) + n * chance + 256)).bit_length()
+    if kind == "host":
+        return {"kind": kind, "matcher": matcher, "data": data.cpu().numpy().tobytes(),
+                "table": np.zeros((cap, 3), dtype=np.int64)}
+    if kind == "stream":
+        return {"kind": kind, "pipeline": ws.StreamPipeline.new(matcher), "data": data.cpu().numpy(),
+                "piece": case["piece"], "table": np.zeros((cap, 3), dtype=np.int64)}
     state = {"kind": kind, "matcher": matcher, "data": data, "bytes": n, "cap": cap,
              "count": torch.zeros(1, dtype=torch.int64, device=dev), "place": torch.arange(cap, device=dev),
              "last": torch.full((1,), LAST, device=dev)}
@@ -391,10 +392,14 @@ def prepare(case, seed):
 
 def run(state):
     kind = state["kind"]
-    if kind == "host":
-        return state["matcher"].scan_array(state["data"])
-    if kind == "stream":
-        return state["pipeline"].scan_array(state["data"], block=state["piece"])
+    if kind in ("host", "stream"):  # the rows go into the program's own table
+        if kind == "host":
+            rows = state["matcher"].scan_array(state["data"])
+        else:
+            rows = state["pipeline"].scan_array(state["data"], block=state["piece"])
+        state["table"][:len(rows)] = rows
+        state["table"][len(rows):] = 0
+        return {"count": len(rows), "matches": state["table"]}
     m, stream = state["matcher"], torch.cuda.current_stream().cuda_stream
     data, out, count = state["data"].data_ptr(), state["out"].data_ptr(), state["count"].data_ptr()
     if kind == "batch":
