@@ -412,10 +412,8 @@ def build_matchers(ws, wl, config, walk_chunk=None, proposer=True, dfa_max_state
 def roofline_of(config, infos, n_bytes, count, n_items, batch, has_regex, peak, peak_kind):
     """The dominant kernel's achieved algorithmic bandwidth against the
     measured HBM peak (N input bytes + 12 B per match + 16 B per item)."""
-    # the literal phase (index 0) spans the filter and the verify kernel; the
-    # 10,000-literal set takes the large-set layout (stage-1b table, no literals
-    # under 4 bytes), whose filter is literal_lean_kernel
-    lit_name = "literal_lean_kernel" if config == "literals_large" else "literal_filter_kernel"
+    # the literal phase (index 0) spans the filter and the verify kernel
+    lit_name = "literal_gram_kernel"
 
     def phase(k):
         return statistics.mean(i["last_kernel_ms"][k] for i in infos) if infos else 0.0

@@ -92,21 +92,34 @@ struct DeviceBuffer {
 };
 
 // ------------------------------------------------------- literal device plan
-// Stage 1 of the literal scan: a sampled q-gram filter.  Every long literal
-// (length >= 4) registers its 4-byte grams at offsets k = 0..P-1 in a table of
-// 2^bits nibbles; bit (P-1-k) of entry hash(gram) records offset k.  A scan
-// position s can start a long literal only if the entry of the gram at the
-// first P-aligned position a >= s has bit (P-1-(a-s)) set.  Short literals
-// (length 1..3) register their first two bytes in a 64 Ki-bit table checked at
-// every position.  Stage 2 runs the reference's own FNV-1a probe of the
-// LiteralPrefilterTable at each surviving position and verifies exactly.
+// Stage 1 of the literal scan is a sampled q-gram filter: every string of the
+// set (the literals, and the prefixes the regexes' matches begin with) holds,
+// wherever it starts, one G-byte gram at a position that is a multiple of P, so
+// only those positions are looked up.  Two kernels:
+//   - the gram kernel (gram_kernel): sets without strings of one or two bytes,
+//     whose grams cover little of their alphabet's.  Stage 1 is a bitmap
+//     or a two-bit Bloom filter of the grams in shared memory, the phase bits (which
+//     offsets of a string have this gram) are a byte table in L2;
+//   - the compacting kernel for the others: 4-byte grams in a table of 2^bits
+//     nibbles (bit P - 1 - k of entry hash(gram) records offset k), strings of
+//     one to three bytes by their first two bytes in a 64 Ki-bit table checked
+//     at every position, and for low-entropy sets longer grams.
+// Stage 2 runs the reference's own FNV-1a probe of the LiteralPrefilterTable at
+// each surviving position and verifies exactly.
 struct LiteralPlan {
   uint32_t n_literals = 0;
+  uint32_t n_strings = 0;    // literals and regex prefixes: what the filter looks for
   uint32_t period = 4;       // P: 1, 2 or 4
   uint32_t table_bits = 18;  // 2^bits nibble entries
   uint32_t has_long = 0, has_short = 0;
   uint32_t max_len = 0;
   uint32_t parts = 0;                 // bit i: some literal has prefix length i+1
+  uint32_t bloom_parts = 0;           // the same over the literals and the regex prefixes
+  // Gram kernel: bitmap (gram_bits = 1) or two-bit blocked Bloom filter of the
+  // grams (2^gram_word_bits words) and their phase bits (2^phase_bits bytes).
+  bool gram_kernel = false;
+  uint32_t gram_bits = 1, gram_word_bits = 0, phase_bits = 0;
+  DeviceBuffer d_gram, d_phase;
   std::vector<uint32_t> filter;       // 2^bits nibbles packed 8 per word
   std::vector<uint32_t> bloom;        // 2^18-bit Bloom bitmap of prefix hashes
   std::vector<uint32_t> short_bits;   // 65536 bits
@@ -115,7 +128,7 @@ struct LiteralPlan {
   // Low-entropy pattern sets (e.g. nucleotide k-mers) saturate 4-byte grams:
   // stage 1 then hashes longer grams (gram_len 8 or 16 bytes) and stage 1.5
   // adds a second, L2-resident Bloom bitmap of the first min(len, 16) bytes.
-  uint32_t gram_len = 4;
+  uint32_t gram_len = 4;              // (3 when the gram kernel serves a set whose shortest literal has 3 bytes)
   uint32_t parts16 = 0;               // bit i: some literal has a key of i+1 bytes (<= 16)
   std::vector<uint32_t> bloom2;       // 2^kBloom2Bits bits, only when gram_len > 4
   // Large pattern sets fill the shared-memory gram table: a second table of
@@ -155,9 +168,37 @@ __host__ __device__ inline uint32_t ascii_fold4(uint32_t w) {
   return w | (upper >> 2);
 }
 
+// Gram hash of the gram kernel: a multiplicative hash of 3 or 4 bytes (the
+// constant is 2^32 / phi, shifted for three bytes so that the word's top byte
+// drops out) or the sum of four such products for 16 bytes.  (The high half of
+// a 64-bit product mixes better but measured slower: three more instructions a
+// gram.)  The filter's word comes from the top bits, the one or two bits in it
+// from the five-bit fields below.
+__host__ __device__ inline uint32_t gram_hash32(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, int gram_len) {
+  if (gram_len == 3) return w0 * 0x3779B100u;
+  if (gram_len == 4) return w0 * 0x9E3779B1u;
+  return w0 * 0x9E3779B1u + w1 * 0x85EBCA77u + w2 * 0xC2B2AE3Du + w3 * 0x27D4EB2Fu;
+}
+constexpr uint32_t kGramWords = 15;  // log2 of the filter's words at most (128 KiB of shared memory)
+
+// Multiply-add hash of 2 or 4 words with a final avalanche (xor-shift,
+// multiply, xor-shift), for long grams and 16-byte prefix keys.
+__host__ __device__ inline uint32_t mix_words(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t salt) {
+  uint32_t h = w0 * 0x9E3779B1u + w1 * 0x85EBCA77u + w2 * 0xC2B2AE3Du + w3 * 0x27D4EB2Fu + salt * 0x165667B1u;
+  h ^= h >> 15;
+  h *= 0x2C1B3C6Du;
+  h ^= h >> 12;
+  return h;
+}
+
+// Key of the gram kernel's phase table (its top phase_bits bits).
+__host__ __device__ inline uint32_t phase_key(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, int gram_len) {
+  return mix_words(gram_len == 3 ? w0 & 0xFFFFFFu : w0, w1, w2, w3, (uint32_t)gram_len);
+}
+
 constexpr uint32_t kBloom2Bits = 24;  // 2 MiB, read through L2
 constexpr uint32_t kBigBits = 25;     // stage-1b table: 2^25 bytes, 32 MiB, read through L2
-constexpr uint32_t kLeanBits = 20;    // stage 1 of the lean kernel: a 2^20-bit bitmap, 128 KiB of shared memory
+constexpr uint32_t kLeanBits = 20;    // its stage 1: a 2^20-bit bitmap, 128 KiB of shared memory
 
 // Blocked Bloom filter of stage 1 for long grams with the stage-1b table: the
 // word of 32-bit gram hash hf (its top kLeanBits - 5 bits) and the two bits
@@ -170,16 +211,6 @@ __host__ __device__ inline uint32_t lean2_mask(uint32_t hf) {
 
 // Gram hash of stage 1 (a multiplicative hash; the constant is 2^32 / phi).
 inline uint32_t gram_hash(uint32_t gram, uint32_t bits) { return (gram * 0x9E3779B1u) >> (32 - bits); }
-
-// Multiply-add hash of 2 or 4 words with a final avalanche (xor-shift,
-// multiply, xor-shift), for long grams and 16-byte prefix keys.
-__host__ __device__ inline uint32_t mix_words(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t salt) {
-  uint32_t h = w0 * 0x9E3779B1u + w1 * 0x85EBCA77u + w2 * 0xC2B2AE3Du + w3 * 0x27D4EB2Fu + salt * 0x165667B1u;
-  h ^= h >> 15;
-  h *= 0x2C1B3C6Du;
-  h ^= h >> 12;
-  return h;
-}
 
 // Stage-1 key of a gram of 4, 8 or 16 bytes (g[0..gram_len/4)).
 __host__ __device__ inline uint32_t long_gram_hash(uint32_t g0, uint32_t g1, uint32_t g2, uint32_t g3, uint32_t gram_len,
@@ -200,7 +231,9 @@ __host__ __device__ inline uint32_t prefix16_key(uint32_t x0, uint32_t x1, uint3
          (32 - kBloom2Bits);
 }
 
-void plan_literals(const ws_pattern_tables& t, LiteralPlan& plan);
+// `prefixes`: strings of at least 4 bytes that are filtered with the literals
+// (regex prefixes); positions where one starts are survivors.
+void plan_literals(const ws_pattern_tables& t, LiteralPlan& plan, const std::vector<std::string>& prefixes = {});
 
 // Kernel launchers (ws_literal.cu).
 struct LiteralLaunch {

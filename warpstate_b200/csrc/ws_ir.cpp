@@ -95,9 +95,75 @@ void DeviceBuffer::upload(const void* src, size_t n) {
   if (n && src) check_cuda(cudaMemcpy(ptr, src, n, cudaMemcpyHostToDevice), "cudaMemcpy H2D");
 }
 
-void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan) {
+namespace {
+
+struct FilterString {
+  const uint8_t* p;
+  uint32_t len;
+};
+
+// Distinct G-byte grams of the strings at offsets 0..P-1, as a share of all
+// G-byte grams over the bytes the strings use (G <= 4).
+double gram_coverage(const std::vector<FilterString>& strings, uint32_t P, uint32_t G) {
+  bool seen[256] = {};
+  std::vector<uint32_t> grams;
+  for (const FilterString& f : strings) {
+    for (uint32_t k = 0; k < f.len; ++k) seen[f.p[k]] = true;
+    for (uint32_t k = 0; f.len >= G && k < P && k + G <= f.len; ++k) {
+      uint32_t g = 0;
+      std::memcpy(&g, f.p + k, G);
+      grams.push_back(g);
+    }
+  }
+  std::sort(grams.begin(), grams.end());
+  const double distinct = (double)(std::unique(grams.begin(), grams.end()) - grams.begin());
+  double alphabet = 0, all = 1;
+  for (bool b : seen) alphabet += b ? 1.0 : 0.0;
+  for (uint32_t k = 0; k < G; ++k) all *= alphabet;
+  return distinct / std::min(std::max(all, 1.0), 4294967296.0);
+}
+
+// Tables of the gram kernel.  Stage 1 has 1,024 bits a gram (0.1% of other
+// grams pass), from 4 KiB for small sets (it is staged per block) up to
+// 128 KiB; from 8,192 grams on, where one bit of that would let 0.8% pass, two
+// bits per gram.  The phase table has 64 bytes a gram, up to 32 MiB.
+void build_gram_tables(const std::vector<FilterString>& strings, LiteralPlan& plan) {
+  const uint32_t P = plan.period, G = plan.gram_len;
+  struct Gram {
+    uint32_t hash, key;
+    uint8_t phase;
+  };
+  std::vector<Gram> grams;
+  for (const FilterString& f : strings)
+    for (uint32_t k = 0; k < P; ++k) {
+      uint32_t g[4] = {0, 0, 0, 0};
+      std::memcpy(g, f.p + k, G);
+      grams.push_back({gram_hash32(g[0], g[1], g[2], g[3], (int)G), phase_key(g[0], g[1], g[2], g[3], (int)G),
+                       (uint8_t)(1u << (P - 1 - k))});
+    }
+  uint32_t bits = 0;
+  while (bits < 25 && ((size_t)1 << bits) < grams.size()) ++bits;
+  plan.gram_bits = grams.size() >= 8192 ? 2 : 1;
+  plan.gram_word_bits = std::min<uint32_t>(std::max<uint32_t>(bits + 5, 10), kGramWords);
+  std::vector<uint32_t> words((size_t)1 << plan.gram_word_bits, 0u);
+  const uint32_t wb = plan.gram_word_bits;
+  for (const Gram& g : grams) {
+    words[g.hash >> (32 - wb)] |= 1u << ((g.hash >> (27 - wb)) & 31u);
+    if (plan.gram_bits == 2) words[g.hash >> (32 - wb)] |= 1u << ((g.hash >> (22 - wb)) & 31u);
+  }
+  plan.d_gram.upload(words.data(), words.size() * 4);
+  plan.phase_bits = std::min<uint32_t>(std::max<uint32_t>(bits + 6, 12), kBigBits);
+  std::vector<uint8_t> phase((size_t)1 << plan.phase_bits, 0);
+  for (const Gram& g : grams) phase[g.key >> (32 - plan.phase_bits)] |= g.phase;
+  plan.d_phase.upload(phase.data(), phase.size());
+}
+
+}  // namespace
+
+void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan, const std::vector<std::string>& prefixes) {
   plan.n_literals = given.n_literals;
-  if (given.n_literals == 0) return;
+  plan.n_strings = given.n_literals + (uint32_t)prefixes.size();
+  if (plan.n_strings == 0) return;
   // ASCII case-insensitive sets (PatternSetBuilder::case_insensitive,
   // core/src/pattern/compiler.rs:66-76, an Aho-Corasick automaton with
   // ascii_case_insensitive): every table below is planned on the literals
@@ -105,11 +171,14 @@ void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan) {
   // hashes, and the kernels fold the input the same way.
   ws_pattern_tables t = given;
   std::vector<uint8_t> folded;
+  std::vector<std::string> pre = prefixes;
   std::vector<uint32_t> foffsets, fhashes, fmeta, franges, fentries;
   plan.fold = given.case_insensitive != 0;
   if (plan.fold) {
     folded.assign(given.packed_bytes, given.packed_bytes + given.packed_len);
     for (uint8_t& c : folded) c = ascii_fold(c);
+    for (std::string& x : pre)
+      for (char& c : x) c = (char)ascii_fold((uint8_t)c);
     foffsets.assign(given.offsets, given.offsets + 2 * (size_t)given.n_literals);
     for (uint32_t li = 0; li < given.n_literals; ++li)
       fhashes.push_back(fnv1a(folded.data() + foffsets[2 * li], foffsets[2 * li + 1], HASH_WINDOW));
@@ -121,131 +190,116 @@ void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan) {
     t.n_buckets = (uint32_t)(franges.size() / 2);
     t.entries = fentries.data();
   }
-  uint32_t min_long = UINT32_MAX;
+  std::vector<FilterString> strings;
+  for (uint32_t li = 0; li < t.n_literals; ++li)
+    strings.push_back({t.packed_bytes + t.offsets[2 * li], t.offsets[2 * li + 1]});
+  for (const std::string& x : pre) strings.push_back({reinterpret_cast<const uint8_t*>(x.data()), (uint32_t)x.size()});
+  uint32_t min_len = UINT32_MAX, min_long = UINT32_MAX;
   plan.max_len = 0;
-  for (uint32_t li = 0; li < t.n_literals; ++li) {
-    uint32_t len = t.offsets[2 * li + 1];
-    plan.max_len = std::max(plan.max_len, len);
-    if (len >= 4) { plan.has_long = 1; min_long = std::min(min_long, len); }
+  for (const FilterString& f : strings) {
+    plan.max_len = std::max(plan.max_len, f.len);
+    min_len = std::min(min_len, f.len);
+    if (f.len >= 4) { plan.has_long = 1; min_long = std::min(min_long, f.len); }
     else plan.has_short = 1;
   }
-  // P grams at offsets 0..P-1 must fit inside every long literal: P + 3 <= len.
+  // P grams at offsets 0..P-1 must fit inside every long string: P + 3 <= len.
   plan.period = !plan.has_long ? 4 : (min_long >= 7) ? 4 : (min_long >= 5) ? 2 : 1;
   plan.table_bits = 18;
-  const uint32_t P = plan.period, bits = plan.table_bits;
-  plan.filter.assign((size_t)1 << (bits - 3), 0);
-  plan.bloom.assign((size_t)1 << (18 - 5), 0);
-  plan.short_bits.assign(65536 / 32, 0);
-  plan.parts = 0;
+  // A low-entropy set (a small alphabet whose 4-grams the strings mostly
+  // cover, e.g. nucleotide k-mers) lets most input positions through 4-byte
+  // grams: it takes the longest gram every long string holds at all P phases.
+  const bool low_entropy = plan.has_long && plan.period == 4 && min_long >= 11 && gram_coverage(strings, 4, 4) > 0.25;
+  if (low_entropy) plan.gram_len = min_long >= 19 ? 16 : 8;
+  // The gram kernel verifies in a later kernel what passes, from a list of one
+  // survivor per 64 bytes of input.  Where an input over the set's own
+  // alphabet would crowd that list (the grams cover more than 1/64 of the
+  // alphabet's; a quarter for P = 4, whose lookups are a quarter as many),
+  // the compacting kernel checks prefixes inside the filter instead.  Shortest
+  // string of three bytes: 3-byte grams at every position.
+  if (low_entropy) {
+    plan.gram_kernel = plan.gram_len == 16 && !plan.has_short;
+  } else if (min_len == 3) {
+    plan.gram_kernel = gram_coverage(strings, 1, 3) <= 1.0 / 64;
+    if (plan.gram_kernel) {
+      plan.period = 1;
+      plan.gram_len = 3;
+    }
+  } else if (min_len >= 4) {
+    plan.gram_kernel = gram_coverage(strings, plan.period, 4) <= (plan.period == 4 ? 0.25 : 1.0 / 64);
+  }
+  const uint32_t P = plan.period, G = plan.gram_len, bits = plan.table_bits;
+  plan.parts = plan.bloom_parts = 0;
   plan.lit_info.assign(4 * (size_t)t.n_literals, 0);
   plan.lit_bytes.clear();
-  for (uint32_t li = 0; li < t.n_literals; ++li) {
-    uint32_t off = t.offsets[2 * li], len = t.offsets[2 * li + 1];
-    const uint8_t* lit = t.packed_bytes + off;
+  plan.bloom.assign((size_t)1 << (18 - 5), 0);
+  for (size_t k = 0; k < strings.size(); ++k) {
+    const uint32_t len = strings[k].len;
+    const uint8_t* lit = strings[k].p;
+    // Bloom bitmap of the first min(len, 8) bytes (the kernel's prefix_key)
+    const uint32_t pl = std::max<uint32_t>(std::min<uint32_t>(len, HASH_WINDOW), 1);
+    uint32_t x[2] = {0, 0};
+    std::memcpy(x, lit, pl);
+    const uint32_t key = (x[0] * 0x9E3779B1u + x[1] * 0x85EBCA77u + pl * 0xC2B2AE3Du) >> (32 - 18);
+    plan.bloom[key >> 5] |= 1u << (key & 31);
+    plan.bloom_parts |= 1u << (pl - 1);
+    if (k >= t.n_literals) continue;
+    plan.parts |= 1u << (pl - 1);
     while (plan.lit_bytes.size() % 4) plan.lit_bytes.push_back(0);
-    plan.lit_info[4 * li + 0] = (uint32_t)plan.lit_bytes.size();
-    plan.lit_info[4 * li + 1] = len;
-    plan.lit_info[4 * li + 2] = t.literal_pattern_ids[li];
+    plan.lit_info[4 * k + 0] = (uint32_t)plan.lit_bytes.size();
+    plan.lit_info[4 * k + 1] = len;
+    plan.lit_info[4 * k + 2] = t.literal_pattern_ids[k];
     plan.lit_bytes.insert(plan.lit_bytes.end(), lit, lit + len);
-    plan.parts16 |= 1u << (std::min<uint32_t>(std::max<uint32_t>(len, 1), 16) - 1);
-    {
-      // Bloom bitmap of the first min(len, 8) bytes (the kernel's prefix_key)
-      uint32_t pl = std::max<uint32_t>(std::min<uint32_t>(len, HASH_WINDOW), 1);
-      uint8_t x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      std::memcpy(x, lit, pl);
-      uint32_t lo, hi;
-      std::memcpy(&lo, x, 4);
-      std::memcpy(&hi, x + 4, 4);
-      uint32_t k = (lo * 0x9E3779B1u + hi * 0x85EBCA77u + pl * 0xC2B2AE3Du) >> (32 - 18);
-      plan.bloom[k >> 5] |= 1u << (k & 31);
-      plan.parts |= 1u << (pl - 1);
-    }
-    if (len >= 4) {
-      for (uint32_t k = 0; k < P; ++k) {
-        uint32_t gram;
-        std::memcpy(&gram, lit + k, 4);
-        uint32_t h = gram_hash(gram, bits);
-        plan.filter[h >> 3] |= (1u << (P - 1 - k)) << ((h & 7) * 4);
-      }
-    } else {
-      uint32_t b0 = lit[0];
-      if (len == 1) {
-        for (uint32_t b1 = 0; b1 < 256; ++b1) {
-          uint32_t key = b0 | (b1 << 8);
-          plan.short_bits[key >> 5] |= 1u << (key & 31);
-        }
-      } else {
-        uint32_t key = b0 | ((uint32_t)lit[1] << 8);
-        plan.short_bits[key >> 5] |= 1u << (key & 31);
-      }
-    }
   }
   while (plan.lit_bytes.size() % 16) plan.lit_bytes.push_back(0);
-  // A low-entropy pattern set (a small alphabet whose 4-grams the literals
-  // mostly cover, e.g. nucleotide k-mers) lets most input positions through
-  // 4-byte grams: then switch to the longest gram every long literal holds at
-  // all P phases, and add the 16-byte-prefix Bloom.
-  if (plan.has_long && P == 4) {
-    bool seen_byte[256] = {};
-    std::vector<uint32_t> grams;
-    for (uint32_t li = 0; li < t.n_literals; ++li) {
-      const uint32_t len = t.offsets[2 * li + 1];
-      const uint8_t* lit = t.packed_bytes + t.offsets[2 * li];
-      for (uint32_t k = 0; k < len; ++k) seen_byte[lit[k]] = true;
-      for (uint32_t k = 0; len >= 4 && k < P; ++k) {
-        uint32_t g;
-        std::memcpy(&g, lit + k, 4);
-        grams.push_back(g);
+  if (plan.gram_kernel) {
+    build_gram_tables(strings, plan);
+  } else {
+    // the compacting kernel's tables
+    plan.filter.assign((size_t)1 << (bits - 3), 0);
+    plan.short_bits.assign(65536 / 32, 0);
+    if (G > 4) plan.bloom2.assign((size_t)1 << (kBloom2Bits - 5), 0u);
+    plan.parts16 = 0;
+    for (const FilterString& f : strings) {
+      for (uint32_t k = 0; f.len >= 4 && k < P; ++k) {
+        uint32_t g[4] = {0, 0, 0, 0};
+        std::memcpy(g, f.p + k, G);
+        const uint32_t h = G == 4 ? gram_hash(g[0], bits) : long_gram_hash(g[0], g[1], g[2], g[3], G, bits);
+        plan.filter[h >> 3] |= (1u << (P - 1 - k)) << ((h & 7) * 4);
       }
-    }
-    std::sort(grams.begin(), grams.end());
-    const double distinct = (double)(std::unique(grams.begin(), grams.end()) - grams.begin());
-    double alphabet = 0;
-    for (bool b : seen_byte) alphabet += b ? 1.0 : 0.0;
-    const double coverage = distinct / std::min(alphabet * alphabet * alphabet * alphabet, 4294967296.0);
-    const uint32_t G = min_long >= 19 ? 16 : min_long >= 11 ? 8 : 4;
-    if (coverage > 0.25 && G > 4) {
-      plan.gram_len = G;
-      std::fill(plan.filter.begin(), plan.filter.end(), 0u);
-      plan.bloom2.assign((size_t)1 << (kBloom2Bits - 5), 0u);
-      for (uint32_t li = 0; li < t.n_literals; ++li) {
-        const uint32_t len = t.offsets[2 * li + 1];
-        const uint8_t* lit = t.packed_bytes + t.offsets[2 * li];
-        for (uint32_t k = 0; len >= 4 && k < P; ++k) {
-          uint32_t g[4] = {0, 0, 0, 0};
-          std::memcpy(g, lit + k, G);
-          uint32_t h = long_gram_hash(g[0], g[1], g[2], g[3], G, bits);
-          plan.filter[h >> 3] |= (1u << (P - 1 - k)) << ((h & 7) * 4);
+      if (f.len < 4) {
+        const uint32_t b0 = f.p[0];
+        for (uint32_t b1 = f.len == 1 ? 0 : f.p[1]; b1 < (f.len == 1 ? 256u : f.p[1] + 1u); ++b1) {
+          const uint32_t key = b0 | (b1 << 8);
+          plan.short_bits[key >> 5] |= 1u << (key & 31);
         }
-        // every literal (short ones too) is in the prefix Bloom
+      }
+      plan.parts16 |= 1u << (std::min<uint32_t>(std::max<uint32_t>(f.len, 1), 16) - 1);
+      if (G > 4) {  // every string (short ones too) is in the 16-byte-prefix Bloom
         uint32_t x[4] = {0, 0, 0, 0};
-        const uint32_t pl = std::min<uint32_t>(len, 16);
-        std::memcpy(x, lit, pl);
-        uint32_t key = prefix16_key(x[0], x[1], x[2], x[3], pl);
+        const uint32_t pl = std::min<uint32_t>(f.len, 16);
+        std::memcpy(x, f.p, pl);
+        const uint32_t key = prefix16_key(x[0], x[1], x[2], x[3], pl);
         plan.bloom2[key >> 5] |= 1u << (key & 31);
       }
-      plan.d_bloom2.upload(plan.bloom2.data(), plan.bloom2.size() * 4);
     }
+    if (G > 4) plan.d_bloom2.upload(plan.bloom2.data(), plan.bloom2.size() * 4);
   }
-  // Stage 1b: when more than 0.5% (P = 4) or 0.1% (P = 2: nine grams per
-  // 16 bytes, each passing one sends the warp block to compaction) of the
-  // shared table's phase bits are set, a 2^kBigBits-byte table in L2 (the
-  // same full 32-bit gram hashes, more of their bits) re-checks each passing
-  // gram.
-  if (plan.has_long && (P == 4 || P == 2)) {
+  // Stage 1b of the compacting kernel: when more than 0.5% (P = 4) or 0.1%
+  // (P = 2: nine grams per 16 bytes, each passing one sends the warp block to
+  // compaction) of the shared table's phase bits are set, a 2^kBigBits-byte
+  // table in L2 (the same full 32-bit gram hashes, more of their bits)
+  // re-checks each passing gram.
+  if (!plan.gram_kernel && plan.has_long && (P == 4 || P == 2)) {
     uint64_t set = 0;
     for (uint32_t w : plan.filter) set += (uint64_t)__builtin_popcount(w);
     if ((double)set / (double)((uint64_t)plan.filter.size() * 32) > (P == 4 ? 0.005 : 0.001)) {
-      const uint32_t G = plan.gram_len;
       plan.big.assign((size_t)1 << kBigBits, 0);
       std::vector<uint32_t> lean2(G > 4 ? (size_t)1 << (kLeanBits - 5) : 0, 0u);
-      for (uint32_t li = 0; li < t.n_literals; ++li) {
-        const uint32_t len = t.offsets[2 * li + 1];
-        const uint8_t* lit = t.packed_bytes + t.offsets[2 * li];
-        if (len < 4) continue;
+      for (const FilterString& f : strings) {
+        if (f.len < 4) continue;
         for (uint32_t k = 0; k < P; ++k) {
           uint32_t g[4] = {0, 0, 0, 0};
-          std::memcpy(g, lit + k, G);
+          std::memcpy(g, f.p + k, G);
           const uint32_t hf = G == 4 ? g[0] * 0x9E3779B1u
                               : G == 8 ? mix_words(g[0], g[1], 0, 0, 8)
                                        : mix_words(g[0], g[1], g[2], g[3], 16);

@@ -18,8 +18,10 @@
 //   survivors are appended to a compact position list with one atomic per warp
 //             (ballot + popc).  If the list is full, the position is verified in
 //             place instead, so results never depend on the list's capacity.
-// Kernel 1 for large sets, literal_lean_kernel (see its comment): stages 1 and
-//             1b only, no compaction; stage 1.5 moves to kernel 2.
+// Kernel 1 of most sets is literal_gram_kernel (see its comment): stage 1 only,
+//             no compaction; stage 1.5 moves to kernel 2.  The kernel above is
+//             for sets with literals of one or two bytes and for sets whose
+//             grams crowd their alphabet.
 // Kernel 2, literal_verify_kernel: the reference's per-position algorithm on the
 //             surviving positions only: FNV-1a probe of the LiteralPrefilterTable
 //             partition at each non-empty prefix length (shader.rs:59-98) and an
@@ -49,6 +51,7 @@ struct LitArgs {
   uint32_t has_long;
   uint32_t has_short;
   uint32_t parts;            // bit i: prefix length i+1 has literals
+  uint32_t bloom_parts;      // bit i: prefix length i+1 is in the prefix Bloom (literals, regex prefixes)
   const uint32_t* short_bits;
   const uint32_t* bloom;
   const uint4* info;
@@ -68,12 +71,18 @@ struct LitArgs {
   uint32_t n_items;
   uint64_t min_end;          // stream: matches ending at or before it were reported
   uint64_t max_start;        // shard: matches starting at or after it belong to the next shard
-  uint32_t gram_len;        // stage-1 gram bytes: 4, 8 or 16 (8 and 16 with P = 4)
+  uint32_t gram_len;        // stage-1 gram bytes: 3, 4, 8 or 16 (8 and 16 with P = 4)
   uint32_t parts16;          // stage-1.5b key lengths (bit i: i+1 bytes)
   const uint32_t* bloom2;    // stage-1.5b bitmap (2^kBloom2Bits bits, L2), or null
-  const uint8_t* big;        // stage-1b gram table (2^kBigBits bytes, L2), or null
-  const uint32_t* lean_bits; // stage 1 with the stage-1b table (2^kLeanBits bits), or null
+  const uint8_t* big;        // stage-1b gram table (2^kBigBits bytes, L2), or null (compacting kernel)
   uint32_t verify_bloom;     // the verify kernel runs stage 1.5 first
+  // gram kernel: stage 1 has 2^gram_word_bits words, the phase table
+  // 2^(32 - phase_shift) bytes
+  const uint32_t* gram_bloom;
+  uint32_t gram_word_bits;
+  const uint8_t* phase;
+  uint32_t phase_shift;
+  uint32_t slot_chunk;       // survivor slots a warp reserves at a time
   uint32_t fold;             // ASCII case-insensitive: input bytes A-Z read as a-z
 };
 
@@ -293,7 +302,7 @@ __device__ __forceinline__ void process_block(const LitArgs& a, uint32_t* blk, u
       const uint32_t wi = off >> 2, sh = (off & 3) * 8;
       const uint32_t x0 = blk[wi], x1 = blk[wi + 1], x2 = blk[wi + 2];
       const uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
-      for (uint32_t m = a.parts; m; m &= m - 1) {  // prefix lengths that have literals
+      for (uint32_t m = a.bloom_parts; m; m &= m - 1) {  // prefix lengths of the set
         const uint32_t key = prefix_key(lo, hi, __ffs(m));
         keep |= (bloom[key >> 5] >> (key & 31)) & 1u;
       }
@@ -574,62 +583,46 @@ __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(LitA
   }
 }
 
-// ------------------------------------------------------------- lean kernel
-// P = 4, 4-byte grams, stage-1b table present, no literals shorter than 4
-// bytes (the large-set layout).  Stage 1.5 moves to the verify kernel, so the
-// filter only hashes, looks up and appends:
-//   - ownership is shifted by 3: the lane with the 16 bytes at `base` owns the
-//     start positions base-3 .. base+12, whose first 4-aligned position is one
-//     of its own four words, so its own four grams decide all of them (bit t of
-//     n0 | n1 << 4 | n2 << 8 | n3 << 12 is position base - 3 + t) and no lane
-//     needs its neighbour's bytes.  The last three positions of the input start
-//     no literal of 4 or more bytes;
-//   - a warp step covers kLeanVecs coalesced 512-byte halves (32 bytes per
-//     lane), so the per-step overhead is paid once per kLeanVecs x 512 bytes;
-//   - stage 1 and the stage-1b loads run one warp step ahead of the step
-//     being finished, the input two steps ahead;
-//   - the stage-1b survivors of a warp step (about 0.15 per 512 bytes on
-//     10,000 literals) are appended into the warp's reserved slots of the
-//     list, one atomic per kLeanChunk slots (see lean_append).
-constexpr int kLeanThreads = 1024;
-constexpr int kLeanVecs = 2;  // 16-byte vectors per lane per warp step (a step covers kLeanVecs x 512 bytes)
+// ------------------------------------------------------------- gram kernel
+// Stage 1 for every set without literals of one or two bytes whose grams are
+// sparse enough in their alphabet (LiteralPlan::gram_kernel).  The filter only
+// hashes, looks up and appends; stage 1.5 moves to the verify kernel.
+//   - a literal of at least P + G - 1 bytes holds, wherever it starts, one
+//     G-byte gram at a position that is a multiple of P (G = 16 has P = 4), so
+//     16 / P grams per 16 bytes are tested.  A lane's grams are those at
+//     base - OFF + P * j (base the offset of its 16 bytes), all inside its own
+//     bytes and the few bytes before them, which come from the lane below;
+//   - stage 1 is a bitmap in shared memory (BITS = 1), or for crowded sets a
+//     blocked Bloom filter of two bits of one word per gram (BITS = 2), word
+//     and bits all from one multiplicative hash: the second bit costs two
+//     instructions and no second load, and squares the pass rate (10,000
+//     literals: 0.6% of the grams pass where one bit let 3.4% pass);
+//   - the warp takes kGramBits / NG vectors of 512 coalesced bytes in a row,
+//     one pass bit per gram in a 32-bit mask, and looks at the mask once: the
+//     passing grams go into the warp's queue in shared memory;
+//   - with 32 or more queued, every lane takes one: its phase bits (which
+//     offsets of a literal have this gram, a byte of a table in L2) give the
+//     start positions, which are appended to the warp's reserved slots of the
+//     list, one global atomic per slot_chunk slots.
+// One CTA of 1,024 threads per SM, four 512-byte loads in flight per warp.
+// What bounds it: the shared-memory lookups (a warp's 32 random words meet in
+// 3.4 wavefronts of the data pipe: 0.86 of it busy with P = 2, 0.91 with P = 1)
+// and, for P = 4, instruction issue (70 warp instructions per 512 bytes, the
+// data pipe 0.71 busy).  Measured, us per 256 MiB: 10,000 literals (P = 4) 57,
+// where the kernel before it (one bit, a vote and an append per 1 KiB step, its
+// candidates' L2 loads in the main loop) took 65; 500 literals of 5 bytes and
+// more (P = 2) 78, of 4 (P = 1) 134; 20,000 k-mers (G = 16) 81 against 164 for
+// the compacting kernel; 1,000 caseless literals of 3 and more over 97 MiB 69
+// against 184.
+constexpr int kGramThreads = 1024;
+constexpr uint32_t kGramWarps = kGramThreads / 32;
+constexpr uint32_t kGramQueue = 512;  // u32 positions per warp
+constexpr uint32_t kGramBits = 32;    // grams per lane and mask
+constexpr uint32_t kNoSurvivor = 0xFFFFFFFFu;  // no position: inputs are shorter than 2^32 bytes
 
-struct LeanGrams {
-  uint32_t bw[4];  // the stage-1b phase bits of the four grams (0: rejected by stage 1)
-};
-
-// Stage 1 of a lane's four aligned grams from the bitmap in shared memory
-// (top kLeanBits bits of the hash); the stage-1b loads from the byte table in
-// L2 (top kBigBits bits, the P phase bits) are issued for the grams that pass.
-__device__ __forceinline__ void lean_issue(const uint32_t* filt, const uint8_t* big, const uint4& v, LeanGrams& g) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const uint32_t hf = w[q] * 0x9E3779B1u;
-    const uint32_t b = hf >> (32 - kLeanBits);
-    const bool pass = (filt[b >> 5] >> (b & 31)) & 1u;
-    g.bw[q] = pass ? (uint32_t)__ldg(big + (hf >> (32 - kBigBits))) : 0u;
-  }
-}
-
-// Candidate mask of positions base-3 .. base+12 inside [0, len).
-__device__ __forceinline__ uint32_t lean_finish(const LeanGrams& g, uint32_t base, uint32_t len) {
-  uint32_t mask = 0;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) mask |= g.bw[q] << (4 * q);
-  if (base == 0) mask &= ~7u;  // positions -3 .. -1
-  if (base + 13 > len) {
-    const uint32_t valid = len + 3 > base ? len + 3 - base : 0;
-    mask &= valid >= 16 ? 0xFFFFu : ((1u << valid) - 1u);
-  }
-  return mask;
-}
-
-// Survivor slots are reserved per warp, kLeanChunk at a time, so that the
-// single global counter sees one atomic per chunk rather than one per warp
-// block; slots a warp reserved but did not fill hold kNoSurvivor.
-constexpr uint32_t kLeanChunk = 32;
-constexpr uint32_t kNoSurvivor = 0xFFFFFFFFu;  // no position: inputs end below 2^32 - 64
+// Bytes before its own that a lane's grams start at.
+template <int P, int G>
+__host__ __device__ constexpr int gram_off() { return G == 16 ? 12 : P == 4 ? 0 : P == 2 ? 2 : G == 3 ? 2 : 3; }
 
 struct LeanSlots {
   unsigned long long next = 0, end = 0;  // the warp's reserved range [next, end)
@@ -640,100 +633,229 @@ __device__ __forceinline__ void lean_holes(const LitArgs& a, const LeanSlots& r,
   for (unsigned long long k = r.next + lane; k < r.end && k < a.survivor_cap; k += 32) a.survivors[k] = kNoSurvivor;
 }
 
-template <int V>
-__device__ __forceinline__ void lean_append(const LitArgs& a, LeanSlots& r, const uint32_t (&mask)[V],
-                                            const uint32_t (&base)[V], uint32_t lane) {
-  uint32_t any = 0, cnt = 0;
-#pragma unroll
-  for (int h = 0; h < V; ++h) {
-    any |= mask[h];
-    cnt += __popc(mask[h]);
+// Stage 1.5 of position s: its first min(len, 8) bytes against the Bloom bitmap
+// of the literals' prefixes.
+__device__ __forceinline__ bool prefix_bloom(const LitArgs& a, uint32_t s) {
+  const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
+  const uint32_t x0 = input_word(a, len, w0), x1 = input_word(a, len, w0 + 4), x2 = input_word(a, len, w0 + 8);
+  const uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
+  bool keep = false;
+  for (uint32_t m = a.bloom_parts; m; m &= m - 1) {
+    const uint32_t key = prefix_key(lo, hi, __ffs(m));
+    keep |= (__ldg(a.bloom + (key >> 5)) >> (key & 31)) & 1u;
   }
-  if (__ballot_sync(0xFFFFFFFFu, any != 0) == 0) return;
-  uint32_t incl = cnt;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-    if (lane >= (uint32_t)d) incl += y;
+  return keep;
+}
+
+// Key of the phase table for the gram at position at: a hash independent of
+// stage 1's, so that what stage 1 lets through by chance does not pass again.
+template <int G>
+__device__ __forceinline__ uint32_t phase_key_at(const LitArgs& a, uint32_t at) {
+  const uint32_t len = (uint32_t)a.len, w0 = at & ~3u, sh = (at & 3) * 8;
+  if (G == 16) {  // aligned
+    return phase_key(input_word(a, len, w0), input_word(a, len, w0 + 4), input_word(a, len, w0 + 8),
+                     input_word(a, len, w0 + 12), 16);
   }
-  const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-  if (r.next + total > r.end) {  // warp-uniform: reserve a new chunk
-    lean_holes(a, r, lane);
-    const unsigned long long want = total > kLeanChunk ? total : kLeanChunk;
-    unsigned long long wb = 0;
-    if (lane == 0) wb = atomicAdd(a.survivor_count, want);
-    wb = __shfl_sync(0xFFFFFFFFu, wb, 0);
-    r.next = wb;
-    r.end = wb + want;
-  }
-  unsigned long long slot = r.next + incl - cnt;
-  r.next += total;
+  const uint32_t g = __funnelshift_r(input_word(a, len, w0), sh ? input_word(a, len, w0 + 4) : 0u, sh);
+  return phase_key(g, 0, 0, 0, G);
+}
+
+// Takes the queued grams [0, n), 32 at a time: phase bits, start positions,
+// append.
+template <int P, int G>
+__device__ __forceinline__ void gram_flush(const LitArgs& a, const uint32_t* queue, uint32_t n, LeanSlots& r,
+                                           uint32_t lane) {
+  const uint32_t len = (uint32_t)a.len;
+  for (uint32_t k0 = 0; k0 < n; k0 += 32) {
+    uint32_t at = 0, bits = 0;
+    if (k0 + lane < n) {
+      at = queue[k0 + lane];
+      bits = (uint32_t)__ldg(a.phase + (phase_key_at<G>(a, at) >> a.phase_shift));
 #pragma unroll
-  for (int h = 0; h < V; ++h) {
-    for (uint32_t m = mask[h]; m; m &= m - 1) {
-      const uint32_t s = base[h] - 3 + (__ffs(m) - 1);
+      for (int k = 0; k < P; ++k)  // bit P - 1 - k: the literal starts k bytes before the gram
+        if (at < (uint32_t)k || at - k >= len) bits &= ~(1u << (P - 1 - k));
+    }
+    const uint32_t cnt = __popc(bits);
+    if (__ballot_sync(0xFFFFFFFFu, cnt != 0) == 0) continue;
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= (uint32_t)d) incl += y;
+    }
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    if (r.next + total > r.end) {  // warp-uniform: reserve more slots
+      lean_holes(a, r, lane);
+      const unsigned long long want = total > a.slot_chunk ? total : a.slot_chunk;
+      unsigned long long wb = 0;
+      if (lane == 0) wb = atomicAdd(a.survivor_count, want);
+      wb = __shfl_sync(0xFFFFFFFFu, wb, 0);
+      r.next = wb;
+      r.end = wb + want;
+    }
+    unsigned long long slot = r.next + incl - cnt;
+    r.next += total;
+    for (; bits; bits &= bits - 1) {
+      const uint32_t s = at - (P - 1) + (__ffs(bits) - 1);
       if (slot < a.survivor_cap) a.survivors[slot] = s;
-      else verify_position(a, s);  // list full: verify in place
+      else if (prefix_bloom(a, s)) verify_position(a, s);  // list full: verify in place
       ++slot;
     }
   }
 }
 
-__global__ void __launch_bounds__(kLeanThreads, 1) literal_lean_kernel(LitArgs a) {
-  constexpr uint32_t W = kLeanThreads / 32, V = kLeanVecs;
-  extern __shared__ __align__(16) uint32_t filt[];
+// Queues the passing grams of a run of vectors (bit i of `pass`: gram i % NG of
+// vector i / NG) and flushes whole groups of 32.
+template <int P, int G>
+__device__ __forceinline__ uint32_t gram_queue(const LitArgs& a, uint32_t* queue, uint32_t queued, uint32_t pass,
+                                               uint32_t base, LeanSlots& slots, uint32_t lane) {
+  constexpr uint32_t NG = 16 / P;
+  for (uint32_t ball = __ballot_sync(0xFFFFFFFFu, pass != 0); ball; ball = __ballot_sync(0xFFFFFFFFu, pass != 0)) {
+    if (pass) {  // one gram of every lane that has one left
+      const uint32_t i = __ffs(pass) - 1;
+      pass &= pass - 1;
+      queue[queued + __popc(ball & ((1u << lane) - 1u))] = base + (i / NG) * 512 + (i % NG) * P;
+    }
+    queued += __popc(ball);
+    if (queued > kGramQueue - 32 || (queued >= 32 && !__any_sync(0xFFFFFFFFu, pass != 0))) {
+      __syncwarp();
+      const uint32_t whole = queued & ~31u, left = queued & 31u;
+      gram_flush<P, G>(a, queue, whole, slots, lane);
+      const uint32_t keep = lane < left ? queue[whole + lane] : 0u;
+      __syncwarp();
+      if (lane < left) queue[lane] = keep;
+      queued = left;
+    }
+  }
+  __syncwarp();
+  return queued;
+}
+
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t x;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(addr));
+  return x;
+}
+
+// Pass bits of one vector: gram j shifts into the top of `pass`.  w[k] is word
+// k - NPRE of the lane's bytes; `below` holds the words before the vector for
+// lane 0 and receives those of the next one.
+template <int P, int G, int BITS, int NPRE>
+__device__ __forceinline__ uint32_t gram_test(uint32_t filt, uint32_t wsh, uint32_t lane, const uint4& v,
+                                              uint32_t (&below)[NPRE ? NPRE : 1], uint32_t pass) {
+  constexpr int NG = 16 / P, OFF = gram_off<P, G>();
+  uint32_t w[NPRE + 4];
+  w[NPRE] = v.x;
+  w[NPRE + 1] = v.y;
+  w[NPRE + 2] = v.z;
+  w[NPRE + 3] = v.w;
+#pragma unroll
+  for (int k = 0; k < NPRE; ++k) {
+    // lane 31's word goes to lane 0, which keeps it for the next vector
+    const uint32_t x = __shfl_sync(0xFFFFFFFFu, k == 0 ? v.w : k == 1 ? v.z : v.y, (lane + 31) & 31);
+    w[NPRE - 1 - k] = lane == 0 ? below[k] : x;
+    below[k] = x;
+  }
+  uint32_t h[NG], x[NG];
+#pragma unroll
+  for (int j = 0; j < NG; ++j) {
+    const int o = P * j - OFF + 4 * NPRE;  // byte offset of gram j in w
+    if (G == 16) {
+      h[j] = gram_hash32(w[o / 4], w[o / 4 + 1], w[o / 4 + 2], w[o / 4 + 3], 16);
+    } else {
+      const uint32_t g =
+          (o & 3) ? __funnelshift_r(w[o / 4], w[o / 4 + 1 < NPRE + 4 ? o / 4 + 1 : o / 4], 8 * (o & 3)) : w[o / 4];
+      h[j] = gram_hash32(g, 0, 0, 0, G);
+    }
+    x[j] = lds32(filt + ((h[j] >> (wsh - 2)) & ~3u));
+  }
+#pragma unroll
+  for (int j = 0; j < NG; ++j) {
+    uint32_t bit = __funnelshift_r(x[j], x[j], h[j] >> (wsh - 5));
+    if (BITS == 2) bit &= __funnelshift_r(x[j], x[j], h[j] >> (wsh - 10));
+    pass = __funnelshift_r(pass, bit, 1);
+  }
+  return pass;
+}
+
+template <int P, int G, int BITS>
+__global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __grid_constant__ LitArgs a) {
+  constexpr int NG = 16 / P, OFF = gram_off<P, G>(), NPRE = (OFF + 3) / 4;
+  constexpr uint32_t VECS = kGramBits / NG;                // 512-byte vectors of a run
+  constexpr uint32_t RING = VECS < 4 ? VECS : 4;           // vectors loaded ahead
+  extern __shared__ __align__(16) uint32_t gsm[];
+  uint32_t* queue = gsm + (1u << a.gram_word_bits) + (threadIdx.x >> 5) * kGramQueue;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   {
-    const uint4* src = reinterpret_cast<const uint4*>(a.lean_bits);
-    uint4* dst = reinterpret_cast<uint4*>(filt);
-    for (uint32_t k = threadIdx.x; k < (1u << (kLeanBits - 7)); k += kLeanThreads) dst[k] = __ldg(src + k);
+    const uint4* src = reinterpret_cast<const uint4*>(a.gram_bloom);
+    uint4* dst = reinterpret_cast<uint4*>(gsm);
+    for (uint32_t k = threadIdx.x; k < (1u << a.gram_word_bits) / 4; k += kGramThreads) dst[k] = __ldg(src + k);
   }
   __syncthreads();
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warp = threadIdx.x >> 5;
+  const uint32_t filt = (uint32_t)__cvta_generic_to_shared(gsm), wsh = 32 - a.gram_word_bits;
   const uint32_t len = (uint32_t)a.len;
   const uint32_t nvec = (uint32_t)((a.len + 15) >> 4);
-  const uint32_t full_vecs = len >> 4;
-  const uint32_t nblk = (nvec + 32 * V - 1) / (32 * V);  // warp steps of V * 512 bytes
-  const uint32_t nw = gridDim.x * W;
-  const uint8_t* big = a.big;
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-  // half h of warp step blk: the 512 coalesced bytes at (blk * V + h) * 512
-  auto load = [&](uint32_t blk, uint32_t h) -> uint4 {
-    const uint32_t v = (blk * V + h) * 32 + lane;
-    const uint4 x = v < full_vecs ? __ldg(reinterpret_cast<const uint4*>(a.data) + v)
-                    : v < nvec ? load_vec(a.data, a.len, v) : zero;
-    return a.fold ? fold16(x) : x;
-  };
-  uint32_t b = blockIdx.x * W + warp;
+  const uint32_t runs = len / (VECS * 512);                // runs entirely inside the input
+  // neighbouring runs go to different SMs, so that a small input spreads out
+  const uint32_t first = warp * gridDim.x + blockIdx.x, nw = gridDim.x * kGramWarps;
+  const bool fold = a.fold != 0;
   LeanSlots slots;
-  // stage 1 and the stage-1b loads of step b + nw run while step b finishes;
-  // the input is loaded two steps ahead
-  uint4 vn[V];
-  LeanGrams gc[V];
+  uint32_t queued = 0;
+  uint32_t below[NPRE ? NPRE : 1];
+  auto run_ptr = [&](uint32_t r) { return reinterpret_cast<const uint4*>(a.data + (uint64_t)r * (VECS * 512)) + lane; };
+  auto before = [&](uint32_t at, uint32_t (&x)[NPRE ? NPRE : 1]) {  // the words before byte `at` (lane 0)
 #pragma unroll
-  for (uint32_t h = 0; h < V; ++h) {
-    vn[h] = b + nw < nblk ? load(b + nw, h) : zero;
-    if (b < nblk) lean_issue(filt, big, load(b, h), gc[h]);
+    for (int k = 0; k < NPRE; ++k)
+      x[k] = lane == 0 && at ? __ldg(reinterpret_cast<const uint32_t*>(a.data + at) - 1 - k) : 0u;
+  };
+  auto folded = [&](uint32_t (&x)[NPRE ? NPRE : 1]) {
+#pragma unroll
+    for (int k = 0; k < NPRE; ++k) x[k] = ascii_fold4(x[k]);
+  };
+  uint4 ring[RING];
+  uint32_t ahead[NPRE ? NPRE : 1];
+  if (first < runs) {
+    const uint4* p = run_ptr(first);
+#pragma unroll
+    for (uint32_t i = 0; i < RING; ++i) ring[i] = __ldg(p + i * 32);
+    before(first * (VECS * 512), ahead);
   }
-  for (; b < nblk; b += nw) {
-    const uint32_t b1 = b + nw, b2 = b1 + nw;
-    uint4 vn2[V];
-    LeanGrams gn[V];
-    uint32_t mask[V], base[V];
+  for (uint32_t r = first; r < runs; r += nw) {
+    const uint4* p = run_ptr(r);
+    const bool more = r + nw < runs;
+    const uint4* pn = more ? run_ptr(r + nw) : p;
 #pragma unroll
-    for (uint32_t h = 0; h < V; ++h) {
-      vn2[h] = b2 < nblk ? load(b2, h) : zero;
-      if (b1 < nblk) lean_issue(filt, big, vn[h], gn[h]);
-      base[h] = (b * V + h) * 512 + lane * 16;
-      mask[h] = lean_finish(gc[h], base[h], len);
-    }
-    lean_append<V>(a, slots, mask, base, lane);
+    for (int k = 0; k < NPRE; ++k) below[k] = ahead[k];
+    if (NPRE && more) before((r + nw) * (VECS * 512), ahead);
+    if (fold) folded(below);
+    uint32_t pass = 0;
 #pragma unroll
-    for (uint32_t h = 0; h < V; ++h) {
-      gc[h] = gn[h];
-      vn[h] = vn2[h];
+    for (uint32_t i = 0; i < VECS; ++i) {
+      uint4 v = ring[i % RING];
+      if (i + RING < VECS) ring[i % RING] = __ldg(p + (i + RING) * 32);
+      else if (more) ring[i % RING] = __ldg(pn + (i + RING - VECS) * 32);
+      if (fold) v = fold16(v);
+      pass = gram_test<P, G, BITS, NPRE>(filt, wsh, lane, v, below, pass);
     }
+    if (OFF && r == 0 && lane == 0) pass &= ~((1u << ((OFF + P - 1) / P)) - 1u);  // grams that begin before the input
+    if (__any_sync(0xFFFFFFFFu, pass != 0))
+      queued = gram_queue<P, G>(a, queue, queued, pass, r * (VECS * 512) + lane * 16 - OFF, slots, lane);
   }
+  // the vectors after the last whole run, one warp each
+  const uint32_t v0 = runs * VECS, nv = (nvec + 31) >> 5;
+  if (first < nv - v0) {
+    const uint32_t b = v0 + first, vec = b * 32 + lane;
+    uint4 v = vec < nvec ? load_vec(a.data, a.len, vec) : make_uint4(0, 0, 0, 0);
+    before(b * 512, below);
+    if (fold) {
+      v = fold16(v);
+      folded(below);
+    }
+    uint32_t pass = gram_test<P, G, BITS, NPRE>(filt, wsh, lane, v, below, 0u) >> (32 - NG);
+    if (OFF && b == 0 && lane == 0) pass &= ~((1u << ((OFF + P - 1) / P)) - 1u);
+    queued = gram_queue<P, G>(a, queue, queued, pass, b * 512 + lane * 16 - OFF, slots, lane);
+  }
+  if (queued) gram_flush<P, G>(a, queue, queued, slots, lane);
   lean_holes(a, slots, lane);
 }
 
@@ -743,18 +865,8 @@ __global__ void __launch_bounds__(256) literal_verify_kernel(LitArgs a) {
   for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (unsigned long long)gridDim.x * blockDim.x) {
     const uint32_t s = a.survivors[k];
-    if (s == kNoSurvivor) continue;  // a slot the lean kernel reserved but did not fill
-    if (a.verify_bloom) {  // stage 1.5 for survivors of the lean kernel
-      const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
-      const uint32_t x0 = input_word(a, len, w0), x1 = input_word(a, len, w0 + 4), x2 = input_word(a, len, w0 + 8);
-      const uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
-      bool keep = false;
-      for (uint32_t m = a.parts; m; m &= m - 1) {
-        const uint32_t key = prefix_key(lo, hi, __ffs(m));
-        keep |= (__ldg(a.bloom + (key >> 5)) >> (key & 31)) & 1u;
-      }
-      if (!keep) continue;
-    }
+    if (s == kNoSurvivor) continue;  // a slot the gram kernel reserved but did not fill
+    if (a.verify_bloom && !prefix_bloom(a, s)) continue;  // stage 1.5 for survivors of the gram kernel
     verify_position(a, s);
   }
 }
@@ -770,7 +882,7 @@ size_t literal_smem_bytes(const LiteralPlan& plan) {
 size_t literal_scratch_bytes(uint64_t survivor_cap) { return 64 + survivor_cap * 4; }
 
 void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaStream_t st, int sm_count) {
-  if (plan.n_literals == 0 || l.len == 0) return;
+  if (plan.n_strings == 0 || l.len == 0) return;
   LitArgs a;
   a.data = l.data;
   a.len = l.len;
@@ -805,8 +917,12 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   a.parts16 = plan.parts16;
   a.bloom2 = plan.gram_len > 4 ? plan.d_bloom2.as<uint32_t>() : nullptr;
   a.big = plan.has_big ? plan.d_big.as<uint8_t>() : nullptr;
-  a.lean_bits = plan.has_big ? plan.d_lean_bits.as<uint32_t>() : nullptr;
-  a.verify_bloom = 0;
+  a.verify_bloom = plan.gram_kernel ? 1 : 0;
+  a.bloom_parts = plan.bloom_parts;
+  a.gram_bloom = plan.d_gram.as<uint32_t>();
+  a.gram_word_bits = plan.gram_word_bits;
+  a.phase = plan.d_phase.as<uint8_t>();
+  a.phase_shift = 32 - plan.phase_bits;
   a.fold = plan.fold ? 1 : 0;
   check_cuda(cudaMemsetAsync(a.survivor_count, 0, 8, st), "memset survivors");
   if (l.len > 0xFFFFFFFFull) raise(WS_ERR_INPUT_TOO_LARGE, "literal scan launch beyond 32-bit offsets", 0, l.len,
@@ -829,22 +945,36 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
     kernel<<<grid, kBigThreads, smem, st>>>(a);
     check_cuda(cudaGetLastError(), "literal_filter_big_kernel launch");
   };
-  // large sets with 4-byte grams: the lean kernel, or with literals shorter
-  // than 4 bytes the pipelined compacting kernel; long grams, whose hashing
+  auto run_gram = [&](auto kernel, uint32_t run_bytes) {
+    // a warp per run of run_bytes, or per 512-byte vector after the last one
+    const uint64_t units = l.len / run_bytes + (l.len % run_bytes + 511) / 512;
+    const int blocks = (int)std::min<uint64_t>((uint64_t)sm_count, units);
+    // a warp reserves 32 list slots at a time when it has many runs (one
+    // atomic in place of several), else what it appends: the unfilled slots
+    // of all warps stay well below the list's capacity
+    a.slot_chunk = l.len >= 16384ull * blocks * kGramWarps ? 32 : 1;
+    const size_t gsmem = ((size_t)4 << plan.gram_word_bits) + (size_t)kGramWarps * kGramQueue * 4;
+    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem),
+               "cudaFuncSetAttribute(literal gram)");
+    kernel<<<blocks, kGramThreads, gsmem, st>>>(a);
+    check_cuda(cudaGetLastError(), "literal_gram_kernel launch");
+  };
+  // sparse sets: the gram kernel; else with literals shorter than 4 bytes and
+  // a stage-1b table the pipelined compacting kernel; long grams, whose hashing
   // dominates, keep 32 warps per SM
-  if (lg && !sh && a.big && a.lean_bits && plan.period == 4 && plan.gram_len == 4) {
-    a.verify_bloom = 1;
-    const size_t lsmem = (size_t)1 << (kLeanBits - 3);
-    check_cuda(cudaFuncSetAttribute(literal_lean_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem),
-               "cudaFuncSetAttribute(literal lean)");
-    literal_lean_kernel<<<sm_count, kLeanThreads, lsmem, st>>>(a);
-    check_cuda(cudaGetLastError(), "literal_lean_kernel launch");
+  if (plan.gram_kernel) {
+    const bool two = plan.gram_bits == 2;
+    if (plan.gram_len == 16) two ? run_gram(literal_gram_kernel<4, 16, 2>, 4096) : run_gram(literal_gram_kernel<4, 16, 1>, 4096);
+    else if (plan.gram_len == 3) two ? run_gram(literal_gram_kernel<1, 3, 2>, 1024) : run_gram(literal_gram_kernel<1, 3, 1>, 1024);
+    else if (plan.period == 4) two ? run_gram(literal_gram_kernel<4, 4, 2>, 4096) : run_gram(literal_gram_kernel<4, 4, 1>, 4096);
+    else if (plan.period == 2) two ? run_gram(literal_gram_kernel<2, 4, 2>, 2048) : run_gram(literal_gram_kernel<2, 4, 1>, 2048);
+    else two ? run_gram(literal_gram_kernel<1, 4, 2>, 1024) : run_gram(literal_gram_kernel<1, 4, 1>, 1024);
   } else if (lg && sh && a.big && plan.period == 4 && plan.gram_len == 4) {
     run_big(literal_filter_big_kernel<4, true>);
   } else if (!lg) {
     run(literal_filter_kernel<4, 4, false, true>);
   } else if (plan.gram_len == 16) {
-    sh ? run(literal_filter_kernel<4, 16, true, true>) : run(literal_filter_kernel<4, 16, true, false>);
+    run(literal_filter_kernel<4, 16, true, true>);  // (without short literals the gram kernel has it)
   } else if (plan.gram_len == 8) {
     sh ? run(literal_filter_kernel<4, 8, true, true>) : run(literal_filter_kernel<4, 8, true, false>);
   } else if (plan.period == 4) {
@@ -854,9 +984,11 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   } else {
     sh ? run(literal_filter_kernel<1, 4, true, true>) : run(literal_filter_kernel<1, 4, true, false>);
   }
-  // the verify pass is a chain of dependent loads per survivor: the lean
-  // path's longer survivor list (stage 1.5 runs here) gets more threads
-  literal_verify_kernel<<<sm_count * (a.verify_bloom ? 16 : 4), 256, 0, st>>>(a);
+  // the verify pass is a chain of dependent loads per survivor: the gram
+  // kernel's longer survivor list (stage 1.5 runs here) gets more threads, a
+  // short list no more blocks than it can fill
+  const uint64_t vgrid = std::min<uint64_t>((uint64_t)sm_count * (a.verify_bloom ? 16 : 4), (l.survivor_cap + 255) / 256);
+  literal_verify_kernel<<<(unsigned)vgrid, 256, 0, st>>>(a);
   check_cuda(cudaGetLastError(), "literal_verify_kernel launch");
 }
 
