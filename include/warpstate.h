@@ -173,6 +173,11 @@ typedef struct {
 } ws_config;
 
 enum { WS_REGEX_SPECULATIVE = 0, WS_REGEX_PLAIN = 1 };
+/* Regexes whose every match begins with one of a few strings of at least 4
+ * bytes are found through the literal filter (their groups are walked only when
+ * an input makes that the worse way); the others by the walk of their groups,
+ * whose chunk starts the proposer may guess.  WS_PROPOSER_NONE pins the walk:
+ * every group is walked, guessing the unanchored start.  Matches never change. */
 enum { WS_PROPOSER_MLP = 0, WS_PROPOSER_NONE = 1 };
 /* WS_FLAG_PROFILE: record CUDA events around every kernel phase of a scan so
  * ws_matcher_get_info reports per-phase device times (one caller at a time). */
@@ -364,8 +369,8 @@ ws_status ws_matcher_tune(ws_matcher* m, const uint8_t* corpus, uint64_t len, ui
 /* Pins the speculative walk's chunk (bytes, a multiple of 256; 0 keeps the
  * current one) and whether the trained proposer (WS_PROPOSER_MLP) or the
  * unanchored start (WS_PROPOSER_NONE) supplies each chunk's start state in the
- * groups without exact chunk starts, overriding the autotuner's choice.  Matches never change.  No counterpart in
- * the reference.  Call it between scans, not while scans run. */
+ * groups without exact chunk starts, overriding the autotuner's choice; scans then walk every speculative group.
+ * Matches never change.  No counterpart in the reference.  Call it between scans, not while scans run. */
 ws_status ws_matcher_set_walk(ws_matcher* m, uint32_t walk_chunk, uint32_t proposer, ws_error_info* err);
 
 /* Introspection for tests and the benchmark. */

@@ -595,7 +595,8 @@ class GpuMatcher:
     def set_walk(self, walk_chunk: int = 0, proposer: int = PROPOSER_MLP):
         """Pins the speculative walk's chunk (0 keeps it) and its boundary
         guess: the trained proposer (PROPOSER_MLP) or the unanchored start
-        (PROPOSER_NONE), overriding the autotuner.  Matches never change."""
+        (PROPOSER_NONE), overriding the autotuner; scans then walk every
+        speculative group.  Matches never change."""
         _call(N.lib().ws_matcher_set_walk, self._h, int(walk_chunk), int(proposer))
 
     def regex_candidates(self, data, mode: int, distinct: bool = False) -> np.ndarray:

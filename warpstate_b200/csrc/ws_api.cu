@@ -16,6 +16,7 @@
 
 #include "ws_matcher.h"
 #include "ws_proposer.h"
+#include "ws_scan.h"
 
 using namespace ws;
 
@@ -114,20 +115,12 @@ uint32_t enqueue_scan(ws_matcher* m, Scratch& s, cudaStream_t st, const uint8_t*
   m->use_summed = false;
   check_cuda(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st), "memset counter");
   if (prof) check_cuda(cudaEventRecord(m->pev[0], st), "event");
-  if (m->lit.n_literals && x.literals) {
-    uint64_t scap = literal_survivor_cap(len);
-    ensure(s.lit, literal_scratch_bytes(scap));
-    LiteralLaunch ll{d_data, len, d_out, cap, d_counter, s.lit.ptr, scap};
-    ll.item_end = x.item_end;
-    ll.n_items = x.n_items;
-    ll.min_end = x.lit_min_end;
-    ll.max_start = x.lit_max_start;
-    launch_literal_scan(m->lit, ll, st, m->ctx->sm_count);
-    launches += 2;
-  }
-  if (prof) check_cuda(cudaEventRecord(m->pev[1], st), "event");
+  RegexLaunch rl{d_data, len, d_out, cap, d_counter, m->cfg.regex_mode};
+  RegexScan rs;
+  // the literal filter also looks for the regexes' prefixes, unless the walk
+  // is pinned
+  const bool prefixes = m->rx.n_regex && m->lit.n_prefixes && m->cfg.regex_mode == WS_REGEX_SPECULATIVE && !m->walk_pinned;
   if (m->rx.n_regex) {
-    RegexLaunch rl{d_data, len, d_out, cap, d_counter, m->cfg.regex_mode};
     rl.item_end = x.item_end;
     rl.n_items = x.n_items;
     rl.cursor = x.cursor;
@@ -142,8 +135,24 @@ uint32_t enqueue_scan(ws_matcher* m, Scratch& s, cudaStream_t st, const uint8_t*
       rl.k_min = k ? k + k / 4 : 0;
       rl.ev_min = e ? e + e / 4 : 0;
     }
-    launches += run_regex_scan(m->rx, rl, st, s.rx, m->ctx->sm_count, prof ? m->rx_events : nullptr);
+    regex_begin(m->rx, rl, st, s.rx, m->ctx->sm_count, prof, prefixes, rs);
   }
+  if ((m->lit.n_literals && x.literals) || prefixes) {
+    uint64_t scap = literal_survivor_cap(len);
+    ensure(s.lit, literal_scratch_bytes(scap));
+    LiteralLaunch ll{d_data, len, d_out, cap, d_counter, s.lit.ptr, scap};
+    ll.item_end = x.item_end;
+    ll.n_items = x.n_items;
+    ll.min_end = x.lit_min_end;
+    ll.max_start = x.lit_max_start;
+    ll.literals = m->lit.n_literals && x.literals;
+    ll.rx = prefixes ? &rs : nullptr;
+    launch_literal_scan(m->lit, ll, st, m->ctx->sm_count);
+    launches += 2;
+  }
+  if (prof) check_cuda(cudaEventRecord(m->pev[1], st), "event");
+  if (m->rx.n_regex)
+    launches += regex_finish(m->rx, rs, rl, st, m->ctx->sm_count, prof ? m->rx_events : nullptr);
   if (prof) check_cuda(cudaEventRecord(m->pev[2], st), "event");
   check_cuda(cudaEventRecord(s.busy, st), "event");
   std::lock_guard<std::mutex> g(m->info_mu);
@@ -331,8 +340,8 @@ ws_status ws_matcher_create(ws_ctx* ctx, const ws_pattern_tables* t, const ws_co
     }
     for (uint32_t i = 0; i < t->n_literals; ++i) m->max_literal_len = std::max(m->max_literal_len, t->offsets[2 * i + 1]);
     std::memset(&m->info, 0, sizeof(m->info));
-    plan_literals(*t, m->lit);
     plan_regex(*t, m->cfg, ctx->sm_count, m->rx);
+    plan_filter(*t, m->rx, m->lit);
     m->info.n_literals = t->n_literals;
     m->info.n_regex = t->n_regex;
     m->info.filter_q = m->lit.gram_len;

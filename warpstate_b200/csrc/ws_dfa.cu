@@ -13,6 +13,7 @@
 #include "ws_dfa.h"
 #include "ws_async.h"
 #include "ws_proposer.h"
+#include "ws_scan.h"
 
 namespace cg = cooperative_groups;
 
@@ -20,9 +21,6 @@ namespace ws {
 
 namespace {
 
-constexpr uint32_t F_MATCH = 0x80000000u;
-constexpr uint32_t F_DEAD = 0x40000000u;
-constexpr uint32_t F_MASK = 0x3FFFFFFFu;
 constexpr uint32_t kCkpt = 256;       // bytes between recorded walk states
 constexpr int kFixRounds = 3;         // parallel fix-up rounds before the serial sweep
 constexpr int kWalkThreads = 1024;    // threads (= chunks) per walk block
@@ -33,12 +31,7 @@ constexpr int kWalkThreads = 1024;    // threads (= chunks) per walk block
 // linear instead of quadratic.  2^kRmarkBits slots of 8 bytes, cleared per scan.
 constexpr uint32_t kRmarkBits = 20;
 constexpr uint32_t kRmarkStateBits = 20;  // states below 2^20, groups below 2^12
-// Leftmost-first walks in the parallel pass stop after kLfCap bytes; the
-// chain kernel finishes such a walk only if it picks that start (picked
-// matches do not overlap, so that work is bounded by the input).
-constexpr uint64_t kLfCap = 1024;
-constexpr uint32_t kLfNone = 0xFFFFFFFFu;  // no match from this start (or a duplicate start)
-constexpr uint32_t kLfLong = 0xFFFFFFFEu;  // the walk reached kLfCap bytes
+static_assert(C_ROUND + kFixRounds < C_FIX, "counter slots overlap");
 
 // ------------------------------------------------------------ scratch layout
 struct RxLayout {
@@ -47,19 +40,6 @@ struct RxLayout {
   size_t off_ctr, off_k, off_ev, off_guess, off_used, off_end, off_spec, off_conv, off_round, off_ckpt,
       off_count, off_offs, off_cursor, off_starts, off_lfend, off_rmark, total;
 };
-
-struct KCand { uint32_t r, s, e; };
-struct Event { uint32_t e, state, q, tag; };
-
-// counters block (unsigned long long[16]):
-//  [0] K count  [1] event count  [2] error flags  [3..3+kFixRounds] round-changed flags
-//  [8] chunk re-walks of the fix-up  [9] bytes those re-walks stepped
-//  [10] boundary guesses that were the true state  [11] boundary guesses
-enum { C_K = 0, C_EV = 1, C_ERR = 2, C_ROUND = 3, C_FIX = 8, C_REWALK = 9, C_HITS = 10, C_GUESSES = 11 };
-// error bits in ctr[C_ERR]: 1 candidate overflow, 2 event overflow, 4 a
-// bounded device-side wait ran out
-constexpr unsigned long long kErrTimeout = 4;
-static_assert(C_ROUND + kFixRounds < C_FIX, "counter slots overlap");
 
 // Candidate and event buffers hold at most this many entries (the per-regex
 // offsets of the resolution are 32-bit).
@@ -79,6 +59,7 @@ RxLayout layout(const RegexPlan& p, uint64_t len, uint32_t chunk, uint64_t max_m
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t r = o; o = (o + bytes + 255) & ~(size_t)255; return r; };
   L.off_ctr = take(16 * 8);
+  L.off_count = take((size_t)p.n_regex * 4);  // (cleared together with the counters)
   L.off_k = take(L.k_cap * sizeof(KCand));
   L.off_ev = take(L.ev_cap * sizeof(Event));
   L.off_guess = take(L.n_q * 4);
@@ -88,7 +69,6 @@ RxLayout layout(const RegexPlan& p, uint64_t len, uint32_t chunk, uint64_t max_m
   L.off_conv = take(L.n_q * 4);
   L.off_round = take(L.n_q * 4);
   L.off_ckpt = take(L.n_q * L.nck * 4);
-  L.off_count = take((size_t)p.n_regex * 4);
   L.off_offs = take(((size_t)p.n_regex + 1) * 4);
   L.off_cursor = take((size_t)p.n_regex * 4);
   L.off_starts = take(L.k_cap * 4);
@@ -97,56 +77,6 @@ RxLayout layout(const RegexPlan& p, uint64_t len, uint32_t chunk, uint64_t max_m
   L.total = o;
   return L;
 }
-
-struct DevTables {
-  const GroupDev* groups;
-  const uint32_t* fwd;
-  const uint32_t* hot;
-  const uint32_t* rev;
-  const uint32_t* lf;
-  const uint8_t* cls;
-  const uint32_t* mptr;
-  const uint32_t* mlist;
-  const uint32_t* rmptr;
-  const uint32_t* rmlist;
-  const uint4* lfinfo;   // per regex: {lf_off, lf_start row, group, classes}
-  const uint32_t* lfx;   // per regex: context DFA starts and end-step flags (8 words)
-  const uint32_t* pid;
-  uint32_t n_groups, n_regex, n_spec;
-};
-
-struct ScanPtrs {
-  const uint8_t* data;
-  uint64_t len;
-  unsigned long long* ctr;
-  KCand* k;
-  uint64_t k_cap;
-  Event* ev;
-  uint64_t ev_cap;
-  uint32_t* guess;
-  uint32_t* used;
-  uint32_t* end;
-  uint32_t* spec;
-  uint32_t* conv;
-  uint32_t* round;
-  uint32_t* ckpt;
-  uint32_t* count;
-  uint32_t* offs;
-  uint32_t* cursor;
-  uint32_t* starts;
-  uint32_t* lfend;
-  unsigned long long* rmark;    // visited reverse-walk triples, or null (state numbers too large, or full K)
-  uint32_t full_k;              // report every (start, end) of K, not only distinct starts (diagnostics)
-  uint32_t count_guesses;       // profiled speculative scans: the speculative groups whose guesses are counted
-  uint64_t n_chunks, chunk, nck;
-  ws_match* out;
-  uint64_t out_cap;
-  unsigned long long* out_counter;
-  const uint32_t* item_end;     // batch item ends (n_items), else null
-  uint32_t n_items;
-  unsigned long long* cursor64;  // stream: per-regex find_iter position, else null
-  uint64_t base, frontier;
-};
 
 ScanPtrs make_ptrs(const RxLayout& L, void* base, const RegexLaunch& l) {
   uint8_t* b = static_cast<uint8_t*>(base);
@@ -185,27 +115,6 @@ ScanPtrs make_ptrs(const RxLayout& L, void* base, const RegexLaunch& l) {
   p.base = l.base;
   p.frontier = l.frontier;
   return p;
-}
-
-// One slot of an append buffer, one atomic per group of converged lanes.
-__device__ __forceinline__ unsigned long long warp_append(unsigned long long* counter) {
-  cg::coalesced_group g = cg::coalesced_threads();
-  unsigned long long base = 0;
-  if (g.thread_rank() == 0) base = atomicAdd(counter, (unsigned long long)g.size());
-  base = g.shfl(base, 0);
-  return base + g.thread_rank();
-}
-
-// Appends a candidate and counts it for its regex (the per-regex counts size
-// the resolution's start lists).
-__device__ __forceinline__ void emit_k(const ScanPtrs& p, uint32_t r, uint32_t s, uint32_t e) {
-  unsigned long long i = warp_append(&p.ctr[C_K]);
-  if (i < p.k_cap) {
-    p.k[i] = KCand{r, s, e};
-    atomicAdd(&p.count[r], 1u);
-  } else {
-    atomicOr(&p.ctr[C_ERR], 1ull);
-  }
 }
 
 __device__ __forceinline__ void emit_event(const ScanPtrs& p, uint32_t e, uint32_t st, uint32_t q, uint32_t tag) {
@@ -443,13 +352,6 @@ __global__ void __launch_bounds__(kWalkThreads, 1) dfa_plain_kernel(DevTables t,
 }
 
 // --------------------------------------------------------- context groups
-// Context of a byte for the assertions (byte_context in ws_regex.h).
-__device__ __forceinline__ uint32_t ctx_of(uint32_t b) {
-  if (b == '\n') return CTX_NL;
-  const bool w = (b - '0' < 10u) || ((b | 0x20u) - 'a' < 26u) || b == '_';
-  return w ? CTX_WORD : CTX_OTHER;
-}
-
 // Context groups: one thread per start position, the anchored walk of the
 // group's context DFA (build_context_all_dfa): the start row chosen by the
 // byte before the start (CTX_BEGIN at the start of the input or item), the
@@ -463,6 +365,7 @@ __device__ __forceinline__ uint32_t ctx_of(uint32_t b) {
 __global__ void __launch_bounds__(256) dfa_context_kernel(DevTables t, ScanPtrs p) {
   __shared__ uint8_t cls_s[256];
   const uint32_t g = t.n_spec + blockIdx.y;
+  if (g >= t.n_ctx_walk && p.ctr[C_GATE] == 0) return;
   const GroupDev gd = t.groups[g];
   for (uint32_t k = threadIdx.x; k < 256; k += blockDim.x) cls_s[k] = t.cls[g * 256 + k];
   __syncthreads();
@@ -529,6 +432,14 @@ __global__ void __launch_bounds__(kWalkThreads, 1)
   // blockIdx.x = group (fastest), so the groups' blocks over the same chunks
   // run together and the input is read from HBM once, then from L2
   const uint32_t g = blockIdx.x;
+  const bool gated = g >= t.n_walk;
+  if (gated && p.ctr[C_GATE] == 0) return;
+  if (t.n_walk == 0 && p.rmark) {  // every group is gated: the marks were not cleared for this scan
+    const uint64_t n = (uint64_t)gridDim.x * gridDim.y * blockDim.x;
+    for (uint64_t k = ((uint64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+         k < (1ull << kRmarkBits); k += n)
+      p.rmark[k] = ~0ull;
+  }
   const GroupDev gd = t.groups[g];
   uint32_t* img = smem;
   uint8_t* stages = reinterpret_cast<uint8_t*>(smem) + kWalkImgBytes;
@@ -569,7 +480,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1)
   // before the chunk (exact); other groups start from the boundary guess
   const bool exact = warm_exact(gd, p.chunk);
   uint32_t start = gd.start_unanchored;
-  if (active && i != 0 && !exact) start = p.guess[q];
+  if (active && i != 0 && !exact && !gated) start = p.guess[q];  // (no guesses are made for gated groups)
   if (start >= gd.n_states) start = gd.start_unanchored;  // a guess never written
   uint32_t* ck = p.ckpt + q * p.nck;
   uint32_t cold_row = 0;
@@ -782,6 +693,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) dfa_fixup_kernel(DevTables t,
   if (round > 0 && p.ctr[C_ROUND + round - 1] == 0) return;  // nothing changed last round
   extern __shared__ __align__(16) uint32_t smem[];
   const uint32_t g = blockIdx.x;
+  if (g >= t.n_walk && p.ctr[C_GATE] == 0) return;
   const uint64_t first = 1 + (uint64_t)blockIdx.y * blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.y * blockDim.x;
   bool need = false;
@@ -804,6 +716,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) dfa_fixup_kernel(DevTables t,
 __global__ void dfa_fixup_serial_kernel(DevTables t, ScanPtrs p) {
   if (p.ctr[C_ROUND + kFixRounds - 1] == 0) return;
   const uint32_t g = blockIdx.x;
+  if (g >= t.n_walk && p.ctr[C_GATE] == 0) return;
   for (uint64_t i = 1; i < p.n_chunks; ++i)
     fix_chunk(t, p, g, i, (uint32_t)kFixRounds + 1, &p.ctr[C_ROUND + kFixRounds]);
 }
@@ -1004,44 +917,6 @@ __global__ void __launch_bounds__(512) k_sort_kernel(ScanPtrs p, uint32_t n_rege
   }
 }
 
-// Leftmost-first end of a match of regex r from start s: the walk of the
-// regex's priority DFA from s, remembering the last match position, until the
-// DFA dies or the item or input ends.  kLfNone when no match starts at s;
-// kLfLong when the walk was cut off after `cap` bytes.
-__device__ uint32_t lf_walk(const DevTables& t, const ScanPtrs& p, uint32_t r, uint32_t s, uint64_t cap) {
-  const uint4 info = t.lfinfo[r];
-  const uint8_t* cm = t.cls + info.z * 256;
-  const uint32_t* tab = t.lf + info.x;
-  uint32_t st = info.y;
-  int64_t last = -1;
-  const uint64_t stop = p.n_items ? min(p.len, (uint64_t)item_end_of(p.item_end, p.n_items, s)) : p.len;
-  const uint32_t* x = t.lfx + 8 * (size_t)r;
-  if (__ldg(x)) {
-    // context DFA (build_context_lf_dfa): start row by the byte before s, a
-    // match flag on the byte at pos ends a match at pos, the end step after
-    // the last byte of the input or item
-    const uint64_t lo = p.n_items ? item_start_of(p.item_end, p.n_items, s) : 0;
-    st = __ldg(x + 1 + (s == lo ? CTX_BEGIN : ctx_of(__ldg(p.data + s - 1))));
-    for (uint64_t pos = s; pos < stop; ++pos) {
-      if (pos - s == cap) return kLfLong;
-      const uint32_t w = __ldg(tab + st * info.w + __ldg(cm + __ldg(p.data + pos)));
-      if (w & F_MATCH) last = (int64_t)pos;
-      if (w & F_DEAD) return last < 0 ? kLfNone : (uint32_t)last;
-      st = w & F_MASK;
-    }
-    if (__ldg(t.lf + __ldg(x + 5) + st)) last = (int64_t)stop;
-    return last < 0 ? kLfNone : (uint32_t)last;
-  }
-  for (uint64_t pos = s; pos < stop; ++pos) {
-    if (pos - s == cap) return kLfLong;
-    uint32_t w = __ldg(tab + st * info.w + __ldg(cm + __ldg(p.data + pos)));
-    if (w & F_DEAD) break;
-    st = w & F_MASK;
-    if (w & F_MATCH) last = (int64_t)pos + 1;
-  }
-  return last < 0 ? kLfNone : (uint32_t)last;
-}
-
 // Leftmost-first end of every distinct candidate start (in parallel), each
 // walk cut off after kLfCap bytes.
 // The regexes' candidate offsets are staged in shared memory when they fit
@@ -1068,7 +943,8 @@ __global__ void k_lf_kernel(DevTables t, ScanPtrs p, uint32_t n_regex) {
     const uint32_t r = lo;
     const uint32_t s = p.starts[j];
     if (j > offs[r] && p.starts[j - 1] == s) { p.lfend[j] = kLfNone; continue; }  // duplicate
-    p.lfend[j] = lf_walk(t, p, r, s, kLfCap);
+    const uint32_t e = lf_walk(t, p, r, s, kLfCap);
+    p.lfend[j] = e == kLfOpen ? kLfLong : e;
   }
 }
 
@@ -1185,6 +1061,8 @@ DevTables dev_tables(const RegexPlan& P) {
   t.n_groups = P.n_groups;
   t.n_regex = P.n_regex;
   t.n_spec = P.n_spec;
+  t.n_walk = P.n_spec;
+  t.n_ctx_walk = P.n_groups;
   return t;
 }
 
@@ -1280,10 +1158,17 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
     return launches;
   }
   dim3 cgrid(P.n_spec, (unsigned)((p.n_chunks + kWalkThreads - 1) / kWalkThreads));
-  // the walk ignores the guesses of groups with exact chunk starts
-  if (P.proposer && P.use_proposer && !regex_all_exact(P, p.chunk)) {
+  // the walk ignores the guesses of groups with exact chunk starts and makes
+  // none for gated ones
+  bool guessed = false, all_exact = true;
+  for (uint32_t g = 0; g < P.n_spec; ++g) {
+    const bool exact = warm_exact(P.groups[g], p.chunk);
+    all_exact &= exact;
+    guessed |= !exact && g < t.n_walk;
+  }
+  if (guessed && P.proposer && P.use_proposer) {
     launches += proposer_predict(*P.proposer, p.data, p.len, p.chunk, p.n_chunks, p.guess, st);
-  } else {
+  } else if (guessed) {
     fill_guess_kernel<<<dim3(std::min<unsigned>((unsigned)((p.n_chunks + 255) / 256), 1024), P.n_spec), 256, 0, st>>>(t, p);
     check_cuda(cudaGetLastError(), "fill_guess_kernel");
     launches++;
@@ -1304,20 +1189,23 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
   check_cuda(cudaGetLastError(), "dfa_walk_kernel");
   launches++;
   mark(2);
-  // one wave of fix-up blocks (one per SM, the walk's shared memory)
-  const uint64_t fper = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sm_count / P.n_spec,
-                                                                  (p.n_chunks + kWalkThreads - 1) / kWalkThreads));
-  dim3 fgrid(P.n_spec, (unsigned)fper);
-  auto fixup = P.class_image ? dfa_fixup_kernel<true> : dfa_fixup_kernel<false>;
-  set_smem(fixup, kFixSmem, "smem(fixup)");
-  for (int r = 0; r < kFixRounds; ++r) {
-    fixup<<<fgrid, kWalkThreads, kFixSmem, st>>>(t, p, r);
-    check_cuda(cudaGetLastError(), "dfa_fixup_kernel");
+  // exact chunk starts are the true states: nothing to fix up
+  if (!all_exact) {
+    // one wave of fix-up blocks (one per SM, the walk's shared memory)
+    const uint64_t fper = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sm_count / P.n_spec,
+                                                                    (p.n_chunks + kWalkThreads - 1) / kWalkThreads));
+    dim3 fgrid(P.n_spec, (unsigned)fper);
+    auto fixup = P.class_image ? dfa_fixup_kernel<true> : dfa_fixup_kernel<false>;
+    set_smem(fixup, kFixSmem, "smem(fixup)");
+    for (int r = 0; r < kFixRounds; ++r) {
+      fixup<<<fgrid, kWalkThreads, kFixSmem, st>>>(t, p, r);
+      check_cuda(cudaGetLastError(), "dfa_fixup_kernel");
+      launches++;
+    }
+    dfa_fixup_serial_kernel<<<P.n_spec, 1, 0, st>>>(t, p);
+    check_cuda(cudaGetLastError(), "dfa_fixup_serial_kernel");
     launches++;
   }
-  dfa_fixup_serial_kernel<<<P.n_spec, 1, 0, st>>>(t, p);
-  check_cuda(cudaGetLastError(), "dfa_fixup_serial_kernel");
-  launches++;
   mark(3);
   dfa_reverse_kernel<<<sm_count * 8, 256, 0, st>>>(t, p);
   check_cuda(cudaGetLastError(), "dfa_reverse_kernel");
@@ -1622,6 +1510,12 @@ void plan_regex(const ws_pattern_tables& t, const ws_config& cfg, int sm_count, 
   // verification of every group (halved while it exceeds the budget).
   std::vector<int> est(t.n_regex);
   std::vector<uint8_t> ctx(t.n_regex, 0);
+  // The prefix filter covers a regex whose matches all begin with one of a few
+  // strings of at least 4 bytes (a config that pins the walk's boundary guess
+  // to the unanchored start walks every regex).
+  P.covered.assign(t.n_regex, 0);
+  for (auto& x : P.prefixes) x.assign(t.n_regex, {});
+  const bool prefixes = cfg.regex_mode == WS_REGEX_SPECULATIVE && cfg.proposer != WS_PROPOSER_NONE;
   for (uint32_t r = 0; r < t.n_regex; ++r) {
     ctx[r] = tree_has_look(trees[r]) ? 1 : 0;
     Nfa n = build_nfa({&trees[r]}, false);
@@ -1632,21 +1526,29 @@ void plan_regex(const ws_pattern_tables& t, const ws_config& cfg, int sm_count, 
                                 std::to_string(max_states) + " DFA states (raise dfa_max_states)",
             t.regex_pattern_ids[r]);
     est[r] = d.n_states;
+    for (int k = 0; prefixes && k < kPrefixLens; ++k) {
+      const bool ok = regex_prefixes(d, bc, ctx[r] != 0, kPrefixLen[k], kPrefixMost[k], P.prefixes[k][r]);
+      if (kPrefixLen[k] == 4) P.covered[r] = ok ? 1 : 0;
+    }
   }
-  // speculative groups first, then the context groups
+  // speculative groups first, then the context groups; among each, the groups
+  // of covered regexes last
   std::vector<GroupBuild> gbs;
-  for (int want_ctx = 0; want_ctx < 2; ++want_ctx) {
+  for (int part = 0; part < 4; ++part) {
+    const int want_ctx = part >> 1, want_cov = part & 1;
     std::vector<std::vector<uint32_t>> packs(1);
     int sum = 0;
     for (uint32_t r = 0; r < t.n_regex; ++r) {
-      if (ctx[r] != want_ctx) continue;
+      if (ctx[r] != want_ctx || P.covered[r] != want_cov) continue;
       if (!packs.back().empty() && 4 * (sum + est[r]) > 3 * max_states) { packs.emplace_back(); sum = 0; }
       packs.back().push_back(r);
       sum += est[r];
     }
     for (auto& pk : packs)
       if (!pk.empty()) build_groups(trees, pk, max_states, gbs, want_ctx != 0);
-    if (!want_ctx) P.n_spec = (uint32_t)gbs.size();
+    if (part == 0) P.n_walk = (uint32_t)gbs.size();
+    if (part == 1) P.n_spec = (uint32_t)gbs.size();
+    if (part == 2) P.n_ctx_walk = (uint32_t)gbs.size();
   }
   P.has_context = P.n_spec < gbs.size();
 
@@ -1820,11 +1722,12 @@ namespace {
 // Reverse-walk marks start empty in every scan (a stale mark would stop a
 // walk that no other walk continues); plans whose state numbers do not fit
 // the mark key run without them.
-void clear_marks(const RegexPlan& P, ScanPtrs& p, cudaStream_t st) {
+void clear_marks(const RegexPlan& P, ScanPtrs& p, const DevTables& t, cudaStream_t st) {
   if (!P.rev_marks || p.full_k) {
     p.rmark = nullptr;
     return;
   }
+  if (t.n_walk == 0) return;  // no group walks unless the prefix filter gives up: the walk clears them then
   check_cuda(cudaMemsetAsync(p.rmark, 0xFF, ((size_t)1 << kRmarkBits) * 8, st), "memset marks");
 }
 
@@ -1858,22 +1761,34 @@ uint32_t effective_chunk(const RegexPlan& P, uint64_t len, int sm_count) {
 
 }  // namespace
 
-uint32_t run_regex_scan(RegexPlan& P, const RegexLaunch& l, cudaStream_t st, DeviceBuffer& scratch, int sm_count,
-                        cudaEvent_t* ev) {
-  if (!P.n_regex || l.len == 0) return 0;
+void regex_begin(RegexPlan& P, const RegexLaunch& l, cudaStream_t st, DeviceBuffer& scratch, int sm_count,
+                 bool profiled, bool prefixes, RegexScan& rs) {
   RxLayout L = layout(P, l.len, effective_chunk(P, l.len, sm_count), l.cap, l.k_min, l.ev_min);
   ensure_scratch(scratch, L.total);
-  ScanPtrs p = make_ptrs(L, scratch.ptr, l);
+  rs.p = make_ptrs(L, scratch.ptr, l);
+  rs.t = dev_tables(P);
+  rs.k_cap = L.k_cap;
+  rs.n_q = L.n_q;
+  rs.prefixes = prefixes;
+  if (prefixes) {
+    rs.t.n_walk = P.n_walk;
+    rs.t.n_ctx_walk = P.n_ctx_walk;
+  }
   // profiled speculative scans count the boundary guesses that held
-  if (ev && l.mode != WS_REGEX_PLAIN) p.count_guesses = P.n_spec;
-  DevTables t = dev_tables(P);
+  if (profiled && l.mode != WS_REGEX_PLAIN) rs.p.count_guesses = rs.t.n_walk;
+  if (l.mode != WS_REGEX_PLAIN && P.n_spec) clear_marks(P, rs.p, rs.t, st);
+  // the counters and the per-regex counts after them
+  check_cuda(cudaMemsetAsync(rs.p.ctr, 0, L.off_count - L.off_ctr + (size_t)P.n_regex * 4, st), "memset");
+}
+
+uint32_t regex_finish(RegexPlan& P, RegexScan& rs, const RegexLaunch& l, cudaStream_t st, int sm_count,
+                      cudaEvent_t* ev) {
+  const ScanPtrs& p = rs.p;
+  const DevTables& t = rs.t;
   uint32_t launches = 0;
-  clear_marks(P, p, st);
-  check_cuda(cudaMemsetAsync(p.ctr, 0, 16 * 8, st), "memset");
-  check_cuda(cudaMemsetAsync(p.count, 0, (size_t)P.n_regex * 4, st), "memset");
   if (ev) check_cuda(cudaEventRecord(ev[0], st), "event");
   launches += candidates_phase(P, t, p, l.mode, st, sm_count, ev);
-  int hg = (int)std::min<uint64_t>((uint64_t)sm_count * 8, (L.k_cap + 255) / 256);
+  int hg = (int)std::min<uint64_t>((uint64_t)sm_count * 8, (rs.k_cap + 255) / 256);
   k_scan_kernel<<<1, 1024, 0, st>>>(p, P.n_regex);
   k_scatter_kernel<<<hg, 256, 0, st>>>(p);
   k_sort_kernel<<<(unsigned)std::min<uint32_t>(P.n_regex, 4096), 512, 0, st>>>(p, P.n_regex);
@@ -1895,9 +1810,17 @@ uint32_t run_regex_scan(RegexPlan& P, const RegexLaunch& l, cudaStream_t st, Dev
     check_cuda(cudaMemcpyAsync(P.prof_ctr.get(), p.ctr, 16 * 8, cudaMemcpyDeviceToHost, st), "D2H counters");
     check_cuda(cudaEventRecord(ev[5], st), "event");
   }
-  P.last_chunks = L.n_q;
+  P.last_chunks = rs.n_q;
   P.last_launches = launches;
   return launches;
+}
+
+uint32_t run_regex_scan(RegexPlan& P, const RegexLaunch& l, cudaStream_t st, DeviceBuffer& scratch, int sm_count,
+                        cudaEvent_t* ev) {
+  if (!P.n_regex || l.len == 0) return 0;
+  RegexScan rs;
+  regex_begin(P, l, st, scratch, sm_count, ev != nullptr, false, rs);
+  return regex_finish(P, rs, l, st, sm_count, ev);
 }
 
 void regex_collect_timing(const RegexPlan& P, cudaEvent_t* ev, ws_matcher_info& info) {
@@ -1932,7 +1855,7 @@ uint64_t regex_candidates(RegexPlan& P, const uint8_t* d_data, uint64_t len, uin
   ScanPtrs p = make_ptrs(L, scratch.ptr, l);
   p.full_k = full ? 1 : 0;
   DevTables t = dev_tables(P);
-  clear_marks(P, p, st);
+  clear_marks(P, p, t, st);
   check_cuda(cudaMemsetAsync(p.ctr, 0, 16 * 8, st), "memset");
   candidates_phase(P, t, p, mode, st, sm_count, nullptr);
   unsigned long long ctr[16];

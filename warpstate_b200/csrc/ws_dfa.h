@@ -75,6 +75,14 @@ struct GroupDev {
 // before it (the walk reads them once per chunk: at most a quarter of a chunk).
 constexpr uint32_t kWarmMax = 512;
 
+// Lengths at which a regex's prefixes are listed (a match shorter than that
+// ends its prefix), and the most a regex may have.  4, 5 and 7 bytes are what
+// the literal filter needs to look at every, every second and every fourth
+// position; 20 is for small alphabets (16-byte grams at every fourth).
+constexpr int kPrefixLens = 4;
+constexpr uint32_t kPrefixLen[kPrefixLens] = {20, 7, 5, 4};
+constexpr uint32_t kPrefixMost[kPrefixLens] = {2048, 1024, 1024, 512};
+
 struct Proposer;
 // Frees a trained proposer (ws_proposer.cu).
 struct ProposerDeleter {
@@ -88,6 +96,13 @@ struct RegexPlan {
   // groups [n_spec, n_groups) are context groups, walked one anchored walk
   // per start position in both modes.
   uint32_t n_spec = 0;
+  // Covered regexes (every match begins with one of a few strings of at least
+  // 4 bytes) have groups of their own: [n_walk, n_spec) and
+  // [n_ctx_walk, n_groups).  When the literal filter looks for their prefixes
+  // those groups walk only if it gives up.
+  uint32_t n_walk = 0, n_ctx_walk = 0;
+  std::vector<uint8_t> covered;          // per regex
+  std::vector<std::vector<std::string>> prefixes[kPrefixLens];  // per length and regex; empty: too many
   bool has_context = false;              // some regex has a look-around assertion
   bool class_image = false;              // the speculative groups' walk images are class-indexed
   uint32_t total_states = 0;
@@ -173,7 +188,16 @@ void regex_fill_info(const RegexPlan& plan, ws_matcher_info& info);
 // True when every speculative group starts its chunks (of `chunk` bytes) from
 // their exact states, so that boundary guesses (and the proposer) are unused.
 bool regex_all_exact(const RegexPlan& plan, uint64_t chunk);
-// Enqueues the regex pipeline on `st`.  `events` (8 CUDA events) is non-null
+// The regex pipeline in two parts, with the literal scan between them when it
+// looks for the covered regexes' prefixes (`prefixes`): regex_begin prepares
+// the scratch and clears the counters, regex_finish runs the walks of the
+// groups that need them and the resolution.
+struct RegexScan;  // ws_scan.h
+void regex_begin(RegexPlan& plan, const RegexLaunch& l, cudaStream_t st, DeviceBuffer& scratch, int sm_count,
+                 bool profiled, bool prefixes, RegexScan& rs);
+uint32_t regex_finish(RegexPlan& plan, RegexScan& rs, const RegexLaunch& l, cudaStream_t st, int sm_count,
+                      cudaEvent_t* events);
+// Enqueues the whole regex pipeline on `st`, every group walked.  `events` (8 CUDA events) is non-null
 // when phase timing is wanted.  Returns the number of kernel launches.
 uint32_t run_regex_scan(RegexPlan& plan, const RegexLaunch& l, cudaStream_t st, DeviceBuffer& scratch,
                         int sm_count, cudaEvent_t* events);

@@ -150,6 +150,10 @@ struct LiteralPlan {
   DeviceBuffer d_filter, d_bloom, d_short, d_info, d_bytes, d_meta, d_ranges, d_entries, d_bloom2, d_big,
       d_lean_bits;
   uint32_t n_buckets = 0;
+  // Regex prefixes: entries {first 4 bytes, next 4, their mask, regex} by
+  // bucket of a hash of the first 4 bytes (prefix_mul = 0) or of all 8.
+  uint32_t n_prefixes = 0, prefix_shift = 0, prefix_mul = 0;
+  DeviceBuffer d_prefix_range, d_prefix_entry;
   // ASCII case-insensitive: the tables hold folded literals and the kernels
   // fold the input (A-Z to a-z) before hashing and comparing.
   bool fold = false;
@@ -234,6 +238,15 @@ __host__ __device__ inline uint32_t prefix16_key(uint32_t x0, uint32_t x1, uint3
 // `prefixes`: strings of at least 4 bytes that are filtered with the literals
 // (regex prefixes); positions where one starts are survivors.
 void plan_literals(const ws_pattern_tables& t, LiteralPlan& plan, const std::vector<std::string>& prefixes = {});
+// Whether 4-byte grams of the literals and `prefixes` cover too much of their
+// alphabet's for the gram kernel.
+bool filter_crowded(const ws_pattern_tables& t, const std::vector<std::string>& prefixes);
+struct RegexPlan;
+// plan_literals with the prefixes of the regexes that have some, and the table
+// the verify kernel finds them in (n_prefixes stays 0 when there are none).
+void plan_filter(const ws_pattern_tables& t, const RegexPlan& rx, LiteralPlan& plan);
+
+struct RegexScan;  // ws_scan.h
 
 // Kernel launchers (ws_literal.cu).
 struct LiteralLaunch {
@@ -252,6 +265,8 @@ struct LiteralLaunch {
   uint64_t min_end = 0;
   // Shard scans: only matches starting before this offset are this shard's.
   uint64_t max_start = ~0ull;
+  bool literals = true;          // report literal matches (else only the regexes' prefixes are looked for)
+  const RegexScan* rx = nullptr;  // the regex scan that takes the prefixes' candidates
 };
 
 // Exclusive end of the item that contains offset `s` (the first end above s).

@@ -158,7 +158,29 @@ void build_gram_tables(const std::vector<FilterString>& strings, LiteralPlan& pl
   plan.d_phase.upload(phase.data(), phase.size());
 }
 
+// P grams at offsets 0..P-1 must fit inside every string: P + 3 <= len.
+uint32_t period_of(uint32_t min_len) { return min_len >= 7 ? 4 : min_len >= 5 ? 2 : 1; }
+
+// Share of its alphabet's 4-byte grams that a set may cover.  The gram kernel
+// verifies in a later kernel what passes, from a list of one survivor per 64
+// bytes of input: an input over the set's own alphabet should not crowd it
+// (for P = 4, whose lookups are a quarter as many, a quarter is allowed).
+double coverage_limit(uint32_t P) { return P == 4 ? 0.25 : 1.0 / 64; }
+
 }  // namespace
+
+bool filter_crowded(const ws_pattern_tables& t, const std::vector<std::string>& prefixes) {
+  std::vector<FilterString> strings;
+  uint32_t min_long = UINT32_MAX;
+  for (uint32_t li = 0; li < t.n_literals; ++li)
+    strings.push_back({t.packed_bytes + t.offsets[2 * li], t.offsets[2 * li + 1]});
+  for (const std::string& x : prefixes)
+    strings.push_back({reinterpret_cast<const uint8_t*>(x.data()), (uint32_t)x.size()});
+  for (const FilterString& f : strings)
+    if (f.len >= 4) min_long = std::min(min_long, f.len);
+  const uint32_t P = period_of(min_long);
+  return gram_coverage(strings, P, 4) > coverage_limit(P);
+}
 
 void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan, const std::vector<std::string>& prefixes) {
   plan.n_literals = given.n_literals;
@@ -202,30 +224,25 @@ void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan, const std:
     if (f.len >= 4) { plan.has_long = 1; min_long = std::min(min_long, f.len); }
     else plan.has_short = 1;
   }
-  // P grams at offsets 0..P-1 must fit inside every long string: P + 3 <= len.
-  plan.period = !plan.has_long ? 4 : (min_long >= 7) ? 4 : (min_long >= 5) ? 2 : 1;
+  plan.period = !plan.has_long ? 4 : period_of(min_long);
   plan.table_bits = 18;
   // A low-entropy set (a small alphabet whose 4-grams the strings mostly
   // cover, e.g. nucleotide k-mers) lets most input positions through 4-byte
   // grams: it takes the longest gram every long string holds at all P phases.
-  const bool low_entropy = plan.has_long && plan.period == 4 && min_long >= 11 && gram_coverage(strings, 4, 4) > 0.25;
+  const bool low_entropy = plan.has_long && plan.period == 4 && min_long >= 11 && gram_coverage(strings, 4, 4) > coverage_limit(4);
   if (low_entropy) plan.gram_len = min_long >= 19 ? 16 : 8;
-  // The gram kernel verifies in a later kernel what passes, from a list of one
-  // survivor per 64 bytes of input.  Where an input over the set's own
-  // alphabet would crowd that list (the grams cover more than 1/64 of the
-  // alphabet's; a quarter for P = 4, whose lookups are a quarter as many),
-  // the compacting kernel checks prefixes inside the filter instead.  Shortest
-  // string of three bytes: 3-byte grams at every position.
+  // Crowded sets take the compacting kernel, which checks prefixes inside the
+  // filter.  Shortest string of three bytes: 3-byte grams at every position.
   if (low_entropy) {
     plan.gram_kernel = plan.gram_len == 16 && !plan.has_short;
   } else if (min_len == 3) {
-    plan.gram_kernel = gram_coverage(strings, 1, 3) <= 1.0 / 64;
+    plan.gram_kernel = gram_coverage(strings, 1, 3) <= coverage_limit(1);
     if (plan.gram_kernel) {
       plan.period = 1;
       plan.gram_len = 3;
     }
   } else if (min_len >= 4) {
-    plan.gram_kernel = gram_coverage(strings, plan.period, 4) <= (plan.period == 4 ? 0.25 : 1.0 / 64);
+    plan.gram_kernel = gram_coverage(strings, plan.period, 4) <= coverage_limit(plan.period);
   }
   const uint32_t P = plan.period, G = plan.gram_len, bits = plan.table_bits;
   plan.parts = plan.bloom_parts = 0;

@@ -32,6 +32,7 @@
 
 
 #include "ws_internal.h"
+#include "ws_scan.h"
 
 namespace ws {
 
@@ -639,12 +640,13 @@ __device__ __forceinline__ bool prefix_bloom(const LitArgs& a, uint32_t s) {
   const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
   const uint32_t x0 = input_word(a, len, w0), x1 = input_word(a, len, w0 + 4), x2 = input_word(a, len, w0 + 8);
   const uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
-  bool keep = false;
-  for (uint32_t m = a.bloom_parts; m; m &= m - 1) {
-    const uint32_t key = prefix_key(lo, hi, __ffs(m));
-    keep |= (__ldg(a.bloom + (key >> 5)) >> (key & 31)) & 1u;
+  uint32_t keep = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < 8; ++i) {  // the loads of all lengths together
+    const uint32_t key = prefix_key(lo, hi, i + 1);
+    if ((a.bloom_parts >> i) & 1u) keep |= __ldg(a.bloom + (key >> 5)) >> (key & 31);
   }
-  return keep;
+  return keep & 1u;
 }
 
 // Key of the phase table for the gram at position at: a hash independent of
@@ -859,15 +861,91 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
   lean_holes(a, slots, lane);
 }
 
-__global__ void __launch_bounds__(256) literal_verify_kernel(LitArgs a) {
+// A position where a covered regex's prefix may start: every regex of which one
+// does (entries of different regexes may share it) runs its leftmost-first walk
+// from there, and a match makes a candidate.  A walk still open after kLfCap
+// bytes, or more long walks than the input has bytes, give the prefix
+// candidates up: the regexes' groups are walked instead (ctr[C_GATE]), whose
+// cost does not depend on the input.
+__device__ __forceinline__ void prefix_position(const LitArgs& a, const DevTables& t, const ScanPtrs& p,
+                                                const PrefixDev& pf, uint32_t s, bool in) {
+  uint32_t k = 0, k1 = 0, lo = 0, hi = 0;
+  if (in) {
+    const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
+    const uint32_t x0 = word_at(a.data, len, w0), x1 = word_at(a.data, len, w0 + 4), x2 = word_at(a.data, len, w0 + 8);
+    lo = __funnelshift_r(x0, x1, sh);
+    hi = __funnelshift_r(x1, x2, sh);
+    const uint32_t* rg = pf.range + ((lo * 0x9E3779B1u + hi * pf.mul) >> pf.shift);
+    k = __ldg(rg);
+    k1 = __ldg(rg + 1);
+  }
+  // every lane finds its next entry, then the lanes that have one walk together
+  while (true) {
+    uint32_t r = 0xFFFFFFFFu;
+    while (k < k1 && r == 0xFFFFFFFFu) {
+      const uint4 e = __ldg(pf.entry + k++);
+      if (e.x == lo && !((e.y ^ hi) & e.z)) r = e.w;
+    }
+    if (__ballot_sync(0xFFFFFFFFu, r != 0xFFFFFFFFu) == 0) return;
+    if (r != 0xFFFFFFFFu) {
+      if (*(volatile unsigned long long*)&p.ctr[C_GATE]) {
+        k = k1;
+      } else {
+        uint32_t steps = 0;
+        const uint32_t end = lf_walk(t, p, r, s, kLfCap, &steps);
+        if (end == kLfOpen || (steps > 64 && atomicAdd(&p.ctr[C_WORK], (unsigned long long)steps) > a.len))
+          atomicOr(&p.ctr[C_GATE], 1ull);
+        else if (end != kLfNone)
+          emit_k(p, r, s, end);
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// RX: the survivors are also looked up among the regex prefixes.  A full list
+// (more than one survivor per 64 bytes) gives the prefix candidates up, like
+// long walks do; the last block then drops the candidates found so far, so that
+// the gated groups start from none.
+template <bool RX>
+__global__ void __launch_bounds__(256) literal_verify_kernel(const __grid_constant__ LitArgs a,
+                                                             const __grid_constant__ DevTables t,
+                                                             const __grid_constant__ ScanPtrs p, PrefixDev pf) {
   unsigned long long n = *a.survivor_count;
-  if (n > a.survivor_cap) n = a.survivor_cap;
-  for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-       k += (unsigned long long)gridDim.x * blockDim.x) {
-    const uint32_t s = a.survivors[k];
-    if (s == kNoSurvivor) continue;  // a slot the gram kernel reserved but did not fill
-    if (a.verify_bloom && !prefix_bloom(a, s)) continue;  // stage 1.5 for survivors of the gram kernel
-    verify_position(a, s);
+  const bool full = n > a.survivor_cap;
+  if (full) n = a.survivor_cap;
+  // Neighbouring survivors go to different warps: a short list (the usual one)
+  // then has a survivor per warp, whose chains of dependent loads do not wait
+  // for one another.
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t w = blockIdx.x + gridDim.x * (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  for (unsigned long long k0 = w; k0 < n; k0 += 32ull * warps) {  // warp-uniform: lane 0 has the first one
+    const unsigned long long k = k0 + (unsigned long long)lane * warps;
+    const uint32_t s = k < n ? a.survivors[k] : kNoSurvivor;
+    // (kNoSurvivor: a slot the gram kernel reserved but did not fill; stage 1.5
+    // for the gram kernel's survivors, unless the prefix table alone decides)
+    bool in = s != kNoSurvivor;
+    if (in && a.verify_bloom && (!RX || a.parts)) in = prefix_bloom(a, s);
+    if (in && (!RX || a.parts)) verify_position(a, s);
+    if (RX && !full) prefix_position(a, t, p, pf, s, in);
+  }
+  if (RX) {
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      last = atomicAdd(&p.ctr[C_TICKET], 1ull) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (!full && *(volatile unsigned long long*)&p.ctr[C_GATE] == 0) return;
+    for (uint32_t r = threadIdx.x; r < t.n_regex; r += blockDim.x) p.count[r] = 0;
+    if (threadIdx.x == 0) {
+      p.ctr[C_K] = 0;
+      p.ctr[C_ERR] = 0;
+      p.ctr[C_GATE] = 1;
+    }
   }
 }
 
@@ -893,7 +971,7 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   a.period = plan.period;
   a.has_long = plan.has_long;
   a.has_short = plan.has_short;
-  a.parts = plan.parts;
+  a.parts = l.literals ? plan.parts : 0;  // (no prefix length, no literal)
   a.short_bits = plan.d_short.as<uint32_t>();
   a.bloom = plan.d_bloom.as<uint32_t>();
   a.info = plan.d_info.as<uint4>();
@@ -988,7 +1066,13 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   // kernel's longer survivor list (stage 1.5 runs here) gets more threads, a
   // short list no more blocks than it can fill
   const uint64_t vgrid = std::min<uint64_t>((uint64_t)sm_count * (a.verify_bloom ? 16 : 4), (l.survivor_cap + 255) / 256);
-  literal_verify_kernel<<<(unsigned)vgrid, 256, 0, st>>>(a);
+  if (l.rx) {
+    const PrefixDev pf{plan.d_prefix_range.as<uint32_t>(), plan.d_prefix_entry.as<uint4>(), plan.prefix_shift,
+                       plan.prefix_mul};
+    literal_verify_kernel<true><<<(unsigned)vgrid, 256, 0, st>>>(a, l.rx->t, l.rx->p, pf);
+  } else {
+    literal_verify_kernel<false><<<(unsigned)vgrid, 256, 0, st>>>(a, DevTables{}, ScanPtrs{}, PrefixDev{});
+  }
   check_cuda(cudaGetLastError(), "literal_verify_kernel launch");
 }
 

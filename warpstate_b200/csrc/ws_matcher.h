@@ -142,6 +142,7 @@ struct ws_matcher {
   std::mutex info_mu;
   ws_matcher_info info;
   bool profile = false;          // record phase events (single caller at a time)
+  bool walk_pinned = false;      // ws_matcher_set_walk was called: every speculative group walks
   // Bumped whenever the launch sequence of a scan may change (walk chunk,
   // proposer on or off, re-planned groups or hot rows): captured graphs of
   // earlier plans are not replayed.

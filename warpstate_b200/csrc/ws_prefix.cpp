@@ -1,0 +1,148 @@
+// Regex prefixes in the literal filter.
+//
+// A regex whose every match begins with one of a few strings needs no walk of
+// its group's DFA over the whole input: the literal filter, which passes over
+// the input at several times the walk's rate and once for all groups, finds
+// where those strings occur, and the verify kernel runs the regex's
+// leftmost-first DFA from there.  The candidates are the same distinct
+// (regex, start) pairs the walk finds.
+//
+// The walk takes one shared-memory lookup per input byte and group, 1.8 T
+// lookups/s over the chip; the filter one per second or fourth byte, once for
+// the literals and all groups.  Measured, us a pass with the walk and with the
+// filter: 500 regexes (9 groups) over 64 MiB 487 -> 171, 160 regexes (1 group)
+// over 1 GiB 939 -> 602, 60 unbounded regexes over 200 MiB 737 -> 273, 40
+// anchored ones over 32 MiB 300 -> 136, 40,000 items with 1,500 literals and
+// 200 regexes 1556 -> 414, 20,000 k-mers and 100 motifs over 2 GiB 2349 -> 892.
+// Where prefixes are dense the filter gives up at run time (ws_literal.cu,
+// literal_verify_kernel) and the walk does what it did before.
+#include <algorithm>
+#include <cstring>
+
+#include "ws_dfa.h"
+
+namespace ws {
+
+namespace {
+
+// All covered regexes' prefixes of one length; false when some regex has none
+// listed there or there are more than `most`.
+bool collect(const RegexPlan& P, int k, size_t most, std::vector<std::pair<std::string, uint32_t>>& out) {
+  out.clear();
+  for (uint32_t r = 0; r < P.n_regex; ++r) {
+    if (!P.covered[r]) continue;
+    if (P.prefixes[k][r].empty()) return false;
+    for (const std::string& x : P.prefixes[k][r]) out.emplace_back(x, r);
+    if (out.size() > most) return false;
+  }
+  return !out.empty();
+}
+
+}  // namespace
+
+// The length is the one that lets the filter look at the fewest positions that
+// the literals allow too: 7 bytes for every fourth, 5 for every second.  Longer
+// prefixes are more strings (a class in the prefix multiplies them): at most
+// 4,096 at 7 bytes and 16,384 at 5, beyond which the crowded filter costs more
+// than the lookups it saves.  A set whose 4-byte grams crowd their alphabet
+// takes 20 bytes (16-byte grams) or, where that is not possible, no prefixes:
+// its regexes are walked.
+void plan_filter(const ws_pattern_tables& t, const RegexPlan& P, LiteralPlan& plan) {
+  uint32_t shortest = UINT32_MAX;
+  for (uint32_t i = 0; i < t.n_literals; ++i) shortest = std::min(shortest, t.offsets[2 * i + 1]);
+  std::vector<std::pair<std::string, uint32_t>> pre;
+  const size_t most[kPrefixLens] = {65536, 4096, 16384, 65536};
+  bool found = false;
+  for (int k = 1; k < kPrefixLens && !found && P.n_regex; ++k)
+    found = (kPrefixLen[k] <= shortest || kPrefixLen[k] == 4) && collect(P, k, most[k], pre);
+  if (found) {
+    std::vector<std::string> strings;
+    for (const auto& x : pre) strings.push_back(x.first);
+    if (filter_crowded(t, strings)) found = shortest >= 19 && collect(P, 0, most[0], pre);
+  }
+  if (!found) pre.clear();
+  std::vector<std::string> strings;
+  for (const auto& x : pre) strings.push_back(x.first);
+  std::sort(strings.begin(), strings.end());
+  strings.erase(std::unique(strings.begin(), strings.end()), strings.end());
+  plan_literals(t, plan, strings);
+  if (pre.empty()) return;
+  // The verify kernel's table: entries by bucket of the first 4 bytes' hash (of
+  // all 8 where every entry has 8).  It needs no more of a regex's prefixes
+  // than tell most false positions apart, the walk decides: the longest listed
+  // with at most 16 different beginnings of up to 8 bytes, else those of 4
+  // bytes (a class after a short word makes hundreds with the same beginning,
+  // and a bucket is read one entry after another).
+  struct Entry {
+    uint32_t bucket, w0, w1, mask, r;
+  };
+  std::vector<Entry> es;
+  bool all8 = true;
+  for (uint32_t r = 0; r < P.n_regex; ++r) {
+    if (!P.covered[r]) continue;
+    std::vector<std::string> heads;
+    for (int k = 0; k < kPrefixLens; ++k) {
+      if (P.prefixes[k][r].empty()) continue;
+      heads.clear();
+      for (const std::string& x : P.prefixes[k][r]) heads.push_back(x.substr(0, 8));
+      heads.erase(std::unique(heads.begin(), heads.end()), heads.end());  // (sorted)
+      if (heads.size() <= 16) break;
+    }
+    for (const std::string& x : heads) {
+      uint32_t w[2] = {0, 0}, m[2] = {0, 0};
+      std::memcpy(w, x.data(), x.size());
+      std::memset(m, 0xFF, x.size());
+      es.push_back({0, w[0], w[1], m[1], r});
+      all8 &= x.size() == 8;
+    }
+  }
+  uint32_t bits = 6;
+  while (bits < 16 && ((size_t)1 << bits) < es.size()) ++bits;
+  plan.prefix_mul = all8 ? 0x85EBCA77u : 0u;
+  for (Entry& e : es) e.bucket = (e.w0 * 0x9E3779B1u + e.w1 * plan.prefix_mul) >> (32 - bits);
+  std::sort(es.begin(), es.end(), [](const Entry& a, const Entry& b) { return a.bucket < b.bucket; });
+  std::vector<uint32_t> range(((size_t)1 << bits) + 1, 0), entry;
+  for (const Entry& e : es) {
+    ++range[e.bucket + 1];
+    entry.insert(entry.end(), {e.w0, e.w1, e.mask, e.r});
+  }
+  for (size_t k = 1; k < range.size(); ++k) range[k] += range[k - 1];
+  plan.prefix_shift = 32 - bits;
+  plan.n_prefixes = (uint32_t)es.size();
+  plan.d_prefix_range.upload(range.data(), range.size() * 4);
+  plan.d_prefix_entry.upload(entry.data(), entry.size() * 4);
+}
+
+}  // namespace ws
+
+// Test hook: the prefixes of one regex at `len` bytes, as lines of hex.
+// Returns their number, -1 when there are too many or one is shorter than 4
+// bytes, -2 for a regex that does not parse; the text is cut at `cap` bytes.
+extern "C" long ws_testing_regex_prefixes(const char* source, unsigned len, unsigned long most, char* out,
+                                          unsigned long cap) {
+  using namespace ws;
+  try {
+    const ReTree tree = parse_regex(source);
+    const bool ctx = tree_has_look(tree);
+    const Nfa n = build_nfa({&tree}, false);
+    const ByteClasses bc = compute_classes({&n});
+    const Dfa d = ctx ? build_context_all_dfa(n, bc, 1 << 16) : build_all_dfa(n, bc, true, 1 << 16);
+    std::vector<std::string> found;
+    if (d.too_big || !regex_prefixes(d, bc, ctx, len, most, found)) return -1;
+    std::string text;
+    for (const std::string& x : found) {
+      for (char c : x) {
+        const char* hex = "0123456789abcdef";
+        text += hex[(uint8_t)c >> 4];
+        text += hex[(uint8_t)c & 15];
+      }
+      text += '\n';
+    }
+    const size_t k = std::min<size_t>(text.size(), cap ? cap - 1 : 0);
+    std::memcpy(out, text.data(), k);
+    if (cap) out[k] = 0;
+    return (long)found.size();
+  } catch (const std::exception&) {
+    return -2;
+  }
+}

@@ -1003,6 +1003,45 @@ Dfa build_context_lf_dfa(const Nfa& nfa, const ByteClasses& cls, int max_states)
   return d;
 }
 
+bool regex_prefixes(const Dfa& d, const ByteClasses& cls, bool context, uint32_t len, size_t most,
+                    std::vector<std::string>& out) {
+  out.clear();
+  std::vector<uint32_t> starts;
+  if (context) starts.assign(d.ctx_start, d.ctx_start + 4);
+  else starts.push_back(d.start_anchored);
+  std::sort(starts.begin(), starts.end());
+  starts.erase(std::unique(starts.begin(), starts.end()), starts.end());
+  typedef std::pair<std::string, uint32_t> Item;  // bytes, state after them
+  std::vector<std::string> found;
+  std::vector<Item> cur, nxt;
+  for (uint32_t s : starts) cur.emplace_back(std::string(), s);
+  for (uint32_t depth = 0; !cur.empty(); ++depth) {
+    nxt.clear();
+    for (const Item& it : cur) {
+      const uint32_t* row = d.trans.data() + (size_t)it.second * d.n_classes;
+      size_t ways = 0;
+      for (int b = 0; b < 256; ++b) ways += (row[cls.map[b]] & DFA_FLAG_DEAD) ? 0 : 1;
+      const bool ends = d.is_match[it.second] != 0;  // (in a context DFA: under some right context)
+      if (ends && depth < 4) return false;
+      if (ends || (depth >= len && (depth >= 8 || ways != 1))) {
+        found.push_back(it.first);
+        if (found.size() > 4 * most) return false;
+        continue;
+      }
+      if (nxt.size() + ways > 4 * most) return false;  // (up to four starts give the same string)
+      for (int b = 0; b < 256; ++b)
+        if (!(row[cls.map[b]] & DFA_FLAG_DEAD))
+          nxt.emplace_back(it.first + (char)(uint8_t)b, row[cls.map[b]] & DFA_MASK_STATE);
+    }
+    cur.swap(nxt);
+  }
+  std::sort(found.begin(), found.end());
+  for (const std::string& x : found)  // sorted: a prefix comes right before what it begins
+    if (out.empty() || x.compare(0, out.back().size(), out.back()) != 0) out.push_back(x);
+  if (out.size() > most) out.clear();
+  return !out.empty();
+}
+
 void renumber_dfa(Dfa& d, const std::vector<uint32_t>& order) {
   const int n = d.n_states, C = d.n_classes;
   std::vector<uint32_t> inv((size_t)n);

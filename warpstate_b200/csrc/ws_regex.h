@@ -140,6 +140,15 @@ Dfa build_leftmost_first_dfa(const Nfa& nfa, const ByteClasses& cls, int max_sta
 Dfa build_context_all_dfa(const Nfa& nfa, const ByteClasses& cls, int max_states);
 Dfa build_context_lf_dfa(const Nfa& nfa, const ByteClasses& cls, int max_states);
 
+// The strings that matches of the DFA's one pattern begin with: bytes along
+// every path from its anchored start (the start rows of every left context in a
+// context DFA), up to `len` bytes or to where a match can end, whichever comes
+// first; past `len`, up to 8 bytes where only one byte continues.  Sorted, none
+// a prefix of another.  False (and empty) when there are more than `most` or
+// one is shorter than 4 bytes.  `d`: build_all_dfa or build_context_all_dfa.
+bool regex_prefixes(const Dfa& d, const ByteClasses& cls, bool context, uint32_t len, size_t most,
+                    std::vector<std::string>& out);
+
 // Reorders states so that `order` (old ids, dead state first) becomes 0..n-1.
 void renumber_dfa(Dfa& d, const std::vector<uint32_t>& order);
 

@@ -196,6 +196,7 @@ extern "C" ws_status ws_matcher_set_walk(ws_matcher* m, uint32_t walk_chunk, uin
       m->cfg.walk_chunk = walk_chunk;
     }
     m->rx.use_proposer = proposer == WS_PROPOSER_MLP;
+    m->walk_pinned = true;
     m->plan_gen++;
   });
 }
