@@ -38,7 +38,7 @@ struct RxLayout {
   uint64_t n_chunks = 0, chunk = 0, nck = 0, n_q = 0;
   uint64_t k_cap = 0, ev_cap = 0;
   size_t off_ctr, off_k, off_ev, off_guess, off_used, off_end, off_spec, off_conv, off_round, off_ckpt,
-      off_count, off_offs, off_cursor, off_starts, off_lfend, off_rmark, total;
+      off_count, off_offs, off_pair, off_pair2, off_rmark, total;
 };
 
 // Candidate and event buffers hold at most this many entries (the per-regex
@@ -70,9 +70,8 @@ RxLayout layout(const RegexPlan& p, uint64_t len, uint32_t chunk, uint64_t max_m
   L.off_round = take(L.n_q * 4);
   L.off_ckpt = take(L.n_q * L.nck * 4);
   L.off_offs = take(((size_t)p.n_regex + 1) * 4);
-  L.off_cursor = take((size_t)p.n_regex * 4);
-  L.off_starts = take(L.k_cap * 4);
-  L.off_lfend = take(L.k_cap * 4);
+  L.off_pair = take(L.k_cap * 8);
+  L.off_pair2 = take(L.k_cap * 8);
   L.off_rmark = take(((size_t)1 << kRmarkBits) * 8);
   L.total = o;
   return L;
@@ -97,9 +96,8 @@ ScanPtrs make_ptrs(const RxLayout& L, void* base, const RegexLaunch& l) {
   p.ckpt = reinterpret_cast<uint32_t*>(b + L.off_ckpt);
   p.count = reinterpret_cast<uint32_t*>(b + L.off_count);
   p.offs = reinterpret_cast<uint32_t*>(b + L.off_offs);
-  p.cursor = reinterpret_cast<uint32_t*>(b + L.off_cursor);
-  p.starts = reinterpret_cast<uint32_t*>(b + L.off_starts);
-  p.lfend = reinterpret_cast<uint32_t*>(b + L.off_lfend);
+  p.pair = reinterpret_cast<unsigned long long*>(b + L.off_pair);
+  p.pair2 = reinterpret_cast<unsigned long long*>(b + L.off_pair2);
   p.rmark = reinterpret_cast<unsigned long long*>(b + L.off_rmark);
   p.full_k = 0;
   p.count_guesses = 0;
@@ -797,13 +795,14 @@ __global__ void __launch_bounds__(256) dfa_reverse_kernel(DevTables t, ScanPtrs 
 }
 
 // ---------------------------------------------------------------- resolution
-__global__ void k_scan_kernel(ScanPtrs p, uint32_t n_regex) {
-  // single-block exclusive scan (blockDim.x a multiple of 32, at most 1024):
-  // each thread sums a run of regexes, the runs are scanned across the block
-  // with warp shuffles, then each thread writes its run's offsets
+// Exclusive scan of the per-regex candidate counts into offs[0, n_regex] by one
+// block (blockDim.x a multiple of 32, at most 1024): each thread sums a run of
+// regexes, the runs are scanned across the block with warp shuffles, then each
+// thread writes its run's offsets.
+__device__ void scan_counts(const ScanPtrs& p, uint32_t n_regex, uint32_t* offs) {
   __shared__ uint32_t wsum[32];
   const uint32_t per = (n_regex + blockDim.x - 1) / blockDim.x;
-  const uint32_t a = threadIdx.x * per, b = min(n_regex, a + per);
+  const uint32_t a = min(n_regex, threadIdx.x * per), b = min(n_regex, a + per);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   uint32_t sum = 0;
   for (uint32_t r = a; r < b; ++r) sum += p.count[r];
@@ -825,29 +824,52 @@ __global__ void k_scan_kernel(ScanPtrs p, uint32_t n_regex) {
     wsum[lane] = v;  // inclusive sums of the warps' runs
   }
   __syncthreads();
-  if (threadIdx.x == 0) p.offs[n_regex] = wsum[nw - 1];
+  if (threadIdx.x == 0) offs[n_regex] = wsum[nw - 1];
   uint32_t acc = incl - sum + (warp ? wsum[warp - 1] : 0u);
-  for (uint32_t r = a; r < b; ++r) { p.offs[r] = acc; p.cursor[r] = acc; acc += p.count[r]; }
+  for (uint32_t r = a; r < b; ++r) {
+    offs[r] = acc;
+    acc += p.count[r];
+  }
 }
 
-__global__ void k_scatter_kernel(ScanPtrs p) {
-  unsigned long long n = min(p.ctr[C_K], (unsigned long long)p.k_cap);
+__global__ void k_scan_kernel(ScanPtrs p, uint32_t n_regex) { scan_counts(p, n_regex, p.offs); }
+
+// The regexes' candidate offsets are staged in shared memory when they fit.
+constexpr uint32_t kOffsShared = 8192;
+
+// Every candidate to its place in its regex's list: the regex's offset plus the
+// rank it drew when it was counted.  Each block that has candidates scans the
+// counts itself (a few hundred of them: less than a launch), the first one
+// also for the later kernels; sets of kOffsShared regexes and more have them
+// scanned before.
+__global__ void __launch_bounds__(256) k_scatter_kernel(ScanPtrs p, uint32_t n_regex) {
+  extern __shared__ uint32_t offs_s[];
+  const unsigned long long n = min(p.ctr[C_K], (unsigned long long)p.k_cap);
+  const bool staged = n_regex < kOffsShared;
+  if (blockIdx.x && (unsigned long long)blockIdx.x * blockDim.x >= n) return;
+  if (staged) {
+    scan_counts(p, n_regex, offs_s);
+    __syncthreads();
+    if (blockIdx.x == 0)
+      for (uint32_t r = threadIdx.x; r <= n_regex; r += blockDim.x) p.offs[r] = offs_s[r];
+  }
+  const uint32_t* offs = staged ? offs_s : p.offs;
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-    KCand c = p.k[k];
-    uint32_t slot = atomicAdd(&p.cursor[c.r], 1u);
-    p.starts[slot] = c.s;
+    const KCand c = p.k[k];
+    p.pair[offs[c.r] + (c.rank & ~kEndKnown)] =
+        ((unsigned long long)c.s << 32) | ((c.rank & kEndKnown) ? c.e : kLfTodo);
   }
 }
 
 // Block-wide bitonic sort of buf[0, m) in shared memory (m a power of two).
-__device__ void bitonic_smem(uint32_t* buf, uint32_t m) {
+__device__ void bitonic_smem(unsigned long long* buf, uint32_t m) {
   for (uint32_t size = 2; size <= m; size <<= 1) {
     for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
       for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) {
         uint32_t j = k ^ stride;
         if (j > k) {
           bool up = (k & size) == 0;
-          uint32_t x = buf[k], y = buf[j];
+          unsigned long long x = buf[k], y = buf[j];
           if ((x > y) == up) { buf[k] = y; buf[j] = x; }
         }
       }
@@ -856,20 +878,21 @@ __device__ void bitonic_smem(uint32_t* buf, uint32_t m) {
   }
 }
 
-// Sorts src[0, n), n <= 4096, in place through shared memory.
-__device__ void sort_tile(uint32_t* buf, uint32_t* src, uint32_t n) {
+constexpr uint32_t kSortTile = 4096;
+
+// Sorts src[0, n), n <= kSortTile, into buf (shared memory).
+__device__ void sort_into(unsigned long long* buf, const unsigned long long* src, uint32_t n) {
   uint32_t m = 1;
   while (m < n) m <<= 1;
-  for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) buf[k] = (k < n) ? src[k] : 0xFFFFFFFFu;
+  for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) buf[k] = (k < n) ? src[k] : ~0ull;
   __syncthreads();
   bitonic_smem(buf, m);
-  for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) src[k] = buf[k];
-  __syncthreads();
 }
 
 // Number of elements taken from A among the first `diag` of the merge of
 // sorted A and B (ties from A first).
-__device__ uint32_t merge_path(const uint32_t* A, uint32_t na, const uint32_t* B, uint32_t nb, uint32_t diag) {
+__device__ uint32_t merge_path(const unsigned long long* A, uint32_t na, const unsigned long long* B, uint32_t nb,
+                               uint32_t diag) {
   uint32_t lo = diag > nb ? diag - nb : 0, hi = min(diag, na);
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
@@ -878,55 +901,62 @@ __device__ uint32_t merge_path(const uint32_t* A, uint32_t na, const uint32_t* B
   return lo;
 }
 
-// Sorts each regex's starts ascending: a bitonic sort in shared memory for
-// segments of up to 4096; beyond that, sorted 4096-tiles merged pairwise in
-// global memory (merge-path split of each merge across the block), with the
-// lfend array -- written only after this kernel -- as the other buffer.
-__global__ void __launch_bounds__(512) k_sort_kernel(ScanPtrs p, uint32_t n_regex) {
-  __shared__ uint32_t buf[4096];
-  for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
-    const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
-    if (n <= 1) continue;
-    uint32_t* src = p.starts + a;
-    if (n <= 4096) {
-      sort_tile(buf, src, n);
-      continue;
+// Sorts regex candidates list[0, n) ascending by start: a bitonic sort in
+// shared memory for up to kSortTile; beyond that, sorted tiles merged pairwise
+// in global memory (merge-path split of each merge across the block), with
+// other[0, n) as the other buffer.
+__device__ void sort_list(unsigned long long* buf, unsigned long long* list, unsigned long long* other, uint32_t n) {
+  for (uint32_t t0 = 0; t0 < n; t0 += kSortTile) {
+    const uint32_t m = min(kSortTile, n - t0);
+    sort_into(buf, list + t0, m);
+    for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) list[t0 + k] = buf[k];
+    __syncthreads();
+  }
+  unsigned long long *src = list, *dst = other;
+  for (uint32_t w = kSortTile; w < n; w <<= 1) {
+    for (uint32_t lo = 0; lo < n; lo += 2 * w) {
+      const uint32_t mid = min(lo + w, n), hi = min(lo + 2 * w, n);
+      const unsigned long long *A = src + lo, *B = src + mid;
+      const uint32_t na = mid - lo, nb = hi - mid, total = hi - lo;
+      const uint32_t per = (total + blockDim.x - 1) / blockDim.x;
+      const uint32_t d0 = min(total, threadIdx.x * per), d1 = min(total, d0 + per);
+      uint32_t i = merge_path(A, na, B, nb, d0), j = d0 - i;
+      for (uint32_t d = d0; d < d1; ++d) dst[lo + d] = (j >= nb || (i < na && A[i] <= B[j])) ? A[i++] : B[j++];
     }
-    for (uint32_t t0 = 0; t0 < n; t0 += 4096) sort_tile(buf, src + t0, min(4096u, n - t0));
-    uint32_t* dst = p.lfend + a;
-    for (uint32_t w = 4096; w < n; w <<= 1) {
-      for (uint32_t lo = 0; lo < n; lo += 2 * w) {
-        const uint32_t mid = min(lo + w, n), hi = min(lo + 2 * w, n);
-        const uint32_t* A = src + lo;
-        const uint32_t* B = src + mid;
-        const uint32_t na = mid - lo, nb = hi - mid, total = hi - lo;
-        const uint32_t per = (total + blockDim.x - 1) / blockDim.x;
-        const uint32_t d0 = min(total, threadIdx.x * per), d1 = min(total, d0 + per);
-        uint32_t i = merge_path(A, na, B, nb, d0), j = d0 - i;
-        for (uint32_t d = d0; d < d1; ++d) dst[lo + d] = (j >= nb || (i < na && A[i] <= B[j])) ? A[i++] : B[j++];
-      }
-      __syncthreads();
-      uint32_t* t = src;
-      src = dst;
-      dst = t;
-    }
-    if (src != p.starts + a) {
-      for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) p.starts[a + k] = src[k];
-      __syncthreads();
-    }
+    __syncthreads();
+    unsigned long long* t = src;
+    src = dst;
+    dst = t;
+  }
+  if (src != list) {
+    for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) list[k] = src[k];
+    __syncthreads();
   }
 }
 
-// Leftmost-first end of every distinct candidate start (in parallel), each
-// walk cut off after kLfCap bytes.
-// The regexes' candidate offsets are staged in shared memory when they fit
-// (kLfOffsShared regexes), so that finding a candidate's regex is a binary
-// search in shared memory rather than a chain of dependent global loads.
-constexpr uint32_t kLfOffsShared = 8192;
+__global__ void __launch_bounds__(512) k_sort_kernel(ScanPtrs p, uint32_t n_regex) {
+  __shared__ unsigned long long buf[kSortTile];
+  for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
+    const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
+    if (n > 1) sort_list(buf, p.pair + a, p.pair2 + a, n);
+  }
+}
 
+// Leftmost-first end of candidate j of a sorted list, its walk cut off after
+// kLfCap bytes; a start listed before has none.
+__device__ __forceinline__ uint32_t list_end(const DevTables& t, const ScanPtrs& p, uint32_t r,
+                                             const unsigned long long* list, uint32_t j) {
+  const uint32_t s = (uint32_t)(list[j] >> 32);
+  if (j && (uint32_t)(list[j - 1] >> 32) == s) return kLfNone;
+  const uint32_t e = lf_walk(t, p, r, s, kLfCap);
+  return e == kLfOpen ? kLfLong : e;
+}
+
+// The ends that are not known yet, in parallel over all candidates.  A
+// candidate's regex comes from a binary search over the offsets.
 __global__ void k_lf_kernel(DevTables t, ScanPtrs p, uint32_t n_regex) {
   extern __shared__ uint32_t offs_s[];
-  const bool staged = n_regex < kLfOffsShared;
+  const bool staged = n_regex < kOffsShared;
   if (staged) {
     for (uint32_t r = threadIdx.x; r <= n_regex; r += blockDim.x) offs_s[r] = p.offs[r];
     __syncthreads();
@@ -934,61 +964,90 @@ __global__ void k_lf_kernel(DevTables t, ScanPtrs p, uint32_t n_regex) {
   const uint32_t* offs = staged ? offs_s : p.offs;
   const uint32_t total = offs[n_regex];
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
-    // owning regex: binary search in offs
+    if ((uint32_t)p.pair[j] != kLfTodo) continue;
     uint32_t lo = 0, hi = n_regex;
     while (hi - lo > 1) {
       uint32_t mid = (lo + hi) >> 1;
       if (offs[mid] <= j) lo = mid; else hi = mid;
     }
-    const uint32_t r = lo;
-    const uint32_t s = p.starts[j];
-    if (j > offs[r] && p.starts[j - 1] == s) { p.lfend[j] = kLfNone; continue; }  // duplicate
-    const uint32_t e = lf_walk(t, p, r, s, kLfCap);
-    p.lfend[j] = e == kLfOpen ? kLfLong : e;
+    // (only the low half is written: the neighbour reads this start)
+    reinterpret_cast<uint32_t*>(p.pair + j)[0] = list_end(t, p, lo, p.pair + offs[lo], j - offs[lo]);
   }
 }
 
-// find_iter chain per regex: leftmost candidate start with its leftmost-first
-// end, then the next candidate at or after that end.
-// One warp per regex: the warp loads 32 sorted candidates at a time and picks
-// the chain's next match among them with a ballot (the first candidate whose
-// start is at or after the current end), so the serial part is one ballot per
-// reported match.
-__global__ void k_chain_kernel(DevTables t, ScanPtrs p) {
-  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31;
-  if (r >= t.n_regex) return;  // whole warps exit together
-  const uint32_t a = p.offs[r], b = p.offs[r + 1];
+// After a candidate or event buffer overflow the scan's match count is not
+// known: the count becomes kCountUnknown (larger than any capacity), and the
+// capacities the scan would have needed are recorded in `need` (host-mapped
+// memory of the matcher, read by the next launch), so the same scan run again
+// fits.  By one thread of the last kernel, whose other threads then add
+// nothing: true when the scan has failed.
+__device__ bool finalize(const ScanPtrs& p, unsigned long long* need) {
+  const unsigned long long err = p.ctr[C_ERR];
+  if (!err) return false;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *p.out_counter = (err & kErrTimeout) ? kCountTimeout : kCountUnknown;
+    if (!(err & kErrTimeout) && need) {
+      volatile unsigned long long* v = need;
+      if (p.ctr[C_K] > v[0]) v[0] = p.ctr[C_K];
+      if (p.ctr[C_EV] > v[1]) v[1] = p.ctr[C_EV];
+    }
+  }
+  return true;
+}
+
+// find_iter chain of one regex over its sorted candidates, by one warp:
+// leftmost candidate start with its leftmost-first end, then the next candidate
+// at or after that end.  32 candidates at a time; where none of them overlaps
+// the one before it (the usual case) all are taken at once, else a ballot per
+// reported match picks the first one at or after the current end.
+__device__ void chain_list(const DevTables& t, const ScanPtrs& p, uint32_t r, const unsigned long long* list,
+                           uint32_t n, uint32_t lane) {
   const uint32_t pid = t.pid[r];
   // stream scans: resume at the regex's cursor, decide only starts before the
   // frontier (both in stream offsets; the buffer starts at p.base <= cursor)
   uint64_t last_end = (p.cursor64 && p.cursor64[r] > p.base) ? p.cursor64[r] - p.base : 0;
   const uint64_t limit = p.cursor64 ? p.frontier - p.base : ~0ull;
   // each window's candidates are loaded while the previous window is decided
-  uint32_t e_nx = a + lane < b ? p.lfend[a + lane] : kLfNone;
-  uint32_t s_nx = a + lane < b ? p.starts[a + lane] : 0xFFFFFFFFu;
-  for (uint32_t j0 = a; j0 < b; j0 += 32) {
-    const uint32_t j = j0 + lane;
-    const bool in = j < b;
-    uint32_t e = e_nx;
-    const uint32_t s = s_nx;
-    e_nx = j + 32 < b ? p.lfend[j + 32] : kLfNone;
-    s_nx = j + 32 < b ? p.starts[j + 32] : 0xFFFFFFFFu;
+  const unsigned long long none = ((unsigned long long)0xFFFFFFFFu << 32) | kLfNone;
+  unsigned long long next = lane < n ? list[lane] : none;
+  for (uint32_t j0 = 0; j0 < n; j0 += 32) {
+    const bool in = j0 + lane < n;
+    const unsigned long long c = next;
+    next = j0 + 32 + lane < n ? list[j0 + 32 + lane] : none;
+    const uint32_t s = (uint32_t)(c >> 32);
+    uint32_t e = (uint32_t)c;
     const bool past = in && (uint64_t)s >= limit;
     bool picked = false;
-    while (true) {
-      const bool ok = in && e != kLfNone && (uint64_t)s >= last_end && !past;
-      const unsigned m = __ballot_sync(0xFFFFFFFFu, ok);
-      if (!m) break;
-      const int k = __ffs(m) - 1;
-      uint32_t ek = __shfl_sync(0xFFFFFFFFu, e, k);
-      if (ek == kLfLong) {  // the parallel walk was cut off: finish it here
-        if ((int)lane == k) e = lf_walk(t, p, r, s, ~0ull);
-        ek = __shfl_sync(0xFFFFFFFFu, e, k);
-        if (ek == kLfNone) continue;  // no match from that start after all
+    const bool valid = in && e != kLfNone && (uint64_t)s >= last_end && !past;
+    // ends of the valid candidates before this lane's
+    uint32_t before = valid && e != kLfLong ? e : 0u;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, before, d);
+      if (lane >= (uint32_t)d) before = max(before, y);
+    }
+    const uint32_t upto = before;
+    before = __shfl_up_sync(0xFFFFFFFFu, upto, 1);
+    if (lane == 0) before = 0;
+    if (!__any_sync(0xFFFFFFFFu, valid && (s < before || e == kLfLong))) {
+      picked = valid;
+      const uint32_t top = __shfl_sync(0xFFFFFFFFu, upto, 31);
+      last_end = max(last_end, (uint64_t)top);
+    } else {
+      while (true) {
+        const bool ok = in && e != kLfNone && (uint64_t)s >= last_end && !past;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, ok);
+        if (!m) break;
+        const int k = __ffs(m) - 1;
+        uint32_t ek = __shfl_sync(0xFFFFFFFFu, e, k);
+        if (ek == kLfLong) {  // the parallel walk was cut off: finish it here
+          if ((int)lane == k) e = lf_walk(t, p, r, s, ~0ull);
+          ek = __shfl_sync(0xFFFFFFFFu, e, k);
+          if (ek == kLfNone) continue;  // no match from that start after all
+        }
+        picked |= (int)lane == k;
+        last_end = ek;
       }
-      picked |= (int)lane == k;
-      last_end = ek;
     }
     // one output reservation per window of 32 candidates
     const unsigned pm = __ballot_sync(0xFFFFFFFFu, picked);
@@ -1006,6 +1065,39 @@ __global__ void k_chain_kernel(DevTables t, ScanPtrs p) {
   if (p.cursor64 && lane == 0) p.cursor64[r] = max(p.base + last_end, p.frontier);
 }
 
+// A warp per regex.
+__global__ void k_chain_kernel(DevTables t, ScanPtrs p, unsigned long long* need) {
+  if (finalize(p, need)) return;
+  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (r >= t.n_regex) return;  // whole warps exit together
+  chain_list(t, p, r, p.pair + p.offs[r], p.offs[r + 1] - p.offs[r], threadIdx.x & 31);
+}
+
+// Sort, missing ends and chain of a regex by one block, in shared memory for up
+// to kSortTile candidates: the resolution of scans whose candidates came from
+// prefixes, ends known (three kernels and a pass through global memory between
+// each took 8 us more on small lists).
+__global__ void __launch_bounds__(256) k_resolve_kernel(DevTables t, ScanPtrs p, uint32_t n_regex,
+                                                        unsigned long long* need) {
+  __shared__ unsigned long long buf[kSortTile];
+  if (finalize(p, need)) return;
+  for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
+    const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
+    unsigned long long* list = p.pair + a;
+    if (n > kSortTile) {
+      sort_list(buf, list, p.pair2 + a, n);
+    } else if (n) {
+      sort_into(buf, list, n);
+      list = buf;
+    }
+    for (uint32_t j = threadIdx.x; j < n; j += blockDim.x)
+      if ((uint32_t)list[j] == kLfTodo) reinterpret_cast<uint32_t*>(list + j)[0] = list_end(t, p, r, list, j);
+    __syncthreads();
+    if (threadIdx.x < 32) chain_list(t, p, r, list, n, threadIdx.x);
+    __syncthreads();  // the next regex's sort overwrites buf
+  }
+}
+
 // Copies K candidates into a ws_match buffer (diagnostics).
 __global__ void k_export_kernel(DevTables t, ScanPtrs p, ws_match* out, uint64_t cap) {
   unsigned long long n = min(p.ctr[C_K], (unsigned long long)p.k_cap);
@@ -1013,24 +1105,6 @@ __global__ void k_export_kernel(DevTables t, ScanPtrs p, ws_match* out, uint64_t
        k += (uint64_t)gridDim.x * blockDim.x) {
     KCand c = p.k[k];
     out[k] = ws_match{t.pid[c.r], c.s, c.e};
-  }
-}
-
-// After a candidate or event buffer overflow the scan's match count is not
-// known: the count becomes kCountUnknown (larger than any capacity), and the
-// capacities the scan would have needed are recorded in `need` (host-mapped
-// memory of the matcher, read by the next launch), so the same scan run again
-// fits.  One thread, after every other kernel of the scan.
-__global__ void finalize_kernel(ScanPtrs p, unsigned long long* need) {
-  if (p.ctr[C_ERR] & kErrTimeout) {
-    *p.out_counter = kCountTimeout;
-  } else if (p.ctr[C_ERR]) {
-    *p.out_counter = kCountUnknown;
-    if (need) {
-      volatile unsigned long long* v = need;
-      if (p.ctr[C_K] > v[0]) v[0] = p.ctr[C_K];
-      if (p.ctr[C_EV] > v[1]) v[1] = p.ctr[C_EV];
-    }
   }
 }
 
@@ -1788,17 +1862,25 @@ uint32_t regex_finish(RegexPlan& P, RegexScan& rs, const RegexLaunch& l, cudaStr
   uint32_t launches = 0;
   if (ev) check_cuda(cudaEventRecord(ev[0], st), "event");
   launches += candidates_phase(P, t, p, l.mode, st, sm_count, ev);
-  int hg = (int)std::min<uint64_t>((uint64_t)sm_count * 8, (rs.k_cap + 255) / 256);
-  k_scan_kernel<<<1, 1024, 0, st>>>(p, P.n_regex);
-  k_scatter_kernel<<<hg, 256, 0, st>>>(p);
-  k_sort_kernel<<<(unsigned)std::min<uint32_t>(P.n_regex, 4096), 512, 0, st>>>(p, P.n_regex);
-  k_lf_kernel<<<sm_count * 8, 128, P.n_regex < kLfOffsShared ? (P.n_regex + 1) * 4 : 0, st>>>(t, p, P.n_regex);
-  k_chain_kernel<<<(P.n_regex + 3) / 4, 128, 0, st>>>(t, p);  // a warp per regex
-  check_cuda(cudaGetLastError(), "resolution kernels");
-  launches += 5;
-  finalize_kernel<<<1, 1, 0, st>>>(p, l.need);
-  check_cuda(cudaGetLastError(), "finalize_kernel");
+  const bool staged = P.n_regex < kOffsShared;
+  const size_t osmem = staged ? ((size_t)P.n_regex + 1) * 4 : 0;
+  const int hg = (int)std::min<uint64_t>((uint64_t)sm_count * 4, (rs.k_cap + 255) / 256);
+  if (!staged) {
+    k_scan_kernel<<<1, 1024, 0, st>>>(p, P.n_regex);
+    launches += 1;
+  }
+  k_scatter_kernel<<<hg, 256, osmem, st>>>(p, P.n_regex);
   launches += 1;
+  if (rs.prefixes && t.n_walk == 0 && t.n_ctx_walk == P.n_spec) {
+    k_resolve_kernel<<<(unsigned)std::min<uint32_t>(P.n_regex, 4096), 256, 0, st>>>(t, p, P.n_regex, l.need);
+    launches += 1;
+  } else {
+    k_sort_kernel<<<(unsigned)std::min<uint32_t>(P.n_regex, 4096), 512, 0, st>>>(p, P.n_regex);
+    k_lf_kernel<<<sm_count * 8, 128, osmem, st>>>(t, p, P.n_regex);
+    k_chain_kernel<<<(P.n_regex + 3) / 4, 128, 0, st>>>(t, p, l.need);  // a warp per regex
+    launches += 3;
+  }
+  check_cuda(cudaGetLastError(), "resolution kernels");
   if (ev) {
     // profiled scans read the counters back for ws_matcher_get_info
     if (!P.prof_ctr) {

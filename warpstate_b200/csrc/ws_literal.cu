@@ -128,7 +128,8 @@ __device__ __forceinline__ uint32_t input_word(const LitArgs& a, uint32_t len, u
 // one launch are below 4 GiB.  The hashed bytes come from two words read
 // once, and a candidate literal is compared a word at a time (literal bytes
 // start 4-aligned in a buffer padded to 16 bytes).
-__device__ void verify_position(const LitArgs& a, uint64_t s64) {
+template <class Sink>
+__device__ void verify_position(const LitArgs& a, uint64_t s64, Sink&& sink) {
   if (s64 >= a.max_start) return;
   const uint32_t s = (uint32_t)s64, len = (uint32_t)a.len;
   const uint32_t w0 = s & ~3u, sh = (s & 3) * 8;
@@ -161,16 +162,20 @@ __device__ void verify_position(const LitArgs& a, uint64_t s64) {
       if (!eq) continue;
       if (s + info.y <= a.min_end) continue;
       if (a.n_items && s + info.y > item_end_of(a.item_end, a.n_items, (uint32_t)s)) continue;  // crosses items
-      unsigned long long idx = atomicAdd(a.counter, 1ull);
-      if (idx < a.cap) {
-        ws_match mm;
-        mm.pattern_id = info.z;
-        mm.start = (uint32_t)s;
-        mm.end = (uint32_t)(s + info.y);
-        a.out[idx] = mm;
-      }
+      sink(info.z, s, s + info.y);
     }
   }
+}
+
+// A match straight to the output.
+__device__ __forceinline__ void report_match(const LitArgs& a, uint32_t pid, uint32_t s, uint32_t e) {
+  const unsigned long long idx = atomicAdd(a.counter, 1ull);
+  if (idx < a.cap) a.out[idx] = ws_match{pid, s, e};
+}
+
+// Verifies a position in the filter kernel (the survivor list is full).
+__device__ __forceinline__ void verify_in_place(const LitArgs& a, uint32_t s) {
+  verify_position(a, s, [&](uint32_t pid, uint32_t at, uint32_t e) { report_match(a, pid, at, e); });
 }
 
 // 16-bit mask of owned positions that may start a literal (stage 1).  w[0..3]
@@ -328,7 +333,7 @@ __device__ __forceinline__ void process_block(const LitArgs& a, uint32_t* blk, u
         const unsigned long long slot = wbase + __popc(ball & ((1u << lane) - 1u));
         const uint32_t s = blk_base + off;
         if (slot < a.survivor_cap) a.survivors[slot] = s;
-        else verify_position(a, s);  // list full: verify in place
+        else verify_in_place(a, s);  // list full
       }
     }
   }
@@ -700,7 +705,7 @@ __device__ __forceinline__ void gram_flush(const LitArgs& a, const uint32_t* que
     for (; bits; bits &= bits - 1) {
       const uint32_t s = at - (P - 1) + (__ffs(bits) - 1);
       if (slot < a.survivor_cap) a.survivors[slot] = s;
-      else if (prefix_bloom(a, s)) verify_position(a, s);  // list full: verify in place
+      else if (prefix_bloom(a, s)) verify_in_place(a, s);  // list full
       ++slot;
     }
   }
@@ -867,8 +872,9 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
 // bytes, or more long walks than the input has bytes, give the prefix
 // candidates up: the regexes' groups are walked instead (ctr[C_GATE]), whose
 // cost does not depend on the input.
+template <class Sink>
 __device__ __forceinline__ void prefix_position(const LitArgs& a, const DevTables& t, const ScanPtrs& p,
-                                                const PrefixDev& pf, uint32_t s, bool in) {
+                                                const PrefixDev& pf, uint32_t s, bool in, Sink&& sink) {
   uint32_t k = 0, k1 = 0, lo = 0, hi = 0;
   if (in) {
     const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
@@ -896,7 +902,7 @@ __device__ __forceinline__ void prefix_position(const LitArgs& a, const DevTable
         if (end == kLfOpen || (steps > 64 && atomicAdd(&p.ctr[C_WORK], (unsigned long long)steps) > a.len))
           atomicOr(&p.ctr[C_GATE], 1ull);
         else if (end != kLfNone)
-          emit_k(p, r, s, end);
+          sink(r, s, end);
       }
     }
     __syncwarp();
@@ -907,10 +913,30 @@ __device__ __forceinline__ void prefix_position(const LitArgs& a, const DevTable
 // (more than one survivor per 64 bytes) gives the prefix candidates up, like
 // long walks do; the last block then drops the candidates found so far, so that
 // the gated groups start from none.
+constexpr uint32_t kVerifyBuf = 512;
+
 template <bool RX>
 __global__ void __launch_bounds__(256) literal_verify_kernel(const __grid_constant__ LitArgs a,
                                                              const __grid_constant__ DevTables t,
                                                              const __grid_constant__ ScanPtrs p, PrefixDev pf) {
+  // Matches and candidates collect in shared memory: one atomic per block and
+  // counter instead of one per match (65,536 on one address took 35 us).
+  __shared__ uint3 mbuf[kVerifyBuf];
+  __shared__ uint3 kbuf[RX ? kVerifyBuf : 1];
+  __shared__ uint32_t held[2];
+  __shared__ unsigned long long first[2];
+  if (threadIdx.x < 2) held[threadIdx.x] = 0;
+  __syncthreads();
+  auto match = [&](uint32_t pid, uint32_t s, uint32_t e) {
+    const uint32_t i = atomicAdd(&held[0], 1u);
+    if (i < kVerifyBuf) mbuf[i] = make_uint3(pid, s, e);
+    else report_match(a, pid, s, e);
+  };
+  auto candidate = [&](uint32_t r, uint32_t s, uint32_t e) {
+    const uint32_t i = atomicAdd(&held[1], 1u);
+    if (i < kVerifyBuf) kbuf[RX ? i : 0] = make_uint3(r, s, e);
+    else emit_k(p, r, s, e, kEndKnown);
+  };
   unsigned long long n = *a.survivor_count;
   const bool full = n > a.survivor_cap;
   if (full) n = a.survivor_cap;
@@ -919,15 +945,30 @@ __global__ void __launch_bounds__(256) literal_verify_kernel(const __grid_consta
   // for one another.
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const uint32_t w = blockIdx.x + gridDim.x * (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  for (unsigned long long k0 = w; k0 < n; k0 += 32ull * warps) {  // warp-uniform: lane 0 has the first one
-    const unsigned long long k = k0 + (unsigned long long)lane * warps;
+  for (unsigned long long k0 = 0; k0 < n; k0 += 32ull * warps) {  // the same for all threads
+    const unsigned long long k = k0 + (unsigned long long)lane * warps + w;
     const uint32_t s = k < n ? a.survivors[k] : kNoSurvivor;
     // (kNoSurvivor: a slot the gram kernel reserved but did not fill; stage 1.5
     // for the gram kernel's survivors, unless the prefix table alone decides)
     bool in = s != kNoSurvivor;
     if (in && a.verify_bloom && (!RX || a.parts)) in = prefix_bloom(a, s);
-    if (in && (!RX || a.parts)) verify_position(a, s);
-    if (RX && !full) prefix_position(a, t, p, pf, s, in);
+    if (in && (!RX || a.parts)) verify_position(a, s, match);
+    if (RX && !full) prefix_position(a, t, p, pf, s, in, candidate);
+    __syncthreads();
+    const uint32_t nm = min(held[0], kVerifyBuf), nk = min(held[1], kVerifyBuf);
+    const bool done = k0 + 32ull * warps >= n;
+    if ((nm | nk) && (done || nm > kVerifyBuf - 256 || nk > kVerifyBuf - 256)) {
+      if (threadIdx.x == 0 && nm) first[0] = atomicAdd(a.counter, (unsigned long long)nm);
+      if (RX && threadIdx.x == 32 && nk) first[1] = atomicAdd(&p.ctr[C_K], (unsigned long long)nk);
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < nm; i += blockDim.x)
+        if (first[0] + i < a.cap) a.out[first[0] + i] = ws_match{mbuf[i].x, mbuf[i].y, mbuf[i].z};
+      for (uint32_t i = threadIdx.x; RX && i < nk; i += blockDim.x)
+        store_k(p, first[1] + i, kbuf[i].x, kbuf[i].y, kbuf[i].z, kEndKnown);
+      __syncthreads();
+      if (threadIdx.x < 2) held[threadIdx.x] = 0;
+      __syncthreads();
+    }
   }
   if (RX) {
     __shared__ bool last;
@@ -1062,10 +1103,11 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   } else {
     sh ? run(literal_filter_kernel<1, 4, true, true>) : run(literal_filter_kernel<1, 4, true, false>);
   }
-  // the verify pass is a chain of dependent loads per survivor: the gram
-  // kernel's longer survivor list (stage 1.5 runs here) gets more threads, a
-  // short list no more blocks than it can fill
-  const uint64_t vgrid = std::min<uint64_t>((uint64_t)sm_count * (a.verify_bloom ? 16 : 4), (l.survivor_cap + 255) / 256);
+  // the verify pass is a chain of dependent loads per survivor: as many threads
+  // as are resident at once (six blocks per SM; with 16 a second wave doubled
+  // the latency: 160 regexes over 1 GiB 367 -> 351 us a scan), and for a short
+  // list no more blocks than it can fill
+  const uint64_t vgrid = std::min<uint64_t>((uint64_t)sm_count * (a.verify_bloom ? 6 : 4), (l.survivor_cap + 255) / 256);
   if (l.rx) {
     const PrefixDev pf{plan.d_prefix_range.as<uint32_t>(), plan.d_prefix_entry.as<uint4>(), plan.prefix_shift,
                        plan.prefix_mul};

@@ -19,8 +19,13 @@ constexpr uint64_t kLfCap = 1024;
 constexpr uint32_t kLfNone = 0xFFFFFFFFu;  // no match from this start (or a duplicate start)
 constexpr uint32_t kLfLong = 0xFFFFFFFEu;  // cut off after a match
 constexpr uint32_t kLfOpen = 0xFFFFFFFDu;  // cut off before any match
+constexpr uint32_t kLfTodo = 0xFFFFFFFCu;  // (in a sorted candidate) the walk is still to be done
 
-struct KCand { uint32_t r, s, e; };
+// A candidate: regex, start, end of a match from there, and its rank among the
+// regex's candidates, with kEndKnown when the end is the leftmost-first one (or
+// kLfLong).
+struct KCand { uint32_t r, s, e, rank; };
+constexpr uint32_t kEndKnown = 0x80000000u;
 struct Event { uint32_t e, state, q, tag; };
 
 // counters block (unsigned long long[16]):
@@ -73,9 +78,8 @@ struct ScanPtrs {
   uint32_t* ckpt;
   uint32_t* count;
   uint32_t* offs;
-  uint32_t* cursor;
-  uint32_t* starts;
-  uint32_t* lfend;
+  unsigned long long* pair;     // candidates by regex: start << 32 | leftmost-first end
+  unsigned long long* pair2;    // the same size, for merging
   unsigned long long* rmark;    // visited reverse-walk triples, or null (state numbers too large, or full K)
   uint32_t full_k;              // report every (start, end) of K, not only distinct starts (diagnostics)
   uint32_t count_guesses;       // profiled speculative scans: the speculative groups whose guesses are counted
@@ -98,16 +102,16 @@ __device__ __forceinline__ unsigned long long warp_append(unsigned long long* co
   return base + g.thread_rank();
 }
 
-// Appends a candidate and counts it for its regex (the per-regex counts size
-// the resolution's start lists).
-__device__ __forceinline__ void emit_k(const ScanPtrs& p, uint32_t r, uint32_t s, uint32_t e) {
-  unsigned long long i = warp_append(&p.ctr[C_K]);
-  if (i < p.k_cap) {
-    p.k[i] = KCand{r, s, e};
-    atomicAdd(&p.count[r], 1u);
-  } else {
-    atomicOr(&p.ctr[C_ERR], 1ull);
-  }
+// Stores candidate i of K and counts it for its regex (the per-regex counts
+// size the resolution's lists, the rank is its place in one).
+__device__ __forceinline__ void store_k(const ScanPtrs& p, unsigned long long i, uint32_t r, uint32_t s, uint32_t e,
+                                        uint32_t known) {
+  if (i < p.k_cap) p.k[i] = KCand{r, s, e, atomicAdd(&p.count[r], 1u) | known};
+  else atomicOr(&p.ctr[C_ERR], 1ull);
+}
+
+__device__ __forceinline__ void emit_k(const ScanPtrs& p, uint32_t r, uint32_t s, uint32_t e, uint32_t known = 0) {
+  store_k(p, warp_append(&p.ctr[C_K]), r, s, e, known);
 }
 
 // Context of a byte for the assertions (byte_context in ws_regex.h).
