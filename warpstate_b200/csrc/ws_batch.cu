@@ -322,14 +322,16 @@ extern "C" ws_status ws_scan_batch(ws_matcher* m, const ws_item* items, uint64_t
                                                                     reinterpret_cast<const uint64_t*>(aux + ids_off),
                                                                     (uint32_t)ni, d_tag);
           check_cuda(cudaGetLastError(), "tag_kernel");
+          enqueue_results(*s, d_tag, d_counter, dcap, s->stream);
           if (attempt == 0 && gi + 1 < groups.size()) gather(gi + 1);
-          check_cuda(cudaMemcpyAsync(&count, d_counter, sizeof(count), cudaMemcpyDeviceToHost, s->stream),
-                     "D2H count");
           check_cuda(cudaStreamSynchronize(s->stream), "batch scan");
+          count = result_count(*s);
           if (!repeat_scan(m, count, attempt)) break;  // else the regex candidates overflowed: scan again
         }
         if (count > dcap) raise(WS_ERR_OVERFLOW, "too many matches in one batch launch", 0, count, dcap);
-        if (total + count <= cap && count) {
+        if (total + count <= cap && count <= kSmallTagged) {
+          std::memcpy(out + total, result_rows<ws_tagged_match>(*s), count * sizeof(ws_tagged_match));
+        } else if (total + count <= cap) {
           const ws_tagged_match* res = d_tag;
           if (count > 1 && count <= kMaxDeviceSorted) {  // this group's matches in their final order
             ensure(s->sorted, count * sizeof(ws_tagged_match));

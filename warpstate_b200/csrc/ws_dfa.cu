@@ -1852,7 +1852,7 @@ void regex_begin(RegexPlan& P, const RegexLaunch& l, cudaStream_t st, DeviceBuff
   if (profiled && l.mode != WS_REGEX_PLAIN) rs.p.count_guesses = rs.t.n_walk;
   if (l.mode != WS_REGEX_PLAIN && P.n_spec) clear_marks(P, rs.p, rs.t, st);
   // the counters and the per-regex counts after them
-  check_cuda(cudaMemsetAsync(rs.p.ctr, 0, L.off_count - L.off_ctr + (size_t)P.n_regex * 4, st), "memset");
+  rs.clear_words = (uint32_t)((L.off_count - L.off_ctr) / 4 + P.n_regex);
 }
 
 uint32_t regex_finish(RegexPlan& P, RegexScan& rs, const RegexLaunch& l, cudaStream_t st, int sm_count,
@@ -1902,6 +1902,7 @@ uint32_t run_regex_scan(RegexPlan& P, const RegexLaunch& l, cudaStream_t st, Dev
   if (!P.n_regex || l.len == 0) return 0;
   RegexScan rs;
   regex_begin(P, l, st, scratch, sm_count, ev != nullptr, false, rs);
+  check_cuda(cudaMemsetAsync(rs.p.ctr, 0, (size_t)rs.clear_words * 4, st), "memset");
   return regex_finish(P, rs, l, st, sm_count, ev);
 }
 

@@ -190,7 +190,8 @@ void regex_fill_info(const RegexPlan& plan, ws_matcher_info& info);
 bool regex_all_exact(const RegexPlan& plan, uint64_t chunk);
 // The regex pipeline in two parts, with the literal scan between them when it
 // looks for the covered regexes' prefixes (`prefixes`): regex_begin prepares
-// the scratch and clears the counters, regex_finish runs the walks of the
+// the scratch (the caller clears rs.clear_words from the counters on before
+// anything else runs), regex_finish runs the walks of the
 // groups that need them and the resolution.
 struct RegexScan;  // ws_scan.h
 void regex_begin(RegexPlan& plan, const RegexLaunch& l, cudaStream_t st, DeviceBuffer& scratch, int sm_count,

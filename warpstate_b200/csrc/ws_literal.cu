@@ -1043,7 +1043,7 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   a.phase = plan.d_phase.as<uint8_t>();
   a.phase_shift = 32 - plan.phase_bits;
   a.fold = plan.fold ? 1 : 0;
-  check_cuda(cudaMemsetAsync(a.survivor_count, 0, 8, st), "memset survivors");
+  if (!l.cleared) check_cuda(cudaMemsetAsync(a.survivor_count, 0, 8, st), "memset survivors");
   if (l.len > 0xFFFFFFFFull) raise(WS_ERR_INPUT_TOO_LARGE, "literal scan launch beyond 32-bit offsets", 0, l.len,
                                    0xFFFFFFFFull);
   const size_t smem = literal_smem_bytes(plan);

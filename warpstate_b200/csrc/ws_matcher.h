@@ -73,7 +73,12 @@ struct Scratch {
   size_t pinned_bytes = 0;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // [0], [1]: window copies; [2], [3]: staging slots drained
   bool pin_busy[2] = {false, false};                         // a DMA may still read the slot
+  int pin_turn = 0;                                          // slot of the next small copy
   cudaEvent_t busy = nullptr;  // recorded after the last use
+  uint8_t* result = nullptr;   // host-mapped count and rows of a small result (enqueue_results)
+  // A stream's windows and regex cursors (a stream holds its scratch from
+  // begin to destroy); windows above kKeepWindow are freed when it ends.
+  DeviceBuffer win[2], cursor, cursor_bak;
   cudaStream_t copy = nullptr;  // host-to-device copies overlapped with scans (created on first use)
   BatchGraph batch_graph;       // the last device batch scan's launch sequence
   ~Scratch() {
@@ -81,6 +86,7 @@ struct Scratch {
     if (copy) cudaStreamDestroy(copy);
     if (stream) cudaStreamDestroy(stream);
     if (pinned) cudaFreeHost(pinned);
+    if (result) cudaFreeHost(result);
     for (auto e : ev) if (e) cudaEventDestroy(e);
   }
 };
@@ -111,6 +117,21 @@ void sort_matches(ws_match* p, uint64_t n);
 // Device ordering of results (ws_sort.cu), for counts up to kMaxDeviceSorted;
 // larger counts are ordered on the host.  Input and output must not alias.
 constexpr uint64_t kMaxDeviceSorted = 0x7FFFFFFFull;
+// Small results: enqueued behind a scan, the kernel writes the true count and,
+// up to kSmallResults matches (kSmallTagged tagged ones), the rows in their
+// final order into the scratch's host-mapped result, valid once the stream has
+// been waited for.
+constexpr uint32_t kSmallResults = 2048, kSmallTagged = 1024;
+// `cap`: rows that d_res holds.
+void enqueue_results(Scratch& s, const ws_match* d_res, const unsigned long long* d_count, uint64_t cap,
+                     cudaStream_t st);
+void enqueue_results(Scratch& s, const ws_tagged_match* d_res, const unsigned long long* d_count, uint64_t cap,
+                     cudaStream_t st);
+inline unsigned long long result_count(const Scratch& s) {
+  return *reinterpret_cast<const volatile unsigned long long*>(s.result);
+}
+template <class R> const R* result_rows(const Scratch& s) { return reinterpret_cast<const R*>(s.result + 64); }
+constexpr size_t kKeepWindow = 64ull << 20;
 // By (start, pattern_id, end).
 void sort_matches_device(Scratch& s, const ws_match* d_in, ws_match* d_out, uint64_t n, cudaStream_t st);
 // By (source_id, start, pattern_id, end).

@@ -182,6 +182,7 @@ struct RegexScan {
   ScanPtrs p;
   DevTables t;
   uint64_t k_cap = 0, n_q = 0;
+  uint32_t clear_words = 0;  // u32 words from p.ctr on that start as zero
   bool prefixes = false;  // the literal scan finds the covered groups' candidates
 };
 

@@ -28,15 +28,15 @@ using namespace ws;
 
 struct ws_stream {
   ws_matcher* m = nullptr;
+  // holds the ping-pong windows (win), the per-regex find_iter positions
+  // (cursor, u64) and those before the window scan in flight (cursor_bak,
+  // restored to repeat it)
   std::unique_ptr<Scratch> s;
-  DeviceBuffer win[2];      // ping-pong windows
   int cur = 0;
   uint64_t win_base = 0;    // stream offset of the window's first byte
   uint64_t win_len = 0;
   uint64_t seen = 0;        // bytes fed so far
   uint64_t frontier = 0;    // regex starts below it are decided
-  DeviceBuffer cursor;      // per-regex find_iter position (u64)
-  DeviceBuffer cursor_bak;  // the cursors before the window scan in flight (restored to repeat it)
   std::vector<ws_match64> pending;  // decided, not yet delivered
   size_t delivered = 0;
   std::vector<ws_match> host;       // per-step readback
@@ -44,7 +44,10 @@ struct ws_stream {
   bool failed = false;
   bool ended = false;
   ~ws_stream() {
-    if (s && m) m->give(std::move(s));
+    if (!s || !m) return;
+    for (auto& w : s->win)
+      if (w.bytes > kKeepWindow) w = DeviceBuffer();
+    m->give(std::move(s));
   }
 };
 
@@ -66,16 +69,15 @@ bool enqueue_window(ws_stream* st, bool literals, uint64_t lit_min_end, uint64_t
   ScanExtras x;
   x.literals = literals;
   x.lit_min_end = lit_min_end;
-  x.cursor = m->rx.n_regex ? st->cursor.as<unsigned long long>() : nullptr;
+  x.cursor = m->rx.n_regex ? st->s->cursor.as<unsigned long long>() : nullptr;
   x.base = st->win_base;
   x.frontier = frontier;
   if (!literals && !m->rx.n_regex) return false;
   if (m->rx.n_regex)
-    check_cuda(cudaMemcpyAsync(st->cursor_bak.ptr, st->cursor.ptr, (size_t)m->rx.n_regex * 8,
+    check_cuda(cudaMemcpyAsync(st->s->cursor_bak.ptr, st->s->cursor.ptr, (size_t)m->rx.n_regex * 8,
                                cudaMemcpyDeviceToDevice, s.stream), "D2D cursor");
-  enqueue_scan(m, s, s.stream, st->win[st->cur].as<uint8_t>(), st->win_len, s.out.as<ws_match>(), dcap, d_counter, x);
-  check_cuda(cudaMemcpyAsync(&st->count, d_counter, sizeof(st->count), cudaMemcpyDeviceToHost, s.stream),
-             "D2H count");
+  enqueue_scan(m, s, s.stream, st->s->win[st->cur].as<uint8_t>(), st->win_len, s.out.as<ws_match>(), dcap, d_counter, x);
+  enqueue_results(s, s.out.as<ws_match>(), d_counter, dcap, s.stream);
   return true;
 }
 
@@ -86,8 +88,9 @@ bool window_done(ws_stream* st, int attempt) {
   ws_matcher* m = st->m;
   Scratch& s = *st->s;
   check_cuda(cudaStreamSynchronize(s.stream), "stream scan");
+  st->count = result_count(s);
   if (!repeat_scan(m, st->count, attempt)) return true;
-  check_cuda(cudaMemcpyAsync(st->cursor.ptr, st->cursor_bak.ptr, (size_t)m->rx.n_regex * 8,
+  check_cuda(cudaMemcpyAsync(st->s->cursor.ptr, st->s->cursor_bak.ptr, (size_t)m->rx.n_regex * 8,
                              cudaMemcpyDeviceToDevice, s.stream), "D2D cursor");
   return false;
 }
@@ -100,9 +103,14 @@ void finish_window(ws_stream* st) {
   const unsigned long long count = st->count;
   if (count > dcap) raise(WS_ERR_OVERFLOW, "too many matches in one stream piece", 0, count, dcap);
   if (count) {
-    st->host.resize(count);
-    read_sorted(s, s.out.as<ws_match>(), count, st->host.data());
-    for (const ws_match& mm : st->host) {
+    const ws_match* rows = result_rows<ws_match>(s);
+    if (count > kSmallResults) {
+      st->host.resize(count);
+      read_sorted(s, s.out.as<ws_match>(), count, st->host.data());
+      rows = st->host.data();
+    }
+    for (unsigned long long k = 0; k < count; ++k) {
+      const ws_match& mm = rows[k];
       ws_match64 o;
       o.pattern_id = mm.pattern_id;
       o.reserved = 0;
@@ -164,10 +172,10 @@ StepPlan copy_step(ws_stream* st, const uint8_t* data, uint64_t len, cudaStream_
   const uint64_t old_seen = st->seen;
   const StepPlan plan = plan_step(m, st->win_base, old_seen, old_seen + len, st->frontier, false);
   const uint64_t carry = old_seen - plan.keep;
-  DeviceBuffer& dst = st->win[st->cur ^ 1];
+  DeviceBuffer& dst = st->s->win[st->cur ^ 1];
   ensure(dst, carry + len + 64);
   if (carry)
-    check_cuda(cudaMemcpyAsync(dst.ptr, st->win[st->cur].as<uint8_t>() + (plan.keep - st->win_base), carry,
+    check_cuda(cudaMemcpyAsync(dst.ptr, st->s->win[st->cur].as<uint8_t>() + (plan.keep - st->win_base), carry,
                                cudaMemcpyDeviceToDevice, cs), "D2D carry");
   if (cs == s.stream)
     stage_copy(s, dst.as<uint8_t>() + carry, data, len);
@@ -343,9 +351,9 @@ ws_status ws_stream_begin(ws_matcher* m, ws_stream** out, ws_error_info* err) {
     st->s = m->take();
     check_cuda(cudaStreamWaitEvent(st->s->stream, st->s->busy, 0), "wait");
     if (m->rx.n_regex) {
-      st->cursor.alloc((size_t)m->rx.n_regex * 8);
-      st->cursor_bak.alloc((size_t)m->rx.n_regex * 8);
-      check_cuda(cudaMemsetAsync(st->cursor.ptr, 0, (size_t)m->rx.n_regex * 8, st->s->stream), "memset cursor");
+      ensure(st->s->cursor, (size_t)m->rx.n_regex * 8);
+      ensure(st->s->cursor_bak, (size_t)m->rx.n_regex * 8);
+      check_cuda(cudaMemsetAsync(st->s->cursor.ptr, 0, (size_t)m->rx.n_regex * 8, st->s->stream), "memset cursor");
     }
     *out = st.release();
   });
