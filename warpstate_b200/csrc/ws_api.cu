@@ -14,6 +14,7 @@
 #include <chrono>
 #include <cstring>
 
+#include "ws_launch.h"
 #include "ws_matcher.h"
 #include "ws_proposer.h"
 #include "ws_scan.h"
@@ -127,6 +128,7 @@ namespace {
 // regex counters (three memsets were 3 us more on the device).
 __global__ void clear_counters_kernel(unsigned long long* count, unsigned long long* survivors,
                                       unsigned long long* rx, uint32_t rx_words) {
+  pdl_trigger();
   uint32_t* w = reinterpret_cast<uint32_t*>(rx);
   for (uint32_t k = threadIdx.x; k < rx_words; k += blockDim.x) w[k] = 0;
   if (threadIdx.x == 0) *count = 0;

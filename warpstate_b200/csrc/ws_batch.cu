@@ -23,6 +23,7 @@
 #include <cstring>
 #include <numeric>
 
+#include "ws_launch.h"
 #include "ws_matcher.h"
 
 using namespace ws;
@@ -33,6 +34,7 @@ namespace {
 // item-relative offsets.
 __global__ void tag_kernel(const ws_match* in, const unsigned long long* count, uint64_t cap, const uint32_t* ends,
                            const uint64_t* ids, uint32_t n_items, ws_tagged_match* out) {
+  pdl_begin();
   unsigned long long n = *count;
   if (n > cap) n = cap;
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
@@ -135,9 +137,8 @@ extern "C" ws_status ws_scan_batch_device(ws_matcher* m, const uint8_t* d_data, 
       x.item_end = d_item_end;
       x.n_items = (uint32_t)n_items;
       const uint32_t n = enqueue_scan(m, *s, st, d_data, len, s->out.as<ws_match>(), dcap, d_counter, x);
-      tag_kernel<<<m->ctx->sm_count * 4, 256, 0, st>>>(s->out.as<ws_match>(), d_counter, std::min(dcap, cap),
-                                                        d_item_end, d_ids, (uint32_t)n_items, d_out);
-      check_cuda(cudaGetLastError(), "tag_kernel");
+      launch_pdl(tag_kernel, m->ctx->sm_count * 4, 256, 0, st, s->out.as<ws_match>(), d_counter, std::min(dcap, cap),
+                 d_item_end, d_ids, (uint32_t)n_items, d_out);
       return n + 1;
     };
     // The launch sequence of a call is replayed from a CUDA graph when the
@@ -317,11 +318,9 @@ extern "C" ws_status ws_scan_batch(ws_matcher* m, const ws_item* items, uint64_t
         for (int attempt = 0;; ++attempt) {
           enqueue_scan(m, *s, s->stream, inbuf[gi & 1]->as<uint8_t>(), G.bytes, s->out.as<ws_match>(), dcap,
                        d_counter, x);
-          tag_kernel<<<m->ctx->sm_count * 4, 256, 0, s->stream>>>(s->out.as<ws_match>(), d_counter, dcap,
-                                                                    reinterpret_cast<const uint32_t*>(aux + ends_off),
-                                                                    reinterpret_cast<const uint64_t*>(aux + ids_off),
-                                                                    (uint32_t)ni, d_tag);
-          check_cuda(cudaGetLastError(), "tag_kernel");
+          launch_pdl(tag_kernel, m->ctx->sm_count * 4, 256, 0, s->stream, s->out.as<ws_match>(), d_counter, dcap,
+                     reinterpret_cast<const uint32_t*>(aux + ends_off), reinterpret_cast<const uint64_t*>(aux + ids_off),
+                     (uint32_t)ni, d_tag);
           enqueue_results(*s, d_tag, d_counter, dcap, s->stream);
           if (attempt == 0 && gi + 1 < groups.size()) gather(gi + 1);
           check_cuda(cudaStreamSynchronize(s->stream), "batch scan");

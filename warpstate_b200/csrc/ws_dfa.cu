@@ -12,6 +12,7 @@
 
 #include "ws_dfa.h"
 #include "ws_async.h"
+#include "ws_launch.h"
 #include "ws_proposer.h"
 #include "ws_scan.h"
 
@@ -307,6 +308,7 @@ __device__ __forceinline__ uint32_t step_l2(uint32_t st, uint32_t b, const uint8
 // group DFA, reporting every match instead of stopping at the first).
 // blockIdx.y = group; the group's hottest anchored rows sit in shared memory.
 __global__ void __launch_bounds__(kWalkThreads, 1) dfa_plain_kernel(DevTables t, ScanPtrs p) {
+  pdl_begin();
   extern __shared__ __align__(16) uint32_t smem[];
   const uint32_t g = blockIdx.y;
   const GroupDev gd = t.groups[g];
@@ -361,6 +363,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) dfa_plain_kernel(DevTables t,
 // tables are read through L1/L2: these groups hold the patterns with
 // assertions, whose anchored walks mostly die within a few bytes.
 __global__ void __launch_bounds__(256) dfa_context_kernel(DevTables t, ScanPtrs p) {
+  pdl_begin();
   __shared__ uint8_t cls_s[256];
   const uint32_t g = t.n_spec + blockIdx.y;
   if (g >= t.n_ctx_walk && p.ctr[C_GATE] == 0) return;
@@ -426,6 +429,7 @@ __host__ __device__ __forceinline__ bool warm_exact(const GroupDev& gd, uint64_t
 template <bool kCls>
 __global__ void __launch_bounds__(kWalkThreads, 1)
     dfa_walk_kernel(DevTables t, ScanPtrs p, const __grid_constant__ CUtensorMap rows, uint64_t n_full) {
+  pdl_begin();
   extern __shared__ __align__(128) uint32_t smem[];
   // blockIdx.x = group (fastest), so the groups' blocks over the same chunks
   // run together and the input is read from HBM once, then from L2
@@ -688,6 +692,7 @@ __device__ void fix_chunk_img(const DevTables& t, const ScanPtrs& p, const Group
 // differs from its predecessor's end.
 template <bool kCls>
 __global__ void __launch_bounds__(kWalkThreads, 1) dfa_fixup_kernel(DevTables t, ScanPtrs p, int round) {
+  pdl_begin();
   if (round > 0 && p.ctr[C_ROUND + round - 1] == 0) return;  // nothing changed last round
   extern __shared__ __align__(16) uint32_t smem[];
   const uint32_t g = blockIdx.x;
@@ -712,6 +717,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) dfa_fixup_kernel(DevTables t,
 // Final sweep, one thread per group, in chunk order: exact whatever happened
 // in the parallel rounds (runs only if the last round still changed something).
 __global__ void dfa_fixup_serial_kernel(DevTables t, ScanPtrs p) {
+  pdl_begin();
   if (p.ctr[C_ROUND + kFixRounds - 1] == 0) return;
   const uint32_t g = blockIdx.x;
   if (g >= t.n_walk && p.ctr[C_GATE] == 0) return;
@@ -749,6 +755,7 @@ __device__ void count_guess_hits(const DevTables& t, const ScanPtrs& p) {
 // Valid match events -> reverse walk -> K candidates (and, in profiled
 // speculative scans, the guess count).
 __global__ void __launch_bounds__(256) dfa_reverse_kernel(DevTables t, ScanPtrs p) {
+  pdl_begin();
   if (p.count_guesses && p.n_chunks > 1) count_guess_hits(t, p);
   unsigned long long n = p.ctr[C_EV];
   if (n > p.ev_cap) n = p.ev_cap;
@@ -832,7 +839,10 @@ __device__ void scan_counts(const ScanPtrs& p, uint32_t n_regex, uint32_t* offs)
   }
 }
 
-__global__ void k_scan_kernel(ScanPtrs p, uint32_t n_regex) { scan_counts(p, n_regex, p.offs); }
+__global__ void k_scan_kernel(ScanPtrs p, uint32_t n_regex) {
+  pdl_begin();
+  scan_counts(p, n_regex, p.offs);
+}
 
 // The regexes' candidate offsets are staged in shared memory when they fit.
 constexpr uint32_t kOffsShared = 8192;
@@ -843,6 +853,7 @@ constexpr uint32_t kOffsShared = 8192;
 // also for the later kernels; sets of kOffsShared regexes and more have them
 // scanned before.
 __global__ void __launch_bounds__(256) k_scatter_kernel(ScanPtrs p, uint32_t n_regex) {
+  pdl_begin();
   extern __shared__ uint32_t offs_s[];
   const unsigned long long n = min(p.ctr[C_K], (unsigned long long)p.k_cap);
   const bool staged = n_regex < kOffsShared;
@@ -935,6 +946,7 @@ __device__ void sort_list(unsigned long long* buf, unsigned long long* list, uns
 }
 
 __global__ void __launch_bounds__(512) k_sort_kernel(ScanPtrs p, uint32_t n_regex) {
+  pdl_begin();
   __shared__ unsigned long long buf[kSortTile];
   for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
     const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
@@ -955,6 +967,7 @@ __device__ __forceinline__ uint32_t list_end(const DevTables& t, const ScanPtrs&
 // The ends that are not known yet, in parallel over all candidates.  A
 // candidate's regex comes from a binary search over the offsets.
 __global__ void k_lf_kernel(DevTables t, ScanPtrs p, uint32_t n_regex) {
+  pdl_begin();
   extern __shared__ uint32_t offs_s[];
   const bool staged = n_regex < kOffsShared;
   if (staged) {
@@ -1067,6 +1080,7 @@ __device__ void chain_list(const DevTables& t, const ScanPtrs& p, uint32_t r, co
 
 // A warp per regex.
 __global__ void k_chain_kernel(DevTables t, ScanPtrs p, unsigned long long* need) {
+  pdl_begin();
   if (finalize(p, need)) return;
   const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (r >= t.n_regex) return;  // whole warps exit together
@@ -1079,6 +1093,7 @@ __global__ void k_chain_kernel(DevTables t, ScanPtrs p, unsigned long long* need
 // each took 8 us more on small lists).
 __global__ void __launch_bounds__(256) k_resolve_kernel(DevTables t, ScanPtrs p, uint32_t n_regex,
                                                         unsigned long long* need) {
+  pdl_begin();
   __shared__ unsigned long long buf[kSortTile];
   if (finalize(p, need)) return;
   for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
@@ -1111,6 +1126,7 @@ __global__ void k_export_kernel(DevTables t, ScanPtrs p, ws_match* out, uint64_t
 // Counts the chunk boundaries whose guess (the proposer's, or the unanchored
 // start) was the true state: the predecessor's end state after the fix-up.
 __global__ void fill_guess_kernel(DevTables t, ScanPtrs p) {
+  pdl_begin();
   const uint32_t g = blockIdx.y;
   const uint32_t st = t.groups[g].start_unanchored;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.n_chunks; i += (uint64_t)gridDim.x * blockDim.x)
@@ -1201,7 +1217,7 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
     const uint64_t want = (p.len + 255) / 256;
     const uint64_t per_group = std::max<uint64_t>(1, (uint64_t)sm_count * 8 / nc);
     dim3 grid((unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, per_group)), nc);
-    dfa_context_kernel<<<grid, 256, 0, st>>>(t, p);
+    launch_pdl(dfa_context_kernel, grid, 256, 0, st, t, p);
     check_cuda(cudaGetLastError(), "dfa_context_kernel");
     launches++;
   };
@@ -1213,7 +1229,7 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
       uint64_t per_group = std::max<uint64_t>(1, (uint64_t)sm_count / P.n_spec);
       uint64_t want = (p.len + kWalkThreads - 1) / kWalkThreads;
       dim3 grid((unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, per_group * 2)), P.n_spec);
-      dfa_plain_kernel<<<grid, kWalkThreads, smem, st>>>(t, p);
+      launch_pdl(dfa_plain_kernel, grid, kWalkThreads, smem, st, t, p);
       check_cuda(cudaGetLastError(), "dfa_plain_kernel");
       launches++;
     }
@@ -1243,7 +1259,7 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
   if (guessed && P.proposer && P.use_proposer) {
     launches += proposer_predict(*P.proposer, p.data, p.len, p.chunk, p.n_chunks, p.guess, st);
   } else if (guessed) {
-    fill_guess_kernel<<<dim3(std::min<unsigned>((unsigned)((p.n_chunks + 255) / 256), 1024), P.n_spec), 256, 0, st>>>(t, p);
+    launch_pdl(fill_guess_kernel, dim3(std::min<unsigned>((unsigned)((p.n_chunks + 255) / 256), 1024), P.n_spec), 256, 0, st, t, p);
     check_cuda(cudaGetLastError(), "fill_guess_kernel");
     launches++;
   }
@@ -1255,10 +1271,10 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
   if (n_full) encode_chunk_rows(&rows, p.data, p.chunk, n_full);
   if (P.class_image) {
     set_smem(dfa_walk_kernel<true>, kWalkSmem, "smem(walk)");
-    dfa_walk_kernel<true><<<cgrid, kWalkThreads, kWalkSmem, st>>>(t, p, rows, n_full);
+    launch_pdl(dfa_walk_kernel<true>, cgrid, kWalkThreads, kWalkSmem, st, t, p, rows, n_full);
   } else {
     set_smem(dfa_walk_kernel<false>, kWalkSmem, "smem(walk)");
-    dfa_walk_kernel<false><<<cgrid, kWalkThreads, kWalkSmem, st>>>(t, p, rows, n_full);
+    launch_pdl(dfa_walk_kernel<false>, cgrid, kWalkThreads, kWalkSmem, st, t, p, rows, n_full);
   }
   check_cuda(cudaGetLastError(), "dfa_walk_kernel");
   launches++;
@@ -1272,16 +1288,16 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
     auto fixup = P.class_image ? dfa_fixup_kernel<true> : dfa_fixup_kernel<false>;
     set_smem(fixup, kFixSmem, "smem(fixup)");
     for (int r = 0; r < kFixRounds; ++r) {
-      fixup<<<fgrid, kWalkThreads, kFixSmem, st>>>(t, p, r);
+      launch_pdl(fixup, fgrid, kWalkThreads, kFixSmem, st, t, p, r);
       check_cuda(cudaGetLastError(), "dfa_fixup_kernel");
       launches++;
     }
-    dfa_fixup_serial_kernel<<<P.n_spec, 1, 0, st>>>(t, p);
+    launch_pdl(dfa_fixup_serial_kernel, P.n_spec, 1, 0, st, t, p);
     check_cuda(cudaGetLastError(), "dfa_fixup_serial_kernel");
     launches++;
   }
   mark(3);
-  dfa_reverse_kernel<<<sm_count * 8, 256, 0, st>>>(t, p);
+  launch_pdl(dfa_reverse_kernel, sm_count * 8, 256, 0, st, t, p);
   check_cuda(cudaGetLastError(), "dfa_reverse_kernel");
   launches++;
   context_groups();
@@ -1866,18 +1882,18 @@ uint32_t regex_finish(RegexPlan& P, RegexScan& rs, const RegexLaunch& l, cudaStr
   const size_t osmem = staged ? ((size_t)P.n_regex + 1) * 4 : 0;
   const int hg = (int)std::min<uint64_t>((uint64_t)sm_count * 4, (rs.k_cap + 255) / 256);
   if (!staged) {
-    k_scan_kernel<<<1, 1024, 0, st>>>(p, P.n_regex);
+    launch_pdl(k_scan_kernel, 1, 1024, 0, st, p, P.n_regex);
     launches += 1;
   }
-  k_scatter_kernel<<<hg, 256, osmem, st>>>(p, P.n_regex);
+  launch_pdl(k_scatter_kernel, hg, 256, osmem, st, p, P.n_regex);
   launches += 1;
   if (rs.prefixes && t.n_walk == 0 && t.n_ctx_walk == P.n_spec) {
-    k_resolve_kernel<<<(unsigned)std::min<uint32_t>(P.n_regex, 4096), 256, 0, st>>>(t, p, P.n_regex, l.need);
+    launch_pdl(k_resolve_kernel, (unsigned)std::min<uint32_t>(P.n_regex, 4096), 256, 0, st, t, p, P.n_regex, l.need);
     launches += 1;
   } else {
-    k_sort_kernel<<<(unsigned)std::min<uint32_t>(P.n_regex, 4096), 512, 0, st>>>(p, P.n_regex);
-    k_lf_kernel<<<sm_count * 8, 128, osmem, st>>>(t, p, P.n_regex);
-    k_chain_kernel<<<(P.n_regex + 3) / 4, 128, 0, st>>>(t, p, l.need);  // a warp per regex
+    launch_pdl(k_sort_kernel, (unsigned)std::min<uint32_t>(P.n_regex, 4096), 512, 0, st, p, P.n_regex);
+    launch_pdl(k_lf_kernel, sm_count * 8, 128, osmem, st, t, p, P.n_regex);
+    launch_pdl(k_chain_kernel, (P.n_regex + 3) / 4, 128, 0, st, t, p, l.need);  // a warp per regex
     launches += 3;
   }
   check_cuda(cudaGetLastError(), "resolution kernels");

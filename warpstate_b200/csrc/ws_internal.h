@@ -147,7 +147,8 @@ struct LiteralPlan {
   // lean2_mask), which passes 11% instead of 17% of the grams of a
   // 200,000-gram set.
   std::vector<uint8_t> lean_bits;
-  DeviceBuffer d_filter, d_bloom, d_short, d_info, d_bytes, d_meta, d_ranges, d_entries, d_bloom2, d_big,
+  std::vector<uint32_t> meta;         // LiteralPrefilterTable partitions: 4 words per prefix length
+  DeviceBuffer d_filter, d_bloom, d_short, d_info, d_bytes, d_ranges, d_entries, d_bloom2, d_big,
       d_lean_bits;
   uint32_t n_buckets = 0;
   // Regex prefixes: entries {first 4 bytes, next 4, their mask, regex} by

@@ -347,7 +347,9 @@ void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan, const std:
   plan.d_short.upload(plan.short_bits.data(), plan.short_bits.size() * 4);
   plan.d_info.upload(plan.lit_info.data(), plan.lit_info.size() * 4);
   plan.d_bytes.upload(plan.lit_bytes.data(), plan.lit_bytes.size());
-  plan.d_meta.upload(t.prefix_meta, 4 * (size_t)t.hash_window_len * 4);
+  plan.meta.assign(4 * HASH_WINDOW, 0u);
+  if (t.prefix_meta)
+    std::copy(t.prefix_meta, t.prefix_meta + 4 * std::min(t.hash_window_len, HASH_WINDOW), plan.meta.begin());
   plan.d_ranges.upload(t.bucket_ranges, 2 * (size_t)t.n_buckets * 4);
   plan.d_entries.upload(t.entries, 2 * (size_t)t.n_literals * 4);
 }

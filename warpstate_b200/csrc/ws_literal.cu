@@ -32,6 +32,7 @@
 
 
 #include "ws_internal.h"
+#include "ws_launch.h"
 #include "ws_scan.h"
 
 namespace ws {
@@ -57,10 +58,9 @@ struct LitArgs {
   const uint32_t* bloom;
   const uint4* info;
   const uint8_t* lit_bytes;
-  const uint4* meta;
+  uint2 meta[HASH_WINDOW];  // per prefix length: {first bucket, bucket mask} (LiteralPrefilterTable partition)
   const uint2* ranges;
   const uint2* entries;
-  uint32_t window;
   ws_match* out;
   uint64_t cap;
   unsigned long long* counter;
@@ -76,11 +76,11 @@ struct LitArgs {
   uint32_t parts16;          // stage-1.5b key lengths (bit i: i+1 bytes)
   const uint32_t* bloom2;    // stage-1.5b bitmap (2^kBloom2Bits bits, L2), or null
   const uint8_t* big;        // stage-1b gram table (2^kBigBits bytes, L2), or null (compacting kernel)
-  uint32_t verify_bloom;     // the verify kernel runs stage 1.5 first
   // gram kernel: stage 1 has 2^gram_word_bits words, the phase table
   // 2^(32 - phase_shift) bytes
   const uint32_t* gram_bloom;
   uint32_t gram_word_bits;
+  uint32_t gram_bits;        // bits per gram in it; 0: the compacting kernel ran
   const uint8_t* phase;
   uint32_t phase_shift;
   uint32_t slot_chunk;       // survivor slots a warp reserves at a time
@@ -124,58 +124,87 @@ __device__ __forceinline__ uint32_t input_word(const LitArgs& a, uint32_t len, u
   return a.fold ? ascii_fold4(w) : w;
 }
 
-// The reference's per-position probe and exact verify (stage 2).  Inputs of
-// one launch are below 4 GiB.  The hashed bytes come from two words read
-// once, and a candidate literal is compared a word at a time (literal bytes
-// start 4-aligned in a buffer padded to 16 bytes).
-template <class Sink>
-__device__ void verify_position(const LitArgs& a, uint64_t s64, Sink&& sink) {
-  if (s64 >= a.max_start) return;
-  const uint32_t s = (uint32_t)s64, len = (uint32_t)a.len;
-  const uint32_t w0 = s & ~3u, sh = (s & 3) * 8;
-  const uint32_t x0 = input_word(a, len, w0), x1 = input_word(a, len, w0 + 4), x2 = input_word(a, len, w0 + 8);
-  const uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
+// The reference's per-position probe and exact verify (stage 2), in two parts
+// so that a survivor's loads go out together: probe_literals hashes the
+// position's first eight bytes and reads the bucket of every prefix length that
+// has literals, verify_literals walks the buckets and compares.  Inputs of one
+// launch are below 4 GiB.
+struct Probe {
+  uint32_t h[8];
+  uint2 r[8];
+};
+
+__device__ __forceinline__ void probe_literals(const LitArgs& a, uint32_t lo, uint32_t hi, uint32_t rem, Probe& pr) {
   uint32_t h = 2166136261u;
-  const uint32_t rem = len - s;
-  const uint32_t maxp = rem < a.window ? rem : a.window;
-  for (uint32_t i = 0; i < maxp; ++i) {
+#pragma unroll
+  for (uint32_t i = 0; i < HASH_WINDOW; ++i) {
     h = (h ^ (((i < 4 ? lo : hi) >> (8 * (i & 3))) & 0xFFu)) * 16777619u;
-    if (!((a.parts >> i) & 1u)) continue;
-    uint4 m = __ldg(a.meta + i);
-    uint2 r = __ldg(a.ranges + m.x + (h & m.y));
-    for (uint32_t e = 0; e < r.y; ++e) {
-      uint2 ent = __ldg(a.entries + r.x + e);
-      if (ent.x != h) continue;
-      uint4 info = __ldg(a.info + ent.y);  // {offset, len, pattern id, 0}
-      if (info.y > rem) continue;
-      const uint32_t* lit = reinterpret_cast<const uint32_t*>(a.lit_bytes + info.x);
-      bool eq = true;
-      uint32_t cur = x0;
-      for (uint32_t k = 0; k < info.y; k += 4) {
-        const uint32_t nxt = input_word(a, len, w0 + k + 4);
-        const uint32_t dw = __funnelshift_r(cur, nxt, sh);
-        const uint32_t left = info.y - k;
-        const uint32_t m = left >= 4 ? 0xFFFFFFFFu : ((1u << (8 * left)) - 1u);
-        if ((__ldg(lit + (k >> 2)) ^ dw) & m) { eq = false; break; }
-        cur = nxt;
+    pr.h[i] = h;
+    pr.r[i] = ((a.parts >> i) & 1u) && i < rem ? __ldg(a.ranges + a.meta[i].x + (h & a.meta[i].y)) : make_uint2(0, 0);
+  }
+}
+
+// Compares literals of the probed buckets at s; x0 is the (folded) word at
+// s & ~3.  Literal bytes start 4-aligned in a buffer padded to 16 bytes; four
+// words of literal and input are read together.
+template <class Sink>
+__device__ __forceinline__ void verify_literals(const LitArgs& a, uint32_t s, uint32_t x0, const Probe& pr, Sink&& sink) {
+  const uint32_t len = (uint32_t)a.len, rem = len - s, w0 = s & ~3u, sh = (s & 3) * 8;
+  uint32_t part = 0, e = 0;  // the next entry: bucket `part`, place e
+  while (true) {
+    uint32_t found = 0xFFFFFFFFu;
+#pragma unroll
+    for (uint32_t i = 0; i < HASH_WINDOW; ++i) {
+      if (i < part || found != 0xFFFFFFFFu) continue;
+      for (; e < pr.r[i].y && found == 0xFFFFFFFFu; ++e) {
+        const uint2 ent = __ldg(a.entries + pr.r[i].x + e);
+        if (ent.x == pr.h[i]) found = ent.y;
       }
-      if (!eq) continue;
-      if (s + info.y <= a.min_end) continue;
-      if (a.n_items && s + info.y > item_end_of(a.item_end, a.n_items, (uint32_t)s)) continue;  // crosses items
-      sink(info.z, s, s + info.y);
+      part = i;
+      if (found == 0xFFFFFFFFu) e = 0;
     }
+    if (found == 0xFFFFFFFFu) return;
+    const uint4 info = __ldg(a.info + found);  // {offset, len, pattern id, 0}
+    if (info.y > rem) continue;
+    const uint32_t* lit = reinterpret_cast<const uint32_t*>(a.lit_bytes + info.x);
+    uint32_t differ = 0, cur = x0;
+    for (uint32_t k = 0; k < info.y && !differ; k += 16) {
+      uint32_t l[4], d[5];
+      d[0] = cur;
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j) {
+        const bool on = k + 4 * j < info.y;
+        l[j] = on ? __ldg(lit + (k >> 2) + j) : 0u;
+        d[j + 1] = on ? input_word(a, len, w0 + k + 4 * j + 4) : 0u;
+      }
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j) {
+        const uint32_t left = info.y > k + 4 * j ? info.y - k - 4 * j : 0u;
+        const uint32_t m = left >= 4 ? 0xFFFFFFFFu : ((1u << (8 * left)) - 1u);
+        differ |= (l[j] ^ __funnelshift_r(d[j], d[j + 1], sh)) & m;
+      }
+      cur = d[4];
+    }
+    if (differ || s + info.y <= a.min_end) continue;
+    if (a.n_items && s + info.y > item_end_of(a.item_end, a.n_items, s)) continue;  // crosses items
+    sink(info.z, s, s + info.y);
   }
 }
 
 // A match straight to the output.
 __device__ __forceinline__ void report_match(const LitArgs& a, uint32_t pid, uint32_t s, uint32_t e) {
-  const unsigned long long idx = atomicAdd(a.counter, 1ull);
+  const unsigned long long idx = warp_append(a.counter);
   if (idx < a.cap) a.out[idx] = ws_match{pid, s, e};
 }
 
-// Verifies a position in the filter kernel (the survivor list is full).
+// Verifies a position in the compacting kernel (the survivor list is full).
 __device__ __forceinline__ void verify_in_place(const LitArgs& a, uint32_t s) {
-  verify_position(a, s, [&](uint32_t pid, uint32_t at, uint32_t e) { report_match(a, pid, at, e); });
+  if (!a.parts || s >= a.max_start) return;
+  const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
+  const uint32_t x0 = input_word(a, len, w0), x1 = input_word(a, len, w0 + 4), x2 = input_word(a, len, w0 + 8);
+  Probe pr;
+  probe_literals(a, __funnelshift_r(x0, x1, sh), __funnelshift_r(x1, x2, sh), len - s, pr);
+  verify_literals(a, s, x0, pr, [&](uint32_t pid, uint32_t at, uint32_t e) { report_match(a, pid, at, e); });
 }
 
 // 16-bit mask of owned positions that may start a literal (stage 1).  w[0..3]
@@ -344,6 +373,7 @@ __device__ __forceinline__ void process_block(const LitArgs& a, uint32_t* blk, u
 // 32-bit.
 template <int P, int G, bool LONG, bool SHORT>
 __global__ void __launch_bounds__(kThreads, 1) literal_filter_kernel(LitArgs a) {
+  pdl_begin();
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* filt = smem;                                 // filter_words
   uint32_t* bloom = filt + a.filter_words;               // 2^kBloomBits / 32 words
@@ -495,6 +525,7 @@ constexpr int kBigWarps = kBigThreads / 32;
 // 16 warps per CTA leave room for the pipeline's registers.
 template <int G, bool SHORT>
 __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(LitArgs a) {
+  pdl_begin();
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* filt = smem;
   uint32_t* bloom = filt + a.filter_words;
@@ -639,21 +670,6 @@ __device__ __forceinline__ void lean_holes(const LitArgs& a, const LeanSlots& r,
   for (unsigned long long k = r.next + lane; k < r.end && k < a.survivor_cap; k += 32) a.survivors[k] = kNoSurvivor;
 }
 
-// Stage 1.5 of position s: its first min(len, 8) bytes against the Bloom bitmap
-// of the literals' prefixes.
-__device__ __forceinline__ bool prefix_bloom(const LitArgs& a, uint32_t s) {
-  const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
-  const uint32_t x0 = input_word(a, len, w0), x1 = input_word(a, len, w0 + 4), x2 = input_word(a, len, w0 + 8);
-  const uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
-  uint32_t keep = 0;
-#pragma unroll
-  for (uint32_t i = 0; i < 8; ++i) {  // the loads of all lengths together
-    const uint32_t key = prefix_key(lo, hi, i + 1);
-    if ((a.bloom_parts >> i) & 1u) keep |= __ldg(a.bloom + (key >> 5)) >> (key & 31);
-  }
-  return keep & 1u;
-}
-
 // Key of the phase table for the gram at position at: a hash independent of
 // stage 1's, so that what stage 1 lets through by chance does not pass again.
 template <int G>
@@ -703,9 +719,9 @@ __device__ __forceinline__ void gram_flush(const LitArgs& a, const uint32_t* que
     unsigned long long slot = r.next + incl - cnt;
     r.next += total;
     for (; bits; bits &= bits - 1) {
-      const uint32_t s = at - (P - 1) + (__ffs(bits) - 1);
-      if (slot < a.survivor_cap) a.survivors[slot] = s;
-      else if (prefix_bloom(a, s)) verify_in_place(a, s);  // list full
+      // (a full list: the count alone says so, and the verify kernel looks at
+      // every gram again; verifying here cost the loop its registers)
+      if (slot < a.survivor_cap) a.survivors[slot] = at - (P - 1) + (__ffs(bits) - 1);
       ++slot;
     }
   }
@@ -799,6 +815,9 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
     for (uint32_t k = threadIdx.x; k < (1u << a.gram_word_bits) / 4; k += kGramThreads) dst[k] = __ldg(src + k);
   }
   __syncthreads();
+  // (the tables above are no kernel's output; the verify kernel is not let in
+  // early, its waiting blocks cost the last runs 1%)
+  pdl_wait();
   const uint32_t filt = (uint32_t)__cvta_generic_to_shared(gsm), wsh = 32 - a.gram_word_bits;
   const uint32_t len = (uint32_t)a.len;
   const uint32_t nvec = (uint32_t)((a.len + 15) >> 4);
@@ -873,18 +892,9 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
 // candidates up: the regexes' groups are walked instead (ctr[C_GATE]), whose
 // cost does not depend on the input.
 template <class Sink>
-__device__ __forceinline__ void prefix_position(const LitArgs& a, const DevTables& t, const ScanPtrs& p,
-                                                const PrefixDev& pf, uint32_t s, bool in, Sink&& sink) {
-  uint32_t k = 0, k1 = 0, lo = 0, hi = 0;
-  if (in) {
-    const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
-    const uint32_t x0 = word_at(a.data, len, w0), x1 = word_at(a.data, len, w0 + 4), x2 = word_at(a.data, len, w0 + 8);
-    lo = __funnelshift_r(x0, x1, sh);
-    hi = __funnelshift_r(x1, x2, sh);
-    const uint32_t* rg = pf.range + ((lo * 0x9E3779B1u + hi * pf.mul) >> pf.shift);
-    k = __ldg(rg);
-    k1 = __ldg(rg + 1);
-  }
+__device__ __forceinline__ void verify_prefixes(const LitArgs& a, const DevTables& t, const ScanPtrs& p,
+                                                const PrefixDev& pf, uint32_t s, uint32_t lo, uint32_t hi, uint32_t k,
+                                                uint32_t k1, bool gate, Sink&& sink) {
   // every lane finds its next entry, then the lanes that have one walk together
   while (true) {
     uint32_t r = 0xFFFFFFFFu;
@@ -893,32 +903,58 @@ __device__ __forceinline__ void prefix_position(const LitArgs& a, const DevTable
       if (e.x == lo && !((e.y ^ hi) & e.z)) r = e.w;
     }
     if (__ballot_sync(0xFFFFFFFFu, r != 0xFFFFFFFFu) == 0) return;
-    if (r != 0xFFFFFFFFu) {
-      if (*(volatile unsigned long long*)&p.ctr[C_GATE]) {
-        k = k1;
-      } else {
-        uint32_t steps = 0;
-        const uint32_t end = lf_walk(t, p, r, s, kLfCap, &steps);
-        if (end == kLfOpen || (steps > 64 && atomicAdd(&p.ctr[C_WORK], (unsigned long long)steps) > a.len))
-          atomicOr(&p.ctr[C_GATE], 1ull);
-        else if (end != kLfNone)
-          sink(r, s, end);
+    if (r != 0xFFFFFFFFu && !gate) {
+      uint32_t steps = 0;
+      const uint32_t end = lf_walk(t, p, r, s, kLfCap, &steps);
+      if (end == kLfOpen || (steps > 64 && atomicAdd(&p.ctr[C_WORK], (unsigned long long)steps) > a.len)) {
+        atomicOr(&p.ctr[C_GATE], 1ull);
+        gate = true;
+      } else if (end != kLfNone) {
+        sink(r, s, end);
       }
     }
     __syncwarp();
   }
 }
 
-// RX: the survivors are also looked up among the regex prefixes.  A full list
-// (more than one survivor per 64 bytes) gives the prefix candidates up, like
-// long walks do; the last block then drops the candidates found so far, so that
-// the gated groups start from none.
+// The gram at `at` and, when it passes stage 1 and the phase table, the literals
+// that start at its phases: the gram kernel's test of one position, from global
+// memory (inputs whose survivors did not fit the list).
+template <class Sink>
+__device__ __noinline__ void verify_gram(const LitArgs& a, uint32_t at, Sink& sink) {
+  const uint32_t len = (uint32_t)a.len, w0 = at & ~3u, sh = (at & 3) * 8, wsh = 32 - a.gram_word_bits;
+  uint32_t g[4] = {0, 0, 0, 0};
+  g[0] = __funnelshift_r(input_word(a, len, w0), input_word(a, len, w0 + 4), sh);
+  if (a.gram_len == 16)  // (aligned)
+    for (uint32_t k = 1; k < 4; ++k) g[k] = input_word(a, len, w0 + 4 * k);
+  const uint32_t h = gram_hash32(g[0], g[1], g[2], g[3], (int)a.gram_len);
+  const uint32_t x = __ldg(a.gram_bloom + (h >> wsh));
+  if (!((x >> ((h >> (wsh - 5)) & 31u)) & 1u)) return;
+  if (a.gram_bits == 2 && !((x >> ((h >> (wsh - 10)) & 31u)) & 1u)) return;
+  uint32_t bits = __ldg(a.phase + (phase_key(g[0], g[1], g[2], g[3], (int)a.gram_len) >> a.phase_shift));
+  for (; bits; bits &= bits - 1) {
+    const uint32_t k = a.period - __ffs(bits);  // bit period - 1 - k: the literal starts k bytes before the gram
+    if (at < k || at - k >= len || at - k >= a.max_start) continue;
+    const uint32_t s = at - k, v0 = s & ~3u, vs = (s & 3) * 8;
+    const uint32_t x0 = input_word(a, len, v0), x1 = input_word(a, len, v0 + 4), x2 = input_word(a, len, v0 + 8);
+    Probe pr;
+    probe_literals(a, __funnelshift_r(x0, x1, vs), __funnelshift_r(x1, x2, vs), len - s, pr);
+    verify_literals(a, s, x0, pr, sink);
+  }
+}
+
+// Kernel 2.  When the gram kernel's list was full, every gram of the input is
+// tested again here and verified at once.  RX: the survivors are also looked up
+// among the regex prefixes.  A full list (more than one survivor per 64 bytes)
+// gives the prefix candidates up, like long walks do; the last block then drops
+// the candidates found so far, so that the gated groups start from none.
 constexpr uint32_t kVerifyBuf = 512;
 
 template <bool RX>
-__global__ void __launch_bounds__(256) literal_verify_kernel(const __grid_constant__ LitArgs a,
+__global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_constant__ LitArgs a,
                                                              const __grid_constant__ DevTables t,
                                                              const __grid_constant__ ScanPtrs p, PrefixDev pf) {
+  pdl_begin();
   // Matches and candidates collect in shared memory: one atomic per block and
   // counter instead of one per match (65,536 on one address took 35 us).
   __shared__ uint3 mbuf[kVerifyBuf];
@@ -940,23 +976,16 @@ __global__ void __launch_bounds__(256) literal_verify_kernel(const __grid_consta
   unsigned long long n = *a.survivor_count;
   const bool full = n > a.survivor_cap;
   if (full) n = a.survivor_cap;
+  // the gram kernel drops what does not fit (the compacting kernel verifies it)
+  const bool dense = full && a.gram_bits;
   // Neighbouring survivors go to different warps: a short list (the usual one)
   // then has a survivor per warp, whose chains of dependent loads do not wait
   // for one another.
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const uint32_t w = blockIdx.x + gridDim.x * (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  for (unsigned long long k0 = 0; k0 < n; k0 += 32ull * warps) {  // the same for all threads
-    const unsigned long long k = k0 + (unsigned long long)lane * warps + w;
-    const uint32_t s = k < n ? a.survivors[k] : kNoSurvivor;
-    // (kNoSurvivor: a slot the gram kernel reserved but did not fill; stage 1.5
-    // for the gram kernel's survivors, unless the prefix table alone decides)
-    bool in = s != kNoSurvivor;
-    if (in && a.verify_bloom && (!RX || a.parts)) in = prefix_bloom(a, s);
-    if (in && (!RX || a.parts)) verify_position(a, s, match);
-    if (RX && !full) prefix_position(a, t, p, pf, s, in, candidate);
+  auto flush = [&](bool done) {  // by all threads of the block
     __syncthreads();
     const uint32_t nm = min(held[0], kVerifyBuf), nk = min(held[1], kVerifyBuf);
-    const bool done = k0 + 32ull * warps >= n;
     if ((nm | nk) && (done || nm > kVerifyBuf - 256 || nk > kVerifyBuf - 256)) {
       if (threadIdx.x == 0 && nm) first[0] = atomicAdd(a.counter, (unsigned long long)nm);
       if (RX && threadIdx.x == 32 && nk) first[1] = atomicAdd(&p.ctr[C_K], (unsigned long long)nk);
@@ -968,6 +997,46 @@ __global__ void __launch_bounds__(256) literal_verify_kernel(const __grid_consta
       __syncthreads();
       if (threadIdx.x < 2) held[threadIdx.x] = 0;
       __syncthreads();
+    }
+  };
+  for (unsigned long long k0 = 0; k0 < n && !dense; k0 += 32ull * warps) {  // the same for all threads
+    const unsigned long long k = k0 + (unsigned long long)lane * warps + w;
+    const uint32_t s = k < n ? a.survivors[k] : kNoSurvivor;
+    const bool in = s != kNoSurvivor;  // (else a slot the gram kernel reserved but did not fill)
+    // the first words, then the buckets of the literals' table and of the
+    // prefixes', in flight together
+    const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
+    uint32_t x0 = 0, x1 = 0, x2 = 0;
+    if (in) {
+      x0 = word_at(a.data, len, w0);
+      x1 = word_at(a.data, len, w0 + 4);
+      x2 = word_at(a.data, len, w0 + 8);
+    }
+    const uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
+    const bool literals = in && a.parts && s < a.max_start;
+    uint32_t pk = 0, pk1 = 0;
+    bool gate = true;
+    if (RX && in && !full) {
+      const uint32_t* rg = pf.range + ((lo * 0x9E3779B1u + hi * pf.mul) >> pf.shift);
+      pk = __ldg(rg);
+      pk1 = __ldg(rg + 1);
+      gate = *(volatile unsigned long long*)&p.ctr[C_GATE] != 0;
+    }
+    if (literals) {
+      Probe pr;
+      if (a.fold) probe_literals(a, ascii_fold4(lo), ascii_fold4(hi), len - s, pr);
+      else probe_literals(a, lo, hi, len - s, pr);
+      verify_literals(a, s, a.fold ? ascii_fold4(x0) : x0, pr, match);
+    }
+    if (RX) verify_prefixes(a, t, p, pf, s, lo, hi, pk, pk1, gate, candidate);
+    flush(k0 + 32ull * warps >= n);
+  }
+  if (dense && a.parts) {
+    const uint64_t grams = (a.len + a.period - 1) / a.period;
+    for (uint64_t k0 = (uint64_t)blockIdx.x * blockDim.x; k0 < grams; k0 += (uint64_t)gridDim.x * blockDim.x) {
+      const uint64_t k = k0 + threadIdx.x;
+      if (k < grams) verify_gram(a, (uint32_t)(k * a.period), match);
+      flush(k0 + (uint64_t)gridDim.x * blockDim.x >= grams);
     }
   }
   if (RX) {
@@ -1017,10 +1086,9 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   a.bloom = plan.d_bloom.as<uint32_t>();
   a.info = plan.d_info.as<uint4>();
   a.lit_bytes = plan.d_bytes.as<uint8_t>();
-  a.meta = plan.d_meta.as<uint4>();
+  for (uint32_t i = 0; i < HASH_WINDOW; ++i) a.meta[i] = make_uint2(plan.meta[4 * i], plan.meta[4 * i + 1]);
   a.ranges = plan.d_ranges.as<uint2>();
   a.entries = plan.d_entries.as<uint2>();
-  a.window = HASH_WINDOW;
   a.out = l.out;
   a.cap = l.cap;
   a.counter = l.counter;
@@ -1036,10 +1104,10 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   a.parts16 = plan.parts16;
   a.bloom2 = plan.gram_len > 4 ? plan.d_bloom2.as<uint32_t>() : nullptr;
   a.big = plan.has_big ? plan.d_big.as<uint8_t>() : nullptr;
-  a.verify_bloom = plan.gram_kernel ? 1 : 0;
   a.bloom_parts = plan.bloom_parts;
   a.gram_bloom = plan.d_gram.as<uint32_t>();
   a.gram_word_bits = plan.gram_word_bits;
+  a.gram_bits = plan.gram_kernel ? plan.gram_bits : 0;
   a.phase = plan.d_phase.as<uint8_t>();
   a.phase_shift = 32 - plan.phase_bits;
   a.fold = plan.fold ? 1 : 0;
@@ -1054,14 +1122,14 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   auto run = [&](auto kernel) {
     check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "cudaFuncSetAttribute(literal)");
-    kernel<<<grid, kThreads, smem, st>>>(a);
+    launch_pdl(kernel, grid, kThreads, smem, st, a);
     check_cuda(cudaGetLastError(), "literal_filter_kernel launch");
   };
   const bool lg = plan.has_long != 0, sh = plan.has_short != 0;
   auto run_big = [&](auto kernel) {
     check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "cudaFuncSetAttribute(literal)");
-    kernel<<<grid, kBigThreads, smem, st>>>(a);
+    launch_pdl(kernel, grid, kBigThreads, smem, st, a);
     check_cuda(cudaGetLastError(), "literal_filter_big_kernel launch");
   };
   auto run_gram = [&](auto kernel, uint32_t run_bytes) {
@@ -1075,7 +1143,7 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
     const size_t gsmem = ((size_t)4 << plan.gram_word_bits) + (size_t)kGramWarps * kGramQueue * 4;
     check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem),
                "cudaFuncSetAttribute(literal gram)");
-    kernel<<<blocks, kGramThreads, gsmem, st>>>(a);
+    launch_pdl(kernel, blocks, kGramThreads, gsmem, st, a);
     check_cuda(cudaGetLastError(), "literal_gram_kernel launch");
   };
   // sparse sets: the gram kernel; else with literals shorter than 4 bytes and
@@ -1104,16 +1172,16 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
     sh ? run(literal_filter_kernel<1, 4, true, true>) : run(literal_filter_kernel<1, 4, true, false>);
   }
   // the verify pass is a chain of dependent loads per survivor: as many threads
-  // as are resident at once (six blocks per SM; with 16 a second wave doubled
-  // the latency: 160 regexes over 1 GiB 367 -> 351 us a scan), and for a short
-  // list no more blocks than it can fill
-  const uint64_t vgrid = std::min<uint64_t>((uint64_t)sm_count * (a.verify_bloom ? 6 : 4), (l.survivor_cap + 255) / 256);
+  // as are resident at once (four blocks per SM; a second wave doubled the
+  // latency: 40,000 items 65 -> 39 us in this kernel), and for a short list no
+  // more blocks than it can fill
+  const uint64_t vgrid = std::min<uint64_t>((uint64_t)sm_count * 4, (l.survivor_cap + 255) / 256);
   if (l.rx) {
     const PrefixDev pf{plan.d_prefix_range.as<uint32_t>(), plan.d_prefix_entry.as<uint4>(), plan.prefix_shift,
                        plan.prefix_mul};
-    literal_verify_kernel<true><<<(unsigned)vgrid, 256, 0, st>>>(a, l.rx->t, l.rx->p, pf);
+    launch_pdl(literal_verify_kernel<true>, (unsigned)vgrid, 256, 0, st, a, l.rx->t, l.rx->p, pf);
   } else {
-    literal_verify_kernel<false><<<(unsigned)vgrid, 256, 0, st>>>(a, DevTables{}, ScanPtrs{}, PrefixDev{});
+    launch_pdl(literal_verify_kernel<false>, (unsigned)vgrid, 256, 0, st, a, DevTables{}, ScanPtrs{}, PrefixDev{});
   }
   check_cuda(cudaGetLastError(), "literal_verify_kernel launch");
 }

@@ -15,6 +15,7 @@
 
 #include <cub/device/device_radix_sort.cuh>
 
+#include "ws_launch.h"
 #include "ws_matcher.h"
 
 namespace ws {
@@ -140,6 +141,7 @@ __device__ __forceinline__ void from_key(const SmallKey& k, ws_tagged_match& r) 
 template <class R, uint32_t kMost>
 __global__ void __launch_bounds__(1024) small_results_kernel(const R* rec, const unsigned long long* count, uint64_t cap,
                                                              unsigned long long* host_count, R* host_rows) {
+  pdl_begin();
   constexpr bool kTagged = sizeof(R) == sizeof(ws_tagged_match);
   __shared__ uint64_t src[kTagged ? kMost : 1], key[kMost];
   __shared__ uint32_t end[kMost];
@@ -196,7 +198,7 @@ uint8_t* result_buffer(Scratch& s) {
 void enqueue_results(Scratch& s, const ws_match* d_res, const unsigned long long* d_count, uint64_t cap,
                      cudaStream_t st) {
   uint8_t* d = result_buffer(s);
-  small_results_kernel<ws_match, kSmallResults><<<1, 1024, 0, st>>>(
+  launch_pdl(small_results_kernel<ws_match, kSmallResults>, 1, 1024, 0, st, 
       d_res, d_count, cap, reinterpret_cast<unsigned long long*>(d), reinterpret_cast<ws_match*>(d + 64));
   check_cuda(cudaGetLastError(), "small_results_kernel");
 }
@@ -204,7 +206,7 @@ void enqueue_results(Scratch& s, const ws_match* d_res, const unsigned long long
 void enqueue_results(Scratch& s, const ws_tagged_match* d_res, const unsigned long long* d_count, uint64_t cap,
                      cudaStream_t st) {
   uint8_t* d = result_buffer(s);
-  small_results_kernel<ws_tagged_match, kSmallTagged><<<1, 1024, 0, st>>>(
+  launch_pdl(small_results_kernel<ws_tagged_match, kSmallTagged>, 1, 1024, 0, st, 
       d_res, d_count, cap, reinterpret_cast<unsigned long long*>(d), reinterpret_cast<ws_tagged_match*>(d + 64));
   check_cuda(cudaGetLastError(), "small_results_kernel");
 }

@@ -22,6 +22,7 @@
 
 #include <algorithm>
 
+#include "ws_launch.h"
 #include "ws_matcher.h"
 
 using namespace ws;
@@ -243,6 +244,7 @@ void feed_pipelined(ws_stream* st, const uint8_t* data, uint64_t len) {
 __global__ void __launch_bounds__(1024) widen_kernel(const ws_match* in, const unsigned long long* step_count,
                                                      uint64_t step_cap, uint64_t base, ws_match64* out, uint64_t cap,
                                                      unsigned long long* total) {
+  pdl_begin();
   const unsigned long long n = *step_count;
   const unsigned long long at = *total;
   if (n >= kCountTimeout || at >= kCountTimeout) {  // a timeout or an unknown count stays in the total
@@ -315,7 +317,7 @@ uint32_t enqueue_windows(ws_matcher* m, Scratch& s, cudaStream_t cs, const uint8
     x.frontier = plan.frontier;
     before_window(seen + n);
     launches += enqueue_scan(m, s, cs, d_data + keep, seen + n - keep, s.out.as<ws_match>(), scap, step_count, x);
-    widen_kernel<<<1, 1024, 0, cs>>>(s.out.as<ws_match>(), step_count, scap, keep, d_out, cap, total);
+    launch_pdl(widen_kernel, 1, 1024, 0, cs, s.out.as<ws_match>(), step_count, scap, keep, d_out, cap, total);
     check_cuda(cudaGetLastError(), "widen_kernel");
     launches += 1;
     if (m->profile) {  // profiling: phase times summed over the windows
@@ -459,7 +461,7 @@ ws_status ws_scan_shard(ws_matcher* m, const uint8_t* d_data, uint64_t len, uint
     x.base = base;
     x.frontier = own_end;
     uint32_t launches = enqueue_scan(m, *s, cs, d_data, len, s->out.as<ws_match>(), scap, step_count, x);
-    widen_kernel<<<1, 1024, 0, cs>>>(s->out.as<ws_match>(), step_count, scap, base, d_out, cap, total);
+    launch_pdl(widen_kernel, 1, 1024, 0, cs, s->out.as<ws_match>(), step_count, scap, base, d_out, cap, total);
     check_cuda(cudaGetLastError(), "widen_kernel");
     check_cuda(cudaEventRecord(s->busy, cs), "event");
     std::lock_guard<std::mutex> g(m->info_mu);
