@@ -1012,14 +1012,11 @@ __device__ bool finalize(const ScanPtrs& p, unsigned long long* need) {
 // leftmost candidate start with its leftmost-first end, then the next candidate
 // at or after that end.  32 candidates at a time; where none of them overlaps
 // the one before it (the usual case) all are taken at once, else a ballot per
-// reported match picks the first one at or after the current end.
-__device__ void chain_list(const DevTables& t, const ScanPtrs& p, uint32_t r, const unsigned long long* list,
-                           uint32_t n, uint32_t lane) {
-  const uint32_t pid = t.pid[r];
-  // stream scans: resume at the regex's cursor, decide only starts before the
-  // frontier (both in stream offsets; the buffer starts at p.base <= cursor)
-  uint64_t last_end = (p.cursor64 && p.cursor64[r] > p.base) ? p.cursor64[r] - p.base : 0;
-  const uint64_t limit = p.cursor64 ? p.frontier - p.base : ~0ull;
+// reported match picks the first one at or after the current end.  The picks
+// stay in the list (with their ends), the others get kLfNone.  Returns the end
+// of the last pick (at least `last_end`).
+__device__ uint64_t chain_list(const DevTables& t, const ScanPtrs& p, uint32_t r, unsigned long long* list, uint32_t n,
+                               uint64_t last_end, uint64_t limit, uint32_t lane) {
   // each window's candidates are loaded while the previous window is decided
   const unsigned long long none = ((unsigned long long)0xFFFFFFFFu << 32) | kLfNone;
   unsigned long long next = lane < n ? list[lane] : none;
@@ -1062,54 +1059,120 @@ __device__ void chain_list(const DevTables& t, const ScanPtrs& p, uint32_t r, co
         last_end = ek;
       }
     }
-    // one output reservation per window of 32 candidates
-    const unsigned pm = __ballot_sync(0xFFFFFFFFu, picked);
-    if (pm) {
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(p.out_counter, (unsigned long long)__popc(pm));
-      base = __shfl_sync(0xFFFFFFFFu, base, 0);
-      if (picked) {
-        const unsigned long long idx = base + __popc(pm & ((1u << lane) - 1u));
-        if (idx < p.out_cap) p.out[idx] = ws_match{pid, s, e};
-      }
-    }
-    if (__any_sync(0xFFFFFFFFu, past)) break;  // sorted: every later start is past too
+    if (in) reinterpret_cast<uint32_t*>(list + j0 + lane)[0] = picked ? e : kLfNone;
   }
-  if (p.cursor64 && lane == 0) p.cursor64[r] = max(p.base + last_end, p.frontier);
+  return last_end;
+}
+
+// Stream scans: the chain resumes at the regex's cursor and decides only starts
+// before the frontier (both in stream offsets; the buffer starts at p.base).
+__device__ __forceinline__ uint64_t chain_start(const ScanPtrs& p, uint32_t r) {
+  return (p.cursor64 && p.cursor64[r] > p.base) ? p.cursor64[r] - p.base : 0;
+}
+__device__ __forceinline__ uint64_t chain_limit(const ScanPtrs& p) {
+  return p.cursor64 ? p.frontier - p.base : ~0ull;
+}
+
+// The picks of a list to the output: by `width` threads (a warp or a block,
+// thread i of them), one reservation per `width` candidates.
+__device__ __forceinline__ void report_window(const ScanPtrs& p, uint32_t pid, unsigned long long c, bool picked,
+                                              unsigned long long at) {
+  if (picked && at < p.out_cap) p.out[at] = ws_match{pid, (uint32_t)(c >> 32), (uint32_t)c};
 }
 
 // A warp per regex.
 __global__ void k_chain_kernel(DevTables t, ScanPtrs p, unsigned long long* need) {
   pdl_begin();
   if (finalize(p, need)) return;
-  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= t.n_regex) return;  // whole warps exit together
-  chain_list(t, p, r, p.pair + p.offs[r], p.offs[r + 1] - p.offs[r], threadIdx.x & 31);
+  unsigned long long* list = p.pair + p.offs[r];
+  const uint32_t n = p.offs[r + 1] - p.offs[r], pid = t.pid[r];
+  const uint64_t last_end = chain_list(t, p, r, list, n, chain_start(p, r), chain_limit(p), lane);
+  for (uint32_t j0 = 0; j0 < n; j0 += 32) {  // (every lane wrote its own candidates)
+    const unsigned long long c = j0 + lane < n ? list[j0 + lane] : kLfNone;
+    const bool picked = (uint32_t)c != kLfNone;
+    const unsigned pm = __ballot_sync(0xFFFFFFFFu, picked);
+    if (!pm) continue;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(p.out_counter, (unsigned long long)__popc(pm));
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    report_window(p, pid, c, picked, base + __popc(pm & ((1u << lane) - 1u)));
+  }
+  if (p.cursor64 && lane == 0) p.cursor64[r] = max(p.base + last_end, p.frontier);
 }
 
 // Sort, missing ends and chain of a regex by one block, in shared memory for up
 // to kSortTile candidates: the resolution of scans whose candidates came from
 // prefixes, ends known (three kernels and a pass through global memory between
-// each took 8 us more on small lists).
+// each took 8 us more on small lists).  A list in which no candidate overlaps
+// the next needs no chain: all of it is reported at once, with one reservation
+// per block-width of candidates (a reservation per 32, each waiting for the one
+// before, took 14 of 23 us on 400 candidates a regex).
 __global__ void __launch_bounds__(256) k_resolve_kernel(DevTables t, ScanPtrs p, uint32_t n_regex,
                                                         unsigned long long* need) {
-  pdl_begin();
   __shared__ unsigned long long buf[kSortTile];
+  __shared__ uint32_t wcount[8];
+  __shared__ unsigned long long first;
+  __shared__ uint64_t chain_end;
+  pdl_begin();
   if (finalize(p, need)) return;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t limit = chain_limit(p);
   for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
     const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
+    const uint64_t from = chain_start(p, r);
+    if (n == 0) {
+      if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + from, p.frontier);
+      continue;
+    }
     unsigned long long* list = p.pair + a;
     if (n > kSortTile) {
       sort_list(buf, list, p.pair2 + a, n);
-    } else if (n) {
+    } else {
       sort_into(buf, list, n);
       list = buf;
     }
     for (uint32_t j = threadIdx.x; j < n; j += blockDim.x)
       if ((uint32_t)list[j] == kLfTodo) reinterpret_cast<uint32_t*>(list + j)[0] = list_end(t, p, r, list, j);
     __syncthreads();
-    if (threadIdx.x < 32) chain_list(t, p, r, list, n, threadIdx.x);
-    __syncthreads();  // the next regex's sort overwrites buf
+    bool apart = true;
+    for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+      const unsigned long long c = list[j];
+      const uint32_t s = (uint32_t)(c >> 32), e = (uint32_t)c;
+      apart &= e < kLfTodo && (uint64_t)s >= from && (uint64_t)s < limit &&
+               (j + 1 == n || (uint32_t)(list[j + 1] >> 32) >= e);
+    }
+    if (!__syncthreads_and(apart)) {
+      if (warp == 0) {
+        const uint64_t end = chain_list(t, p, r, list, n, from, limit, lane);
+        if (lane == 0) chain_end = end;
+      }
+    } else if (threadIdx.x == 0) {
+      chain_end = max(from, (uint64_t)(uint32_t)list[n - 1]);
+    }
+    __syncthreads();
+    if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + chain_end, p.frontier);
+    for (uint32_t j0 = 0; j0 < n; j0 += blockDim.x) {
+      const uint32_t j = j0 + threadIdx.x;
+      const unsigned long long c = j < n ? list[j] : kLfNone;
+      const bool picked = (uint32_t)c != kLfNone;
+      const unsigned pm = __ballot_sync(0xFFFFFFFFu, picked);
+      if (lane == 0) wcount[warp] = __popc(pm);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        uint32_t sum = 0;
+        for (uint32_t k = 0; k < blockDim.x >> 5; ++k) {
+          const uint32_t x = wcount[k];
+          wcount[k] = sum;
+          sum += x;
+        }
+        first = sum ? atomicAdd(p.out_counter, (unsigned long long)sum) : 0;
+      }
+      __syncthreads();
+      report_window(p, t.pid[r], c, picked, first + wcount[warp] + __popc(pm & ((1u << lane) - 1u)));
+      __syncthreads();  // (wcount, first; and buf before the next regex)
+    }
   }
 }
 
@@ -1297,7 +1360,8 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
     launches++;
   }
   mark(3);
-  launch_pdl(dfa_reverse_kernel, sm_count * 8, 256, 0, st, t, p);
+  // (as a fallback, a quarter of the blocks: they usually find no event and exit)
+  launch_pdl(dfa_reverse_kernel, t.n_walk ? sm_count * 8 : sm_count * 2, 256, 0, st, t, p);
   check_cuda(cudaGetLastError(), "dfa_reverse_kernel");
   launches++;
   context_groups();
@@ -1880,7 +1944,7 @@ uint32_t regex_finish(RegexPlan& P, RegexScan& rs, const RegexLaunch& l, cudaStr
   launches += candidates_phase(P, t, p, l.mode, st, sm_count, ev);
   const bool staged = P.n_regex < kOffsShared;
   const size_t osmem = staged ? ((size_t)P.n_regex + 1) * 4 : 0;
-  const int hg = (int)std::min<uint64_t>((uint64_t)sm_count * 4, (rs.k_cap + 255) / 256);
+  const int hg = (int)std::min<uint64_t>((uint64_t)sm_count * (t.n_walk ? 4 : 1), (rs.k_cap + 255) / 256);
   if (!staged) {
     launch_pdl(k_scan_kernel, 1, 1024, 0, st, p, P.n_regex);
     launches += 1;

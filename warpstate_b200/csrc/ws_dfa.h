@@ -120,8 +120,8 @@ struct RegexPlan {
   // host copies
   std::vector<uint32_t> fwd, rev, lf, mptr, mlist, rmptr, rmlist, lfinfo, pid;
   // per regex, 8 words: {context, start row per left context (4), offset in
-  // `lf` of the end-step flags, 0, 0}; context 0 for regexes without
-  // assertions
+  // `lf` of the end-step flags, 0, 0}; context 0 for regexes
+  // without assertions
   std::vector<uint32_t> lfx;
   std::vector<uint32_t> hot;   // shared-memory images, one per (group, part)
   std::vector<uint8_t> cls;

@@ -653,7 +653,9 @@ __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(LitA
 // against 184.
 constexpr int kGramThreads = 1024;
 constexpr uint32_t kGramWarps = kGramThreads / 32;
-constexpr uint32_t kGramQueue = 512;  // u32 positions per warp
+// u32 positions per warp.  (512 of them left less L1 for the flush, which reads
+// the queued grams again: 10,000 literals over 1 GiB 204 -> 200 us a scan.)
+constexpr uint32_t kGramQueue = 128;
 constexpr uint32_t kGramBits = 32;    // grams per lane and mask
 constexpr uint32_t kNoSurvivor = 0xFFFFFFFFu;  // no position: inputs are shorter than 2^32 bytes
 
