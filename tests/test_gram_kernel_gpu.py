@@ -70,3 +70,26 @@ def test_gram_kernel_list_overflow():
         exp = oracle.scan_patterns([(0, p) for p in lits], d)
         assert len(exp) > (1 << 20)
         assert np.array_equal(m.scan_array(d), exp), run
+
+
+@pytest.mark.parametrize("fold", [False, True])
+@pytest.mark.parametrize("unit,n", [(b"zqz", 300_001), (b"zqzq", 262_144), (b"zqzqz", 300_013), (b"zqzqzqz", 524_303),
+                                    (b"ACGTACGGTACCATGCATG", 400_007)])
+def test_gram_kernel_full_list_forms(unit, n, fold):
+    # the second look at every gram: each gram form, short and long literals,
+    # runs of matches with gaps, both cases of a caseless set, an odd tail
+    import warpstate_b200 as ws
+    lits = sorted({unit, unit + unit[:2], unit + unit} | set(_set(len(unit), 200, LETTERS, 7)))
+    b = ws.PatternSet.builder().case_insensitive(fold)
+    for p in lits:
+        b = b.literal_bytes(p)
+    m = ws.GpuMatcher.with_config(b.build(), ws.AutoMatcherConfig().max_matches(1 << 20))
+    period = len(unit) if len(unit) > 7 else 2
+    d = np.frombuffer((unit[:period] * (n // period + 1))[:n], dtype=np.uint8).copy()
+    d[np.random.default_rng(3).integers(0, n, n // 200)] = ord("~")
+    if fold:
+        d[::3] = np.frombuffer(d[::3].tobytes().swapcase(), dtype=np.uint8)
+    pats = [(0, p) for p in lits]
+    exp = oracle.scan_patterns(pats, d, case_insensitive=True) if fold else oracle.scan_patterns(pats, d)
+    assert len(exp) > n // 32
+    assert np.array_equal(m.scan_array(d), exp)

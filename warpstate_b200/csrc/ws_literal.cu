@@ -65,7 +65,6 @@ struct LitArgs {
   uint64_t cap;
   unsigned long long* counter;
   uint32_t* survivors;       // candidate start positions (low 32 bits)
-  uint32_t* survivor_hi;     // unused for inputs < 4 GiB
   unsigned long long* survivor_count;
   uint64_t survivor_cap;
   const uint32_t* item_end;  // batch: ascending item ends (n_items), else null
@@ -197,14 +196,44 @@ __device__ __forceinline__ void report_match(const LitArgs& a, uint32_t pid, uin
   if (idx < a.cap) a.out[idx] = ws_match{pid, s, e};
 }
 
-// Verifies a position in the compacting kernel (the survivor list is full).
-__device__ __forceinline__ void verify_in_place(const LitArgs& a, uint32_t s) {
-  if (!a.parts || s >= a.max_start) return;
-  const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
+// probe_literals and verify_literals one prefix length and one word at a time,
+// for inputs whose survivors do not fit the list.  The probes in flight together
+// are more code and registers: inlined in the compacting kernels they spilled
+// the main loop (11-mers over 128 MiB 313 us a scan, this way 246).
+template <class Sink>
+__device__ __forceinline__ void verify_lean(const LitArgs& a, uint32_t s, Sink&& sink) {
+  if (s >= a.max_start) return;
+  const uint32_t len = (uint32_t)a.len, rem = len - s, w0 = s & ~3u, sh = (s & 3) * 8;
   const uint32_t x0 = input_word(a, len, w0), x1 = input_word(a, len, w0 + 4), x2 = input_word(a, len, w0 + 8);
-  Probe pr;
-  probe_literals(a, __funnelshift_r(x0, x1, sh), __funnelshift_r(x1, x2, sh), len - s, pr);
-  verify_literals(a, s, x0, pr, [&](uint32_t pid, uint32_t at, uint32_t e) { report_match(a, pid, at, e); });
+  const uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
+  const uint32_t window = rem < HASH_WINDOW ? rem : HASH_WINDOW;
+  uint32_t h = 2166136261u;
+#pragma unroll 1
+  for (uint32_t i = 0; i < window; ++i) {
+    h = (h ^ (((i < 4 ? lo : hi) >> (8 * (i & 3))) & 0xFFu)) * 16777619u;
+    if (!((a.parts >> i) & 1u)) continue;
+    const uint2 r = __ldg(a.ranges + a.meta[i].x + (h & a.meta[i].y));
+#pragma unroll 1
+    for (uint32_t e = 0; e < r.y; ++e) {
+      const uint2 ent = __ldg(a.entries + r.x + e);
+      if (ent.x != h) continue;
+      const uint4 info = __ldg(a.info + ent.y);  // {offset, len, pattern id, 0}
+      if (info.y > rem) continue;
+      const uint32_t* lit = reinterpret_cast<const uint32_t*>(a.lit_bytes + info.x);
+      bool eq = true;
+      uint32_t cur = x0;
+#pragma unroll 1
+      for (uint32_t k = 0; k < info.y && eq; k += 4) {
+        const uint32_t nxt = input_word(a, len, w0 + k + 4), left = info.y - k;
+        const uint32_t m = left >= 4 ? 0xFFFFFFFFu : ((1u << (8 * left)) - 1u);
+        eq = ((__ldg(lit + (k >> 2)) ^ __funnelshift_r(cur, nxt, sh)) & m) == 0;
+        cur = nxt;
+      }
+      if (!eq || s + info.y <= a.min_end) continue;
+      if (a.n_items && s + info.y > item_end_of(a.item_end, a.n_items, s)) continue;  // crosses items
+      sink(info.z, s, s + info.y);
+    }
+  }
 }
 
 // 16-bit mask of owned positions that may start a literal (stage 1).  w[0..3]
@@ -362,7 +391,11 @@ __device__ __forceinline__ void process_block(const LitArgs& a, uint32_t* blk, u
         const unsigned long long slot = wbase + __popc(ball & ((1u << lane) - 1u));
         const uint32_t s = blk_base + off;
         if (slot < a.survivor_cap) a.survivors[slot] = s;
-        else verify_in_place(a, s);  // list full
+        else verify_lean(a, s, [&](uint32_t pid, uint32_t at, uint32_t e) {  // list full
+          // (not report_match, whose code held registers of the loop: 262 -> 246 us)
+          const unsigned long long idx = atomicAdd(a.counter, 1ull);
+          if (idx < a.cap) a.out[idx] = ws_match{pid, at, e};
+        });
       }
     }
   }
@@ -372,7 +405,7 @@ __device__ __forceinline__ void process_block(const LitArgs& a, uint32_t* blk, u
 // Inputs of one launch are below 4 GiB, so block, vector and byte indices are
 // 32-bit.
 template <int P, int G, bool LONG, bool SHORT>
-__global__ void __launch_bounds__(kThreads, 1) literal_filter_kernel(LitArgs a) {
+__global__ void __launch_bounds__(kThreads, 1) literal_filter_kernel(const __grid_constant__ LitArgs a) {
   pdl_begin();
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* filt = smem;                                 // filter_words
@@ -524,7 +557,7 @@ constexpr int kBigWarps = kBigThreads / 32;
 // block i is finished -- so that the L2 latency overlaps useful work.
 // 16 warps per CTA leave room for the pipeline's registers.
 template <int G, bool SHORT>
-__global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(LitArgs a) {
+__global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(const __grid_constant__ LitArgs a) {
   pdl_begin();
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* filt = smem;
@@ -674,8 +707,7 @@ __device__ __forceinline__ void lean_holes(const LitArgs& a, const LeanSlots& r,
 
 // Key of the phase table for the gram at position at: a hash independent of
 // stage 1's, so that what stage 1 lets through by chance does not pass again.
-template <int G>
-__device__ __forceinline__ uint32_t phase_key_at(const LitArgs& a, uint32_t at) {
+__device__ __forceinline__ uint32_t phase_key_at(const LitArgs& a, uint32_t at, int G) {
   const uint32_t len = (uint32_t)a.len, w0 = at & ~3u, sh = (at & 3) * 8;
   if (G == 16) {  // aligned
     return phase_key(input_word(a, len, w0), input_word(a, len, w0 + 4), input_word(a, len, w0 + 8),
@@ -686,16 +718,17 @@ __device__ __forceinline__ uint32_t phase_key_at(const LitArgs& a, uint32_t at) 
 }
 
 // Takes the queued grams [0, n), 32 at a time: phase bits, start positions,
-// append.
+// append.  True when the list was full before: the verify kernel then looks at
+// every gram of the input again, and this kernel has nothing more to add.
 template <int P, int G>
-__device__ __forceinline__ void gram_flush(const LitArgs& a, const uint32_t* queue, uint32_t n, LeanSlots& r,
+__device__ __forceinline__ bool gram_flush(const LitArgs& a, const uint32_t* queue, uint32_t n, LeanSlots& r,
                                            uint32_t lane) {
   const uint32_t len = (uint32_t)a.len;
   for (uint32_t k0 = 0; k0 < n; k0 += 32) {
     uint32_t at = 0, bits = 0;
     if (k0 + lane < n) {
       at = queue[k0 + lane];
-      bits = (uint32_t)__ldg(a.phase + (phase_key_at<G>(a, at) >> a.phase_shift));
+      bits = (uint32_t)__ldg(a.phase + (phase_key_at(a, at, G) >> a.phase_shift));
 #pragma unroll
       for (int k = 0; k < P; ++k)  // bit P - 1 - k: the literal starts k bytes before the gram
         if (at < (uint32_t)k || at - k >= len) bits &= ~(1u << (P - 1 - k));
@@ -717,20 +750,23 @@ __device__ __forceinline__ void gram_flush(const LitArgs& a, const uint32_t* que
       wb = __shfl_sync(0xFFFFFFFFu, wb, 0);
       r.next = wb;
       r.end = wb + want;
+      if (wb >= a.survivor_cap) return true;
     }
     unsigned long long slot = r.next + incl - cnt;
     r.next += total;
     for (; bits; bits &= bits - 1) {
-      // (a full list: the count alone says so, and the verify kernel looks at
-      // every gram again; verifying here cost the loop its registers)
+      // (verifying here when the list is full cost the loop its registers)
       if (slot < a.survivor_cap) a.survivors[slot] = at - (P - 1) + (__ffs(bits) - 1);
       ++slot;
     }
   }
+  return false;
 }
 
 // Queues the passing grams of a run of vectors (bit i of `pass`: gram i % NG of
-// vector i / NG) and flushes whole groups of 32.
+// vector i / NG) and flushes whole groups of 32; kListFull when the list was.
+constexpr uint32_t kListFull = 0xFFFFFFFFu;
+
 template <int P, int G>
 __device__ __forceinline__ uint32_t gram_queue(const LitArgs& a, uint32_t* queue, uint32_t queued, uint32_t pass,
                                                uint32_t base, LeanSlots& slots, uint32_t lane) {
@@ -745,7 +781,7 @@ __device__ __forceinline__ uint32_t gram_queue(const LitArgs& a, uint32_t* queue
     if (queued > kGramQueue - 32 || (queued >= 32 && !__any_sync(0xFFFFFFFFu, pass != 0))) {
       __syncwarp();
       const uint32_t whole = queued & ~31u, left = queued & 31u;
-      gram_flush<P, G>(a, queue, whole, slots, lane);
+      if (gram_flush<P, G>(a, queue, whole, slots, lane)) return kListFull;
       const uint32_t keep = lane < left ? queue[whole + lane] : 0u;
       __syncwarp();
       if (lane < left) queue[lane] = keep;
@@ -866,8 +902,10 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
       pass = gram_test<P, G, BITS, NPRE>(filt, wsh, lane, v, below, pass);
     }
     if (OFF && r == 0 && lane == 0) pass &= ~((1u << ((OFF + P - 1) / P)) - 1u);  // grams that begin before the input
-    if (__any_sync(0xFFFFFFFFu, pass != 0))
+    if (__any_sync(0xFFFFFFFFu, pass != 0)) {
       queued = gram_queue<P, G>(a, queue, queued, pass, r * (VECS * 512) + lane * 16 - OFF, slots, lane);
+      if (queued == kListFull) return;
+    }
   }
   // the vectors after the last whole run, one warp each
   const uint32_t v0 = runs * VECS, nv = (nvec + 31) >> 5;
@@ -882,6 +920,7 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
     uint32_t pass = gram_test<P, G, BITS, NPRE>(filt, wsh, lane, v, below, 0u) >> (32 - NG);
     if (OFF && b == 0 && lane == 0) pass &= ~((1u << ((OFF + P - 1) / P)) - 1u);
     queued = gram_queue<P, G>(a, queue, queued, pass, b * 512 + lane * 16 - OFF, slots, lane);
+    if (queued == kListFull) return;
   }
   if (queued) gram_flush<P, G>(a, queue, queued, slots, lane);
   lean_holes(a, slots, lane);
@@ -919,38 +958,48 @@ __device__ __forceinline__ void verify_prefixes(const LitArgs& a, const DevTable
   }
 }
 
-// The gram at `at` and, when it passes stage 1 and the phase table, the literals
-// that start at its phases: the gram kernel's test of one position, from global
-// memory (inputs whose survivors did not fit the list).
-template <class Sink>
-__device__ __noinline__ void verify_gram(const LitArgs& a, uint32_t at, Sink& sink) {
-  const uint32_t len = (uint32_t)a.len, w0 = at & ~3u, sh = (at & 3) * 8, wsh = 32 - a.gram_word_bits;
-  uint32_t g[4] = {0, 0, 0, 0};
-  g[0] = __funnelshift_r(input_word(a, len, w0), input_word(a, len, w0 + 4), sh);
-  if (a.gram_len == 16)  // (aligned)
-    for (uint32_t k = 1; k < 4; ++k) g[k] = input_word(a, len, w0 + 4 * k);
-  const uint32_t h = gram_hash32(g[0], g[1], g[2], g[3], (int)a.gram_len);
-  const uint32_t x = __ldg(a.gram_bloom + (h >> wsh));
-  if (!((x >> ((h >> (wsh - 5)) & 31u)) & 1u)) return;
-  if (a.gram_bits == 2 && !((x >> ((h >> (wsh - 10)) & 31u)) & 1u)) return;
-  uint32_t bits = __ldg(a.phase + (phase_key(g[0], g[1], g[2], g[3], (int)a.gram_len) >> a.phase_shift));
-  for (; bits; bits &= bits - 1) {
-    const uint32_t k = a.period - __ffs(bits);  // bit period - 1 - k: the literal starts k bytes before the gram
-    if (at < k || at - k >= len || at - k >= a.max_start) continue;
-    const uint32_t s = at - k, v0 = s & ~3u, vs = (s & 3) * 8;
-    const uint32_t x0 = input_word(a, len, v0), x1 = input_word(a, len, v0 + 4), x2 = input_word(a, len, v0 + 8);
-    Probe pr;
-    probe_literals(a, __funnelshift_r(x0, x1, vs), __funnelshift_r(x1, x2, vs), len - s, pr);
-    verify_literals(a, s, x0, pr, sink);
+// Stage 1 of the grams that start in the 16 bytes of vector v, by tables in
+// global memory: bit j of the result is the gram at byte j.
+__device__ __forceinline__ uint32_t grams_pass(const LitArgs& a, uint32_t v) {
+  const uint32_t len = (uint32_t)a.len, at = v * 16, wsh = 32 - a.gram_word_bits;
+  uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const uint4 x = load_vec(a.data, a.len, v);
+  w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k) {
+    if (a.fold) w[k] = ascii_fold4(w[k]);
+    if ((k == 0 || a.gram_len == 16) && at + 16 + 4 * k < len) w[4 + k] = input_word(a, len, at + 16 + 4 * k);
   }
+  uint32_t pass = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < 16; ++j) {
+    if (j & (a.period - 1)) continue;
+    uint32_t h;
+    if (a.gram_len == 16) {
+      const uint32_t i = j >> 2;
+      h = gram_hash32(w[i], w[i + 1], w[i + 2], w[i + 3], 16);
+    } else {
+      h = __funnelshift_r(w[j >> 2], w[(j >> 2) + 1], 8 * (j & 3)) * (a.gram_len == 3 ? gram_hash32(1, 0, 0, 0, 3) : gram_hash32(1, 0, 0, 0, 4));
+    }
+    const uint32_t x = __ldg(a.gram_bloom + (h >> wsh));
+    uint32_t bit = x >> ((h >> (wsh - 5)) & 31u);
+    if (a.gram_bits == 2) bit &= x >> ((h >> (wsh - 10)) & 31u);
+    pass |= (bit & 1u) << j;
+  }
+  const uint32_t left = len - at;
+  return left < 16 ? pass & ((1u << left) - 1u) : pass;
 }
 
-// Kernel 2.  When the gram kernel's list was full, every gram of the input is
-// tested again here and verified at once.  RX: the survivors are also looked up
+// Kernel 2.  When the gram kernel's list was full (it then stopped early), every
+// gram of the input is tested again here: a warp takes 16 bytes per lane, queues
+// the grams that pass in shared memory and verifies their literals with all its
+// lanes busy.  (One gram per thread, verified where it was found, took 2,300 us
+// for the 4 M literals of 64 MiB; a queue per block, with its barriers, 340.)  RX: the survivors are also looked up
 // among the regex prefixes.  A full list (more than one survivor per 64 bytes)
 // gives the prefix candidates up, like long walks do; the last block then drops
 // the candidates found so far, so that the gated groups start from none.
 constexpr uint32_t kVerifyBuf = 512;
+constexpr uint32_t kDenseBuf = kVerifyBuf / 8;  // matches and grams a warp of the dense pass holds
 
 template <bool RX>
 __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_constant__ LitArgs a,
@@ -960,7 +1009,8 @@ __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_con
   // Matches and candidates collect in shared memory: one atomic per block and
   // counter instead of one per match (65,536 on one address took 35 us).
   __shared__ uint3 mbuf[kVerifyBuf];
-  __shared__ uint3 kbuf[RX ? kVerifyBuf : 1];
+  // (kbuf also holds the dense pass's positions: a full list makes no candidates)
+  __shared__ uint3 kbuf[kVerifyBuf];
   __shared__ uint32_t held[2];
   __shared__ unsigned long long first[2];
   if (threadIdx.x < 2) held[threadIdx.x] = 0;
@@ -972,7 +1022,7 @@ __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_con
   };
   auto candidate = [&](uint32_t r, uint32_t s, uint32_t e) {
     const uint32_t i = atomicAdd(&held[1], 1u);
-    if (i < kVerifyBuf) kbuf[RX ? i : 0] = make_uint3(r, s, e);
+    if (i < kVerifyBuf) kbuf[i] = make_uint3(r, s, e);
     else emit_k(p, r, s, e, kEndKnown);
   };
   unsigned long long n = *a.survivor_count;
@@ -1034,12 +1084,62 @@ __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_con
     flush(k0 + 32ull * warps >= n);
   }
   if (dense && a.parts) {
-    const uint64_t grams = (a.len + a.period - 1) / a.period;
-    for (uint64_t k0 = (uint64_t)blockIdx.x * blockDim.x; k0 < grams; k0 += (uint64_t)gridDim.x * blockDim.x) {
-      const uint64_t k = k0 + threadIdx.x;
-      if (k < grams) verify_gram(a, (uint32_t)(k * a.period), match);
-      flush(k0 + (uint64_t)gridDim.x * blockDim.x >= grams);
+    __shared__ uint32_t wheld[8];
+    const uint32_t len = (uint32_t)a.len, nvec = (uint32_t)((a.len + 15) >> 4), wi = threadIdx.x >> 5;
+    uint3* mine = mbuf + wi * kDenseBuf;
+    uint32_t* grams = reinterpret_cast<uint32_t*>(kbuf) + wi * kDenseBuf;
+    uint32_t* mine_held = wheld + wi;
+    if (lane == 0) *mine_held = 0;
+    __syncwarp();
+    auto warp_match = [&](uint32_t pid, uint32_t s, uint32_t e) {
+      const uint32_t i = atomicAdd(mine_held, 1u);
+      if (i < kDenseBuf) mine[i] = make_uint3(pid, s, e);
+      else report_match(a, pid, s, e);
+    };
+    auto verify_grams = [&](uint32_t n, bool end) {  // grams[0, n), n <= 32
+      if (lane < n) {
+        const uint32_t at = grams[lane];
+        uint32_t bits = __ldg(a.phase + (phase_key_at(a, at, (int)a.gram_len) >> a.phase_shift));
+        for (; bits; bits &= bits - 1) {
+          const uint32_t k = a.period - __ffs(bits);  // bit period - 1 - k: the literal starts k bytes before
+          if (at >= k && at - k < len) verify_lean(a, at - k, warp_match);
+        }
+      }
+      __syncwarp();
+      const uint32_t nm = min(*mine_held, kDenseBuf);
+      if (nm > kDenseBuf - 32 || (end && nm)) {
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(a.counter, (unsigned long long)nm);
+        at = __shfl_sync(0xFFFFFFFFu, at, 0);
+        for (uint32_t i = lane; i < nm; i += 32)
+          if (at + i < a.cap) a.out[at + i] = ws_match{mine[i].x, mine[i].y, mine[i].z};
+        __syncwarp();
+        if (lane == 0) *mine_held = 0;
+      }
+      __syncwarp();
+    };
+    uint32_t queued = 0;
+    for (uint64_t v0 = (uint64_t)w * 32; v0 < nvec; v0 += (uint64_t)warps * 32) {
+      const uint32_t v = (uint32_t)v0 + lane;
+      uint32_t pass = v < nvec ? grams_pass(a, v) : 0u;
+      for (uint32_t ball; (ball = __ballot_sync(0xFFFFFFFFu, pass != 0)) != 0;) {
+        if (pass) {  // one gram of every lane that has one left
+          grams[queued + __popc(ball & ((1u << lane) - 1u))] = v * 16 + __ffs(pass) - 1;
+          pass &= pass - 1;
+        }
+        queued += __popc(ball);
+        __syncwarp();
+        if (queued >= 32) {
+          verify_grams(32, false);
+          queued -= 32;
+          const uint32_t keep = lane < queued ? grams[32 + lane] : 0u;
+          __syncwarp();
+          if (lane < queued) grams[lane] = keep;
+          __syncwarp();
+        }
+      }
     }
+    verify_grams(queued, true);
   }
   if (RX) {
     __shared__ bool last;
@@ -1096,7 +1196,6 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   a.counter = l.counter;
   a.survivor_count = reinterpret_cast<unsigned long long*>(l.scratch);
   a.survivors = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(l.scratch) + 64);
-  a.survivor_hi = nullptr;
   a.survivor_cap = l.survivor_cap;
   a.item_end = l.item_end;
   a.n_items = l.n_items;
