@@ -912,17 +912,9 @@ __device__ uint32_t merge_path(const unsigned long long* A, uint32_t na, const u
   return lo;
 }
 
-// Sorts regex candidates list[0, n) ascending by start: a bitonic sort in
-// shared memory for up to kSortTile; beyond that, sorted tiles merged pairwise
-// in global memory (merge-path split of each merge across the block), with
-// other[0, n) as the other buffer.
-__device__ void sort_list(unsigned long long* buf, unsigned long long* list, unsigned long long* other, uint32_t n) {
-  for (uint32_t t0 = 0; t0 < n; t0 += kSortTile) {
-    const uint32_t m = min(kSortTile, n - t0);
-    sort_into(buf, list + t0, m);
-    for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) list[t0 + k] = buf[k];
-    __syncthreads();
-  }
+// Merges the sorted tiles of list[0, n) pairwise in global memory (merge-path
+// split of each merge across the block), with other[0, n) as the other buffer.
+__device__ void merge_tiles(unsigned long long* list, unsigned long long* other, uint32_t n) {
   unsigned long long *src = list, *dst = other;
   for (uint32_t w = kSortTile; w < n; w <<= 1) {
     for (uint32_t lo = 0; lo < n; lo += 2 * w) {
@@ -945,12 +937,39 @@ __device__ void sort_list(unsigned long long* buf, unsigned long long* list, uns
   }
 }
 
+// Sorts tile k of regex candidates list[0, n) by start.
+__device__ void sort_tile(unsigned long long* buf, unsigned long long* list, uint32_t n, uint32_t k) {
+  const uint32_t t0 = k * kSortTile, m = min(kSortTile, n - t0);
+  sort_into(buf, list + t0, m);
+  for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) list[t0 + i] = buf[i];
+  __syncthreads();
+}
+
+// A list of up to kSortTile candidates by one block.  The tiles of longer lists
+// are shared by the gridDim.y blocks of the regex, and the block that finishes
+// the last one merges them (its ticket is the regex's count, which nothing reads
+// after the scatter).  The same three regexes: 2,110 us with a block per regex,
+// 1,025 this way.
 __global__ void __launch_bounds__(512) k_sort_kernel(ScanPtrs p, uint32_t n_regex) {
   pdl_begin();
   __shared__ unsigned long long buf[kSortTile];
+  __shared__ bool last;
   for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
-    const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
-    if (n > 1) sort_list(buf, p.pair + a, p.pair2 + a, n);
+    const uint32_t a = p.offs[r], n = p.offs[r + 1] - a, tiles = (n + kSortTile - 1) / kSortTile;
+    if (n < 2) continue;
+    uint32_t done = 0;
+    for (uint32_t k = blockIdx.y; k < tiles; k += gridDim.y, ++done) sort_tile(buf, p.pair + a, n, k);
+    if (tiles < 2 || !done) continue;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      last = atomicAdd(&p.count[r], done) + done == n + tiles;
+    }
+    __syncthreads();
+    if (last) {
+      __threadfence();
+      merge_tiles(p.pair + a, p.pair2 + a, n);
+    }
+    __syncthreads();
   }
 }
 
@@ -1008,58 +1027,126 @@ __device__ bool finalize(const ScanPtrs& p, unsigned long long* need) {
   return true;
 }
 
-// find_iter chain of one regex over its sorted candidates, by one warp:
-// leftmost candidate start with its leftmost-first end, then the next candidate
-// at or after that end.  32 candidates at a time; where none of them overlaps
-// the one before it (the usual case) all are taken at once, else a ballot per
-// reported match picks the first one at or after the current end.  The picks
-// stay in the list (with their ends), the others get kLfNone.  Returns the end
-// of the last pick (at least `last_end`).
-__device__ uint64_t chain_list(const DevTables& t, const ScanPtrs& p, uint32_t r, unsigned long long* list, uint32_t n,
-                               uint64_t last_end, uint64_t limit, uint32_t lane) {
-  // each window's candidates are loaded while the previous window is decided
-  const unsigned long long none = ((unsigned long long)0xFFFFFFFFu << 32) | kLfNone;
-  unsigned long long next = lane < n ? list[lane] : none;
-  for (uint32_t j0 = 0; j0 < n; j0 += 32) {
-    const bool in = j0 + lane < n;
+// find_iter chain of one regex over its sorted candidates, and its report, by a
+// block: leftmost candidate start with its leftmost-first end, then the next
+// candidate at or after that end.  kChainThreads candidates at a time: one that
+// starts at or after the ends of all candidates before it is picked whatever was
+// picked before, so it heads a cluster that its thread decides alone, going from
+// pick to pick.  (Three regexes without prefixes over 128 MiB of log text, whose
+// lists hold every start inside a digit run: 3,190 us by a warp that picked one
+// candidate after the other by a ballot, 775 this way.)
+constexpr uint32_t kChainThreads = 256;
+constexpr uint32_t kChainWarps = kChainThreads / 32;
+
+struct ChainShared {
+  unsigned long long win[kChainThreads];  // the window's candidates
+  uint32_t pick[kChainThreads];           // their ends when picked, else kLfNone
+  uint32_t valid[kChainWarps], head[kChainWarps], most[kChainWarps], picked[kChainWarps];
+  uint32_t end;                           // of the last cluster
+  unsigned long long first;
+};
+
+// The picks of the cluster headed by the thread's candidate: from each pick the
+// first valid candidate at or after its end, up to the next head.  The last
+// cluster of a window goes on in the next one, from sh.end.
+template <class Walk>
+__device__ __forceinline__ void decide(ChainShared& sh, Walk&& walk) {
+  auto next_valid = [&](uint32_t k) {
+    for (; k < kChainThreads; k = (k | 31) + 1)
+      if (const uint32_t m = sh.valid[k >> 5] >> (k & 31)) return k + __ffs(m) - 1;
+    return kChainThreads;
+  };
+  auto start = [&](uint32_t k) { return (uint32_t)(sh.win[k] >> 32); };
+  uint32_t k = threadIdx.x, end = 0;
+  do {
+    uint32_t e = (uint32_t)sh.win[k];
+    if (e == kLfLong) e = walk(start(k));          // the parallel walk was cut off: finish it here
+    if (e != kLfNone) sh.pick[k] = end = e;        // (else no match from that start after all)
+    k = next_valid(k + 1);
+    for (uint32_t tries = 0; k < kChainThreads && start(k) < end; ++tries) {
+      if (tries < 4) {
+        k = next_valid(k + 1);
+        continue;
+      }
+      uint32_t hi = kChainThreads;  // many candidates inside the match: bisection
+      while (k < hi) {
+        const uint32_t m = (k + hi) >> 1;
+        if (start(m) < end) k = m + 1; else hi = m;
+      }
+      k = next_valid(k);
+    }
+  } while (k < kChainThreads && !((sh.head[k >> 5] >> (k & 31)) & 1u));
+  if (k >= kChainThreads) sh.end = end;
+}
+
+// Returns the end of the last pick (at least `last_end`).
+__device__ uint64_t chain_list(const DevTables& t, const ScanPtrs& p, uint32_t r, const unsigned long long* list,
+                               uint32_t n, uint64_t last_end, uint64_t limit, ChainShared& sh) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, pid = t.pid[r];
+  // a window's candidates are loaded while the one before is decided
+  const unsigned long long none = ~0ull;  // (end kLfNone)
+  unsigned long long next = tid < n ? list[tid] : none;
+  for (uint32_t j0 = 0; j0 < n; j0 += kChainThreads) {
     const unsigned long long c = next;
-    next = j0 + 32 + lane < n ? list[j0 + 32 + lane] : none;
-    const uint32_t s = (uint32_t)(c >> 32);
-    uint32_t e = (uint32_t)c;
-    const bool past = in && (uint64_t)s >= limit;
-    bool picked = false;
-    const bool valid = in && e != kLfNone && (uint64_t)s >= last_end && !past;
-    // ends of the valid candidates before this lane's
-    uint32_t before = valid && e != kLfLong ? e : 0u;
+    next = j0 + kChainThreads + tid < n ? list[j0 + kChainThreads + tid] : none;
+    const uint32_t s = (uint32_t)(c >> 32), e = (uint32_t)c;
+    const bool valid = e != kLfNone && (uint64_t)s >= last_end && (uint64_t)s < limit;
+    // the largest end of the valid candidates before (kLfLong: beyond any start)
+    uint32_t upto = valid ? e : 0u;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, before, d);
-      if (lane >= (uint32_t)d) before = max(before, y);
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, upto, d);
+      if (lane >= (uint32_t)d) upto = max(upto, y);
     }
-    const uint32_t upto = before;
-    before = __shfl_up_sync(0xFFFFFFFFu, upto, 1);
+    sh.win[tid] = c;
+    sh.pick[tid] = kLfNone;
+    const unsigned vm = __ballot_sync(0xFFFFFFFFu, valid);
+    if (lane == 31) {
+      sh.most[warp] = upto;
+      sh.valid[warp] = vm;
+    }
+    if (tid == 0) sh.end = 0;
+    uint32_t before = __shfl_up_sync(0xFFFFFFFFu, upto, 1);
     if (lane == 0) before = 0;
-    if (!__any_sync(0xFFFFFFFFu, valid && (s < before || e == kLfLong))) {
-      picked = valid;
-      const uint32_t top = __shfl_sync(0xFFFFFFFFu, upto, 31);
-      last_end = max(last_end, (uint64_t)top);
-    } else {
-      while (true) {
-        const bool ok = in && e != kLfNone && (uint64_t)s >= last_end && !past;
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, ok);
-        if (!m) break;
-        const int k = __ffs(m) - 1;
-        uint32_t ek = __shfl_sync(0xFFFFFFFFu, e, k);
-        if (ek == kLfLong) {  // the parallel walk was cut off: finish it here
-          if ((int)lane == k) e = lf_walk(t, p, r, s, ~0ull);
-          ek = __shfl_sync(0xFFFFFFFFu, e, k);
-          if (ek == kLfNone) continue;  // no match from that start after all
-        }
-        picked |= (int)lane == k;
-        last_end = ek;
-      }
+    __syncthreads();
+    uint32_t all = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kChainWarps; ++k) {
+      const uint32_t m = sh.most[k];
+      if (k < warp) before = max(before, m);
+      all = max(all, m);
     }
-    if (in) reinterpret_cast<uint32_t*>(list + j0 + lane)[0] = picked ? e : kLfNone;
+    // the usual window: no valid candidate overlaps another, all are picked
+    const bool head = valid && s >= before;
+    const bool apart = __syncthreads_and(!valid || (head && e != kLfLong));
+    uint32_t ek = valid ? e : kLfNone;
+    const uint32_t* picked = sh.valid;
+    if (apart) {
+      last_end = max(last_end, (uint64_t)all);
+    } else {
+      const unsigned hm = __ballot_sync(0xFFFFFFFFu, head);
+      if (lane == 0) sh.head[warp] = hm;
+      __syncthreads();
+      if (head) decide(sh, [&](uint32_t s) { return lf_walk(t, p, r, s, ~0ull); });
+      __syncthreads();
+      last_end = max(last_end, (uint64_t)sh.end);
+      ek = sh.pick[tid];
+      const unsigned pm = __ballot_sync(0xFFFFFFFFu, ek != kLfNone);
+      if (lane == 0) sh.picked[warp] = pm;
+      picked = sh.picked;
+      __syncthreads();
+    }
+    uint32_t sum = 0, below = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kChainWarps; ++k) {
+      if (k == warp) below = sum;
+      sum += __popc(picked[k]);
+    }
+    if (tid == 0) sh.first = sum ? atomicAdd(p.out_counter, (unsigned long long)sum) : 0;
+    __syncthreads();
+    const unsigned long long at = sh.first + below + __popc(picked[warp] & ((1u << lane) - 1u));
+    if (ek != kLfNone && at < p.out_cap) p.out[at] = ws_match{pid, s, ek};
+    __syncthreads();  // (sh, before the next window)
   }
   return last_end;
 }
@@ -1073,106 +1160,45 @@ __device__ __forceinline__ uint64_t chain_limit(const ScanPtrs& p) {
   return p.cursor64 ? p.frontier - p.base : ~0ull;
 }
 
-// The picks of a list to the output: by `width` threads (a warp or a block,
-// thread i of them), one reservation per `width` candidates.
-__device__ __forceinline__ void report_window(const ScanPtrs& p, uint32_t pid, unsigned long long c, bool picked,
-                                              unsigned long long at) {
-  if (picked && at < p.out_cap) p.out[at] = ws_match{pid, (uint32_t)(c >> 32), (uint32_t)c};
-}
-
-// A warp per regex.
-__global__ void k_chain_kernel(DevTables t, ScanPtrs p, unsigned long long* need) {
+// A block per regex.
+__global__ void __launch_bounds__(kChainThreads) k_chain_kernel(DevTables t, ScanPtrs p, uint32_t n_regex,
+                                                                unsigned long long* need) {
+  __shared__ ChainShared sh;
   pdl_begin();
   if (finalize(p, need)) return;
-  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (r >= t.n_regex) return;  // whole warps exit together
-  unsigned long long* list = p.pair + p.offs[r];
-  const uint32_t n = p.offs[r + 1] - p.offs[r], pid = t.pid[r];
-  const uint64_t last_end = chain_list(t, p, r, list, n, chain_start(p, r), chain_limit(p), lane);
-  for (uint32_t j0 = 0; j0 < n; j0 += 32) {  // (every lane wrote its own candidates)
-    const unsigned long long c = j0 + lane < n ? list[j0 + lane] : kLfNone;
-    const bool picked = (uint32_t)c != kLfNone;
-    const unsigned pm = __ballot_sync(0xFFFFFFFFu, picked);
-    if (!pm) continue;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(p.out_counter, (unsigned long long)__popc(pm));
-    base = __shfl_sync(0xFFFFFFFFu, base, 0);
-    report_window(p, pid, c, picked, base + __popc(pm & ((1u << lane) - 1u)));
+  for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
+    const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
+    const uint64_t end = chain_list(t, p, r, p.pair + a, n, chain_start(p, r), chain_limit(p), sh);
+    if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + end, p.frontier);
   }
-  if (p.cursor64 && lane == 0) p.cursor64[r] = max(p.base + last_end, p.frontier);
 }
 
 // Sort, missing ends and chain of a regex by one block, in shared memory for up
 // to kSortTile candidates: the resolution of scans whose candidates came from
 // prefixes, ends known (three kernels and a pass through global memory between
-// each took 8 us more on small lists).  A list in which no candidate overlaps
-// the next needs no chain: all of it is reported at once, with one reservation
-// per block-width of candidates (a reservation per 32, each waiting for the one
-// before, took 14 of 23 us on 400 candidates a regex).
-__global__ void __launch_bounds__(256) k_resolve_kernel(DevTables t, ScanPtrs p, uint32_t n_regex,
-                                                        unsigned long long* need) {
+// each took 8 us more on small lists).
+__global__ void __launch_bounds__(kChainThreads) k_resolve_kernel(DevTables t, ScanPtrs p, uint32_t n_regex,
+                                                                  unsigned long long* need) {
   __shared__ unsigned long long buf[kSortTile];
-  __shared__ uint32_t wcount[8];
-  __shared__ unsigned long long first;
-  __shared__ uint64_t chain_end;
+  __shared__ ChainShared sh;
   pdl_begin();
   if (finalize(p, need)) return;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint64_t limit = chain_limit(p);
   for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
     const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
-    const uint64_t from = chain_start(p, r);
-    if (n == 0) {
-      if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + from, p.frontier);
-      continue;
-    }
     unsigned long long* list = p.pair + a;
     if (n > kSortTile) {
-      sort_list(buf, list, p.pair2 + a, n);
-    } else {
+      for (uint32_t k = 0; k * kSortTile < n; ++k) sort_tile(buf, list, n, k);
+      merge_tiles(list, p.pair2 + a, n);
+    } else if (n) {
       sort_into(buf, list, n);
       list = buf;
     }
     for (uint32_t j = threadIdx.x; j < n; j += blockDim.x)
       if ((uint32_t)list[j] == kLfTodo) reinterpret_cast<uint32_t*>(list + j)[0] = list_end(t, p, r, list, j);
     __syncthreads();
-    bool apart = true;
-    for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
-      const unsigned long long c = list[j];
-      const uint32_t s = (uint32_t)(c >> 32), e = (uint32_t)c;
-      apart &= e < kLfTodo && (uint64_t)s >= from && (uint64_t)s < limit &&
-               (j + 1 == n || (uint32_t)(list[j + 1] >> 32) >= e);
-    }
-    if (!__syncthreads_and(apart)) {
-      if (warp == 0) {
-        const uint64_t end = chain_list(t, p, r, list, n, from, limit, lane);
-        if (lane == 0) chain_end = end;
-      }
-    } else if (threadIdx.x == 0) {
-      chain_end = max(from, (uint64_t)(uint32_t)list[n - 1]);
-    }
-    __syncthreads();
-    if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + chain_end, p.frontier);
-    for (uint32_t j0 = 0; j0 < n; j0 += blockDim.x) {
-      const uint32_t j = j0 + threadIdx.x;
-      const unsigned long long c = j < n ? list[j] : kLfNone;
-      const bool picked = (uint32_t)c != kLfNone;
-      const unsigned pm = __ballot_sync(0xFFFFFFFFu, picked);
-      if (lane == 0) wcount[warp] = __popc(pm);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        uint32_t sum = 0;
-        for (uint32_t k = 0; k < blockDim.x >> 5; ++k) {
-          const uint32_t x = wcount[k];
-          wcount[k] = sum;
-          sum += x;
-        }
-        first = sum ? atomicAdd(p.out_counter, (unsigned long long)sum) : 0;
-      }
-      __syncthreads();
-      report_window(p, t.pid[r], c, picked, first + wcount[warp] + __popc(pm & ((1u << lane) - 1u)));
-      __syncthreads();  // (wcount, first; and buf before the next regex)
-    }
+    const uint64_t end = chain_list(t, p, r, list, n, chain_start(p, r), chain_limit(p), sh);
+    if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + end, p.frontier);
+    __syncthreads();  // (buf, before the next regex)
   }
 }
 
@@ -1952,12 +1978,14 @@ uint32_t regex_finish(RegexPlan& P, RegexScan& rs, const RegexLaunch& l, cudaStr
   launch_pdl(k_scatter_kernel, hg, 256, osmem, st, p, P.n_regex);
   launches += 1;
   if (rs.prefixes && t.n_walk == 0 && t.n_ctx_walk == P.n_spec) {
-    launch_pdl(k_resolve_kernel, (unsigned)std::min<uint32_t>(P.n_regex, 4096), 256, 0, st, t, p, P.n_regex, l.need);
+    launch_pdl(k_resolve_kernel, (unsigned)std::min<uint32_t>(P.n_regex, 4096), kChainThreads, 0, st, t, p, P.n_regex, l.need);
     launches += 1;
   } else {
-    launch_pdl(k_sort_kernel, (unsigned)std::min<uint32_t>(P.n_regex, 4096), 512, 0, st, p, P.n_regex);
+    const uint32_t rows = std::min<uint32_t>(P.n_regex, 4096);
+    // (a set of few regexes may have long lists: enough blocks to fill the chip)
+    launch_pdl(k_sort_kernel, dim3(rows, std::max(1u, 4u * sm_count / rows)), 512, 0, st, p, P.n_regex);
     launch_pdl(k_lf_kernel, sm_count * 8, 128, osmem, st, t, p, P.n_regex);
-    launch_pdl(k_chain_kernel, (P.n_regex + 3) / 4, 128, 0, st, t, p, l.need);  // a warp per regex
+    launch_pdl(k_chain_kernel, rows, kChainThreads, 0, st, t, p, P.n_regex, l.need);
     launches += 3;
   }
   check_cuda(cudaGetLastError(), "resolution kernels");
