@@ -130,7 +130,7 @@ double gram_coverage(const std::vector<FilterString>& strings, uint32_t P, uint3
 void build_gram_tables(const std::vector<FilterString>& strings, LiteralPlan& plan) {
   const uint32_t P = plan.period, G = plan.gram_len;
   struct Gram {
-    uint32_t hash, key;
+    uint32_t word, bit[2], key;
     uint8_t phase;
   };
   std::vector<Gram> grams;
@@ -138,19 +138,18 @@ void build_gram_tables(const std::vector<FilterString>& strings, LiteralPlan& pl
     for (uint32_t k = 0; k < P; ++k) {
       uint32_t g[4] = {0, 0, 0, 0};
       std::memcpy(g, f.p + k, G);
-      grams.push_back({gram_hash32(g[0], g[1], g[2], g[3], (int)G), phase_key(g[0], g[1], g[2], g[3], (int)G),
-                       (uint8_t)(1u << (P - 1 - k))});
+      grams.push_back({gram_word(g[0], g[1], g[2], g[3], (int)G),
+                       {gram_bit(g[0], g[1], g[2], (int)G, 0), gram_bit(g[0], g[1], g[2], (int)G, 1)},
+                       phase_key(g[0], g[1], g[2], g[3], (int)G), (uint8_t)(1u << (P - 1 - k))});
     }
   uint32_t bits = 0;
   while (bits < 25 && ((size_t)1 << bits) < grams.size()) ++bits;
   plan.gram_bits = grams.size() >= 8192 ? 2 : 1;
   plan.gram_word_bits = std::min<uint32_t>(std::max<uint32_t>(bits + 5, 10), kGramWords);
   std::vector<uint32_t> words((size_t)1 << plan.gram_word_bits, 0u);
-  const uint32_t wb = plan.gram_word_bits;
-  for (const Gram& g : grams) {
-    words[g.hash >> (32 - wb)] |= 1u << ((g.hash >> (27 - wb)) & 31u);
-    if (plan.gram_bits == 2) words[g.hash >> (32 - wb)] |= 1u << ((g.hash >> (22 - wb)) & 31u);
-  }
+  for (const Gram& g : grams)
+    for (uint32_t b = 0; b < plan.gram_bits; ++b)
+      words[(g.word & gram_mask(plan.gram_word_bits)) >> 2] |= 1u << (g.bit[b] & 31u);
   plan.d_gram.upload(words.data(), words.size() * 4);
   plan.phase_bits = std::min<uint32_t>(std::max<uint32_t>(bits + 6, 12), kBigBits);
   std::vector<uint8_t> phase((size_t)1 << plan.phase_bits, 0);

@@ -83,6 +83,7 @@ struct LitArgs {
   const uint8_t* phase;
   uint32_t phase_shift;
   uint32_t slot_chunk;       // survivor slots a warp reserves at a time
+  uint32_t two;              // 2, unknown to the compiler: a sum of bits stays on the multiply pipe
   uint32_t fold;             // ASCII case-insensitive: input bytes A-Z read as a-z
 };
 
@@ -663,27 +664,31 @@ __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(cons
 //     base - OFF + P * j (base the offset of its 16 bytes), all inside its own
 //     bytes and the few bytes before them, which come from the lane below;
 //   - stage 1 is a bitmap in shared memory (BITS = 1), or for crowded sets a
-//     blocked Bloom filter of two bits of one word per gram (BITS = 2), word
-//     and bits all from one multiplicative hash: the second bit costs two
-//     instructions and no second load, and squares the pass rate (10,000
-//     literals: 0.6% of the grams pass where one bit let 3.4% pass);
-//   - the warp takes kGramBits / NG vectors of 512 coalesced bytes in a row,
-//     one pass bit per gram in a 32-bit mask, and looks at the mask once: the
-//     passing grams go into the warp's queue in shared memory;
+//     blocked Bloom filter of two bits of one word per gram (BITS = 2): the second
+//     bit costs no second load and squares the pass rate (10,000 literals: 0.6% of
+//     the grams pass where one bit let 3.4% pass).  Word and bits come from dot
+//     products of the gram (gram_word, gram_bit);
+//   - the warp takes kGramBits / NG vectors of 512 coalesced bytes in a row (a
+//     run), one pass bit per gram in a 32-bit mask, and looks at the mask once:
+//     the passing grams go into the warp's queue in shared memory;
 //   - with 32 or more queued, every lane takes one: its phase bits (which
 //     offsets of a literal have this gram, a byte of a table in L2) give the
 //     start positions, which are appended to the warp's reserved slots of the
 //     list, one global atomic per slot_chunk slots.
 // One CTA of 1,024 threads per SM, four 512-byte loads in flight per warp.
-// What bounds it: the shared-memory lookups (a warp's 32 random words meet in
-// 3.4 wavefronts of the data pipe: 0.86 of it busy with P = 2, 0.91 with P = 1)
-// and, for P = 4, instruction issue (70 warp instructions per 512 bytes, the
-// data pipe 0.71 busy).  Measured, us per 256 MiB: 10,000 literals (P = 4) 57,
-// where the kernel before it (one bit, a vote and an append per 1 KiB step, its
-// candidates' L2 loads in the main loop) took 65; 500 literals of 5 bytes and
-// more (P = 2) 78, of 4 (P = 1) 134; 20,000 k-mers (G = 16) 81 against 164 for
-// the compacting kernel; 1,000 caseless literals of 3 and more over 97 MiB 69
-// against 184.
+// What bounds it: with few passing grams HBM for P = 4 (2,100 literals over 1 GiB
+// 170 us a scan, a copy takes 164); each passing gram costs a warp 5 to 6 issue
+// slots (10,000 literals 182, 20,000 216), and 16-byte grams three shuffles a
+// vector (2,100 k-mers 197, 20,000 259).  P = 2 and P = 1 are bound by the shared
+// memory lookups: a warp's 32 random words meet in 3.4 wavefronts of the data
+// pipe, which is 0.88 busy with P = 2.  Measured, us per 256 MiB: 10,000 literals
+// (P = 4) 57 -> 52, where the kernel before it (one bit, a vote and an append per
+// 1 KiB step, its candidates' L2 loads in the main loop) took 65; 500 literals of
+// 5 bytes and more (P = 2) 73; 20,000 k-mers (G = 16) 81 -> 74 against 164 for the
+// compacting kernel; 1,000 caseless literals of 3 and more over 97 MiB 69 -> 63
+// against 184.  (The arrows: hashes by multiplication and shifts, which kept the
+// integer pipe 0.8 busy, and positions worked out when a gram was queued, 15 issue
+// slots a passing gram, to the present ones.)
 constexpr int kGramThreads = 1024;
 constexpr uint32_t kGramWarps = kGramThreads / 32;
 // u32 positions per warp.  (512 of them left less L1 for the flush, which reads
@@ -706,35 +711,49 @@ __device__ __forceinline__ void lean_holes(const LitArgs& a, const LeanSlots& r,
 }
 
 // Key of the phase table for the gram at position at: a hash independent of
-// stage 1's, so that what stage 1 lets through by chance does not pass again.
+// stage 1's, so that what stage 1 lets through by chance does not pass again.  No
+// word is read that holds none of the gram's bytes.  EDGE: the last one may reach
+// past the input.
+template <bool EDGE>
 __device__ __forceinline__ uint32_t phase_key_at(const LitArgs& a, uint32_t at, int G) {
   const uint32_t len = (uint32_t)a.len, w0 = at & ~3u, sh = (at & 3) * 8;
-  if (G == 16) {  // aligned
-    return phase_key(input_word(a, len, w0), input_word(a, len, w0 + 4), input_word(a, len, w0 + 8),
-                     input_word(a, len, w0 + 12), 16);
-  }
-  const uint32_t g = __funnelshift_r(input_word(a, len, w0), sh ? input_word(a, len, w0 + 4) : 0u, sh);
-  return phase_key(g, 0, 0, 0, G);
+  auto word = [&](uint32_t x) {
+    if (EDGE) return input_word(a, len, x);
+    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(a.data + x));
+    return a.fold ? ascii_fold4(w) : w;
+  };
+  if (G == 16) return phase_key(word(w0), word(w0 + 4), word(w0 + 8), word(w0 + 12), 16);  // aligned
+  return phase_key(__funnelshift_r(word(w0), sh + 8 * G > 32 ? word(w0 + 4) : 0u, sh), 0, 0, 0, G);
+}
+
+// Position of a queued gram: bit i of lane l's mask in run r is r * 1024 + l * 32
+// + i (a run is 32 grams of every lane, gram i of vector i / NG).
+template <int P, int G>
+__device__ __forceinline__ uint32_t gram_at(uint32_t code) {
+  constexpr uint32_t NG = 16 / P, i_bits = kGramBits - 1;
+  return (code >> 10) * (1024 * P) + ((code & i_bits) / NG) * 512 + ((code >> 5) & 31) * 16 + (code % NG) * P -
+         gram_off<P, G>();
 }
 
 // Takes the queued grams [0, n), 32 at a time: phase bits, start positions,
-// append.  True when the list was full before: the verify kernel then looks at
-// every gram of the input again, and this kernel has nothing more to add.
-template <int P, int G>
+// append.  EDGE: words may lie past the input.  True when the list was full
+// before: the verify kernel then looks at every gram of the input again, and this
+// kernel has nothing more to add.
+template <int P, int G, bool EDGE>
 __device__ __forceinline__ bool gram_flush(const LitArgs& a, const uint32_t* queue, uint32_t n, LeanSlots& r,
                                            uint32_t lane) {
   const uint32_t len = (uint32_t)a.len;
   for (uint32_t k0 = 0; k0 < n; k0 += 32) {
     uint32_t at = 0, bits = 0;
-    if (k0 + lane < n) {
-      at = queue[k0 + lane];
-      bits = (uint32_t)__ldg(a.phase + (phase_key_at(a, at, G) >> a.phase_shift));
-#pragma unroll
-      for (int k = 0; k < P; ++k)  // bit P - 1 - k: the literal starts k bytes before the gram
-        if (at < (uint32_t)k || at - k >= len) bits &= ~(1u << (P - 1 - k));
+    if (!EDGE || k0 + lane < n) {
+      at = gram_at<P, G>(queue[k0 + lane]);
+      bits = (uint32_t)__ldg(a.phase + (phase_key_at<EDGE>(a, at, G) >> a.phase_shift));
     }
+    if (__ballot_sync(0xFFFFFFFFu, bits != 0) == 0) continue;  // the usual group
+#pragma unroll
+    for (int k = 0; k < P; ++k)  // bit P - 1 - k: the literal starts k bytes before the gram
+      if (at < (uint32_t)k || at - k >= len) bits &= ~(1u << (P - 1 - k));
     const uint32_t cnt = __popc(bits);
-    if (__ballot_sync(0xFFFFFFFFu, cnt != 0) == 0) continue;
     uint32_t incl = cnt;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -763,46 +782,41 @@ __device__ __forceinline__ bool gram_flush(const LitArgs& a, const uint32_t* que
   return false;
 }
 
-// Queues the passing grams of a run of vectors (bit i of `pass`: gram i % NG of
-// vector i / NG) and flushes whole groups of 32; kListFull when the list was.
+// Queues the passing grams of a run (bit 31 - i of `pass`: the lane's gram i), the
+// run's codes from `code` on, and flushes whole groups of 32; kListFull when the
+// list was.
 constexpr uint32_t kListFull = 0xFFFFFFFFu;
 
-template <int P, int G>
+template <int P, int G, bool EDGE>
 __device__ __forceinline__ uint32_t gram_queue(const LitArgs& a, uint32_t* queue, uint32_t queued, uint32_t pass,
-                                               uint32_t base, LeanSlots& slots, uint32_t lane) {
-  constexpr uint32_t NG = 16 / P;
-  for (uint32_t ball = __ballot_sync(0xFFFFFFFFu, pass != 0); ball; ball = __ballot_sync(0xFFFFFFFFu, pass != 0)) {
+                                               uint32_t code, LeanSlots& slots, uint32_t lane) {
+  uint32_t ball = __ballot_sync(0xFFFFFFFFu, pass != 0);
+  while (ball) {
     if (pass) {  // one gram of every lane that has one left
-      const uint32_t i = __ffs(pass) - 1;
-      pass &= pass - 1;
-      queue[queued + __popc(ball & ((1u << lane) - 1u))] = base + (i / NG) * 512 + (i % NG) * P;
+      const uint32_t i = __clz(pass);
+      pass ^= 0x80000000u >> i;
+      queue[queued + __popc(ball & ((1u << lane) - 1u))] = code + i;
     }
     queued += __popc(ball);
-    if (queued > kGramQueue - 32 || (queued >= 32 && !__any_sync(0xFFFFFFFFu, pass != 0))) {
+    ball = __ballot_sync(0xFFFFFFFFu, pass != 0);
+    if (queued >= (ball ? kGramQueue - 31 : 32)) {
       __syncwarp();
       const uint32_t whole = queued & ~31u, left = queued & 31u;
-      if (gram_flush<P, G>(a, queue, whole, slots, lane)) return kListFull;
+      if (gram_flush<P, G, EDGE>(a, queue, whole, slots, lane)) return kListFull;
       const uint32_t keep = lane < left ? queue[whole + lane] : 0u;
       __syncwarp();
       if (lane < left) queue[lane] = keep;
       queued = left;
     }
   }
-  __syncwarp();
   return queued;
 }
 
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-  uint32_t x;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(addr));
-  return x;
-}
-
-// Pass bits of one vector: gram j shifts into the top of `pass`.  w[k] is word
+// Pass bits of one vector: gram j shifts into the bottom of `pass`.  w[k] is word
 // k - NPRE of the lane's bytes; `below` holds the words before the vector for
 // lane 0 and receives those of the next one.
 template <int P, int G, int BITS, int NPRE>
-__device__ __forceinline__ uint32_t gram_test(uint32_t filt, uint32_t wsh, uint32_t lane, const uint4& v,
+__device__ __forceinline__ uint32_t gram_test(const uint32_t* filt, uint32_t mask, uint32_t two, uint32_t lane, const uint4& v,
                                               uint32_t (&below)[NPRE ? NPRE : 1], uint32_t pass) {
   constexpr int NG = 16 / P, OFF = gram_off<P, G>();
   uint32_t w[NPRE + 4];
@@ -817,24 +831,23 @@ __device__ __forceinline__ uint32_t gram_test(uint32_t filt, uint32_t wsh, uint3
     w[NPRE - 1 - k] = lane == 0 ? below[k] : x;
     below[k] = x;
   }
-  uint32_t h[NG], x[NG];
+  uint32_t g[NG], x[NG];
 #pragma unroll
   for (int j = 0; j < NG; ++j) {
-    const int o = P * j - OFF + 4 * NPRE;  // byte offset of gram j in w
-    if (G == 16) {
-      h[j] = gram_hash32(w[o / 4], w[o / 4 + 1], w[o / 4 + 2], w[o / 4 + 3], 16);
-    } else {
-      const uint32_t g =
-          (o & 3) ? __funnelshift_r(w[o / 4], w[o / 4 + 1 < NPRE + 4 ? o / 4 + 1 : o / 4], 8 * (o & 3)) : w[o / 4];
-      h[j] = gram_hash32(g, 0, 0, 0, G);
-    }
-    x[j] = lds32(filt + ((h[j] >> (wsh - 2)) & ~3u));
+    const int o = P * j - OFF + 4 * NPRE, i = o / 4;  // byte offset of gram j in w
+    g[j] = (o & 3) ? __funnelshift_r(w[i], w[i + 1 < NPRE + 4 ? i + 1 : i], 8 * (o & 3)) : w[i];
+    const uint32_t at = G == 16 ? gram_word(w[i], w[i + 1], w[i + 2], w[i + 3], G) : gram_word(g[j], 0, 0, 0, G);
+    x[j] = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(filt) + (at & mask));
   }
 #pragma unroll
   for (int j = 0; j < NG; ++j) {
-    uint32_t bit = __funnelshift_r(x[j], x[j], h[j] >> (wsh - 5));
-    if (BITS == 2) bit &= __funnelshift_r(x[j], x[j], h[j] >> (wsh - 10));
-    pass = __funnelshift_r(pass, bit, 1);
+    const int i = (P * j - OFF + 4 * NPRE) / 4;
+    auto bit_of = [&](int k) {
+      return __funnelshift_r(x[j], x[j], gram_bit(g[j], G == 16 ? w[i + 1] : 0, G == 16 ? w[i + 2] : 0, G, k));
+    };
+    uint32_t bit = bit_of(0);
+    if (BITS == 2) bit &= bit_of(1);
+    pass = pass * two + (bit & 1u);
   }
   return pass;
 }
@@ -844,6 +857,7 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
   constexpr int NG = 16 / P, OFF = gram_off<P, G>(), NPRE = (OFF + 3) / 4;
   constexpr uint32_t VECS = kGramBits / NG;                // 512-byte vectors of a run
   constexpr uint32_t RING = VECS < 4 ? VECS : 4;           // vectors loaded ahead
+  const bool fold = a.fold != 0;
   extern __shared__ __align__(16) uint32_t gsm[];
   uint32_t* queue = gsm + (1u << a.gram_word_bits) + (threadIdx.x >> 5) * kGramQueue;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -856,13 +870,12 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
   // (the tables above are no kernel's output; the verify kernel is not let in
   // early, its waiting blocks cost the last runs 1%)
   pdl_wait();
-  const uint32_t filt = (uint32_t)__cvta_generic_to_shared(gsm), wsh = 32 - a.gram_word_bits;
+  const uint32_t mask = gram_mask(a.gram_word_bits);
   const uint32_t len = (uint32_t)a.len;
   const uint32_t nvec = (uint32_t)((a.len + 15) >> 4);
   const uint32_t runs = len / (VECS * 512);                // runs entirely inside the input
   // neighbouring runs go to different SMs, so that a small input spreads out
   const uint32_t first = warp * gridDim.x + blockIdx.x, nw = gridDim.x * kGramWarps;
-  const bool fold = a.fold != 0;
   LeanSlots slots;
   uint32_t queued = 0;
   uint32_t below[NPRE ? NPRE : 1];
@@ -899,13 +912,11 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
       if (i + RING < VECS) ring[i % RING] = __ldg(p + (i + RING) * 32);
       else if (more) ring[i % RING] = __ldg(pn + (i + RING - VECS) * 32);
       if (fold) v = fold16(v);
-      pass = gram_test<P, G, BITS, NPRE>(filt, wsh, lane, v, below, pass);
+      pass = gram_test<P, G, BITS, NPRE>(gsm, mask, a.two, lane, v, below, pass);
     }
-    if (OFF && r == 0 && lane == 0) pass &= ~((1u << ((OFF + P - 1) / P)) - 1u);  // grams that begin before the input
-    if (__any_sync(0xFFFFFFFFu, pass != 0)) {
-      queued = gram_queue<P, G>(a, queue, queued, pass, r * (VECS * 512) + lane * 16 - OFF, slots, lane);
-      if (queued == kListFull) return;
-    }
+    if (OFF && r == 0 && lane == 0) pass &= 0xFFFFFFFFu >> ((OFF + P - 1) / P);  // grams that begin before the input
+    queued = gram_queue<P, G, false>(a, queue, queued, pass, r * 1024 + lane * 32, slots, lane);
+    if (queued == kListFull) return;
   }
   // the vectors after the last whole run, one warp each
   const uint32_t v0 = runs * VECS, nv = (nvec + 31) >> 5;
@@ -917,12 +928,13 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
       v = fold16(v);
       folded(below);
     }
-    uint32_t pass = gram_test<P, G, BITS, NPRE>(filt, wsh, lane, v, below, 0u) >> (32 - NG);
-    if (OFF && b == 0 && lane == 0) pass &= ~((1u << ((OFF + P - 1) / P)) - 1u);
-    queued = gram_queue<P, G>(a, queue, queued, pass, b * 512 + lane * 16 - OFF, slots, lane);
+    uint32_t pass = gram_test<P, G, BITS, NPRE>(gsm, mask, a.two, lane, v, below, 0u) << (32 - NG);
+    if (OFF && b == 0 && lane == 0) pass &= 0xFFFFFFFFu >> ((OFF + P - 1) / P);
+    queued = gram_queue<P, G, true>(a, queue, queued, pass, (b / VECS) * 1024 + lane * 32 + (b % VECS) * NG, slots, lane);
     if (queued == kListFull) return;
   }
-  if (queued) gram_flush<P, G>(a, queue, queued, slots, lane);
+  __syncwarp();
+  if (queued) gram_flush<P, G, true>(a, queue, queued, slots, lane);
   lean_holes(a, slots, lane);
 }
 
@@ -960,30 +972,26 @@ __device__ __forceinline__ void verify_prefixes(const LitArgs& a, const DevTable
 
 // Stage 1 of the grams that start in the 16 bytes of vector v, by tables in
 // global memory: bit j of the result is the gram at byte j.
+template <int G>
 __device__ __forceinline__ uint32_t grams_pass(const LitArgs& a, uint32_t v) {
-  const uint32_t len = (uint32_t)a.len, at = v * 16, wsh = 32 - a.gram_word_bits;
+  const uint32_t len = (uint32_t)a.len, at = v * 16, mask = gram_mask(a.gram_word_bits);
   uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   const uint4 x = load_vec(a.data, a.len, v);
   w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
 #pragma unroll
   for (uint32_t k = 0; k < 4; ++k) {
     if (a.fold) w[k] = ascii_fold4(w[k]);
-    if ((k == 0 || a.gram_len == 16) && at + 16 + 4 * k < len) w[4 + k] = input_word(a, len, at + 16 + 4 * k);
+    if ((k == 0 || G == 16) && at + 16 + 4 * k < len) w[4 + k] = input_word(a, len, at + 16 + 4 * k);
   }
   uint32_t pass = 0;
 #pragma unroll
   for (uint32_t j = 0; j < 16; ++j) {
-    if (j & (a.period - 1)) continue;
-    uint32_t h;
-    if (a.gram_len == 16) {
-      const uint32_t i = j >> 2;
-      h = gram_hash32(w[i], w[i + 1], w[i + 2], w[i + 3], 16);
-    } else {
-      h = __funnelshift_r(w[j >> 2], w[(j >> 2) + 1], 8 * (j & 3)) * (a.gram_len == 3 ? gram_hash32(1, 0, 0, 0, 3) : gram_hash32(1, 0, 0, 0, 4));
-    }
-    const uint32_t x = __ldg(a.gram_bloom + (h >> wsh));
-    uint32_t bit = x >> ((h >> (wsh - 5)) & 31u);
-    if (a.gram_bits == 2) bit &= x >> ((h >> (wsh - 10)) & 31u);
+    if ((G == 16 && (j & 3)) || (j & (a.period - 1))) continue;
+    const uint32_t i = j >> 2, g = G == 16 ? w[i] : __funnelshift_r(w[i], w[i + 1], 8 * (j & 3));
+    const uint32_t word = G == 16 ? gram_word(g, w[i + 1], w[i + 2], w[i + 3], G) : gram_word(g, 0, 0, 0, G);
+    const uint32_t x = __ldg(a.gram_bloom + ((word & mask) >> 2));
+    uint32_t bit = __funnelshift_r(x, x, gram_bit(g, w[i + 1], w[i + 2], G, 0));
+    if (a.gram_bits == 2) bit &= __funnelshift_r(x, x, gram_bit(g, w[i + 1], w[i + 2], G, 1));
     pass |= (bit & 1u) << j;
   }
   const uint32_t left = len - at;
@@ -1099,7 +1107,7 @@ __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_con
     auto verify_grams = [&](uint32_t n, bool end) {  // grams[0, n), n <= 32
       if (lane < n) {
         const uint32_t at = grams[lane];
-        uint32_t bits = __ldg(a.phase + (phase_key_at(a, at, (int)a.gram_len) >> a.phase_shift));
+        uint32_t bits = __ldg(a.phase + (phase_key_at<true>(a, at, (int)a.gram_len) >> a.phase_shift));
         for (; bits; bits &= bits - 1) {
           const uint32_t k = a.period - __ffs(bits);  // bit period - 1 - k: the literal starts k bytes before
           if (at >= k && at - k < len) verify_lean(a, at - k, warp_match);
@@ -1121,7 +1129,8 @@ __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_con
     uint32_t queued = 0;
     for (uint64_t v0 = (uint64_t)w * 32; v0 < nvec; v0 += (uint64_t)warps * 32) {
       const uint32_t v = (uint32_t)v0 + lane;
-      uint32_t pass = v < nvec ? grams_pass(a, v) : 0u;
+      uint32_t pass = 0;
+      if (v < nvec) pass = a.gram_len == 16 ? grams_pass<16>(a, v) : a.gram_len == 3 ? grams_pass<3>(a, v) : grams_pass<4>(a, v);
       for (uint32_t ball; (ball = __ballot_sync(0xFFFFFFFFu, pass != 0)) != 0;) {
         if (pass) {  // one gram of every lane that has one left
           grams[queued + __popc(ball & ((1u << lane) - 1u))] = v * 16 + __ffs(pass) - 1;
@@ -1211,6 +1220,7 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   a.gram_bits = plan.gram_kernel ? plan.gram_bits : 0;
   a.phase = plan.d_phase.as<uint8_t>();
   a.phase_shift = 32 - plan.phase_bits;
+  a.two = 2;
   a.fold = plan.fold ? 1 : 0;
   if (!l.cleared) check_cuda(cudaMemsetAsync(a.survivor_count, 0, 8, st), "memset survivors");
   if (l.len > 0xFFFFFFFFull) raise(WS_ERR_INPUT_TOO_LARGE, "literal scan launch beyond 32-bit offsets", 0, l.len,
@@ -1252,11 +1262,11 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   // dominates, keep 32 warps per SM
   if (plan.gram_kernel) {
     const bool two = plan.gram_bits == 2;
-    if (plan.gram_len == 16) two ? run_gram(literal_gram_kernel<4, 16, 2>, 4096) : run_gram(literal_gram_kernel<4, 16, 1>, 4096);
-    else if (plan.gram_len == 3) two ? run_gram(literal_gram_kernel<1, 3, 2>, 1024) : run_gram(literal_gram_kernel<1, 3, 1>, 1024);
-    else if (plan.period == 4) two ? run_gram(literal_gram_kernel<4, 4, 2>, 4096) : run_gram(literal_gram_kernel<4, 4, 1>, 4096);
-    else if (plan.period == 2) two ? run_gram(literal_gram_kernel<2, 4, 2>, 2048) : run_gram(literal_gram_kernel<2, 4, 1>, 2048);
-    else two ? run_gram(literal_gram_kernel<1, 4, 2>, 1024) : run_gram(literal_gram_kernel<1, 4, 1>, 1024);
+    if (plan.gram_len == 16) run_gram(two ? literal_gram_kernel<4, 16, 2> : literal_gram_kernel<4, 16, 1>, 4096);
+    else if (plan.gram_len == 3) run_gram(two ? literal_gram_kernel<1, 3, 2> : literal_gram_kernel<1, 3, 1>, 1024);
+    else if (plan.period == 4) run_gram(two ? literal_gram_kernel<4, 4, 2> : literal_gram_kernel<4, 4, 1>, 4096);
+    else if (plan.period == 2) run_gram(two ? literal_gram_kernel<2, 4, 2> : literal_gram_kernel<2, 4, 1>, 2048);
+    else run_gram(two ? literal_gram_kernel<1, 4, 2> : literal_gram_kernel<1, 4, 1>, 1024);
   } else if (lg && sh && a.big && plan.period == 4 && plan.gram_len == 4) {
     run_big(literal_filter_big_kernel<4, true>);
   } else if (!lg) {
