@@ -1950,6 +1950,7 @@ void regex_begin(RegexPlan& P, const RegexLaunch& l, cudaStream_t st, DeviceBuff
   rs.k_cap = L.k_cap;
   rs.n_q = L.n_q;
   rs.prefixes = prefixes;
+  rs.walk_tables[0] = &P.d_lf, rs.walk_tables[1] = &P.d_cls, rs.walk_tables[2] = &P.d_lfinfo, rs.walk_tables[3] = &P.d_lfx;
   if (prefixes) {
     rs.t.n_walk = P.n_walk;
     rs.t.n_ctx_walk = P.n_ctx_walk;

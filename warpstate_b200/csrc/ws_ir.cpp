@@ -350,7 +350,17 @@ void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan, const std:
   if (t.prefix_meta)
     std::copy(t.prefix_meta, t.prefix_meta + 4 * std::min(t.hash_window_len, HASH_WINDOW), plan.meta.begin());
   plan.d_ranges.upload(t.bucket_ranges, 2 * (size_t)t.n_buckets * 4);
-  plan.d_entries.upload(t.entries, 2 * (size_t)t.n_literals * 4);
+  // entries {hash, literal} with bytes 8..11 of the literal and their mask
+  std::vector<uint32_t> entries(4 * (size_t)t.n_literals, 0u);
+  for (size_t e = 0; e < t.n_literals; ++e) {
+    const uint32_t li = t.entries[2 * e + 1], len = li < t.n_literals ? t.offsets[2 * li + 1] : 0;
+    entries[4 * e] = t.entries[2 * e];
+    entries[4 * e + 1] = li;
+    if (len <= 8) continue;
+    std::memcpy(&entries[4 * e + 2], t.packed_bytes + t.offsets[2 * li] + 8, std::min<uint32_t>(len - 8, 4));
+    std::memset(&entries[4 * e + 3], 0xFF, std::min<uint32_t>(len - 8, 4));
+  }
+  plan.d_entries.upload(entries.data(), entries.size() * 4);
 }
 
 }  // namespace ws

@@ -50,8 +50,6 @@ struct LitArgs {
   uint32_t filter_words;
   uint32_t bits;
   uint32_t period;
-  uint32_t has_long;
-  uint32_t has_short;
   uint32_t parts;            // bit i: prefix length i+1 has literals
   uint32_t bloom_parts;      // bit i: prefix length i+1 is in the prefix Bloom (literals, regex prefixes)
   const uint32_t* short_bits;
@@ -60,7 +58,7 @@ struct LitArgs {
   const uint8_t* lit_bytes;
   uint2 meta[HASH_WINDOW];  // per prefix length: {first bucket, bucket mask} (LiteralPrefilterTable partition)
   const uint2* ranges;
-  const uint2* entries;
+  const uint4* entries;      // {hash, literal, its bytes 8..11, their mask}
   ws_match* out;
   uint64_t cap;
   unsigned long long* counter;
@@ -145,10 +143,12 @@ __device__ __forceinline__ void probe_literals(const LitArgs& a, uint32_t lo, ui
 }
 
 // Compares literals of the probed buckets at s; x0 is the (folded) word at
-// s & ~3.  Literal bytes start 4-aligned in a buffer padded to 16 bytes; four
+// s & ~3, `next` the four bytes from s + 8 on: an entry tells by four more bytes
+// whether its literal is worth looking at (k-mers share their first eight bytes
+// with a quarter of all positions: 20,000 of them over 2 GiB 596 -> 580 us a scan).  Literal bytes start 4-aligned in a buffer padded to 16 bytes; four
 // words of literal and input are read together.
 template <class Sink>
-__device__ __forceinline__ void verify_literals(const LitArgs& a, uint32_t s, uint32_t x0, const Probe& pr, Sink&& sink) {
+__device__ __forceinline__ void verify_literals(const LitArgs& a, uint32_t s, uint32_t x0, uint32_t next, const Probe& pr, Sink&& sink) {
   const uint32_t len = (uint32_t)a.len, rem = len - s, w0 = s & ~3u, sh = (s & 3) * 8;
   uint32_t part = 0, e = 0;  // the next entry: bucket `part`, place e
   while (true) {
@@ -157,8 +157,8 @@ __device__ __forceinline__ void verify_literals(const LitArgs& a, uint32_t s, ui
     for (uint32_t i = 0; i < HASH_WINDOW; ++i) {
       if (i < part || found != 0xFFFFFFFFu) continue;
       for (; e < pr.r[i].y && found == 0xFFFFFFFFu; ++e) {
-        const uint2 ent = __ldg(a.entries + pr.r[i].x + e);
-        if (ent.x == pr.h[i]) found = ent.y;
+        const uint4 ent = __ldg(a.entries + pr.r[i].x + e);
+        if (ent.x == pr.h[i] && !((ent.z ^ next) & ent.w)) found = ent.y;
       }
       part = i;
       if (found == 0xFFFFFFFFu) e = 0;
@@ -216,7 +216,7 @@ __device__ __forceinline__ void verify_lean(const LitArgs& a, uint32_t s, Sink&&
     const uint2 r = __ldg(a.ranges + a.meta[i].x + (h & a.meta[i].y));
 #pragma unroll 1
     for (uint32_t e = 0; e < r.y; ++e) {
-      const uint2 ent = __ldg(a.entries + r.x + e);
+      const uint4 ent = __ldg(a.entries + r.x + e);
       if (ent.x != h) continue;
       const uint4 info = __ldg(a.info + ent.y);  // {offset, len, pattern id, 0}
       if (info.y > rem) continue;
@@ -998,6 +998,24 @@ __device__ __forceinline__ uint32_t grams_pass(const LitArgs& a, uint32_t v) {
   return left < 16 ? pass & ((1u << left) - 1u) : pass;
 }
 
+// Tables of the verify kernel to be brought into L2 at its start: the filter has
+// just streamed the whole input through L2, and a walk or a bucket's chain that
+// finds its tables gone waits for HBM at each of its steps, all walks at the
+// same ones.  The gain is small, the tables having mostly stayed (us a scan: 160
+// regexes over 1 GiB 323.0 -> 321.9, 60 over 200 MiB 94.9 -> 94.1, 10,000 literals
+// over 1 GiB 191.9 -> 191.2), and so is the cost.
+struct WarmDev {
+  const char* p[10];
+  uint32_t lines[10];  // of 128 bytes
+};
+
+__device__ __forceinline__ void warm_tables(const WarmDev& wd) {
+#pragma unroll
+  for (int q = 0; q < 10; ++q)
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < wd.lines[q]; i += gridDim.x * blockDim.x)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(wd.p[q] + (size_t)i * 128));
+}
+
 // Kernel 2.  When the gram kernel's list was full (it then stopped early), every
 // gram of the input is tested again here: a warp takes 16 bytes per lane, queues
 // the grams that pass in shared memory and verifies their literals with all its
@@ -1006,32 +1024,58 @@ __device__ __forceinline__ uint32_t grams_pass(const LitArgs& a, uint32_t v) {
 // among the regex prefixes.  A full list (more than one survivor per 64 bytes)
 // gives the prefix candidates up, like long walks do; the last block then drops
 // the candidates found so far, so that the gated groups start from none.
-constexpr uint32_t kVerifyBuf = 512;
-constexpr uint32_t kDenseBuf = kVerifyBuf / 8;  // matches and grams a warp of the dense pass holds
+//
+// Matches and candidates collect in shared memory, a buffer per warp that is
+// written out with one atomic when half full, and what is left at the end with
+// one per block (an atomic per match on the one counter: 35 us for 65,536 of
+// them).  No barrier before the end: a warp whose walks are long delays no other
+// (with block buffers and a barrier a step, 40,000 items took 40 us here, with
+// these 34).
+constexpr uint32_t kVerifyThreads = 256, kVerifyWarps = kVerifyThreads / 32;
+constexpr uint32_t kVerifyBuf = 64;  // per warp
 
 template <bool RX>
-__global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_constant__ LitArgs a,
+__global__ void __launch_bounds__(kVerifyThreads, 4) literal_verify_kernel(const __grid_constant__ LitArgs a,
                                                              const __grid_constant__ DevTables t,
-                                                             const __grid_constant__ ScanPtrs p, PrefixDev pf) {
+                                                             const __grid_constant__ ScanPtrs p, PrefixDev pf,
+                                                             const __grid_constant__ WarmDev wd) {
+  warm_tables(wd);
   pdl_begin();
-  // Matches and candidates collect in shared memory: one atomic per block and
-  // counter instead of one per match (65,536 on one address took 35 us).
-  __shared__ uint3 mbuf[kVerifyBuf];
-  // (kbuf also holds the dense pass's positions: a full list makes no candidates)
-  __shared__ uint3 kbuf[kVerifyBuf];
-  __shared__ uint32_t held[2];
-  __shared__ unsigned long long first[2];
-  if (threadIdx.x < 2) held[threadIdx.x] = 0;
-  __syncthreads();
+  __shared__ uint3 mbuf[kVerifyWarps][kVerifyBuf];
+  __shared__ uint3 kbuf[kVerifyWarps][kVerifyBuf];  // (or the grams of the dense pass: a full list makes no candidates)
+  __shared__ uint32_t held[2][kVerifyWarps];
+  const uint32_t lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  if (lane < 2) held[lane][wi] = 0;
+  __syncwarp();
   auto match = [&](uint32_t pid, uint32_t s, uint32_t e) {
-    const uint32_t i = atomicAdd(&held[0], 1u);
-    if (i < kVerifyBuf) mbuf[i] = make_uint3(pid, s, e);
+    const uint32_t i = atomicAdd(&held[0][wi], 1u);
+    if (i < kVerifyBuf) mbuf[wi][i] = make_uint3(pid, s, e);
     else report_match(a, pid, s, e);
   };
   auto candidate = [&](uint32_t r, uint32_t s, uint32_t e) {
-    const uint32_t i = atomicAdd(&held[1], 1u);
-    if (i < kVerifyBuf) kbuf[i] = make_uint3(r, s, e);
+    const uint32_t i = atomicAdd(&held[1][wi], 1u);
+    if (i < kVerifyBuf) kbuf[wi][i] = make_uint3(r, s, e);
     else emit_k(p, r, s, e, kEndKnown);
+  };
+  // the warp's first `nm` matches and `nk` candidates to places at and kat
+  auto write_out = [&](uint32_t nm, unsigned long long at, uint32_t nk, unsigned long long kat) {
+    for (uint32_t i = lane; i < nm; i += 32)
+      if (at + i < a.cap) a.out[at + i] = ws_match{mbuf[wi][i].x, mbuf[wi][i].y, mbuf[wi][i].z};
+    for (uint32_t i = lane; RX && i < nk; i += 32)
+      store_k(p, kat + i, kbuf[wi][i].x, kbuf[wi][i].y, kbuf[wi][i].z, kEndKnown);
+  };
+  auto drain = [&]() {  // by the warp, after each step
+    __syncwarp();
+    const uint32_t nm = min(held[0][wi], kVerifyBuf), nk = RX ? min(held[1][wi], kVerifyBuf) : 0u;
+    if (nm > kVerifyBuf / 2 || nk > kVerifyBuf / 2) {
+      unsigned long long at = 0;
+      if (lane == 0 && nm) at = atomicAdd(a.counter, (unsigned long long)nm);
+      if (RX && lane == 1 && nk) at = atomicAdd(&p.ctr[C_K], (unsigned long long)nk);
+      write_out(nm, __shfl_sync(0xFFFFFFFFu, at, 0), nk, __shfl_sync(0xFFFFFFFFu, at, 1));
+      __syncwarp();
+      if (lane < 2) held[lane][wi] = 0;
+    }
+    __syncwarp();
   };
   unsigned long long n = *a.survivor_count;
   const bool full = n > a.survivor_cap;
@@ -1042,35 +1086,20 @@ __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_con
   // then has a survivor per warp, whose chains of dependent loads do not wait
   // for one another.
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  const uint32_t w = blockIdx.x + gridDim.x * (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  auto flush = [&](bool done) {  // by all threads of the block
-    __syncthreads();
-    const uint32_t nm = min(held[0], kVerifyBuf), nk = min(held[1], kVerifyBuf);
-    if ((nm | nk) && (done || nm > kVerifyBuf - 256 || nk > kVerifyBuf - 256)) {
-      if (threadIdx.x == 0 && nm) first[0] = atomicAdd(a.counter, (unsigned long long)nm);
-      if (RX && threadIdx.x == 32 && nk) first[1] = atomicAdd(&p.ctr[C_K], (unsigned long long)nk);
-      __syncthreads();
-      for (uint32_t i = threadIdx.x; i < nm; i += blockDim.x)
-        if (first[0] + i < a.cap) a.out[first[0] + i] = ws_match{mbuf[i].x, mbuf[i].y, mbuf[i].z};
-      for (uint32_t i = threadIdx.x; RX && i < nk; i += blockDim.x)
-        store_k(p, first[1] + i, kbuf[i].x, kbuf[i].y, kbuf[i].z, kEndKnown);
-      __syncthreads();
-      if (threadIdx.x < 2) held[threadIdx.x] = 0;
-      __syncthreads();
-    }
-  };
-  for (unsigned long long k0 = 0; k0 < n && !dense; k0 += 32ull * warps) {  // the same for all threads
+  const uint32_t w = blockIdx.x + gridDim.x * wi;
+  for (unsigned long long k0 = 0; k0 < n && !dense; k0 += 32ull * warps) {  // the same for all lanes
     const unsigned long long k = k0 + (unsigned long long)lane * warps + w;
     const uint32_t s = k < n ? a.survivors[k] : kNoSurvivor;
     const bool in = s != kNoSurvivor;  // (else a slot the gram kernel reserved but did not fill)
     // the first words, then the buckets of the literals' table and of the
     // prefixes', in flight together
     const uint32_t len = (uint32_t)a.len, w0 = s & ~3u, sh = (s & 3) * 8;
-    uint32_t x0 = 0, x1 = 0, x2 = 0;
+    uint32_t x0 = 0, x1 = 0, x2 = 0, x3 = 0;
     if (in) {
       x0 = word_at(a.data, len, w0);
       x1 = word_at(a.data, len, w0 + 4);
       x2 = word_at(a.data, len, w0 + 8);
+      if (a.parts) x3 = word_at(a.data, len, w0 + 12);
     }
     const uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
     const bool literals = in && a.parts && s < a.max_start;
@@ -1084,47 +1113,27 @@ __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_con
     }
     if (literals) {
       Probe pr;
+      const uint32_t next = __funnelshift_r(x2, x3, sh);
       if (a.fold) probe_literals(a, ascii_fold4(lo), ascii_fold4(hi), len - s, pr);
       else probe_literals(a, lo, hi, len - s, pr);
-      verify_literals(a, s, a.fold ? ascii_fold4(x0) : x0, pr, match);
+      verify_literals(a, s, a.fold ? ascii_fold4(x0) : x0, a.fold ? ascii_fold4(next) : next, pr, match);
     }
     if (RX) verify_prefixes(a, t, p, pf, s, lo, hi, pk, pk1, gate, candidate);
-    flush(k0 + 32ull * warps >= n);
+    drain();
   }
   if (dense && a.parts) {
-    __shared__ uint32_t wheld[8];
-    const uint32_t len = (uint32_t)a.len, nvec = (uint32_t)((a.len + 15) >> 4), wi = threadIdx.x >> 5;
-    uint3* mine = mbuf + wi * kDenseBuf;
-    uint32_t* grams = reinterpret_cast<uint32_t*>(kbuf) + wi * kDenseBuf;
-    uint32_t* mine_held = wheld + wi;
-    if (lane == 0) *mine_held = 0;
-    __syncwarp();
-    auto warp_match = [&](uint32_t pid, uint32_t s, uint32_t e) {
-      const uint32_t i = atomicAdd(mine_held, 1u);
-      if (i < kDenseBuf) mine[i] = make_uint3(pid, s, e);
-      else report_match(a, pid, s, e);
-    };
-    auto verify_grams = [&](uint32_t n, bool end) {  // grams[0, n), n <= 32
+    const uint32_t len = (uint32_t)a.len, nvec = (uint32_t)((a.len + 15) >> 4);
+    uint32_t* grams = reinterpret_cast<uint32_t*>(kbuf[wi]);
+    auto verify_grams = [&](uint32_t n) {  // grams[0, n), n <= 32
       if (lane < n) {
         const uint32_t at = grams[lane];
         uint32_t bits = __ldg(a.phase + (phase_key_at<true>(a, at, (int)a.gram_len) >> a.phase_shift));
         for (; bits; bits &= bits - 1) {
           const uint32_t k = a.period - __ffs(bits);  // bit period - 1 - k: the literal starts k bytes before
-          if (at >= k && at - k < len) verify_lean(a, at - k, warp_match);
+          if (at >= k && at - k < len) verify_lean(a, at - k, match);
         }
       }
-      __syncwarp();
-      const uint32_t nm = min(*mine_held, kDenseBuf);
-      if (nm > kDenseBuf - 32 || (end && nm)) {
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(a.counter, (unsigned long long)nm);
-        at = __shfl_sync(0xFFFFFFFFu, at, 0);
-        for (uint32_t i = lane; i < nm; i += 32)
-          if (at + i < a.cap) a.out[at + i] = ws_match{mine[i].x, mine[i].y, mine[i].z};
-        __syncwarp();
-        if (lane == 0) *mine_held = 0;
-      }
-      __syncwarp();
+      drain();
     };
     uint32_t queued = 0;
     for (uint64_t v0 = (uint64_t)w * 32; v0 < nvec; v0 += (uint64_t)warps * 32) {
@@ -1139,7 +1148,7 @@ __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_con
         queued += __popc(ball);
         __syncwarp();
         if (queued >= 32) {
-          verify_grams(32, false);
+          verify_grams(32);
           queued -= 32;
           const uint32_t keep = lane < queued ? grams[32 + lane] : 0u;
           __syncwarp();
@@ -1148,7 +1157,24 @@ __global__ void __launch_bounds__(256, 4) literal_verify_kernel(const __grid_con
         }
       }
     }
-    verify_grams(queued, true);
+    verify_grams(queued);
+  }
+  // what the warps still hold
+  __shared__ unsigned long long first[2];
+  __syncthreads();
+  uint32_t before[2] = {0, 0}, sum[2] = {0, 0};
+#pragma unroll
+  for (uint32_t i = 0; i < kVerifyWarps; ++i)
+    for (uint32_t q = 0; q < (RX ? 2u : 1u); ++q) {
+      if (i == wi) before[q] = sum[q];
+      sum[q] += min(held[q][i], kVerifyBuf);
+    }
+  if (threadIdx.x == 0 && sum[0]) first[0] = atomicAdd(a.counter, (unsigned long long)sum[0]);
+  if (RX && threadIdx.x == 32 && sum[1]) first[1] = atomicAdd(&p.ctr[C_K], (unsigned long long)sum[1]);
+  if (sum[0] | sum[1]) {
+    __syncthreads();
+    write_out(min(held[0][wi], kVerifyBuf), first[0] + before[0], RX ? min(held[1][wi], kVerifyBuf) : 0u,
+              first[1] + before[1]);
   }
   if (RX) {
     __shared__ bool last;
@@ -1190,8 +1216,6 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   a.filter_words = plan.has_big ? (1u << (kLeanBits - 5)) : (uint32_t)plan.filter.size();
   a.bits = plan.table_bits;
   a.period = plan.period;
-  a.has_long = plan.has_long;
-  a.has_short = plan.has_short;
   a.parts = l.literals ? plan.parts : 0;  // (no prefix length, no literal)
   a.short_bits = plan.d_short.as<uint32_t>();
   a.bloom = plan.d_bloom.as<uint32_t>();
@@ -1199,7 +1223,7 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   a.lit_bytes = plan.d_bytes.as<uint8_t>();
   for (uint32_t i = 0; i < HASH_WINDOW; ++i) a.meta[i] = make_uint2(plan.meta[4 * i], plan.meta[4 * i + 1]);
   a.ranges = plan.d_ranges.as<uint2>();
-  a.entries = plan.d_entries.as<uint2>();
+  a.entries = plan.d_entries.as<uint4>();
   a.out = l.out;
   a.cap = l.cap;
   a.counter = l.counter;
@@ -1287,12 +1311,28 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   // latency: 40,000 items 65 -> 39 us in this kernel), and for a short list no
   // more blocks than it can fill
   const uint64_t vgrid = std::min<uint64_t>((uint64_t)sm_count * 4, (l.survivor_cap + 255) / 256);
+  // (a set whose tables are more than two lines a thread leaves them where they are)
+  WarmDev wd{};
+  uint64_t lines = 0;
+  uint32_t n_warm = 0;
+  auto warm = [&](const DeviceBuffer& b) {
+    const uint64_t n = (b.bytes + 127) / 128;
+    if (!b.ptr || lines + n > 2 * 256 * vgrid) return;
+    wd.p[n_warm] = b.as<char>();
+    wd.lines[n_warm++] = (uint32_t)n;
+    lines += n;
+  };
+  if (l.literals)
+    for (const DeviceBuffer* b : {&plan.d_ranges, &plan.d_entries, &plan.d_info, &plan.d_bytes}) warm(*b);
   if (l.rx) {
+    for (const DeviceBuffer* b : {&plan.d_prefix_range, &plan.d_prefix_entry}) warm(*b);
+    for (const DeviceBuffer* b : l.rx->walk_tables)
+      if (b) warm(*b);
     const PrefixDev pf{plan.d_prefix_range.as<uint32_t>(), plan.d_prefix_entry.as<uint4>(), plan.prefix_shift,
                        plan.prefix_mul};
-    launch_pdl(literal_verify_kernel<true>, (unsigned)vgrid, 256, 0, st, a, l.rx->t, l.rx->p, pf);
+    launch_pdl(literal_verify_kernel<true>, (unsigned)vgrid, 256, 0, st, a, l.rx->t, l.rx->p, pf, wd);
   } else {
-    launch_pdl(literal_verify_kernel<false>, (unsigned)vgrid, 256, 0, st, a, DevTables{}, ScanPtrs{}, PrefixDev{});
+    launch_pdl(literal_verify_kernel<false>, (unsigned)vgrid, 256, 0, st, a, DevTables{}, ScanPtrs{}, PrefixDev{}, wd);
   }
   check_cuda(cudaGetLastError(), "literal_verify_kernel launch");
 }

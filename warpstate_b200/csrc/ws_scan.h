@@ -183,6 +183,7 @@ struct RegexScan {
   DevTables t;
   uint64_t k_cap = 0, n_q = 0;
   uint32_t clear_words = 0;  // u32 words from p.ctr on that start as zero
+  const DeviceBuffer* walk_tables[4] = {};  // what lf_walk reads
   bool prefixes = false;  // the literal scan finds the covered groups' candidates
 };
 
