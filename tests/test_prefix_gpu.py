@@ -113,3 +113,16 @@ def test_prefix_nucleotides_long_grams():
     m = build(pats)
     exp = oracle.scan_patterns(pats, d)
     assert len(exp) >= 200 and np.array_equal(m.scan_array(d), exp)
+
+
+@pytest.mark.parametrize("flags", [0, 3])
+def test_tuned_matcher_keeps_its_prefixes(flags):
+    # the tuner plans the groups anew: the covered ones are still not walked (no
+    # chunk boundary is guessed)
+    pats = [(1, rb"key=[0-9]+"), (1, rb"(?:alpha|beta1|gamma)[ :]{1,3}[a-f]{2,4}"), (1, rb"user_[a-z0-9_]*\.")]
+    d = plant(text(1 << 20, 5), TEXTS, 97, 6)
+    m = build(pats, max_matches=1 << 18, profile=True)
+    exp = oracle.scan_patterns(pats, d)
+    m.tune(text(1 << 20, 9), flags=flags)
+    assert np.array_equal(m.scan_array(d), exp)
+    assert m.info()["last_guesses"] == 0 and m.info()["last_events"] == 0

@@ -145,8 +145,10 @@ uint32_t enqueue_scan(ws_matcher* m, Scratch& s, cudaStream_t st, const uint8_t*
   RegexLaunch rl{d_data, len, d_out, cap, d_counter, m->cfg.regex_mode};
   RegexScan rs;
   // the literal filter also looks for the regexes' prefixes, unless the walk
-  // is pinned
-  const bool prefixes = m->rx.n_regex && m->lit.n_prefixes && m->cfg.regex_mode == WS_REGEX_SPECULATIVE && !m->walk_pinned;
+  // is pinned or goes over every group all the same
+  const bool spared = m->rx.n_walk < m->rx.n_spec || m->rx.n_ctx_walk < m->rx.n_groups;
+  const bool prefixes =
+      spared && m->lit.n_prefixes && m->cfg.regex_mode == WS_REGEX_SPECULATIVE && !m->walk_pinned;
   if (m->rx.n_regex) {
     rl.item_end = x.item_end;
     rl.n_items = x.n_items;

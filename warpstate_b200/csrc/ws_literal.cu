@@ -202,7 +202,7 @@ __device__ __forceinline__ void report_match(const LitArgs& a, uint32_t pid, uin
 // are more code and registers: inlined in the compacting kernels they spilled
 // the main loop (11-mers over 128 MiB 313 us a scan, this way 246).
 template <class Sink>
-__device__ __forceinline__ void verify_lean(const LitArgs& a, uint32_t s, Sink&& sink) {
+__device__ __forceinline__ void verify_by_word(const LitArgs& a, uint32_t s, Sink&& sink) {
   if (s >= a.max_start) return;
   const uint32_t len = (uint32_t)a.len, rem = len - s, w0 = s & ~3u, sh = (s & 3) * 8;
   const uint32_t x0 = input_word(a, len, w0), x1 = input_word(a, len, w0 + 4), x2 = input_word(a, len, w0 + 8);
@@ -392,7 +392,7 @@ __device__ __forceinline__ void process_block(const LitArgs& a, uint32_t* blk, u
         const unsigned long long slot = wbase + __popc(ball & ((1u << lane) - 1u));
         const uint32_t s = blk_base + off;
         if (slot < a.survivor_cap) a.survivors[slot] = s;
-        else verify_lean(a, s, [&](uint32_t pid, uint32_t at, uint32_t e) {  // list full
+        else verify_by_word(a, s, [&](uint32_t pid, uint32_t at, uint32_t e) {  // list full
           // (not report_match, whose code held registers of the loop: 262 -> 246 us)
           const unsigned long long idx = atomicAdd(a.counter, 1ull);
           if (idx < a.cap) a.out[idx] = ws_match{pid, at, e};
@@ -701,12 +701,12 @@ constexpr uint32_t kNoSurvivor = 0xFFFFFFFFu;  // no position: inputs are shorte
 template <int P, int G>
 __host__ __device__ constexpr int gram_off() { return G == 16 ? 12 : P == 4 ? 0 : P == 2 ? 2 : G == 3 ? 2 : 3; }
 
-struct LeanSlots {
+struct WarpSlots {
   unsigned long long next = 0, end = 0;  // the warp's reserved range [next, end)
 };
 
 // Marks the warp's unfilled reserved slots as holes.
-__device__ __forceinline__ void lean_holes(const LitArgs& a, const LeanSlots& r, uint32_t lane) {
+__device__ __forceinline__ void mark_holes(const LitArgs& a, const WarpSlots& r, uint32_t lane) {
   for (unsigned long long k = r.next + lane; k < r.end && k < a.survivor_cap; k += 32) a.survivors[k] = kNoSurvivor;
 }
 
@@ -740,7 +740,7 @@ __device__ __forceinline__ uint32_t gram_at(uint32_t code) {
 // before: the verify kernel then looks at every gram of the input again, and this
 // kernel has nothing more to add.
 template <int P, int G, bool EDGE>
-__device__ __forceinline__ bool gram_flush(const LitArgs& a, const uint32_t* queue, uint32_t n, LeanSlots& r,
+__device__ __forceinline__ bool gram_flush(const LitArgs& a, const uint32_t* queue, uint32_t n, WarpSlots& r,
                                            uint32_t lane) {
   const uint32_t len = (uint32_t)a.len;
   for (uint32_t k0 = 0; k0 < n; k0 += 32) {
@@ -762,7 +762,7 @@ __device__ __forceinline__ bool gram_flush(const LitArgs& a, const uint32_t* que
     }
     const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
     if (r.next + total > r.end) {  // warp-uniform: reserve more slots
-      lean_holes(a, r, lane);
+      mark_holes(a, r, lane);
       const unsigned long long want = total > a.slot_chunk ? total : a.slot_chunk;
       unsigned long long wb = 0;
       if (lane == 0) wb = atomicAdd(a.survivor_count, want);
@@ -789,7 +789,7 @@ constexpr uint32_t kListFull = 0xFFFFFFFFu;
 
 template <int P, int G, bool EDGE>
 __device__ __forceinline__ uint32_t gram_queue(const LitArgs& a, uint32_t* queue, uint32_t queued, uint32_t pass,
-                                               uint32_t code, LeanSlots& slots, uint32_t lane) {
+                                               uint32_t code, WarpSlots& slots, uint32_t lane) {
   uint32_t ball = __ballot_sync(0xFFFFFFFFu, pass != 0);
   while (ball) {
     if (pass) {  // one gram of every lane that has one left
@@ -876,7 +876,7 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
   const uint32_t runs = len / (VECS * 512);                // runs entirely inside the input
   // neighbouring runs go to different SMs, so that a small input spreads out
   const uint32_t first = warp * gridDim.x + blockIdx.x, nw = gridDim.x * kGramWarps;
-  LeanSlots slots;
+  WarpSlots slots;
   uint32_t queued = 0;
   uint32_t below[NPRE ? NPRE : 1];
   auto run_ptr = [&](uint32_t r) { return reinterpret_cast<const uint4*>(a.data + (uint64_t)r * (VECS * 512)) + lane; };
@@ -935,7 +935,7 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
   }
   __syncwarp();
   if (queued) gram_flush<P, G, true>(a, queue, queued, slots, lane);
-  lean_holes(a, slots, lane);
+  mark_holes(a, slots, lane);
 }
 
 // A position where a covered regex's prefix may start: every regex of which one
@@ -1130,7 +1130,7 @@ __global__ void __launch_bounds__(kVerifyThreads, 4) literal_verify_kernel(const
         uint32_t bits = __ldg(a.phase + (phase_key_at<true>(a, at, (int)a.gram_len) >> a.phase_shift));
         for (; bits; bits &= bits - 1) {
           const uint32_t k = a.period - __ffs(bits);  // bit period - 1 - k: the literal starts k bytes before
-          if (at >= k && at - k < len) verify_lean(a, at - k, match);
+          if (at >= k && at - k < len) verify_by_word(a, at - k, match);
         }
       }
       drain();

@@ -110,7 +110,6 @@ extern "C" ws_status ws_matcher_tune(ws_matcher* m, const uint8_t* corpus, uint6
         for (size_t k = 0; k < cands.size(); ++k) {
           ws_config c = m->cfg;
           c.dfa_max_states = cands[k];
-          c.proposer = WS_PROPOSER_NONE;
           RegexPlan cand;
           try {
             plan_regex(t, c, m->ctx->sm_count, cand);
