@@ -442,7 +442,8 @@ def walk_record(info, n_bytes, ms):
     guesses = info["last_guesses"]
     return {"gbs": round(n_bytes / (ms * 1e-3) / 1e9, 3), "ms_per_step": round(ms, 4),
             "walk_ms": round(walk_ms, 4),
-            "lookups_per_s": round(g * n_bytes / (walk_ms * 1e-3), 1) if walk_ms else None,
+            # (no boundary was guessed: the candidates came from the literal filter)
+            "lookups_per_s": round(g * n_bytes / (walk_ms * 1e-3), 1) if walk_ms and guesses else None,
             "guess_hit_rate": round(info["last_guess_hits"] / guesses, 5) if guesses else None,
             "fixup_chunks": info["last_fixup_chunks"], "chunks": info["last_chunks"],
             "rewalk_bytes": info["last_rewalk_bytes"],
