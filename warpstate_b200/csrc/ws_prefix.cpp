@@ -9,11 +9,12 @@
 //
 // The walk takes one shared-memory lookup per input byte and group, 1.8 T
 // lookups/s over the chip; the filter one per second or fourth byte, once for
-// the literals and all groups.  Measured, us a pass with the walk and with the
-// filter: 500 regexes (9 groups) over 64 MiB 487 -> 171, 160 regexes (1 group)
-// over 1 GiB 939 -> 602, 60 unbounded regexes over 200 MiB 737 -> 273, 40
-// anchored ones over 32 MiB 300 -> 136, 40,000 items with 1,500 literals and
-// 200 regexes 1556 -> 414, 20,000 k-mers and 100 motifs over 2 GiB 2349 -> 892.
+// the literals and all groups.  Measured, us a pass with the walk (as it was
+// before there were prefixes) and with the filter: 500 regexes (9 groups) over 64
+// MiB 483 -> 116, 160 regexes (1 group) over 1 GiB 939 -> 474, 60 unbounded
+// regexes over 200 MiB 740 -> 221, 40 anchored ones over 32 MiB 304 -> 98, 40,000
+// items with 1,500 literals and 200 regexes 1734 -> 336, 20,000 k-mers and 100
+// motifs over 2 GiB 3105 -> 715.
 // Where prefixes are dense the filter gives up at run time (ws_literal.cu,
 // literal_verify_kernel) and the walk does what it did before.
 #include <algorithm>
