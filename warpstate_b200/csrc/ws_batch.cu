@@ -142,8 +142,9 @@ extern "C" ws_status ws_scan_batch_device(ws_matcher* m, const uint8_t* d_data, 
       return n + 1;
     };
     // The launch sequence of a call is replayed from a CUDA graph when the
-    // previous calls on this scratch had the same arguments and plan: the
-    // first runs eagerly (it sizes every buffer), the second is captured.
+    // previous calls on this scratch had the same arguments and plan, in the
+    // same buffers: the first runs eagerly (it sizes every buffer), the second
+    // is captured.
     BatchGraphKey key;
     key.data = d_data;
     key.len = len;
@@ -160,6 +161,12 @@ extern "C" ws_status ws_scan_batch_device(ws_matcher* m, const uint8_t* d_data, 
       key.need[1] = m->need_host[1];
     }
     key.profile = m->profile ? 1 : 0;
+    auto scratch_of = [&](BatchGraphKey& k) {
+      k.scratch[0] = s->rx.ptr;
+      k.scratch[1] = s->lit.ptr;
+      k.scratch[2] = s->out.ptr;
+    };
+    scratch_of(key);
     BatchGraph& bg = s->batch_graph;
     if (std::memcmp(&bg.key, &key, sizeof(key)) != 0) {
       bg.reset();
@@ -203,6 +210,7 @@ extern "C" ws_status ws_scan_batch_device(ws_matcher* m, const uint8_t* d_data, 
       launches = body();
       bg.seen++;
     }
+    scratch_of(bg.key);  // (the body sizes the buffers)
     check_cuda(cudaEventRecord(s->busy, st), "event");
     std::lock_guard<std::mutex> g(m->info_mu);
     m->info.last_launches = launches;

@@ -39,6 +39,9 @@ struct BatchGraphKey {
   uint64_t plan_gen = 0;
   uint64_t need[2] = {0, 0};
   uint64_t profile = 0;
+  // the scratch buffers whose addresses the launches hold: a larger scan of
+  // another kind on the same scratch may have replaced them
+  const void* scratch[3] = {nullptr, nullptr, nullptr};
 };
 
 struct BatchGraph {
