@@ -754,7 +754,7 @@ __device__ void count_guess_hits(const DevTables& t, const ScanPtrs& p) {
 
 // Valid match events -> reverse walk -> K candidates (and, in profiled
 // speculative scans, the guess count).
-__global__ void __launch_bounds__(256) dfa_reverse_kernel(DevTables t, ScanPtrs p) {
+__global__ void __launch_bounds__(1024) dfa_reverse_kernel(DevTables t, ScanPtrs p) {
   pdl_begin();
   if (p.count_guesses && p.n_chunks > 1) count_guess_hits(t, p);
   unsigned long long n = p.ctr[C_EV];
@@ -802,17 +802,32 @@ __global__ void __launch_bounds__(256) dfa_reverse_kernel(DevTables t, ScanPtrs 
 }
 
 // ---------------------------------------------------------------- resolution
+// Candidates a block sorts in shared memory, and the longest list that one block
+// of k_resolve_kernel takes from sort to report.  Where the prefix filter gave
+// up, the candidates' ends are still to be walked, up to kLfCap bytes each: a
+// block then takes four per thread, not sixteen.
+constexpr uint32_t kSortTile = 4096, kOpenTile = 1024;
+__device__ __forceinline__ uint32_t resolve_tile(const ScanPtrs& p) { return p.ctr[C_GATE] ? kOpenTile : kSortTile; }
+
 // Exclusive scan of the per-regex candidate counts into offs[0, n_regex] by one
 // block (blockDim.x a multiple of 32, at most 1024): each thread sums a run of
 // regexes, the runs are scanned across the block with warp shuffles, then each
-// thread writes its run's offsets.
+// thread writes its run's offsets.  Notes in ctr[C_LONG] whether some list is
+// longer than resolve_tile.
 __device__ void scan_counts(const ScanPtrs& p, uint32_t n_regex, uint32_t* offs) {
   __shared__ uint32_t wsum[32];
   const uint32_t per = (n_regex + blockDim.x - 1) / blockDim.x;
   const uint32_t a = min(n_regex, threadIdx.x * per), b = min(n_regex, a + per);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint32_t tile = resolve_tile(p);
   uint32_t sum = 0;
-  for (uint32_t r = a; r < b; ++r) sum += p.count[r];
+  bool more = false;
+  for (uint32_t r = a; r < b; ++r) {
+    const uint32_t c = p.count[r];
+    sum += c;
+    more |= c > tile;
+  }
+  if (more) p.ctr[C_LONG] = 1;
   uint32_t incl = sum;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
@@ -865,10 +880,18 @@ __global__ void __launch_bounds__(256) k_scatter_kernel(ScanPtrs p, uint32_t n_r
       for (uint32_t r = threadIdx.x; r <= n_regex; r += blockDim.x) p.offs[r] = offs_s[r];
   }
   const uint32_t* offs = staged ? offs_s : p.offs;
-  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-    const KCand c = p.k[k];
-    p.pair[offs[c.r] + (c.rank & ~kEndKnown)] =
-        ((unsigned long long)c.s << 32) | ((c.rank & kEndKnown) ? c.e : kLfTodo);
+  // four candidates of a thread in flight together
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += 4 * stride) {
+    KCand c[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i)
+      if (k + i * stride < n) c[i] = p.k[k + i * stride];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i)
+      if (k + i * stride < n)
+        p.pair[offs[c[i].r] + (c[i].rank & ~kEndKnown)] =
+            ((unsigned long long)c[i].s << 32) | ((c[i].rank & kEndKnown) ? c[i].e : kLfTodo);
   }
 }
 
@@ -888,8 +911,6 @@ __device__ void bitonic_smem(unsigned long long* buf, uint32_t m) {
     }
   }
 }
-
-constexpr uint32_t kSortTile = 4096;
 
 // Sorts src[0, n), n <= kSortTile, into buf (shared memory).
 __device__ void sort_into(unsigned long long* buf, const unsigned long long* src, uint32_t n) {
@@ -912,11 +933,12 @@ __device__ uint32_t merge_path(const unsigned long long* A, uint32_t na, const u
   return lo;
 }
 
-// Merges the sorted tiles of list[0, n) pairwise in global memory (merge-path
-// split of each merge across the block), with other[0, n) as the other buffer.
-__device__ void merge_tiles(unsigned long long* list, unsigned long long* other, uint32_t n) {
+// Merges the sorted tiles (of `tile` candidates) of list[0, n) pairwise in
+// global memory (merge-path split of each merge across the block), with
+// other[0, n) as the other buffer.
+__device__ void merge_tiles(unsigned long long* list, unsigned long long* other, uint32_t n, uint32_t tile) {
   unsigned long long *src = list, *dst = other;
-  for (uint32_t w = kSortTile; w < n; w <<= 1) {
+  for (uint32_t w = tile; w < n; w <<= 1) {
     for (uint32_t lo = 0; lo < n; lo += 2 * w) {
       const uint32_t mid = min(lo + w, n), hi = min(lo + 2 * w, n);
       const unsigned long long *A = src + lo, *B = src + mid;
@@ -967,7 +989,7 @@ __global__ void __launch_bounds__(512) k_sort_kernel(ScanPtrs p, uint32_t n_rege
     __syncthreads();
     if (last) {
       __threadfence();
-      merge_tiles(p.pair + a, p.pair2 + a, n);
+      merge_tiles(p.pair + a, p.pair2 + a, n, kSortTile);
     }
     __syncthreads();
   }
@@ -1173,32 +1195,88 @@ __global__ void __launch_bounds__(kChainThreads) k_chain_kernel(DevTables t, Sca
   }
 }
 
-// Sort, missing ends and chain of a regex by one block, in shared memory for up
-// to kSortTile candidates: the resolution of scans whose candidates came from
-// prefixes, ends known (three kernels and a pass through global memory between
-// each took 8 us more on small lists).
+// The block's share of the long lists (see k_resolve_kernel) and its regexes with
+// short ones, missing ends included.
+__device__ void resolve_shared(const DevTables& t, const ScanPtrs& p, uint32_t n_regex, unsigned long long* buf,
+                               ChainShared& sh) {
+  __shared__ bool last;
+  const uint32_t tile = resolve_tile(p), total = p.offs[n_regex];
+  uint64_t slot = (uint64_t)blockIdx.x * tile;
+  for (uint32_t r0 = blockIdx.x;; r0 += gridDim.x) {
+    // the block's regexes (tile 0 of a long list), then its slots of the
+    // candidates: a later tile of a list falls to the block whose slot its first
+    // candidate lies in.  The list began more than a tile before, so it holds the
+    // slot's first candidate too, and no other list has a later tile there.
+    uint32_t r = r0, k = 0;
+    if (r0 >= n_regex) {
+      if (slot >= total) return;
+      uint32_t hi = n_regex;
+      for (r = 0; hi - r > 1;) {
+        const uint32_t mid = (r + hi) >> 1;
+        if (p.offs[mid] <= slot) r = mid; else hi = mid;
+      }
+      k = ((uint32_t)slot - p.offs[r] + tile - 1) / tile;
+      slot += (uint64_t)gridDim.x * tile;
+      if (k == 0) continue;
+    }
+    const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
+    if (k && k * tile >= n) continue;
+    unsigned long long* list = p.pair + a;
+    const uint32_t m = min(tile, n - k * tile);
+    if (m) {
+      sort_into(buf, list + k * tile, m);
+      for (uint32_t j = threadIdx.x; j < m; j += blockDim.x)
+        if ((uint32_t)buf[j] == kLfTodo) reinterpret_cast<uint32_t*>(buf + j)[0] = list_end(t, p, r, buf, j);
+      __syncthreads();
+    }
+    if (n > tile) {
+      for (uint32_t j = threadIdx.x; j < m; j += blockDim.x) list[k * tile + j] = buf[j];
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&p.count[r], 1u) + 1 == n + (n + tile - 1) / tile;
+      }
+      __syncthreads();
+      if (!last) continue;
+      __threadfence();
+      merge_tiles(list, p.pair2 + a, n, tile);
+    }
+    const uint64_t end = chain_list(t, p, r, n > tile ? list : buf, n, chain_start(p, r), chain_limit(p), sh);
+    if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + end, p.frontier);
+    __syncthreads();  // (buf, before the next list)
+  }
+}
+
+// Sort and chain of a regex by one block, in shared memory: the resolution of
+// scans whose candidates came from prefixes, ends known (three kernels and a pass
+// through global memory between each took 8 us more on small lists).
+// Lists longer than resolve_tile (dense matches, or the walk's candidates where
+// the filter gave up) are shared by all blocks: each tile is sorted, its missing
+// ends walked, by the block it falls to, and the block that finishes a list's
+// last tile merges and reports it (its ticket is the regex's count, which nothing
+// reads after the scatter).  A tile walks the ends of its own distinct starts, so
+// a start in several tiles is walked in each, to the same end.  By one block per
+// regex -> shared, us a scan: 21 regexes over 64 MiB whose filter gave up 2,150
+// -> 1,450 (with the walk before there were prefixes 1,880), 30 regexes with
+// 671,000 matches in 64 MiB 2,550 -> 1,240, three with 335,000 in 256 MiB 9,600 ->
+// 2,600, one with 335,000 among 301 18,800 -> 9,100.
 __global__ void __launch_bounds__(kChainThreads) k_resolve_kernel(DevTables t, ScanPtrs p, uint32_t n_regex,
                                                                   unsigned long long* need) {
   __shared__ unsigned long long buf[kSortTile];
   __shared__ ChainShared sh;
   pdl_begin();
+  const bool shared = p.ctr[C_LONG] != 0 || p.ctr[C_GATE] != 0;  // (ends are missing when the walk ran)
   if (finalize(p, need)) return;
+  if (shared) {
+    resolve_shared(t, p, n_regex, buf, sh);
+    return;
+  }
   for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
     const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
-    unsigned long long* list = p.pair + a;
-    if (n > kSortTile) {
-      for (uint32_t k = 0; k * kSortTile < n; ++k) sort_tile(buf, list, n, k);
-      merge_tiles(list, p.pair2 + a, n);
-    } else if (n) {
-      sort_into(buf, list, n);
-      list = buf;
-    }
-    for (uint32_t j = threadIdx.x; j < n; j += blockDim.x)
-      if ((uint32_t)list[j] == kLfTodo) reinterpret_cast<uint32_t*>(list + j)[0] = list_end(t, p, r, list, j);
-    __syncthreads();
-    const uint64_t end = chain_list(t, p, r, list, n, chain_start(p, r), chain_limit(p), sh);
+    if (n) sort_into(buf, p.pair + a, n);
+    const uint64_t end = chain_list(t, p, r, buf, n, chain_start(p, r), chain_limit(p), sh);
     if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + end, p.frontier);
-    __syncthreads();  // (buf, before the next regex)
+    __syncthreads();  // (buf, before the next list)
   }
 }
 
@@ -1386,8 +1464,8 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
     launches++;
   }
   mark(3);
-  // (as a fallback, a quarter of the blocks: they usually find no event and exit)
-  launch_pdl(dfa_reverse_kernel, t.n_walk ? sm_count * 8 : sm_count * 2, 256, 0, st, t, p);
+  // (as a fallback, fewer and larger blocks: they usually find no event and exit)
+  launch_pdl(dfa_reverse_kernel, t.n_walk ? sm_count * 8 : sm_count * 2, t.n_walk ? 256 : 1024, 0, st, t, p);
   check_cuda(cudaGetLastError(), "dfa_reverse_kernel");
   launches++;
   context_groups();
@@ -1971,6 +2049,7 @@ uint32_t regex_finish(RegexPlan& P, RegexScan& rs, const RegexLaunch& l, cudaStr
   launches += candidates_phase(P, t, p, l.mode, st, sm_count, ev);
   const bool staged = P.n_regex < kOffsShared;
   const size_t osmem = staged ? ((size_t)P.n_regex + 1) * 4 : 0;
+  // (where all candidates come from prefixes, mostly few: a quarter of the blocks)
   const int hg = (int)std::min<uint64_t>((uint64_t)sm_count * (t.n_walk ? 4 : 1), (rs.k_cap + 255) / 256);
   if (!staged) {
     launch_pdl(k_scan_kernel, 1, 1024, 0, st, p, P.n_regex);
@@ -1979,7 +2058,9 @@ uint32_t regex_finish(RegexPlan& P, RegexScan& rs, const RegexLaunch& l, cudaStr
   launch_pdl(k_scatter_kernel, hg, 256, osmem, st, p, P.n_regex);
   launches += 1;
   if (rs.prefixes && t.n_walk == 0 && t.n_ctx_walk == P.n_spec) {
-    launch_pdl(k_resolve_kernel, (unsigned)std::min<uint32_t>(P.n_regex, 4096), kChainThreads, 0, st, t, p, P.n_regex, l.need);
+    // a block per regex; at least two per SM, for long lists
+    const uint32_t blocks = std::min<uint32_t>(std::max<uint32_t>(P.n_regex, 2 * sm_count), 4096);
+    launch_pdl(k_resolve_kernel, blocks, kChainThreads, 0, st, t, p, P.n_regex, l.need);
     launches += 1;
   } else {
     const uint32_t rows = std::min<uint32_t>(P.n_regex, 4096);
