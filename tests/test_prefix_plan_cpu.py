@@ -1,0 +1,74 @@
+"""Which regexes the literal filter covers (host side): the choice of the prefix
+length over pattern sets, by the planner's own code."""
+import ctypes
+import random
+
+import pytest
+
+
+def prefix_plan(literals, regexes, states=0, fold=False):
+    """(prefix length, 0 for none; per regex whether it is covered)"""
+    import warpstate_b200 as ws
+    from warpstate_b200 import _native as N
+    b = ws.PatternSet.builder().case_insensitive(fold)
+    for x in literals:
+        b = b.literal_bytes(x)
+    for x in regexes:
+        b = b.regex(x)
+    ps = b.build()
+    fn = N.lib().ws_testing_prefix_plan
+    fn.restype = ctypes.c_int
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_uint, ctypes.c_char_p, ctypes.c_ulong]
+    buf = ctypes.create_string_buffer(len(regexes) + 1)
+    n = fn(ps._h, states, buf, len(regexes))
+    assert n >= 0
+    return n, [buf.raw[i] != 0 for i in range(len(regexes))]
+
+
+def nucleotide_set(kmers, motifs, seed=3):
+    r = random.Random(seed)
+    lits = list({bytes(r.choices(b"ACGT", k=r.randint(20, 32))) for _ in range(kmers)})
+    out = []
+    for _ in range(motifs):  # one degenerate base each, 20 to 40 bases
+        m = r.choices("ACGT", k=r.randint(20, 40))
+        m[r.randrange(len(m))] = r.choice(["[AG]", "[CT]", "[ACGT]"])
+        out.append("".join(m))
+    return lits, out
+
+
+SHORT = ["GT[CT][AG]AC", "G[CT]GGCC[AG]C", "GT[CT][AG]ACGGTAC[AT]", "GT[CT][AG]ACGGTAC[AT]ACGT", "AC[AG]TTGCAACGGTTACGT"]
+
+
+@pytest.mark.parametrize("short", SHORT)
+@pytest.mark.parametrize("motifs", [0, 40])
+def test_short_motif_does_not_choose_the_layout(short, motifs):
+    # beside k-mers, a motif of fewer than 19 bases is walked: 16-byte grams stay
+    # possible for the others
+    lits, rx = nucleotide_set(5000, motifs)
+    n, covered = prefix_plan(lits, rx + [short])
+    assert covered == [True] * motifs + [False]
+    assert n == (20 if motifs else 0)
+
+
+@pytest.mark.parametrize("size", [19, 20])
+def test_motif_of_nineteen_bases_is_covered(size):
+    lits, rx = nucleotide_set(5000, 3)
+    assert prefix_plan(lits, rx + [("AC[AG]" + "TTGCAACGGTTACGTACG")[:size + 3]]) == (20, [True] * 4)
+
+
+def test_motif_with_too_many_prefixes_is_walked_alone():
+    lits, rx = nucleotide_set(5000, 10)
+    wide = "ACGT" + "[ACGT]" * 6 + "TTGCAACGGTTACGT"  # 4,096 strings of 20 bases, above the limit of one regex
+    assert prefix_plan(lits, rx + [wide]) == (20, [True] * 10 + [False])
+
+
+def test_short_kmer_keeps_every_motif_walked():
+    lits, rx = nucleotide_set(5000, 10)
+    assert prefix_plan(lits + [b"ACGTACGTACGT"], rx) == (0, [False] * 10)
+
+
+def test_sets_over_letters_are_covered_at_their_length():
+    words = [r"alpha[0-9]{1,3}x", r"(?:gamma|delta)=[a-f]+", r"tailwind [0-9]"]
+    assert prefix_plan([], words) == (7, [True] * 3)
+    assert prefix_plan([], words + [r"[0-9]+px"])[1] == [True] * 3 + [False]
+    assert prefix_plan([], [r"[0-9]+px"]) == (0, [False])

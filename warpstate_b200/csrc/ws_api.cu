@@ -308,6 +308,33 @@ std::unique_ptr<Scratch> ws_matcher::take() {
   return s;
 }
 
+void ws_matcher::keep_patterns(const ws_pattern_tables& t) {
+  IrData& d = patterns.d;
+  uint64_t bytes = 0;
+  for (uint32_t i = 0; i < t.n_literals; ++i)
+    bytes = std::max<uint64_t>(bytes, (uint64_t)t.offsets[2 * i] + t.offsets[2 * i + 1]);
+  auto copy = [](auto& to, const auto* from, size_t n) { if (n && from) to.assign(from, from + n); };
+  copy(d.packed_bytes, t.packed_bytes, bytes);
+  copy(d.offsets, t.offsets, 2 * (size_t)t.n_literals);
+  copy(d.literal_pattern_ids, t.literal_pattern_ids, t.n_literals);
+  copy(d.prefix_meta, t.prefix_meta, 4 * (size_t)t.hash_window_len);
+  copy(d.bucket_ranges, t.bucket_ranges, 2 * (size_t)t.n_buckets);
+  copy(d.entries, t.entries, 2 * (size_t)t.n_literals);
+  for (uint32_t r = 0; r < t.n_regex; ++r) d.regex_sources.emplace_back(t.regex_sources[r]);
+  for (const std::string& x : d.regex_sources) d.regex_ptrs.push_back(x.c_str());
+  copy(d.regex_pattern_ids, t.regex_pattern_ids, t.n_regex);
+  d.n_patterns = t.n_patterns;
+  d.case_insensitive = t.case_insensitive != 0;
+  hash_window = t.hash_window_len;
+}
+
+ws_pattern_tables ws_matcher::tables() const {
+  ws_pattern_tables t;
+  ws_ir_tables(&patterns, &t);
+  t.hash_window_len = hash_window;
+  return t;
+}
+
 void ws_matcher::give(std::unique_ptr<Scratch> s) {
   std::lock_guard<std::mutex> g(pool_mu);
   pool.push_back(std::move(s));
@@ -367,11 +394,9 @@ ws_status ws_matcher_create(ws_ctx* ctx, const ws_pattern_tables* t, const ws_co
     if (cfg) m->cfg = *cfg; else ws_config_default(&m->cfg);
     m->n_patterns = t->n_patterns;
     m->is_regex.assign(t->n_patterns, 0);
-    for (uint32_t r = 0; r < t->n_regex; ++r) {
+    for (uint32_t r = 0; r < t->n_regex; ++r)
       if (t->regex_pattern_ids[r] < t->n_patterns) m->is_regex[t->regex_pattern_ids[r]] = 1;
-      m->rx_src.emplace_back(t->regex_sources[r]);
-      m->rx_ids.push_back(t->regex_pattern_ids[r]);
-    }
+    m->keep_patterns(*t);
     for (uint32_t i = 0; i < t->n_literals; ++i) m->max_literal_len = std::max(m->max_literal_len, t->offsets[2 * i + 1]);
     std::memset(&m->info, 0, sizeof(m->info));
     plan_regex(*t, m->cfg, ctx->sm_count, m->rx);

@@ -1737,16 +1737,16 @@ void build_groups(const std::vector<ReTree>& trees, const std::vector<uint32_t>&
 
 }  // namespace
 
-void plan_regex(const ws_pattern_tables& t, const ws_config& cfg, int sm_count, RegexPlan& P) {
-  (void)sm_count;
+RegexSources read_regexes(const ws_pattern_tables& t, const ws_config& cfg, RegexPlan& P) {
+  RegexSources src;
+  std::vector<ReTree>& trees = src.trees;
+  trees.resize(t.n_regex);
   P.n_regex = t.n_regex;
-  if (!t.n_regex) return;
-  std::vector<ReTree> trees(t.n_regex);
   P.max_len = 0;
   for (uint32_t r = 0; r < t.n_regex; ++r) {
-    std::string src(t.regex_sources[r]);
+    const std::string text(t.regex_sources[r]);
     try {
-      trees[r] = parse_regex(src);
+      trees[r] = parse_regex(text);
     } catch (const CompileError& e) {
       raise(WS_ERR_COMPILE, "invalid regex at index " + std::to_string(t.regex_pattern_ids[r]) + ": " + e.what(),
             t.regex_pattern_ids[r]);
@@ -1763,11 +1763,8 @@ void plan_regex(const ws_pattern_tables& t, const ws_config& cfg, int sm_count, 
     else P.max_len = std::max(P.max_len, ml);
   }
   const int max_states = (int)std::max<uint32_t>(cfg.dfa_max_states, 16);
-  P.walk_chunk = std::max<uint32_t>(256, cfg.walk_chunk / 256 * 256);
-  // Greedy packing by the size of each regex's own unanchored DFA, then exact
-  // verification of every group (halved while it exceeds the budget).
-  std::vector<int> est(t.n_regex);
-  std::vector<uint8_t> ctx(t.n_regex, 0);
+  src.est.resize(t.n_regex);
+  src.ctx.assign(t.n_regex, 0);
   // The prefix filter covers a regex whose matches all begin with one of a few
   // strings of at least 4 bytes (a config that pins the walk's boundary guess
   // to the unanchored start walks every regex).
@@ -1775,20 +1772,36 @@ void plan_regex(const ws_pattern_tables& t, const ws_config& cfg, int sm_count, 
   for (auto& x : P.prefixes) x.assign(t.n_regex, {});
   const bool prefixes = cfg.regex_mode == WS_REGEX_SPECULATIVE && cfg.proposer != WS_PROPOSER_NONE;
   for (uint32_t r = 0; r < t.n_regex; ++r) {
-    ctx[r] = tree_has_look(trees[r]) ? 1 : 0;
+    src.ctx[r] = tree_has_look(trees[r]) ? 1 : 0;
     Nfa n = build_nfa({&trees[r]}, false);
     ByteClasses bc = compute_classes({&n});
-    Dfa d = ctx[r] ? build_context_all_dfa(n, bc, max_states) : build_all_dfa(n, bc, true, max_states);
+    Dfa d = src.ctx[r] ? build_context_all_dfa(n, bc, max_states) : build_all_dfa(n, bc, true, max_states);
     if (d.too_big)
       raise(WS_ERR_COMPILE, "regex " + std::to_string(t.regex_pattern_ids[r]) + " needs more than " +
                                 std::to_string(max_states) + " DFA states (raise dfa_max_states)",
             t.regex_pattern_ids[r]);
-    est[r] = d.n_states;
+    src.est[r] = d.n_states;
     for (int k = 0; prefixes && k < kPrefixLens; ++k) {
-      const bool ok = regex_prefixes(d, bc, ctx[r] != 0, kPrefixLen[k], kPrefixMost[k], P.prefixes[k][r]);
+      const bool ok = regex_prefixes(d, bc, src.ctx[r] != 0, kPrefixLen[k], kPrefixMost[k], P.prefixes[k][r]);
       if (kPrefixLen[k] == 4) P.covered[r] = ok ? 1 : 0;
     }
   }
+  return src;
+}
+
+void plan_regex(const ws_pattern_tables& t, const ws_config& cfg, int sm_count, RegexPlan& P) {
+  (void)sm_count;
+  P.n_regex = t.n_regex;
+  if (!t.n_regex) return;
+  const RegexSources src = read_regexes(t, cfg, P);
+  const std::vector<ReTree>& trees = src.trees;
+  const std::vector<int>& est = src.est;
+  const std::vector<uint8_t>& ctx = src.ctx;
+  choose_prefixes(t, P);
+  const int max_states = (int)std::max<uint32_t>(cfg.dfa_max_states, 16);
+  P.walk_chunk = std::max<uint32_t>(256, cfg.walk_chunk / 256 * 256);
+  // Greedy packing by the size of each regex's own unanchored DFA, then exact
+  // verification of every group (halved while it exceeds the budget):
   // speculative groups first, then the context groups; among each, the groups
   // of covered regexes last
   std::vector<GroupBuild> gbs;

@@ -103,6 +103,7 @@ struct RegexPlan {
   uint32_t n_walk = 0, n_ctx_walk = 0;
   std::vector<uint8_t> covered;          // per regex
   std::vector<std::vector<std::string>> prefixes[kPrefixLens];  // per length and regex; empty: too many
+  int prefix_len = -1;                   // the length the filter looks for (of kPrefixLen), -1: no regex is covered
   bool has_context = false;              // some regex has a look-around assertion
   bool class_image = false;              // the speculative groups' walk images are class-indexed
   uint32_t total_states = 0;
@@ -180,6 +181,18 @@ constexpr unsigned long long kCountUnknown = ~0ull;
 constexpr unsigned long long kCountTimeout = ~0ull - 1;
 
 void plan_regex(const ws_pattern_tables& t, const ws_config& cfg, int sm_count, RegexPlan& plan);
+// The regexes of a plan before they are grouped.
+struct RegexSources {
+  std::vector<ReTree> trees;
+  std::vector<int> est;      // states of the regex's own DFA
+  std::vector<uint8_t> ctx;  // has a look-around assertion
+};
+// Parses and checks the regexes and lists their prefixes; covered: a list of the
+// shortest length exists (ws_dfa.cu).
+RegexSources read_regexes(const ws_pattern_tables& t, const ws_config& cfg, RegexPlan& plan);
+// Picks the length of the prefixes that the literal filter will look for beside
+// the literals of `t`, and leaves covered the regexes it then covers (ws_prefix.cpp).
+void choose_prefixes(const ws_pattern_tables& t, RegexPlan& plan);
 // Re-ranks the forward DFA states of every group by how often a walk over
 // `d_corpus` visits them and rebuilds the hot-row layout: the placement of
 // rows in shared memory versus L2 is learned from the workload.

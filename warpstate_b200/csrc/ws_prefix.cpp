@@ -46,22 +46,41 @@ bool collect(const RegexPlan& P, int k, size_t most, std::vector<std::pair<std::
 // prefixes are more strings (a class in the prefix multiplies them): at most
 // 4,096 at 7 bytes and 16,384 at 5, beyond which the crowded filter costs more
 // than the lookups it saves.  A set whose 4-byte grams crowd their alphabet
-// takes 20 bytes (16-byte grams) or, where that is not possible, no prefixes:
-// its regexes are walked.
-void plan_filter(const ws_pattern_tables& t, const RegexPlan& P, LiteralPlan& plan) {
+// takes 20 bytes (16-byte grams), and there one short string would choose the
+// layout of all: 4-byte grams, nearly all of which a nucleotide input passes.  So
+// a regex is covered there only if each of its strings has the 19 bytes that
+// 16-byte grams at every fourth position need; the others are walked (20,000
+// k-mers and 100 motifs over 512 MiB, us a scan: with one motif more of 8 bases
+// 19,600 -> 1,560, of 12 bases 1,810 -> 950).  Where no length is possible, every
+// regex is walked.
+void choose_prefixes(const ws_pattern_tables& t, RegexPlan& P) {
+  P.prefix_len = -1;
   uint32_t shortest = UINT32_MAX;
   for (uint32_t i = 0; i < t.n_literals; ++i) shortest = std::min(shortest, t.offsets[2 * i + 1]);
   std::vector<std::pair<std::string, uint32_t>> pre;
   const size_t most[kPrefixLens] = {65536, 4096, 16384, 65536};
-  bool found = false;
-  for (int k = 1; k < kPrefixLens && !found && P.n_regex; ++k)
-    found = (kPrefixLen[k] <= shortest || kPrefixLen[k] == 4) && collect(P, k, most[k], pre);
-  if (found) {
+  for (int k = 1; k < kPrefixLens && P.prefix_len < 0; ++k)
+    if ((kPrefixLen[k] <= shortest || kPrefixLen[k] == 4) && collect(P, k, most[k], pre)) P.prefix_len = k;
+  if (P.prefix_len > 0) {
     std::vector<std::string> strings;
     for (const auto& x : pre) strings.push_back(x.first);
-    if (filter_crowded(t, strings)) found = shortest >= 19 && collect(P, 0, most[0], pre);
+    if (filter_crowded(t, strings)) {
+      P.prefix_len = -1;
+      for (uint32_t r = 0; r < P.n_regex; ++r) {
+        const auto& list = P.prefixes[0][r];
+        bool fits = P.covered[r] && !list.empty();
+        for (const std::string& x : list) fits &= x.size() >= 19;
+        P.covered[r] = fits ? 1 : 0;
+      }
+      if (shortest >= 19 && collect(P, 0, most[0], pre)) P.prefix_len = 0;
+    }
   }
-  if (!found) pre.clear();
+  if (P.prefix_len < 0) std::fill(P.covered.begin(), P.covered.end(), 0);
+}
+
+void plan_filter(const ws_pattern_tables& t, const RegexPlan& P, LiteralPlan& plan) {
+  std::vector<std::pair<std::string, uint32_t>> pre;
+  if (P.n_regex && P.prefix_len >= 0) collect(P, P.prefix_len, SIZE_MAX, pre);
   std::vector<std::string> strings;
   for (const auto& x : pre) strings.push_back(x.first);
   std::sort(strings.begin(), strings.end());
@@ -145,5 +164,26 @@ extern "C" long ws_testing_regex_prefixes(const char* source, unsigned len, unsi
     return (long)found.size();
   } catch (const std::exception&) {
     return -2;
+  }
+}
+
+// Test hook: the host part of a matcher's plan for a pattern set.  Writes per
+// regex whether the literal filter covers it; returns the length of the prefixes
+// it looks for, 0 when it looks for none, -1 on an error.
+extern "C" int ws_testing_prefix_plan(const ws_ir* ir, unsigned dfa_max_states, unsigned char* covered, unsigned long n) {
+  using namespace ws;
+  try {
+    ws_pattern_tables t;
+    ws_config c;
+    if (ws_ir_tables(ir, &t) != WS_OK || t.n_regex > n) return -1;
+    ws_config_default(&c);
+    if (dfa_max_states) c.dfa_max_states = dfa_max_states;
+    RegexPlan plan;
+    read_regexes(t, c, plan);
+    choose_prefixes(t, plan);
+    std::copy(plan.covered.begin(), plan.covered.end(), covered);
+    return plan.prefix_len < 0 ? 0 : (int)kPrefixLen[plan.prefix_len];
+  } catch (const std::exception&) {
+    return -1;
   }
 }

@@ -62,19 +62,6 @@ double time_regex(ws_matcher* m, RegexPlan& P, const uint8_t* d, uint64_t len, i
   return ts.empty() ? 0.0 : ts[ts.size() / 2];
 }
 
-ws_pattern_tables regex_tables(const ws_matcher* m, std::vector<const char*>& ptrs) {
-  ws_pattern_tables t;
-  std::memset(&t, 0, sizeof(t));
-  ptrs.clear();
-  for (const auto& s : m->rx_src) ptrs.push_back(s.c_str());
-  t.regex_sources = ptrs.data();
-  t.regex_pattern_ids = m->rx_ids.data();
-  t.n_regex = (uint32_t)m->rx_src.size();
-  t.n_patterns = m->n_patterns;
-  t.hash_window_len = HASH_WINDOW;
-  return t;
-}
-
 }  // namespace
 
 extern "C" ws_status ws_matcher_tune(ws_matcher* m, const uint8_t* corpus, uint64_t len, uint64_t seed, uint32_t flags,
@@ -104,8 +91,7 @@ extern "C" ws_status ws_matcher_tune(ws_matcher* m, const uint8_t* corpus, uint6
         // larger groups mean fewer lookups per input byte, as long as their
         // visited rows stay hot (the class-indexed image holds up to 1,472)
         std::vector<uint32_t> cands = {16384, 32768, 65536, 131072};
-        std::vector<const char*> ptrs;
-        const ws_pattern_tables t = regex_tables(m, ptrs);
+        const ws_pattern_tables t = m->tables();
         double best = 1e300;
         for (size_t k = 0; k < cands.size(); ++k) {
           ws_config c = m->cfg;
