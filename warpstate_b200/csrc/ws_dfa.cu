@@ -1382,7 +1382,9 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
     const uint32_t nc = P.n_groups - P.n_spec;
     if (!nc) return;
     const uint64_t want = (p.len + 255) / 256;
-    const uint64_t per_group = std::max<uint64_t>(1, (uint64_t)sm_count * 8 / nc);
+    // the chip's blocks are for the groups that walk
+    const uint32_t walking = t.n_ctx_walk > P.n_spec ? t.n_ctx_walk - P.n_spec : nc;
+    const uint64_t per_group = std::max<uint64_t>(1, (uint64_t)sm_count * 8 / walking);
     dim3 grid((unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, per_group)), nc);
     launch_pdl(dfa_context_kernel, grid, 256, 0, st, t, p);
     check_cuda(cudaGetLastError(), "dfa_context_kernel");
@@ -1449,7 +1451,7 @@ uint32_t candidates_phase(RegexPlan& P, const DevTables& t, const ScanPtrs& p, u
   // exact chunk starts are the true states: nothing to fix up
   if (!all_exact) {
     // one wave of fix-up blocks (one per SM, the walk's shared memory)
-    const uint64_t fper = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sm_count / P.n_spec,
+    const uint64_t fper = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sm_count / (t.n_walk ? t.n_walk : P.n_spec),
                                                                     (p.n_chunks + kWalkThreads - 1) / kWalkThreads));
     dim3 fgrid(P.n_spec, (unsigned)fper);
     auto fixup = P.class_image ? dfa_fixup_kernel<true> : dfa_fixup_kernel<false>;
@@ -2018,8 +2020,11 @@ namespace {
 // one 1,024-chunk block per SM and group -- so that no SM sits idle while the
 // others walk (one group over 1 GiB in 8 KiB chunks is 128 blocks on 148 SMs;
 // 7 KiB chunks make it 147).
-uint32_t effective_chunk(const RegexPlan& P, uint64_t len, int sm_count) {
-  const uint64_t c0 = P.walk_chunk, G = std::max<uint32_t>(P.n_spec, 1), sm = (uint64_t)std::max(sm_count, 1);
+// `groups`: those that walk.  (Counting gated groups, whose blocks leave at once,
+// left SMs idle: 20 regexes with prefixes and two without over 256 MiB 424 -> 310 us
+// a scan, 151 regexes in four groups of which one walks 428 -> 311.)
+uint32_t effective_chunk(const RegexPlan& P, uint32_t groups, uint64_t len, int sm_count) {
+  const uint64_t c0 = P.walk_chunk, G = std::max<uint32_t>(groups, 1), sm = (uint64_t)std::max(sm_count, 1);
   auto blocks = [&](uint64_t c) { return G * (((len + c - 1) / c + kWalkThreads - 1) / kWalkThreads); };
   const uint64_t waves = (blocks(c0) + sm - 1) / sm;
   const uint64_t per_group = waves * sm / G;  // blocks per group that fill `waves` waves
@@ -2034,7 +2039,8 @@ uint32_t effective_chunk(const RegexPlan& P, uint64_t len, int sm_count) {
 
 void regex_begin(RegexPlan& P, const RegexLaunch& l, cudaStream_t st, DeviceBuffer& scratch, int sm_count,
                  bool profiled, bool prefixes, RegexScan& rs) {
-  RxLayout L = layout(P, l.len, effective_chunk(P, l.len, sm_count), l.cap, l.k_min, l.ev_min);
+  const uint32_t walking = prefixes && P.n_walk ? P.n_walk : P.n_spec;
+  RxLayout L = layout(P, l.len, effective_chunk(P, walking, l.len, sm_count), l.cap, l.k_min, l.ev_min);
   ensure_scratch(scratch, L.total);
   rs.p = make_ptrs(L, scratch.ptr, l);
   rs.t = dev_tables(P);
@@ -2136,7 +2142,7 @@ uint64_t regex_candidates(RegexPlan& P, const uint8_t* d_data, uint64_t len, uin
   mode &= ~(uint32_t)WS_CAND_DISTINCT;
   RegexLaunch l{d_data, len, nullptr, cap, nullptr, mode};
   // every candidate must fit: the buffers are sized for the caller's capacity
-  RxLayout L = layout(P, len, effective_chunk(P, len, sm_count), std::max<uint64_t>(cap, 1), cap, cap);
+  RxLayout L = layout(P, len, effective_chunk(P, P.n_spec, len, sm_count), std::max<uint64_t>(cap, 1), cap, cap);
   ensure_scratch(scratch, L.total);
   ScanPtrs p = make_ptrs(L, scratch.ptr, l);
   p.full_k = full ? 1 : 0;
