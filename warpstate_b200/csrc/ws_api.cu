@@ -138,18 +138,26 @@ __global__ void clear_counters_kernel(unsigned long long* count, unsigned long l
 
 uint32_t enqueue_scan(ws_matcher* m, Scratch& s, cudaStream_t st, const uint8_t* d_data, uint64_t len,
                       ws_match* d_out, uint64_t cap, unsigned long long* d_counter, const ScanExtras& x) {
+  return enqueue_scan(m, m->rx, m->lit, s, st, d_data, len, d_out, cap, d_counter, x);
+}
+
+bool scans_prefixes(const ws_matcher* m, const RegexPlan& rx, const LiteralPlan& lit) {
+  // not where the walk is pinned or goes over every group all the same
+  const bool spared = rx.n_walk < rx.n_spec || rx.n_ctx_walk < rx.n_groups;
+  return spared && lit.n_prefixes && m->cfg.regex_mode == WS_REGEX_SPECULATIVE && !m->walk_pinned;
+}
+
+uint32_t enqueue_scan(ws_matcher* m, RegexPlan& rx, const LiteralPlan& lit, Scratch& s, cudaStream_t st,
+                      const uint8_t* d_data, uint64_t len, ws_match* d_out, uint64_t cap, unsigned long long* d_counter,
+                      const ScanExtras& x) {
   const bool prof = m->profile;
   uint32_t launches = 0;
   m->use_summed = false;
   if (prof) check_cuda(cudaEventRecord(m->pev[0], st), "event");
   RegexLaunch rl{d_data, len, d_out, cap, d_counter, m->cfg.regex_mode};
   RegexScan rs;
-  // the literal filter also looks for the regexes' prefixes, unless the walk
-  // is pinned or goes over every group all the same
-  const bool spared = m->rx.n_walk < m->rx.n_spec || m->rx.n_ctx_walk < m->rx.n_groups;
-  const bool prefixes =
-      spared && m->lit.n_prefixes && m->cfg.regex_mode == WS_REGEX_SPECULATIVE && !m->walk_pinned;
-  if (m->rx.n_regex) {
+  const bool prefixes = scans_prefixes(m, rx, lit);  // the literal filter also looks for the regexes' prefixes
+  if (rx.n_regex) {
     rl.item_end = x.item_end;
     rl.n_items = x.n_items;
     rl.cursor = x.cursor;
@@ -164,13 +172,13 @@ uint32_t enqueue_scan(ws_matcher* m, Scratch& s, cudaStream_t st, const uint8_t*
       rl.k_min = k ? k + k / 4 : 0;
       rl.ev_min = e ? e + e / 4 : 0;
     }
-    regex_begin(m->rx, rl, st, s.rx, m->ctx->sm_count, prof, prefixes, rs);
+    regex_begin(rx, rl, st, s.rx, m->ctx->sm_count, prof, prefixes, rs);
   }
-  const bool filter = (m->lit.n_literals && x.literals) || prefixes;
+  const bool filter = (lit.n_literals && x.literals) || prefixes;
   const uint64_t scap = literal_survivor_cap(len);
   if (filter) ensure(s.lit, literal_scratch_bytes(scap));
   clear_counters_kernel<<<1, 256, 0, st>>>(d_counter, filter ? s.lit.as<unsigned long long>() : nullptr, rs.p.ctr,
-                                           m->rx.n_regex ? rs.clear_words : 0);
+                                           rx.n_regex ? rs.clear_words : 0);
   check_cuda(cudaGetLastError(), "clear_counters_kernel");
   if (filter) {
     LiteralLaunch ll{d_data, len, d_out, cap, d_counter, s.lit.ptr, scap};
@@ -179,19 +187,19 @@ uint32_t enqueue_scan(ws_matcher* m, Scratch& s, cudaStream_t st, const uint8_t*
     ll.min_end = x.lit_min_end;
     ll.max_start = x.lit_max_start;
     ll.cleared = true;
-    ll.literals = m->lit.n_literals && x.literals;
+    ll.literals = lit.n_literals && x.literals;
     ll.rx = prefixes ? &rs : nullptr;
-    launch_literal_scan(m->lit, ll, st, m->ctx->sm_count);
+    launch_literal_scan(lit, ll, st, m->ctx->sm_count);
     launches += 2;
   }
   if (prof) check_cuda(cudaEventRecord(m->pev[1], st), "event");
-  if (m->rx.n_regex)
-    launches += regex_finish(m->rx, rs, rl, st, m->ctx->sm_count, prof ? m->rx_events : nullptr);
+  if (rx.n_regex)
+    launches += regex_finish(rx, rs, rl, st, m->ctx->sm_count, prof ? m->rx_events : nullptr);
   if (prof) check_cuda(cudaEventRecord(m->pev[2], st), "event");
   check_cuda(cudaEventRecord(s.busy, st), "event");
   std::lock_guard<std::mutex> g(m->info_mu);
   m->info.last_launches = launches;
-  m->info.last_chunks = m->rx.last_chunks;
+  m->info.last_chunks = rx.last_chunks;
   return launches;
 }
 
@@ -335,6 +343,12 @@ ws_pattern_tables ws_matcher::tables() const {
   return t;
 }
 
+void ws_matcher::fill_filter_info() {
+  info.filter_q = lit.gram_len;
+  info.filter_period = lit.period;
+  info.filter_bits = lit.table_bits;
+}
+
 void ws_matcher::give(std::unique_ptr<Scratch> s) {
   std::lock_guard<std::mutex> g(pool_mu);
   pool.push_back(std::move(s));
@@ -403,10 +417,8 @@ ws_status ws_matcher_create(ws_ctx* ctx, const ws_pattern_tables* t, const ws_co
     plan_filter(*t, m->rx, m->lit);
     m->info.n_literals = t->n_literals;
     m->info.n_regex = t->n_regex;
-    m->info.filter_q = m->lit.gram_len;
     m->info.max_literal_len = m->max_literal_len;
-    m->info.filter_period = m->lit.period;
-    m->info.filter_bits = m->lit.table_bits;
+    m->fill_filter_info();
     regex_fill_info(m->rx, m->info);
     if (t->n_regex) {
       check_cuda(cudaHostAlloc(reinterpret_cast<void**>(&m->need_host), 2 * sizeof(unsigned long long),

@@ -163,6 +163,7 @@ struct ws_matcher {
   uint32_t hash_window = 0;
   void keep_patterns(const ws_pattern_tables& t);
   ws_pattern_tables tables() const;  // views of the copies
+  void fill_filter_info();           // info's fields of the literal plan
   std::mutex pool_mu;
   std::vector<std::unique_ptr<ws::Scratch>> pool;
   std::mutex info_mu;
@@ -238,6 +239,12 @@ uint64_t device_capacity(const ws_matcher* m);
 uint32_t enqueue_scan(ws_matcher* m, Scratch& s, cudaStream_t st, const uint8_t* d_data, uint64_t len,
                       ws_match* d_out, uint64_t cap, unsigned long long* d_counter,
                       const ScanExtras& x = ScanExtras());
+// The same with other plans of the matcher's patterns (the autotuner's).
+uint32_t enqueue_scan(ws_matcher* m, RegexPlan& rx, const LiteralPlan& lit, Scratch& s, cudaStream_t st,
+                      const uint8_t* d_data, uint64_t len, ws_match* d_out, uint64_t cap, unsigned long long* d_counter,
+                      const ScanExtras& x);
+// Whether the matcher's scans by these plans look for the regexes' prefixes.
+bool scans_prefixes(const ws_matcher* m, const RegexPlan& rx, const LiteralPlan& lit);
 // Waits for the last profiled scan and reads its phase times (ms[8], the
 // layout of ws_matcher_info.last_kernel_ms).
 void read_phases(ws_matcher* m, double* ms);

@@ -31,8 +31,12 @@ namespace {
 // the inputs the matcher is meant for.
 constexpr uint64_t kTuneBytes = 1ull << 30;
 
-// Median device time (ms) of the speculative regex scan of `len` bytes.
-double time_regex(ws_matcher* m, RegexPlan& P, const uint8_t* d, uint64_t len, int reps) {
+// Median device time (ms) of what a scan of `len` bytes does for the regexes by
+// these plans, as the entry points enqueue it: the filter's pass for prefixes, and
+// no walk of the groups that it spares.  Where it covers every regex, scans walk
+// only if it gives up; that walk, of every group, is then what the knobs are
+// chosen by (as in plain mode, whose scans have none of them).
+double time_scan(ws_matcher* m, RegexPlan& P, const LiteralPlan& lit, const uint8_t* d, uint64_t len, int reps) {
   cudaStream_t st = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   check_cuda(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -42,16 +46,32 @@ double time_regex(ws_matcher* m, RegexPlan& P, const uint8_t* d, uint64_t len, i
   } cleanup{st, e0, e1};
   check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
   check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
-  DeviceBuffer scratch, out, ctr;
+  const bool whole = m->cfg.regex_mode != WS_REGEX_SPECULATIVE ||
+                     (scans_prefixes(m, P, lit) && P.n_walk == 0 && P.n_ctx_walk == P.n_spec);
+  ScanExtras x;
+  x.literals = false;
+  Scratch s;  // (of its own: a pooled one would keep buffers of this size)
+  check_cuda(cudaEventCreateWithFlags(&s.busy, cudaEventDisableTiming), "cudaEventCreate");
+  // what an overflow here records is not kept for later scans either
+  struct Need {
+    unsigned long long *at, was[2] = {0, 0};
+    explicit Need(unsigned long long* p) : at(p) { if (at) was[0] = at[0], was[1] = at[1]; }
+    ~Need() { if (at) at[0] = was[0], at[1] = was[1]; }
+  } need(m->need_host);
+  DeviceBuffer out, ctr;
   const uint64_t cap = device_capacity(m);
   out.alloc(cap * sizeof(ws_match));
   ctr.alloc(64);
-  RegexLaunch rl{d, len, out.as<ws_match>(), cap, ctr.as<unsigned long long>(), WS_REGEX_SPECULATIVE};
+  auto* counter = ctr.as<unsigned long long>();
+  RegexLaunch rl{d, len, out.as<ws_match>(), cap, counter, WS_REGEX_SPECULATIVE};
   std::vector<float> ts;
   for (int r = -1; r < reps; ++r) {  // r = -1: warm-up (sizes the scratch)
     check_cuda(cudaMemsetAsync(ctr.ptr, 0, 8, st), "memset");
     check_cuda(cudaEventRecord(e0, st), "event");
-    run_regex_scan(P, rl, st, scratch, m->ctx->sm_count, nullptr);
+    if (whole)
+      run_regex_scan(P, rl, st, s.rx, m->ctx->sm_count, nullptr);
+    else
+      enqueue_scan(m, P, lit, s, st, d, len, out.as<ws_match>(), cap, counter, x);
     check_cuda(cudaEventRecord(e1, st), "event");
     check_cuda(cudaStreamSynchronize(st), "tune scan");
     float ms = 0;
@@ -92,25 +112,42 @@ extern "C" ws_status ws_matcher_tune(ws_matcher* m, const uint8_t* corpus, uint6
         // visited rows stay hot (the class-indexed image holds up to 1,472)
         std::vector<uint32_t> cands = {16384, 32768, 65536, 131072};
         const ws_pattern_tables t = m->tables();
+        // A plan that walks some groups and spares others by their prefixes is
+        // also tried with all of them walked together: where a group more costs
+        // little, that saves the filter's pass.
         double best = 1e300;
+        std::unique_ptr<LiteralPlan> other;  // the filter's plan with prefixes, or without, as m->lit is not
         for (size_t k = 0; k < cands.size(); ++k) {
-          ws_config c = m->cfg;
-          c.dfa_max_states = cands[k];
-          RegexPlan cand;
-          try {
-            plan_regex(t, c, m->ctx->sm_count, cand);
-          } catch (const WsError&) {
-            continue;  // a limit too small for some regex: not a candidate
-          }
-          regex_rerank_from_corpus(cand, dc, rlen);
-          const double ms = time_regex(m, cand, tiled.as<uint8_t>(), tlen, 3);
-          rep.group_candidates[k] = cands[k];
-          rep.group_ms[k] = ms;
-          if (ms < best) {
-            best = ms;
-            cand.use_proposer = m->cfg.proposer == WS_PROPOSER_MLP;
-            m->rx = std::move(cand);
-            m->cfg.dfa_max_states = cands[k];
+          bool mixed = false;
+          for (int joint = 0; joint < (mixed ? 2 : 1); ++joint) {
+            ws_config c = m->cfg;
+            c.dfa_max_states = cands[k];
+            if (joint) c.proposer = WS_PROPOSER_NONE;  // (no regex is covered)
+            RegexPlan cand;
+            try {
+              plan_regex(t, c, m->ctx->sm_count, cand);
+            } catch (const WsError&) {
+              continue;  // a limit too small for some regex: not a candidate
+            }
+            const uint32_t walked = cand.n_walk + cand.n_ctx_walk - cand.n_spec;
+            mixed = mixed || (walked > 0 && walked < cand.n_groups);
+            const bool prefixes = cand.prefix_len >= 0;
+            const bool have = prefixes == (m->lit.n_prefixes != 0);
+            if (!have && !other) {
+              other = std::make_unique<LiteralPlan>();
+              plan_filter(t, cand, *other);
+            }
+            regex_rerank_from_corpus(cand, dc, rlen);
+            const double ms = time_scan(m, cand, have ? m->lit : *other, tiled.as<uint8_t>(), tlen, 3);
+            rep.group_candidates[k] = cands[k];
+            rep.group_ms[k] = joint ? std::min(rep.group_ms[k], ms) : ms;
+            if (ms < best) {
+              best = ms;
+              cand.use_proposer = m->cfg.proposer == WS_PROPOSER_MLP;
+              if (!have) std::swap(m->lit, *other);
+              m->rx = std::move(cand);
+              m->cfg.dfa_max_states = cands[k];
+            }
           }
         }
       } else {
@@ -144,7 +181,7 @@ extern "C" ws_status ws_matcher_tune(ws_matcher* m, const uint8_t* corpus, uint6
           m->rx.walk_chunk = chunks[k];
           for (int p = 0; p < (trained ? 2 : 1); ++p) {
             m->rx.use_proposer = p == 1;
-            const double ms = time_regex(m, m->rx, tiled.as<uint8_t>(), tlen, 3);
+            const double ms = time_scan(m, m->rx, m->lit, tiled.as<uint8_t>(), tlen, 3);
             rep.chunk_ms[k][p] = ms;
             if (ms < best) { best = ms; best_chunk = chunks[k]; best_prop = p == 1; }
           }
@@ -155,6 +192,7 @@ extern "C" ws_status ws_matcher_tune(ws_matcher* m, const uint8_t* corpus, uint6
       }
       std::lock_guard<std::mutex> g(m->info_mu);
       regex_fill_info(m->rx, m->info);
+      m->fill_filter_info();
       m->info.proposer_top1 = rep.proposer_top1;
       m->info.proposer_top4 = rep.proposer_top4;
     }
