@@ -70,3 +70,21 @@ def test_overlapping_ends_merge_across_tiles():
     exp = oracle.scan_patterns([(1, p) for p in pats], d)
     assert len(exp) > 20_000
     assert np.array_equal(build(pats).scan_array(d), exp)
+
+
+@pytest.mark.parametrize("walked", [[], [rb"[0-9]{1,3}px"]])
+def test_candidates_of_prefixes_overflow_and_are_counted(walked):
+    # ten candidate starts per match: more than the candidate buffer holds on the
+    # first try, whose counts size the second
+    unit = b"abcd" * 10 + b" 12px " + b"-" * 754
+    d = np.frombuffer(unit * ((24 << 20) // len(unit)), dtype=np.uint8)
+    pats = [rb"(?:abcd)+", rb"key=[0-9]"] + walked
+    exp = oracle.scan_patterns([(1, p) for p in pats], d)
+    import warpstate_b200 as ws
+    b = ws.PatternSet.builder()
+    for p in pats:
+        b = b.regex(p.decode())
+    m = ws.GpuMatcher.with_config(b.build(), ws.AutoMatcherConfig().max_matches(70_000))
+    assert len(exp) == (1 + len(walked)) * (len(d) // len(unit))
+    assert np.array_equal(m.scan_array(d), exp)
+    assert np.array_equal(m.scan_array(d), exp)

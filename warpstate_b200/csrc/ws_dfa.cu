@@ -888,10 +888,12 @@ __global__ void __launch_bounds__(256) k_scatter_kernel(ScanPtrs p, uint32_t n_r
     for (uint32_t i = 0; i < 4; ++i)
       if (k + i * stride < n) c[i] = p.k[k + i * stride];
 #pragma unroll
-    for (uint32_t i = 0; i < 4; ++i)
-      if (k + i * stride < n)
-        p.pair[offs[c[i].r] + (c[i].rank & ~kEndKnown)] =
-            ((unsigned long long)c[i].s << 32) | ((c[i].rank & kEndKnown) ? c[i].e : kLfTodo);
+    for (uint32_t i = 0; i < 4; ++i) {
+      if (k + i * stride >= n) continue;
+      const uint64_t at = (uint64_t)offs[c[i].r] + (c[i].rank & ~kEndKnown);
+      if (at < p.k_cap)  // (a scan whose candidates did not fit has counted more)
+        p.pair[at] = ((unsigned long long)c[i].s << 32) | ((c[i].rank & kEndKnown) ? c[i].e : kLfTodo);
+    }
   }
 }
 
@@ -976,6 +978,7 @@ __global__ void __launch_bounds__(512) k_sort_kernel(ScanPtrs p, uint32_t n_rege
   pdl_begin();
   __shared__ unsigned long long buf[kSortTile];
   __shared__ bool last;
+  if (p.ctr[C_ERR]) return;
   for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
     const uint32_t a = p.offs[r], n = p.offs[r + 1] - a, tiles = (n + kSortTile - 1) / kSortTile;
     if (n < 2) continue;
@@ -1011,6 +1014,7 @@ __global__ void k_lf_kernel(DevTables t, ScanPtrs p, uint32_t n_regex) {
   pdl_begin();
   extern __shared__ uint32_t offs_s[];
   const bool staged = n_regex < kOffsShared;
+  if (p.ctr[C_ERR]) return;
   if (staged) {
     for (uint32_t r = threadIdx.x; r <= n_regex; r += blockDim.x) offs_s[r] = p.offs[r];
     __syncthreads();

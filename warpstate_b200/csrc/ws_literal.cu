@@ -1062,7 +1062,7 @@ __global__ void __launch_bounds__(kVerifyThreads, 4) literal_verify_kernel(const
     for (uint32_t i = lane; i < nm; i += 32)
       if (at + i < a.cap) a.out[at + i] = ws_match{mbuf[wi][i].x, mbuf[wi][i].y, mbuf[wi][i].z};
     for (uint32_t i = lane; RX && i < nk; i += 32)
-      store_k(p, kat + i, kbuf[wi][i].x, kbuf[wi][i].y, kbuf[wi][i].z, kEndKnown);
+      store_k(p, kat + i, kbuf[wi][i].x, kbuf[wi][i].y, kbuf[wi][i].z, atomicAdd(&p.count[kbuf[wi][i].x], 1u) | kEndKnown);
   };
   auto drain = [&]() {  // by the warp, after each step
     __syncwarp();

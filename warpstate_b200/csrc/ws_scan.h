@@ -103,16 +103,21 @@ __device__ __forceinline__ unsigned long long warp_append(unsigned long long* co
   return base + g.thread_rank();
 }
 
-// Stores candidate i of K and counts it for its regex (the per-regex counts
-// size the resolution's lists, the rank is its place in one).
+// Stores candidate i of K with its rank among its regex's candidates (the
+// per-regex counts size the resolution's lists, the rank is its place in one).
+// A candidate is counted whether it fits or not, so that its two atomics do not
+// wait for one another (1,000 regexes that match at the same places of 256 MiB:
+// 3,000 -> 2,190 us a scan, 2,160 to 2,290 before candidates had ranks); the lists
+// of a scan whose candidates did not fit are not read.
 __device__ __forceinline__ void store_k(const ScanPtrs& p, unsigned long long i, uint32_t r, uint32_t s, uint32_t e,
-                                        uint32_t known) {
-  if (i < p.k_cap) p.k[i] = KCand{r, s, e, atomicAdd(&p.count[r], 1u) | known};
+                                        uint32_t rank_known) {
+  if (i < p.k_cap) p.k[i] = KCand{r, s, e, rank_known};
   else atomicOr(&p.ctr[C_ERR], 1ull);
 }
 
 __device__ __forceinline__ void emit_k(const ScanPtrs& p, uint32_t r, uint32_t s, uint32_t e, uint32_t known = 0) {
-  store_k(p, warp_append(&p.ctr[C_K]), r, s, e, known);
+  const uint32_t rank = atomicAdd(&p.count[r], 1u);
+  store_k(p, warp_append(&p.ctr[C_K]), r, s, e, rank | known);
 }
 
 // Context of a byte for the assertions (byte_context in ws_regex.h).
