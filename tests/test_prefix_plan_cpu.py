@@ -72,3 +72,41 @@ def test_sets_over_letters_are_covered_at_their_length():
     assert prefix_plan([], words) == (7, [True] * 3)
     assert prefix_plan([], words + [r"[0-9]+px"])[1] == [True] * 3 + [False]
     assert prefix_plan([], [r"[0-9]+px"]) == (0, [False])
+
+
+def sharing(n, head, seed=8):
+    r = random.Random(seed)
+    tails = set()
+    while len(tails) < n:
+        tails.add("".join(r.choices("abcdefghij", k=r.randint(5, 10))))
+    return [f"{head}{t}/[a-z0-9]{{1,6}}" for t in sorted(tails)]
+
+
+@pytest.mark.parametrize("n", [1, 24, 25, 300])
+def test_regexes_that_share_a_beginning(n):
+    # up to 24 regexes are walked in turn from a beginning they share; more of
+    # them are left to their groups' walk, the others stay with the filter
+    rx = [r"alpha[0-9]{1,3}x", r"tailwind [0-9]", r"key=[0-9]+"]
+    got, covered = prefix_plan([], sharing(n, "http://www.") + rx)
+    assert got > 0 and covered == [n <= 24] * n + [True] * 3
+    # a shorter beginning of the same words counts with the longer ones
+    got, covered = prefix_plan([], sharing(n, "http://www.") + rx + ["http[0-9s]*:", "http:[/]?x"])
+    assert covered[:n] == [n + 1 <= 24] * n and covered[n:n + 3] == [True] * 3
+
+
+def test_regexes_with_beginnings_of_their_own_are_all_covered():
+    assert prefix_plan([], joined_words(400))[1] == [True] * 400
+
+
+def joined_words(n):
+    r = random.Random(12)
+    return ["".join(r.choices("abcdefghijklmnop", k=9)) + "[0-9]{1,4}x" for _ in range(n)]
+
+
+@pytest.mark.parametrize("n", [20, 70])
+def test_buckets_by_four_bytes_stay_short(n):
+    # n beginnings of 8 bytes with the same first 4, and one regex whose own has
+    # only 4: it would make the table's buckets go by 4 bytes
+    rx = ["user" + "".join(chr(97 + (i // 5 ** k) % 5) for k in range(4)) + "[0-9]{1,3};" for i in range(n)]
+    got, covered = prefix_plan([], rx + [r"abcd[0-9a-f]+;"])
+    assert covered[:n] == [True] * n and covered[n] == (n <= 64)

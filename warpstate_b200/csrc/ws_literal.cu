@@ -941,25 +941,30 @@ __global__ void __launch_bounds__(kGramThreads, 1) literal_gram_kernel(const __g
 // A position where a covered regex's prefix may start: every regex of which one
 // does (entries of different regexes may share it) runs its leftmost-first walk
 // from there, and a match makes a candidate.  A walk still open after kLfCap
-// bytes, or more long walks than the input has bytes, give the prefix
-// candidates up: the regexes' groups are walked instead (ctr[C_GATE]), whose
-// cost does not depend on the input.
+// bytes gives the prefix candidates up: the regexes' groups are walked instead
+// (ctr[C_GATE]), whose cost does not depend on the input.  So do walks of more
+// steps than kWorkPerByte per input byte, entries looked at included; a long
+// walk, which keeps its whole warp waiting, counts for more.  A warp reports its
+// work in pieces of at least kWorkReport.
+constexpr uint32_t kWorkPerByte = 8, kLongWalk = 64, kLongWeight = 8, kWorkReport = 16384;
 template <class Sink>
 __device__ __forceinline__ void verify_prefixes(const LitArgs& a, const DevTables& t, const ScanPtrs& p,
                                                 const PrefixDev& pf, uint32_t s, uint32_t lo, uint32_t hi, uint32_t k,
-                                                uint32_t k1, bool gate, Sink&& sink) {
+                                                uint32_t k1, bool gate, uint32_t& work, Sink&& sink) {
   // every lane finds its next entry, then the lanes that have one walk together
   while (true) {
     uint32_t r = 0xFFFFFFFFu;
     while (k < k1 && r == 0xFFFFFFFFu) {
       const uint4 e = __ldg(pf.entry + k++);
+      ++work;
       if (e.x == lo && !((e.y ^ hi) & e.z)) r = e.w;
     }
     if (__ballot_sync(0xFFFFFFFFu, r != 0xFFFFFFFFu) == 0) return;
     if (r != 0xFFFFFFFFu && !gate) {
       uint32_t steps = 0;
       const uint32_t end = lf_walk(t, p, r, s, kLfCap, &steps);
-      if (end == kLfOpen || (steps > 64 && atomicAdd(&p.ctr[C_WORK], (unsigned long long)steps) > a.len)) {
+      work += steps > kLongWalk ? kLongWeight * steps : steps;
+      if (end == kLfOpen) {
         atomicOr(&p.ctr[C_GATE], 1ull);
         gate = true;
       } else if (end != kLfNone) {
@@ -1087,6 +1092,7 @@ __global__ void __launch_bounds__(kVerifyThreads, 4) literal_verify_kernel(const
   // for one another.
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const uint32_t w = blockIdx.x + gridDim.x * wi;
+  uint32_t warp_work = 0;
   for (unsigned long long k0 = 0; k0 < n && !dense; k0 += 32ull * warps) {  // the same for all lanes
     const unsigned long long k = k0 + (unsigned long long)lane * warps + w;
     const uint32_t s = k < n ? a.survivors[k] : kNoSurvivor;
@@ -1118,7 +1124,16 @@ __global__ void __launch_bounds__(kVerifyThreads, 4) literal_verify_kernel(const
       else probe_literals(a, lo, hi, len - s, pr);
       verify_literals(a, s, a.fold ? ascii_fold4(x0) : x0, a.fold ? ascii_fold4(next) : next, pr, match);
     }
-    if (RX) verify_prefixes(a, t, p, pf, s, lo, hi, pk, pk1, gate, candidate);
+    if (RX) {
+      uint32_t work = 0;
+      verify_prefixes(a, t, p, pf, s, lo, hi, pk, pk1, gate, work, candidate);
+      warp_work += __reduce_add_sync(0xFFFFFFFFu, work);
+      if (warp_work >= kWorkReport) {
+        if (lane == 0 && atomicAdd(&p.ctr[C_WORK], (unsigned long long)warp_work) + warp_work > kWorkPerByte * a.len)
+          atomicOr(&p.ctr[C_GATE], 1ull);
+        warp_work = 0;
+      }
+    }
     drain();
   }
   if (dense && a.parts) {

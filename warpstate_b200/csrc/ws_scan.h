@@ -33,7 +33,7 @@ struct Event { uint32_t e, state, q, tag; };
 //  [8] chunk re-walks of the fix-up  [9] bytes those re-walks stepped
 //  [10] boundary guesses that were the true state  [11] boundary guesses
 //  [12] the prefix candidates were given up (the gated groups walk)
-//  [13] bytes stepped by long walks from prefixes  [14] finished verify blocks
+//  [13] steps of the walks from prefixes (weighted)  [14] finished verify blocks
 //  [15] some regex's candidates are more than a block resolves alone
 enum { C_K = 0, C_EV = 1, C_ERR = 2, C_ROUND = 3, C_FIX = 8, C_REWALK = 9, C_HITS = 10, C_GUESSES = 11, C_GATE = 12,
        C_WORK = 13, C_TICKET = 14, C_LONG = 15 };
