@@ -897,17 +897,16 @@ __global__ void __launch_bounds__(256) k_scatter_kernel(ScanPtrs p, uint32_t n_r
   }
 }
 
-// Block-wide bitonic sort of buf[0, m) in shared memory (m a power of two).
-__device__ void bitonic_smem(unsigned long long* buf, uint32_t m) {
+// Block-wide bitonic sort of buf[0, m) in shared memory (m a power of two), a
+// pair per thread and turn.
+__device__ __forceinline__ void bitonic_smem(unsigned long long* buf, uint32_t m) {
   for (uint32_t size = 2; size <= m; size <<= 1) {
     for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) {
-        uint32_t j = k ^ stride;
-        if (j > k) {
-          bool up = (k & size) == 0;
-          unsigned long long x = buf[k], y = buf[j];
-          if ((x > y) == up) { buf[k] = y; buf[j] = x; }
-        }
+      for (uint32_t i = threadIdx.x; i < m / 2; i += blockDim.x) {
+        const uint32_t k = 2 * i - (i & (stride - 1)), j = k + stride;
+        const bool up = (k & size) == 0;
+        const unsigned long long x = buf[k], y = buf[j];
+        if ((x > y) == up) { buf[k] = y; buf[j] = x; }
       }
       __syncthreads();
     }
@@ -915,7 +914,7 @@ __device__ void bitonic_smem(unsigned long long* buf, uint32_t m) {
 }
 
 // Sorts src[0, n), n <= kSortTile, into buf (shared memory).
-__device__ void sort_into(unsigned long long* buf, const unsigned long long* src, uint32_t n) {
+__device__ __forceinline__ void sort_into(unsigned long long* buf, const unsigned long long* src, uint32_t n) {
   uint32_t m = 1;
   while (m < n) m <<= 1;
   for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) buf[k] = (k < n) ? src[k] : ~0ull;
