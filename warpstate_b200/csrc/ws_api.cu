@@ -180,6 +180,7 @@ uint32_t enqueue_scan(ws_matcher* m, RegexPlan& rx, const LiteralPlan& lit, Scra
   clear_counters_kernel<<<1, 256, 0, st>>>(d_counter, filter ? s.lit.as<unsigned long long>() : nullptr, rs.p.ctr,
                                            rx.n_regex ? rs.clear_words : 0);
   check_cuda(cudaGetLastError(), "clear_counters_kernel");
+  launches += 1;
   if (filter) {
     LiteralLaunch ll{d_data, len, d_out, cap, d_counter, s.lit.ptr, scap};
     ll.item_end = x.item_end;
