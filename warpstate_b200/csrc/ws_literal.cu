@@ -485,33 +485,27 @@ __global__ void __launch_bounds__(kThreads, 1) literal_filter_kernel(const __gri
   }
 }
 
-// Stage 1 of the P = 4 layouts with the stage-1b table, split in two so that
-// the L2 loads of a block are in flight while the previous block finishes:
-// grams_issue hashes the five aligned grams of a lane (the fifth only on lane
-// 31), looks them up in shared memory and starts the L2 loads of the passing
+// Stage 1 of 4-byte grams at every fourth position with the stage-1b table, split
+// in two so that the L2 loads of a block are in flight while the previous block
+// finishes: grams_issue hashes the five aligned grams of a lane (the fifth only on
+// lane 31), looks them up in shared memory and starts the L2 loads of the passing
 // ones; grams_finish combines them into the 16-bit candidate mask.
 struct Grams {
-  uint32_t h[5], n[5], bw[5];
+  uint32_t n[5], bw[5];
 };
 
-template <int G>
-__device__ __forceinline__ void grams_issue(const uint32_t* filt, const uint8_t* big, const uint32_t (&w)[8],
-                                            uint32_t lane, uint32_t bits, Grams& s) {
+__device__ __forceinline__ void grams_issue(const uint32_t* filt, const uint8_t* big, const uint32_t (&w)[5],
+                                            uint32_t lane, Grams& s) {
 #pragma unroll
   for (int j = 0; j < 5; ++j) {
     if (j == 4 && lane != 31) {
-      s.h[4] = 0;
       s.n[4] = 0;
       s.bw[4] = 0;
       break;
     }
-    uint32_t hf;
-    if (G == 4) hf = w[j] * 0x9E3779B1u;
-    else if (G == 8) hf = mix_words(w[j], w[j + 1], 0, 0, 8);
-    else hf = mix_words(w[j], w[j + 1], w[j + 2], w[j + 3], 16);
+    const uint32_t hf = w[j] * 0x9E3779B1u;
     // stage 1: the 2^kLeanBits-bit bitmap derived from the stage-1b table
     const uint32_t b = hf >> (32 - kLeanBits);
-    s.h[j] = hf;
     s.n[j] = ((filt[b >> 5] >> (b & 31)) & 1u) ? 0xFu : 0u;
     s.bw[j] = s.n[j] ? __ldg(big + (hf >> (32 - kBigBits))) : 0u;
   }
@@ -526,45 +520,33 @@ __device__ __forceinline__ uint32_t grams_finish(const Grams& s, uint32_t lane) 
   return (m >> 3) & 0xFFFFu;
 }
 
-// The words a lane needs: its own four and the next lane's four (the tail
-// vector on lane 31).
-template <int G>
-__device__ __forceinline__ void lane_words(const uint4& cur, const uint4& tail, uint32_t lane, uint32_t (&w)[8]) {
+// The words a lane needs: its own four and the next lane's first (the tail
+// vector's on lane 31).
+__device__ __forceinline__ void lane_words(const uint4& cur, const uint4& tail, uint32_t lane, uint32_t (&w)[5]) {
   w[0] = cur.x;
   w[1] = cur.y;
   w[2] = cur.z;
   w[3] = cur.w;
   w[4] = __shfl_down_sync(0xFFFFFFFFu, cur.x, 1);
-  w[5] = w[6] = w[7] = 0;
-  if (G > 4) {
-    w[5] = __shfl_down_sync(0xFFFFFFFFu, cur.y, 1);
-    w[6] = __shfl_down_sync(0xFFFFFFFFu, cur.z, 1);
-    w[7] = __shfl_down_sync(0xFFFFFFFFu, cur.w, 1);
-  }
-  if (lane == 31) {
-    w[4] = tail.x;
-    w[5] = tail.y;
-    w[6] = tail.z;
-    w[7] = tail.w;
-  }
+  if (lane == 31) w[4] = tail.x;
 }
 
 constexpr int kBigThreads = 512;
 constexpr int kBigWarps = kBigThreads / 32;
 
-// P = 4 with the stage-1b table in L2: the same work as literal_filter_kernel
+// 4-byte grams at every fourth position with the stage-1b table in L2, and literals
+// of one to three bytes: the same work as literal_filter_kernel
 // in a three-block software pipeline per warp -- the input of block i+2 is
 // loaded, the grams of block i+1 are hashed and their L2 checks issued, then
 // block i is finished -- so that the L2 latency overlaps useful work.
 // 16 warps per CTA leave room for the pipeline's registers.
-template <int G, bool SHORT>
 __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(const __grid_constant__ LitArgs a) {
   pdl_begin();
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* filt = smem;
   uint32_t* bloom = filt + a.filter_words;
   uint32_t* shortb = bloom + (1u << (kBloomBits - 5));
-  uint32_t* warpmem = shortb + (SHORT ? 2048 : 0);
+  uint32_t* warpmem = shortb + 2048;
   {
     const uint4* src = reinterpret_cast<const uint4*>(a.filter);
     uint4* dst = reinterpret_cast<uint4*>(filt);
@@ -572,11 +554,9 @@ __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(cons
     const uint4* bs = reinterpret_cast<const uint4*>(a.bloom);
     uint4* bd = reinterpret_cast<uint4*>(bloom);
     for (uint32_t k = threadIdx.x; k < (1u << (kBloomBits - 7)); k += kBigThreads) bd[k] = __ldg(bs + k);
-    if (SHORT) {
-      const uint4* s2 = reinterpret_cast<const uint4*>(a.short_bits);
-      uint4* d2 = reinterpret_cast<uint4*>(shortb);
-      for (uint32_t k = threadIdx.x; k < 512; k += kBigThreads) d2[k] = __ldg(s2 + k);
-    }
+    const uint4* s2 = reinterpret_cast<const uint4*>(a.short_bits);
+    uint4* d2 = reinterpret_cast<uint4*>(shortb);
+    for (uint32_t k = threadIdx.x; k < 512; k += kBigThreads) d2[k] = __ldg(s2 + k);
   }
   __syncthreads();
 
@@ -589,7 +569,6 @@ __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(cons
   const uint32_t full_vecs = len >> 4;
   const uint32_t nblk = (nvec + 31) >> 5;
   const uint32_t nwarps = gridDim.x * kBigWarps;
-  const uint32_t bits = a.bits;
   auto load = [&](uint32_t v) -> uint4 {
     const uint4 x = v < full_vecs ? __ldg(reinterpret_cast<const uint4*>(a.data) + v)
                     : v < nvec ? load_vec(a.data, a.len, v) : make_uint4(0, 0, 0, 0);
@@ -604,9 +583,9 @@ __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(cons
   if (b < nblk) {
     cur = load(b * 32 + lane);
     tail_c = lane == 31 ? load(b * 32 + 32) : zero;
-    uint32_t w[8];
-    lane_words<G>(cur, tail_c, lane, w);
-    grams_issue<G>(filt, a.big, w, lane, bits, gc);
+    uint32_t w[5];
+    lane_words(cur, tail_c, lane, w);
+    grams_issue(filt, a.big, w, lane, gc);
   }
   if (b + nwarps < nblk) {
     nxt = load((b + nwarps) * 32 + lane);
@@ -623,20 +602,18 @@ __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(cons
     // grams of block b + nwarps, L2 checks issued
     Grams gn;
     if (bn < nblk) {
-      uint32_t w[8];
-      lane_words<G>(nxt, tail_n, lane, w);
-      grams_issue<G>(filt, a.big, w, lane, bits, gn);
+      uint32_t w[5];
+      lane_words(nxt, tail_n, lane, w);
+      grams_issue(filt, a.big, w, lane, gn);
     }
     // finish block b
     uint32_t mask = grams_finish(gc, lane);
-    if (SHORT) {
-      uint32_t w[8];
-      lane_words<G>(cur, tail_c, lane, w);
+    uint32_t w[5];
+    lane_words(cur, tail_c, lane, w);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const uint32_t g = __funnelshift_r(w[j >> 2], w[(j >> 2) + 1], 8 * (j & 3)) & 0xFFFFu;
-        mask |= ((shortb[g >> 5] >> (g & 31)) & 1u) << j;
-      }
+    for (int j = 0; j < 16; ++j) {
+      const uint32_t g = __funnelshift_r(w[j >> 2], w[(j >> 2) + 1], 8 * (j & 3)) & 0xFFFFu;
+      mask |= ((shortb[g >> 5] >> (g & 31)) & 1u) << j;
     }
     const uint32_t v = b * 32 + lane;
     if (v >= full_vecs) {
@@ -645,7 +622,7 @@ __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(cons
       mask &= (valid >= 16) ? 0xFFFFu : ((1u << valid) - 1u);
     }
     if (__ballot_sync(0xFFFFFFFFu, mask != 0) != 0)
-      process_block<G>(a, blk, queue, bloom, lane, cur, tail_c, mask, b * 512);
+      process_block<4>(a, blk, queue, bloom, lane, cur, tail_c, mask, b * 512);
     cur = nxt;
     tail_c = tail_n;
     gc = gn;
@@ -1269,19 +1246,13 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   uint64_t want = (nblk + kWarps - 1) / kWarps;
   int grid = (int)std::min<uint64_t>((uint64_t)sm_count, std::max<uint64_t>(want, 1));
   // the filter layout is a compile-time choice of the kernel
-  auto run = [&](auto kernel) {
+  auto run = [&](auto kernel, int threads = kThreads) {
     check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "cudaFuncSetAttribute(literal)");
-    launch_pdl(kernel, grid, kThreads, smem, st, a);
+    launch_pdl(kernel, grid, threads, smem, st, a);
     check_cuda(cudaGetLastError(), "literal_filter_kernel launch");
   };
   const bool lg = plan.has_long != 0, sh = plan.has_short != 0;
-  auto run_big = [&](auto kernel) {
-    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-               "cudaFuncSetAttribute(literal)");
-    launch_pdl(kernel, grid, kBigThreads, smem, st, a);
-    check_cuda(cudaGetLastError(), "literal_filter_big_kernel launch");
-  };
   auto run_gram = [&](auto kernel, uint32_t run_bytes) {
     // a warp per run of run_bytes, or per 512-byte vector after the last one
     const uint64_t units = l.len / run_bytes + (l.len % run_bytes + 511) / 512;
@@ -1307,7 +1278,7 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
     else if (plan.period == 2) run_gram(two ? literal_gram_kernel<2, 4, 2> : literal_gram_kernel<2, 4, 1>, 2048);
     else run_gram(two ? literal_gram_kernel<1, 4, 2> : literal_gram_kernel<1, 4, 1>, 1024);
   } else if (lg && sh && a.big && plan.period == 4 && plan.gram_len == 4) {
-    run_big(literal_filter_big_kernel<4, true>);
+    run(literal_filter_big_kernel, kBigThreads);
   } else if (!lg) {
     run(literal_filter_kernel<4, 4, false, true>);
   } else if (plan.gram_len == 16) {
