@@ -290,7 +290,7 @@ struct LiteralLaunch {
   uint64_t min_end = 0;
   // Shard scans: only matches starting before this offset are this shard's.
   uint64_t max_start = ~0ull;
-  bool cleared = false;          // the scratch's survivor count is zero already
+  bool cleared = false;          // by a kernel of this scan (else the filter is the scan's first kernel)
   bool literals = true;          // report literal matches (else only the regexes' prefixes are looked for)
   const RegexScan* rx = nullptr;  // the regex scan that takes the prefixes' candidates
 };

@@ -28,8 +28,9 @@ __device__ __forceinline__ void pdl_begin() {
   pdl_wait();
 }
 
+// `first`: the first kernel of a scan, launched the ordinary way.
 template <class... P, class... A>
-void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+void launch_scan(bool first, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t c{};
   c.gridDim = grid;
   c.blockDim = block;
@@ -39,8 +40,13 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaSt
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   c.attrs = at;
-  c.numAttrs = 1;
+  c.numAttrs = first ? 0 : 1;
   check_cuda(cudaLaunchKernelEx(&c, kernel, static_cast<P>(std::forward<A>(args))...), "kernel launch");
+}
+
+template <class... P, class... A>
+void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  launch_scan(false, kernel, grid, block, smem, st, std::forward<A>(args)...);
 }
 
 }  // namespace ws

@@ -1249,7 +1249,7 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
   auto run = [&](auto kernel, int threads = kThreads) {
     check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "cudaFuncSetAttribute(literal)");
-    launch_pdl(kernel, grid, threads, smem, st, a);
+    launch_scan(!l.cleared, kernel, grid, threads, smem, st, a);
     check_cuda(cudaGetLastError(), "literal_filter_kernel launch");
   };
   const bool lg = plan.has_long != 0, sh = plan.has_short != 0;
@@ -1264,7 +1264,7 @@ void launch_literal_scan(const LiteralPlan& plan, const LiteralLaunch& l, cudaSt
     const size_t gsmem = ((size_t)4 << plan.gram_word_bits) + (size_t)kGramWarps * kGramQueue * 4;
     check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem),
                "cudaFuncSetAttribute(literal gram)");
-    launch_pdl(kernel, blocks, kGramThreads, gsmem, st, a);
+    launch_scan(!l.cleared, kernel, blocks, kGramThreads, gsmem, st, a);
     check_cuda(cudaGetLastError(), "literal_gram_kernel launch");
   };
   // sparse sets: the gram kernel; else with literals shorter than 4 bytes and
