@@ -379,6 +379,17 @@ def boundary_guess(info, tune) -> str:
     return "unanchored start state (the autotuner turned the proposer off)"
 
 
+def candidate_source(info) -> str:
+    """Where a profiled scan's regex candidates came from.  The filter's need no
+    match events and no guessed chunk starts; where it gave up, the walk of its
+    groups leaves events."""
+    if info["n_context_groups"] == info["n_groups"]:
+        return "walk of anchored starts or literal filter"
+    if info["last_guesses"] or info["last_events"]:
+        return "walk" if info["last_guesses"] else "walk (the literal filter gave up)"
+    return "literal filter (no group walked)"
+
+
 def build_matchers(ws, wl, config, walk_chunk=None, proposer=True, dfa_max_states=None, plain_too=True):
     ps = ws.PatternSet.builder()
     for kind, p in wl.patterns:
@@ -412,7 +423,8 @@ def build_matchers(ws, wl, config, walk_chunk=None, proposer=True, dfa_max_state
 def roofline_of(config, infos, n_bytes, count, n_items, batch, has_regex, peak, peak_kind):
     """The dominant kernel's achieved algorithmic bandwidth against the
     measured HBM peak (N input bytes + 12 B per match + 16 B per item)."""
-    # the literal phase (index 0) spans the filter and the verify kernel
+    # the literal phase (index 0) spans the filter and the verify kernel; the sets
+    # of these workloads all take the gram kernel
     lit_name = "literal_gram_kernel"
 
     def phase(k):
@@ -442,7 +454,8 @@ def walk_record(info, n_bytes, ms):
     guesses = info["last_guesses"]
     return {"gbs": round(n_bytes / (ms * 1e-3) / 1e9, 3), "ms_per_step": round(ms, 4),
             "walk_ms": round(walk_ms, 4),
-            # (no boundary was guessed: the candidates came from the literal filter)
+            "candidates_from": candidate_source(info),
+            # (no boundary was guessed: no group was walked)
             "lookups_per_s": round(g * n_bytes / (walk_ms * 1e-3), 1) if walk_ms and guesses else None,
             "guess_hit_rate": round(info["last_guess_hits"] / guesses, 5) if guesses else None,
             "fixup_chunks": info["last_fixup_chunks"], "chunks": info["last_chunks"],
@@ -516,21 +529,6 @@ def main():
     ms_max = max_over_ranks(ms)
     value = world * n_bytes / (ms_max * 1e-3) / 1e9
     has_regex = any(k == 1 for k, _ in wl.patterns)
-
-    # the other boundary guess of the speculative walk, timed the same way:
-    # the trained proposer when the tuner chose the unanchored start, and the
-    # reverse; same chunk, same matches
-    arms = None
-    if has_regex and tune and not args.no_arms and not args.no_proposer and tune["proposer_top1"] > 0:
-        used = tune["proposer_used"]
-        arms = {("proposer" if used else "unanchored"): walk_record(infos[-1], n_bytes, ms)}
-        m.set_walk(0, ws.PROPOSER_NONE if used else ws.PROPOSER_MLP)
-        ams, ainfos = r.timed_steps(m, args.steps, args.warmup)
-        acount = r.count()
-        if acount != count:
-            raise SystemExit(f"match counts differ between boundary guesses: {acount} vs {count}")
-        arms[("unanchored" if used else "proposer")] = walk_record(ainfos[-1], n_bytes, max_over_ranks(ams))
-        m.set_walk(0, ws.PROPOSER_MLP if used else ws.PROPOSER_NONE)
 
     plain_gbs = plain_ms = None
     if plain is not None:
@@ -662,14 +660,44 @@ def main():
     }
     if has_regex:
         last = infos[-1]
-        rec = {"speculative_gbs": round(value, 3),
+        # The speculative walk itself: the scan, or where that took its candidates
+        # from the literal filter, the same steps with the walk pinned.  (The last
+        # uses of this matcher: a pinned walk stays.)
+        def walk_arm(proposer):
+            m.set_walk(0, ws.PROPOSER_MLP if proposer else ws.PROPOSER_NONE)
+            wms, winfos = r.timed_steps(m, args.steps, args.warmup)
+            wcount = r.count()
+            if wcount != count:
+                raise SystemExit(f"match counts differ between the scan and its walk: {wcount} vs {count}")
+            return winfos[-1], max_over_ranks(wms)
+
+        used = bool(tune["proposer_used"])
+        walk_info, walk_ms = last, ms_max
+        if candidate_source(last).startswith("literal filter"):
+            walk_info, walk_ms = walk_arm(used)
+        walk_gbs = world * n_bytes / (walk_ms * 1e-3) / 1e9
+        # the other boundary guess of the walk, timed the same way: the trained
+        # proposer when the tuner chose the unanchored start, and the reverse; same
+        # chunk, same matches
+        arms = None
+        if not args.no_arms and not args.no_proposer and tune["proposer_top1"] > 0:
+            arms = {("proposer" if used else "unanchored"): walk_record(walk_info, n_bytes, walk_ms)}
+            other_info, other_ms = walk_arm(not used)
+            arms["unanchored" if used else "proposer"] = walk_record(other_info, n_bytes, other_ms)
+        rec = {"scan_gbs": round(value, 3),
+               "scan_vs_plain": round(value / plain_gbs, 3) if plain_gbs else None,
+               "speculative_gbs": round(walk_gbs, 3),
                "plain_gbs": round(plain_gbs, 3) if plain_gbs else None,
-               "speedup_vs_plain": round(value / plain_gbs, 3) if plain_gbs else None,
+               "speedup_vs_plain": round(walk_gbs / plain_gbs, 3) if plain_gbs else None,
                "plain_ms_per_step": round(plain_ms, 4) if plain_ms else None,
-               "boundary_guess": boundary_guess(last, tune),
+               "boundary_guess": boundary_guess(walk_info, tune),
                "proposer_top1_heldout": last["proposer_top1"], "proposer_top4_heldout": last["proposer_top4"],
                "tune": tune, "groups": last["n_groups"], "states": last["total_states"]}
         rec.update(walk_record(last, n_bytes, ms_max))
+        if walk_info is not last:  # chunks, guesses and events are those of a walk
+            rec["walk"] = walk_record(walk_info, n_bytes, walk_ms)
+            for k in ("chunks", "fixup_chunks", "rewalk_bytes", "rewalk_frac"):
+                del rec[k]
         rec["step_ms"] = step_ms
         rec["enqueue_ms"] = enqueue_ms
         if arms:
