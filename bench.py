@@ -379,15 +379,15 @@ def boundary_guess(info, tune) -> str:
     return "unanchored start state (the autotuner turned the proposer off)"
 
 
-def candidate_source(info) -> str:
-    """Where a profiled scan's regex candidates came from.  The filter's need no
-    match events and no guessed chunk starts; where it gave up, the walk of its
-    groups leaves events."""
+def candidate_source(info, n_bytes) -> str:
+    """Where a profiled scan's regex candidates came from.  A walk takes at least
+    one lookup per byte, under 2 T/s on the device; the launches of a walk that is
+    left out take a few microseconds."""
     if info["n_context_groups"] == info["n_groups"]:
         return "walk of anchored starts or literal filter"
-    if info["last_guesses"] or info["last_events"]:
-        return "walk" if info["last_guesses"] else "walk (the literal filter gave up)"
-    return "literal filter (no group walked)"
+    if info["last_kernel_ms"][1] * 1e-3 * 4e12 < n_bytes:
+        return "literal filter (no group walked)"
+    return "walk"
 
 
 def build_matchers(ws, wl, config, walk_chunk=None, proposer=True, dfa_max_states=None, plain_too=True):
@@ -454,8 +454,8 @@ def walk_record(info, n_bytes, ms):
     guesses = info["last_guesses"]
     return {"gbs": round(n_bytes / (ms * 1e-3) / 1e9, 3), "ms_per_step": round(ms, 4),
             "walk_ms": round(walk_ms, 4),
-            "candidates_from": candidate_source(info),
-            # (no boundary was guessed: no group was walked)
+            "candidates_from": candidate_source(info, n_bytes),
+            # (guesses are counted where groups were walked)
             "lookups_per_s": round(g * n_bytes / (walk_ms * 1e-3), 1) if walk_ms and guesses else None,
             "guess_hit_rate": round(info["last_guess_hits"] / guesses, 5) if guesses else None,
             "fixup_chunks": info["last_fixup_chunks"], "chunks": info["last_chunks"],
@@ -673,7 +673,7 @@ def main():
 
         used = bool(tune["proposer_used"])
         walk_info, walk_ms = last, ms_max
-        if candidate_source(last).startswith("literal filter"):
+        if candidate_source(last, n_bytes).startswith("literal filter"):
             walk_info, walk_ms = walk_arm(used)
         walk_gbs = world * n_bytes / (walk_ms * 1e-3) / 1e9
         # the other boundary guess of the walk, timed the same way: the trained
