@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <map>
 #include <unordered_map>
 
 namespace ws {
@@ -1011,29 +1012,73 @@ bool regex_prefixes(const Dfa& d, const ByteClasses& cls, bool context, uint32_t
   else starts.push_back(d.start_anchored);
   std::sort(starts.begin(), starts.end());
   starts.erase(std::unique(starts.begin(), starts.end()), starts.end());
-  typedef std::pair<std::string, uint32_t> Item;  // bytes, state after them
-  std::vector<std::string> found;
-  std::vector<Item> cur, nxt;
-  for (uint32_t s : starts) cur.emplace_back(std::string(), s);
-  for (uint32_t depth = 0; !cur.empty(); ++depth) {
+  // The bytes that continue a state, and whether a prefix of `depth` bytes ends there.
+  std::vector<std::vector<uint8_t>> ways(d.n_states);
+  std::vector<uint8_t> known(d.n_states, 0);
+  auto ways_of = [&](uint32_t state) -> const std::vector<uint8_t>& {
+    if (!known[state]) {
+      known[state] = 1;
+      const uint32_t* row = d.trans.data() + (size_t)state * d.n_classes;
+      for (int b = 0; b < 256; ++b)
+        if (!(row[cls.map[b]] & DFA_FLAG_DEAD)) ways[state].push_back((uint8_t)b);
+    }
+    return ways[state];
+  };
+  auto after = [&](uint32_t state, uint8_t b) {
+    return d.trans[(size_t)state * d.n_classes + cls.map[b]] & DFA_MASK_STATE;
+  };
+  auto stops = [&](uint32_t state, size_t depth) {  // (is_match in a context DFA: under some right context)
+    return d.is_match[state] || (depth >= len && (depth >= 8 || ways_of(state).size() != 1));
+  };
+  // First the numbers of paths per state, depth by depth, against the limits; the
+  // strings only of a regex that keeps them.  (A string per path and all 256 bytes
+  // per step, breadth first, were 0.6 of the 1.9 s that a matcher of 500 regexes
+  // took to build; most of them have too many strings of 20 bytes.)
+  std::map<uint32_t, size_t> cur, nxt;
+  for (uint32_t s : starts) cur[s] = 1;
+  size_t ended = 0;
+  for (size_t depth = 0; !cur.empty(); ++depth) {
     nxt.clear();
-    for (const Item& it : cur) {
-      const uint32_t* row = d.trans.data() + (size_t)it.second * d.n_classes;
-      size_t ways = 0;
-      for (int b = 0; b < 256; ++b) ways += (row[cls.map[b]] & DFA_FLAG_DEAD) ? 0 : 1;
-      const bool ends = d.is_match[it.second] != 0;  // (in a context DFA: under some right context)
-      if (ends && depth < 4) return false;
-      if (ends || (depth >= len && (depth >= 8 || ways != 1))) {
-        found.push_back(it.first);
-        if (found.size() > 4 * most) return false;
+    size_t width = 0;
+    for (const auto& c : cur) {
+      if (d.is_match[c.first] && depth < 4) return false;
+      if (stops(c.first, depth)) {
+        if ((ended += c.second) > 4 * most) return false;
         continue;
       }
-      if (nxt.size() + ways > 4 * most) return false;  // (up to four starts give the same string)
-      for (int b = 0; b < 256; ++b)
-        if (!(row[cls.map[b]] & DFA_FLAG_DEAD))
-          nxt.emplace_back(it.first + (char)(uint8_t)b, row[cls.map[b]] & DFA_MASK_STATE);
+      width += c.second * ways_of(c.first).size();
+      if (width > 4 * most) return false;  // (up to four starts give the same string)
+      for (uint8_t b : ways_of(c.first)) nxt[after(c.first, b)] += c.second;
     }
     cur.swap(nxt);
+  }
+  std::vector<std::string> found;
+  std::string path;
+  struct Level {
+    uint32_t state;
+    size_t next;  // of its ways
+  };
+  std::vector<Level> stack;
+  auto enter = [&](uint32_t state) {
+    const bool end = stops(state, path.size());
+    if (end) found.push_back(path);
+    stack.push_back({state, end ? ways_of(state).size() : 0});
+  };
+  for (uint32_t s : starts) {
+    path.clear();
+    enter(s);
+    while (!stack.empty()) {
+      Level& l = stack.back();
+      if (l.next == ways_of(l.state).size()) {
+        stack.pop_back();
+        if (!path.empty()) path.pop_back();
+        continue;
+      }
+      const uint32_t state = l.state;
+      const uint8_t b = ways_of(state)[l.next++];
+      path.push_back((char)b);
+      enter(after(state, b));
+    }
   }
   std::sort(found.begin(), found.end());
   for (const std::string& x : found)  // sorted: a prefix comes right before what it begins
