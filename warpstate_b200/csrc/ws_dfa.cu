@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(1024) dfa_reverse_kernel(DevTables t, ScanPtrs
       }
       if (w & F_MATCH) {
         for (uint32_t j = __ldg(rmp + st); j < __ldg(rmp + st + 1); ++j)
-          emit_k(p, __ldg(t.rmlist + j), (uint32_t)(pos - 1), ev.e);
+          emit_k_ahead(p, __ldg(t.rmlist + j), (uint32_t)(pos - 1), ev.e);
       }
     }
   }

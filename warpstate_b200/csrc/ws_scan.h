@@ -105,10 +105,6 @@ __device__ __forceinline__ unsigned long long warp_append(unsigned long long* co
 
 // Stores candidate i of K with its rank among its regex's candidates (the
 // per-regex counts size the resolution's lists, the rank is its place in one).
-// A candidate is counted whether it fits or not, so that its two atomics do not
-// wait for one another (1,000 regexes that match at the same places of 256 MiB:
-// 3,000 -> 2,190 us a scan, 2,160 to 2,290 before candidates had ranks); the lists
-// of a scan whose candidates did not fit are not read.
 __device__ __forceinline__ void store_k(const ScanPtrs& p, unsigned long long i, uint32_t r, uint32_t s, uint32_t e,
                                         uint32_t rank_known) {
   if (i < p.k_cap) p.k[i] = KCand{r, s, e, rank_known};
@@ -116,8 +112,20 @@ __device__ __forceinline__ void store_k(const ScanPtrs& p, unsigned long long i,
 }
 
 __device__ __forceinline__ void emit_k(const ScanPtrs& p, uint32_t r, uint32_t s, uint32_t e, uint32_t known = 0) {
+  const unsigned long long i = warp_append(&p.ctr[C_K]);
+  if (i < p.k_cap) p.k[i] = KCand{r, s, e, atomicAdd(&p.count[r], 1u) | known};
+  else atomicOr(&p.ctr[C_ERR], 1ull);
+}
+
+// The same where a thread may emit many in turn: a candidate is counted whether it
+// fits or not, so that its two atomics do not wait for one another (1,000 regexes
+// that match at the same places of 256 MiB: 3,000 -> 2,190 us a scan, 2,160 to
+// 2,290 before candidates had ranks); the lists of a scan whose candidates did not
+// fit are not read.  (In the loops of the plain and the context kernel that order
+// cost more than it saved: 20 regexes with assertions over 32 MiB 138 -> 171 us.)
+__device__ __forceinline__ void emit_k_ahead(const ScanPtrs& p, uint32_t r, uint32_t s, uint32_t e) {
   const uint32_t rank = atomicAdd(&p.count[r], 1u);
-  store_k(p, warp_append(&p.ctr[C_K]), r, s, e, rank | known);
+  store_k(p, warp_append(&p.ctr[C_K]), r, s, e, rank);
 }
 
 // Context of a byte for the assertions (byte_context in ws_regex.h).
