@@ -160,11 +160,60 @@ void build_gram_tables(const std::vector<FilterString>& strings, LiteralPlan& pl
 // P grams at offsets 0..P-1 must fit inside every string: P + 3 <= len.
 uint32_t period_of(uint32_t min_len) { return min_len >= 7 ? 4 : min_len >= 5 ? 2 : 1; }
 
-// Share of its alphabet's 4-byte grams that a set may cover.  The gram kernel
-// verifies in a later kernel what passes, from a list of one survivor per 64
-// bytes of input: an input over the set's own alphabet should not crowd it
-// (for P = 4, whose lookups are a quarter as many, a quarter is allowed).
+// Share of its alphabet's 4-byte grams that a set covers before longer grams, or
+// none of the regexes' prefixes, are the better choice.
 double coverage_limit(uint32_t P) { return P == 4 ? 0.25 : 1.0 / 64; }
+
+// Share of its alphabet's G-byte grams that a set of the gram kernel may cover.
+// That kernel passes on every position whose gram is in the set; on an input over
+// the set's own alphabet that is coverage / P of all positions, and the list holds
+// one of 64.  Beyond it every gram is looked up a second time; the compacting
+// kernel, which checks prefixes inside the filter, is then the better one.
+// Measured over 128 MiB of uniform letters, us a scan with the gram and with the
+// compacting kernel, by coverage: P = 4 4.4% 107 and 123 (26 letters), 102 and 107
+// (8 letters), 4.8% 117 and 126, 5.0% 113 and 108 (12 letters), 7% 269 and 132, 10%
+// (8 letters) 269 and 110; P = 1 1.26% 202 and 322, 1.31% 619 and 340; 3-byte grams
+// 1.08% 185 and 260, 1.14% 346 and 259.  P = 2: 1.5% 109 and 184.
+double gram_limit(uint32_t P, uint32_t G) {
+  return P == 4 ? 0.05 : P == 2 ? 1.0 / 64 : G == 3 ? 0.0105 : 0.0125;
+}
+
+struct Layout {
+  bool has_long = false, has_short = false;  // strings of at least, of fewer than 4 bytes
+  bool gram_kernel = false;
+  uint32_t period = 4, gram_len = 4;
+};
+
+Layout choose_layout(const std::vector<FilterString>& strings) {
+  Layout l;
+  uint32_t min_len = UINT32_MAX, min_long = UINT32_MAX;
+  for (const FilterString& f : strings) {
+    min_len = std::min(min_len, f.len);
+    if (f.len >= 4) { l.has_long = true; min_long = std::min(min_long, f.len); }
+    else l.has_short = true;
+  }
+  l.period = !l.has_long ? 4 : period_of(min_long);
+  // A low-entropy set (a small alphabet whose 4-grams the strings mostly
+  // cover, e.g. nucleotide k-mers) lets most input positions through 4-byte
+  // grams: it takes the longest gram every long string holds at all P phases.
+  const bool low_entropy =
+      l.has_long && l.period == 4 && min_long >= 11 && gram_coverage(strings, 4, 4) > coverage_limit(4);
+  if (low_entropy) l.gram_len = min_long >= 19 ? 16 : 8;
+  // Crowded sets take the compacting kernel, which checks prefixes inside the
+  // filter.  Shortest string of three bytes: 3-byte grams at every position.
+  if (low_entropy) {
+    l.gram_kernel = l.gram_len == 16 && !l.has_short;
+  } else if (min_len == 3) {
+    l.gram_kernel = gram_coverage(strings, 1, 3) <= gram_limit(1, 3);
+    if (l.gram_kernel) {
+      l.period = 1;
+      l.gram_len = 3;
+    }
+  } else if (min_len >= 4) {
+    l.gram_kernel = gram_coverage(strings, l.period, 4) <= gram_limit(l.period, 4);
+  }
+  return l;
+}
 
 }  // namespace
 
@@ -215,34 +264,15 @@ void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan, const std:
   for (uint32_t li = 0; li < t.n_literals; ++li)
     strings.push_back({t.packed_bytes + t.offsets[2 * li], t.offsets[2 * li + 1]});
   for (const std::string& x : pre) strings.push_back({reinterpret_cast<const uint8_t*>(x.data()), (uint32_t)x.size()});
-  uint32_t min_len = UINT32_MAX, min_long = UINT32_MAX;
   plan.max_len = 0;
-  for (const FilterString& f : strings) {
-    plan.max_len = std::max(plan.max_len, f.len);
-    min_len = std::min(min_len, f.len);
-    if (f.len >= 4) { plan.has_long = 1; min_long = std::min(min_long, f.len); }
-    else plan.has_short = 1;
-  }
-  plan.period = !plan.has_long ? 4 : period_of(min_long);
+  for (const FilterString& f : strings) plan.max_len = std::max(plan.max_len, f.len);
+  const Layout layout = choose_layout(strings);
+  plan.has_long = layout.has_long;
+  plan.has_short = layout.has_short;
+  plan.period = layout.period;
+  plan.gram_len = layout.gram_len;
+  plan.gram_kernel = layout.gram_kernel;
   plan.table_bits = 18;
-  // A low-entropy set (a small alphabet whose 4-grams the strings mostly
-  // cover, e.g. nucleotide k-mers) lets most input positions through 4-byte
-  // grams: it takes the longest gram every long string holds at all P phases.
-  const bool low_entropy = plan.has_long && plan.period == 4 && min_long >= 11 && gram_coverage(strings, 4, 4) > coverage_limit(4);
-  if (low_entropy) plan.gram_len = min_long >= 19 ? 16 : 8;
-  // Crowded sets take the compacting kernel, which checks prefixes inside the
-  // filter.  Shortest string of three bytes: 3-byte grams at every position.
-  if (low_entropy) {
-    plan.gram_kernel = plan.gram_len == 16 && !plan.has_short;
-  } else if (min_len == 3) {
-    plan.gram_kernel = gram_coverage(strings, 1, 3) <= coverage_limit(1);
-    if (plan.gram_kernel) {
-      plan.period = 1;
-      plan.gram_len = 3;
-    }
-  } else if (min_len >= 4) {
-    plan.gram_kernel = gram_coverage(strings, plan.period, 4) <= coverage_limit(plan.period);
-  }
   const uint32_t P = plan.period, G = plan.gram_len, bits = plan.table_bits;
   plan.parts = plan.bloom_parts = 0;
   plan.lit_info.assign(4 * (size_t)t.n_literals, 0);
@@ -466,4 +496,14 @@ extern "C" ws_status ws_ir_tables(const ws_ir* ir, ws_pattern_tables* t) {
   t->n_patterns = d.n_patterns;
   t->case_insensitive = d.case_insensitive ? 1 : 0;
   return WS_OK;
+}
+
+// Test hook: the literal filter's layout for the literals of a pattern set: bytes
+// between the positions it looks at, bytes of a gram, whether the gram kernel runs.
+extern "C" void ws_testing_literal_layout(const ws_ir* ir, unsigned* out) {
+  std::vector<FilterString> strings;
+  for (size_t k = 0; k < ir->d.literal_pattern_ids.size(); ++k)
+    strings.push_back({ir->d.packed_bytes.data() + ir->d.offsets[2 * k], ir->d.offsets[2 * k + 1]});
+  const Layout l = choose_layout(strings);
+  out[0] = l.period, out[1] = l.gram_len, out[2] = l.gram_kernel ? 1 : 0;
 }
