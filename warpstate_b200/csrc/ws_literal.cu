@@ -407,7 +407,7 @@ __device__ __forceinline__ void process_block(const LitArgs& a, uint32_t* blk, u
 // 32-bit.
 template <int P, int G, bool LONG, bool SHORT>
 __global__ void __launch_bounds__(kThreads, 1) literal_filter_kernel(const __grid_constant__ LitArgs a) {
-  pdl_begin();
+  pdl_wait();  // (the verify kernel is not let in early: its waiting blocks cost up to 60 us of 370)
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* filt = smem;                                 // filter_words
   uint32_t* bloom = filt + a.filter_words;               // 2^kBloomBits / 32 words
@@ -541,7 +541,7 @@ constexpr int kBigWarps = kBigThreads / 32;
 // block i is finished -- so that the L2 latency overlaps useful work.
 // 16 warps per CTA leave room for the pipeline's registers.
 __global__ void __launch_bounds__(kBigThreads, 1) literal_filter_big_kernel(const __grid_constant__ LitArgs a) {
-  pdl_begin();
+  pdl_wait();  // (as in literal_filter_kernel)
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* filt = smem;
   uint32_t* bloom = filt + a.filter_words;
