@@ -110,3 +110,19 @@ def test_buckets_by_four_bytes_stay_short(n):
     rx = ["user" + "".join(chr(97 + (i // 5 ** k) % 5) for k in range(4)) + "[0-9]{1,3};" for i in range(n)]
     got, covered = prefix_plan([], rx + [r"abcd[0-9a-f]+;"])
     assert covered[:n] == [True] * n and covered[n] == (n <= 64)
+
+
+def test_literals_that_crowd_their_alphabet_decide():
+    # '=' and digits at the ends of the prefixes do not make nucleotide literals sparse
+    r = random.Random(4)
+    lits = sorted({bytes(r.choices(b"ACGT", k=r.randint(12, 16))) for _ in range(38)})
+    rx = ["".join(r.choices("ACGT", k=r.randint(4, 7))) + "=[0-9]+" for _ in range(15)]
+    assert prefix_plan(lits, rx) == (0, [False] * 15)
+    assert prefix_plan([b"needle", b"haystack"], rx)[0] > 0
+    assert prefix_plan([], rx)[0] > 0
+
+
+def test_one_byte_literals_leave_the_list_to_themselves():
+    rx = [r"alpha[0-9]{1,3}x", r"tailwind [0-9]"]
+    assert prefix_plan([b"q", b"needle"], rx) == (0, [False] * 2)
+    assert prefix_plan([b"qz", b"needle"], rx)[1] == [True] * 2

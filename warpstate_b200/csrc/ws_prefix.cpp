@@ -125,6 +125,9 @@ void choose_prefixes(const ws_pattern_tables& t, RegexPlan& P) {
   drop_shared(P);
   uint32_t shortest = UINT32_MAX;
   for (uint32_t i = 0; i < t.n_literals; ++i) shortest = std::min(shortest, t.offsets[2 * i + 1]);
+  // (a literal of one byte fills the survivor list by itself: the filter would
+  // give the prefixes up on most inputs)
+  if (shortest < 2) std::fill(P.covered.begin(), P.covered.end(), 0);
   std::vector<std::pair<std::string, uint32_t>> pre;
   const size_t most[kPrefixLens] = {65536, 4096, 16384, 65536};
   for (int k = 1; k < kPrefixLens && P.prefix_len < 0; ++k)
