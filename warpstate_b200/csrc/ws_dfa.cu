@@ -803,29 +803,28 @@ __global__ void __launch_bounds__(1024) dfa_reverse_kernel(DevTables t, ScanPtrs
 
 // ---------------------------------------------------------------- resolution
 // Candidates a block sorts in shared memory, and the longest list that one block
-// of k_resolve_kernel takes from sort to report.  Where the prefix filter gave
-// up, the candidates' ends are still to be walked, up to kLfCap bytes each: a
-// block then takes four per thread, not sixteen.
-constexpr uint32_t kSortTile = 4096, kOpenTile = 1024;
-__device__ __forceinline__ uint32_t resolve_tile(const ScanPtrs& p) { return p.ctr[C_GATE] ? kOpenTile : kSortTile; }
+// of k_resolve_kernel takes from sort to report.  (Tiles of 1,024 where the
+// filter gave up and each candidate's end is still to be walked: 21 regexes over 64
+// MiB 1,520 -> 1,450 us a scan, but two more merges of long lists, 119 regexes over
+// 20 MiB 36 -> 91 ms.)
+constexpr uint32_t kSortTile = 4096;
 
 // Exclusive scan of the per-regex candidate counts into offs[0, n_regex] by one
 // block (blockDim.x a multiple of 32, at most 1024): each thread sums a run of
 // regexes, the runs are scanned across the block with warp shuffles, then each
 // thread writes its run's offsets.  Notes in ctr[C_LONG] whether some list is
-// longer than resolve_tile.
+// longer than kSortTile.
 __device__ void scan_counts(const ScanPtrs& p, uint32_t n_regex, uint32_t* offs) {
   __shared__ uint32_t wsum[32];
   const uint32_t per = (n_regex + blockDim.x - 1) / blockDim.x;
   const uint32_t a = min(n_regex, threadIdx.x * per), b = min(n_regex, a + per);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t tile = resolve_tile(p);
   uint32_t sum = 0;
   bool more = false;
   for (uint32_t r = a; r < b; ++r) {
     const uint32_t c = p.count[r];
     sum += c;
-    more |= c > tile;
+    more |= c > kSortTile;
   }
   if (more) p.ctr[C_LONG] = 1;
   uint32_t incl = sum;
@@ -934,12 +933,13 @@ __device__ uint32_t merge_path(const unsigned long long* A, uint32_t na, const u
   return lo;
 }
 
-// Merges the sorted tiles (of `tile` candidates) of list[0, n) pairwise in
-// global memory (merge-path split of each merge across the block), with
-// other[0, n) as the other buffer.
-__device__ void merge_tiles(unsigned long long* list, unsigned long long* other, uint32_t n, uint32_t tile) {
+// Merges the sorted tiles of list[0, n) pairwise in global memory (merge-path
+// split of each merge across the block), with other[0, n) as the other buffer.
+// (A pair of tiles per warp while there are enough pairs is slower: one regex with
+// 335,000 candidates 9,110 -> 9,670 us a scan.)
+__device__ void merge_tiles(unsigned long long* list, unsigned long long* other, uint32_t n) {
   unsigned long long *src = list, *dst = other;
-  for (uint32_t w = tile; w < n; w <<= 1) {
+  for (uint32_t w = kSortTile; w < n; w <<= 1) {
     for (uint32_t lo = 0; lo < n; lo += 2 * w) {
       const uint32_t mid = min(lo + w, n), hi = min(lo + 2 * w, n);
       const unsigned long long *A = src + lo, *B = src + mid;
@@ -991,7 +991,7 @@ __global__ void __launch_bounds__(512) k_sort_kernel(ScanPtrs p, uint32_t n_rege
     __syncthreads();
     if (last) {
       __threadfence();
-      merge_tiles(p.pair + a, p.pair2 + a, n, kSortTile);
+      merge_tiles(p.pair + a, p.pair2 + a, n);
     }
     __syncthreads();
   }
@@ -1199,20 +1199,48 @@ __global__ void __launch_bounds__(kChainThreads) k_chain_kernel(DevTables t, Sca
 }
 
 // The block's share of the long lists (see k_resolve_kernel) and its regexes with
-// short ones, missing ends included.
+// short ones, missing ends included.  Tiles first, then short lists, then the long
+// lists whose last tile was the block's: a block that merged and reported a list
+// while other lists waited for its tiles held them all up (119 regexes with 18,000
+// candidates each 45 ms by a block per regex, 114 that way).
 __device__ void resolve_shared(const DevTables& t, const ScanPtrs& p, uint32_t n_regex, unsigned long long* buf,
                                ChainShared& sh) {
-  __shared__ bool last;
-  const uint32_t tile = resolve_tile(p), total = p.offs[n_regex];
+  constexpr uint32_t kMine = 64;
+  __shared__ uint32_t mine[kMine], n_mine;
+  constexpr uint32_t tile = kSortTile;
+  const uint32_t total = p.offs[n_regex];
+  if (threadIdx.x == 0) n_mine = 0;
+  auto sort_and_end = [&](uint32_t r, const unsigned long long* src, uint32_t m) {
+    sort_into(buf, src, m);
+    for (uint32_t j = threadIdx.x; j < m; j += blockDim.x)
+      if ((uint32_t)buf[j] == kLfTodo) reinterpret_cast<uint32_t*>(buf + j)[0] = list_end(t, p, r, buf, j);
+    __syncthreads();
+  };
+  auto report = [&](uint32_t r, const unsigned long long* list, uint32_t n) {
+    const uint64_t end = chain_list(t, p, r, list, n, chain_start(p, r), chain_limit(p), sh);
+    if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + end, p.frontier);
+    __syncthreads();  // (buf, before the next list)
+  };
+  auto finish_mine = [&]() {
+    __syncthreads();
+    __threadfence();
+    for (uint32_t i = 0; i < n_mine; ++i) {
+      const uint32_t r = mine[i], a = p.offs[r], n = p.offs[r + 1] - a;
+      merge_tiles(p.pair + a, p.pair2 + a, n);
+      report(r, p.pair + a, n);
+    }
+    if (threadIdx.x == 0) n_mine = 0;
+    __syncthreads();
+  };
   uint64_t slot = (uint64_t)blockIdx.x * tile;
   for (uint32_t r0 = blockIdx.x;; r0 += gridDim.x) {
-    // the block's regexes (tile 0 of a long list), then its slots of the
-    // candidates: a later tile of a list falls to the block whose slot its first
-    // candidate lies in.  The list began more than a tile before, so it holds the
-    // slot's first candidate too, and no other list has a later tile there.
+    // tile 0 of the block's long lists, then its slots of the candidates: a later
+    // tile of a list falls to the block whose slot its first candidate lies in.
+    // The list began more than a tile before, so it holds the slot's first
+    // candidate too, and no other list has a later tile there.
     uint32_t r = r0, k = 0;
     if (r0 >= n_regex) {
-      if (slot >= total) return;
+      if (slot >= total) break;
       uint32_t hi = n_regex;
       for (r = 0; hi - r > 1;) {
         const uint32_t mid = (r + hi) >> 1;
@@ -1223,46 +1251,42 @@ __device__ void resolve_shared(const DevTables& t, const ScanPtrs& p, uint32_t n
       if (k == 0) continue;
     }
     const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
-    if (k && k * tile >= n) continue;
-    unsigned long long* list = p.pair + a;
+    if (n <= tile || k * tile >= n) continue;
+    unsigned long long* src = p.pair + a + k * tile;
     const uint32_t m = min(tile, n - k * tile);
-    if (m) {
-      sort_into(buf, list + k * tile, m);
-      for (uint32_t j = threadIdx.x; j < m; j += blockDim.x)
-        if ((uint32_t)buf[j] == kLfTodo) reinterpret_cast<uint32_t*>(buf + j)[0] = list_end(t, p, r, buf, j);
-      __syncthreads();
-    }
-    if (n > tile) {
-      for (uint32_t j = threadIdx.x; j < m; j += blockDim.x) list[k * tile + j] = buf[j];
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(&p.count[r], 1u) + 1 == n + (n + tile - 1) / tile;
-      }
-      __syncthreads();
-      if (!last) continue;
+    sort_and_end(r, src, m);
+    for (uint32_t j = threadIdx.x; j < m; j += blockDim.x) src[j] = buf[j];
+    __syncthreads();
+    if (threadIdx.x == 0) {
       __threadfence();
-      merge_tiles(list, p.pair2 + a, n, tile);
+      if (atomicAdd(&p.count[r], 1u) + 1 == n + (n + tile - 1) / tile) mine[n_mine++] = r;
     }
-    const uint64_t end = chain_list(t, p, r, n > tile ? list : buf, n, chain_start(p, r), chain_limit(p), sh);
-    if (p.cursor64 && threadIdx.x == 0) p.cursor64[r] = max(p.base + end, p.frontier);
-    __syncthreads();  // (buf, before the next list)
+    __syncthreads();
+    if (n_mine == kMine) finish_mine();
   }
+  for (uint32_t r = blockIdx.x; r < n_regex; r += gridDim.x) {
+    const uint32_t a = p.offs[r], n = p.offs[r + 1] - a;
+    if (n > tile) continue;
+    if (n) sort_and_end(r, p.pair + a, n);
+    report(r, buf, n);
+  }
+  finish_mine();
 }
 
 // Sort and chain of a regex by one block, in shared memory: the resolution of
 // scans whose candidates came from prefixes, ends known (three kernels and a pass
 // through global memory between each took 8 us more on small lists).
-// Lists longer than resolve_tile (dense matches, or the walk's candidates where
+// Lists longer than kSortTile (dense matches, or the walk's candidates where
 // the filter gave up) are shared by all blocks: each tile is sorted, its missing
 // ends walked, by the block it falls to, and the block that finishes a list's
 // last tile merges and reports it (its ticket is the regex's count, which nothing
 // reads after the scatter).  A tile walks the ends of its own distinct starts, so
 // a start in several tiles is walked in each, to the same end.  By one block per
-// regex -> shared, us a scan: 21 regexes over 64 MiB whose filter gave up 2,150
-// -> 1,450 (with the walk before there were prefixes 1,880), 30 regexes with
-// 671,000 matches in 64 MiB 2,550 -> 1,240, three with 335,000 in 256 MiB 9,600 ->
-// 2,600, one with 335,000 among 301 18,800 -> 9,100.
+// regex -> shared, us a scan: 21 regexes over 64 MiB whose filter gave up 2,400
+// -> 1,520 (with the walk before there were prefixes 1,880), 30 regexes with
+// 671,000 matches in 64 MiB 2,580 -> 1,080, three with 335,000 in 256 MiB 9,300 ->
+// 2,600 to 4,200, one with 335,000 among 301 18,700 -> 9,100, 119 over 20 MiB with
+// 3.8 M candidates 47,700 -> 35,500.
 __global__ void __launch_bounds__(kChainThreads) k_resolve_kernel(DevTables t, ScanPtrs p, uint32_t n_regex,
                                                                   unsigned long long* need) {
   __shared__ unsigned long long buf[kSortTile];
