@@ -112,14 +112,25 @@ def test_buckets_by_four_bytes_stay_short(n):
     assert covered[:n] == [True] * n and covered[n] == (n <= 64)
 
 
-def test_literals_that_crowd_their_alphabet_decide():
-    # '=' and digits at the ends of the prefixes do not make nucleotide literals sparse
+def test_literals_with_long_grams_decide():
+    # '=' and digits at the ends of the prefixes do not make nucleotide literals
+    # sparse: those of 11 bytes and more keep their long grams
     r = random.Random(4)
-    lits = sorted({bytes(r.choices(b"ACGT", k=r.randint(12, 16))) for _ in range(38)})
+    lits = sorted({bytes(r.choices(b"ACGT", k=r.randint(12, 16))) for _ in range(4000)})
     rx = ["".join(r.choices("ACGT", k=r.randint(4, 7))) + "=[0-9]+" for _ in range(15)]
     assert prefix_plan(lits, rx) == (0, [False] * 15)
-    assert prefix_plan([b"needle", b"haystack"], rx)[0] > 0
-    assert prefix_plan([], rx)[0] > 0
+    assert prefix_plan(lits[::100], rx) == (0, [False] * 15)
+    assert prefix_plan([b"needle", b"haystack"], rx)[1] == [True] * 15
+    assert prefix_plan([], rx)[1] == [True] * 15
+
+
+@pytest.mark.parametrize("letters", ["abcdefgh", "abcdefghijkl"])
+def test_short_words_over_few_letters_are_covered(letters):
+    # (by the compacting kernel: their grams crowd the alphabet, their beginnings
+    # do not fill the list)
+    r = random.Random(6)
+    rx = sorted({"\\b" + "".join(r.choices(letters, k=r.randint(5, 9))) + "\\b" for _ in range(60)})
+    assert all(prefix_plan([], rx)[1])
 
 
 def test_one_byte_literals_leave_the_list_to_themselves():

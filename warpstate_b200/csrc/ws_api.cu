@@ -141,10 +141,10 @@ uint32_t enqueue_scan(ws_matcher* m, Scratch& s, cudaStream_t st, const uint8_t*
   return enqueue_scan(m, m->rx, m->lit, s, st, d_data, len, d_out, cap, d_counter, x);
 }
 
-bool scans_prefixes(const ws_matcher* m, const RegexPlan& rx, const LiteralPlan& lit) {
+bool scans_prefixes(const ws_matcher* m, const RegexPlan& rx, const LiteralPlan& lit, uint64_t len) {
   // not where the walk is pinned or goes over every group all the same
   const bool spared = rx.n_walk < rx.n_spec || rx.n_ctx_walk < rx.n_groups;
-  return spared && lit.n_prefixes && m->cfg.regex_mode == WS_REGEX_SPECULATIVE && !m->walk_pinned;
+  return spared && lit.n_prefixes && len <= lit.prefix_most && m->cfg.regex_mode == WS_REGEX_SPECULATIVE && !m->walk_pinned;
 }
 
 uint32_t enqueue_scan(ws_matcher* m, RegexPlan& rx, const LiteralPlan& lit, Scratch& s, cudaStream_t st,
@@ -156,7 +156,7 @@ uint32_t enqueue_scan(ws_matcher* m, RegexPlan& rx, const LiteralPlan& lit, Scra
   if (prof) check_cuda(cudaEventRecord(m->pev[0], st), "event");
   RegexLaunch rl{d_data, len, d_out, cap, d_counter, m->cfg.regex_mode};
   RegexScan rs;
-  const bool prefixes = scans_prefixes(m, rx, lit);  // the literal filter also looks for the regexes' prefixes
+  const bool prefixes = scans_prefixes(m, rx, lit, len);  // the literal filter also looks for the regexes' prefixes
   if (rx.n_regex) {
     rl.item_end = x.item_end;
     rl.n_items = x.n_items;

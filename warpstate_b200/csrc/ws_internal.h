@@ -154,6 +154,7 @@ struct LiteralPlan {
   // Regex prefixes: entries {first 4 bytes, next 4, their mask, regex} by
   // bucket of a hash of the first 4 bytes (prefix_mul = 0) or of all 8.
   uint32_t n_prefixes = 0, prefix_shift = 0, prefix_mul = 0;
+  uint64_t prefix_most = 0;  // longest input on which scans look for them
   DeviceBuffer d_prefix_range, d_prefix_entry;
   // ASCII case-insensitive: the tables hold folded literals and the kernels
   // fold the input (A-Z to a-z) before hashing and comparing.
@@ -263,9 +264,13 @@ __host__ __device__ inline uint32_t prefix16_key(uint32_t x0, uint32_t x1, uint3
 // `prefixes`: strings of at least 4 bytes that are filtered with the literals
 // (regex prefixes); positions where one starts are survivors.
 void plan_literals(const ws_pattern_tables& t, LiteralPlan& plan, const std::vector<std::string>& prefixes = {});
-// Whether 4-byte grams of the literals and `prefixes` cover too much of their
-// alphabet's for the gram kernel.
+// Whether the literals and `prefixes` would fill the survivor list on an input over
+// their alphabet, or the literals give up more by the prefixes than these save.
 bool filter_crowded(const ws_pattern_tables& t, const std::vector<std::string>& prefixes);
+// The filter's pass over uniform letters, ms per GiB (rounded; ws_literal.cu and
+// ws_ir.cpp have what was measured): of a plan, of the literals alone.
+double filter_ms_per_gib(const LiteralPlan& plan);
+double literals_ms_per_gib(const ws_pattern_tables& t);
 struct RegexPlan;
 // plan_literals with the prefixes of the regexes that have some, and the table
 // the verify kernel finds them in (n_prefixes stays 0 when there are none).

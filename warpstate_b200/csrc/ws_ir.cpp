@@ -1,6 +1,7 @@
 // Pattern IR: the host half of PatternSetBuilder::build that the GPU path needs,
 // and the literal-scan plan derived from it.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "ws_internal.h"
@@ -160,9 +161,9 @@ void build_gram_tables(const std::vector<FilterString>& strings, LiteralPlan& pl
 // P grams at offsets 0..P-1 must fit inside every string: P + 3 <= len.
 uint32_t period_of(uint32_t min_len) { return min_len >= 7 ? 4 : min_len >= 5 ? 2 : 1; }
 
-// Share of its alphabet's 4-byte grams that a set covers before longer grams, or
-// none of the regexes' prefixes, are the better choice.
-double coverage_limit(uint32_t P) { return P == 4 ? 0.25 : 1.0 / 64; }
+// Share of its alphabet's 4-byte grams that a set covers before longer grams are
+// the better choice.
+constexpr double kLowEntropy = 0.25;
 
 // Share of its alphabet's G-byte grams that a set of the gram kernel may cover.
 // That kernel passes on every position whose gram is in the set; on an input over
@@ -184,8 +185,19 @@ struct Layout {
   uint32_t period = 4, gram_len = 4;
 };
 
-Layout choose_layout(const std::vector<FilterString>& strings) {
+// (fewer literals say little about the alphabet of the input)
+constexpr size_t kOwnAlphabet = 16;
+
+// `n_literals` of the strings, the first, are literals.  Their grams count by
+// their own alphabet too: a few other bytes in the prefixes make the alphabet of
+// all larger, not the input.
+Layout choose_layout(const std::vector<FilterString>& strings, size_t n_literals) {
   Layout l;
+  const std::vector<FilterString> literals(strings.begin(), strings.begin() + n_literals);
+  auto coverage = [&](uint32_t P, uint32_t G) {
+    const double all = gram_coverage(strings, P, G);
+    return n_literals >= kOwnAlphabet && n_literals < strings.size() ? std::max(all, gram_coverage(literals, P, G)) : all;
+  };
   uint32_t min_len = UINT32_MAX, min_long = UINT32_MAX;
   for (const FilterString& f : strings) {
     min_len = std::min(min_len, f.len);
@@ -197,20 +209,20 @@ Layout choose_layout(const std::vector<FilterString>& strings) {
   // cover, e.g. nucleotide k-mers) lets most input positions through 4-byte
   // grams: it takes the longest gram every long string holds at all P phases.
   const bool low_entropy =
-      l.has_long && l.period == 4 && min_long >= 11 && gram_coverage(strings, 4, 4) > coverage_limit(4);
+      l.has_long && l.period == 4 && min_long >= 11 && coverage(4, 4) > kLowEntropy;
   if (low_entropy) l.gram_len = min_long >= 19 ? 16 : 8;
   // Crowded sets take the compacting kernel, which checks prefixes inside the
   // filter.  Shortest string of three bytes: 3-byte grams at every position.
   if (low_entropy) {
     l.gram_kernel = l.gram_len == 16 && !l.has_short;
   } else if (min_len == 3) {
-    l.gram_kernel = gram_coverage(strings, 1, 3) <= gram_limit(1, 3);
+    l.gram_kernel = coverage(1, 3) <= gram_limit(1, 3);
     if (l.gram_kernel) {
       l.period = 1;
       l.gram_len = 3;
     }
   } else if (min_len >= 4) {
-    l.gram_kernel = gram_coverage(strings, l.period, 4) <= gram_limit(l.period, 4);
+    l.gram_kernel = coverage(l.period, 4) <= gram_limit(l.period, 4);
   }
   return l;
 }
@@ -218,24 +230,55 @@ Layout choose_layout(const std::vector<FilterString>& strings) {
 }  // namespace
 
 bool filter_crowded(const ws_pattern_tables& t, const std::vector<std::string>& prefixes) {
-  // The literals also by themselves: a few other bytes in the prefixes make the
-  // alphabet larger, not the input (38 literals and 15 regexes over nucleotides
-  // with an '=' or a digit at the prefixes' ends, 70 MiB of nucleotides: 425 us a
-  // scan before there were prefixes, 790 with them).
   std::vector<FilterString> strings;
-  uint32_t min_long = UINT32_MAX;
-  auto crowded = [&]() {
-    for (const FilterString& f : strings)
-      if (f.len >= 4) min_long = std::min(min_long, f.len);
-    const uint32_t P = period_of(min_long);
-    return gram_coverage(strings, P, 4) > coverage_limit(P);
-  };
   for (uint32_t li = 0; li < t.n_literals; ++li)
     strings.push_back({t.packed_bytes + t.offsets[2 * li], t.offsets[2 * li + 1]});
-  if (t.n_literals && crowded()) return true;
+  const Layout alone = choose_layout(strings, strings.size());
   for (const std::string& x : prefixes)
     strings.push_back({reinterpret_cast<const uint8_t*>(x.data()), (uint32_t)x.size()});
-  return crowded();
+  const Layout l = choose_layout(strings, t.n_literals);
+  if (l.gram_kernel) return false;  // (its list holds, or it would not run)
+  // the literals' long grams are worth more than the walks (4-byte ones let nearly
+  // every position of such an input through)
+  if (t.n_literals && alone.gram_len > l.gram_len) return true;
+  // The compacting kernel lets a position through whose first bytes (8 of them, 16
+  // with longer grams) a string begins with: as a share of all positions of an
+  // input over the strings' alphabet, and over the literals' for theirs.
+  const uint32_t most = l.gram_len > 4 ? 16 : 8;
+  auto share = [&](size_t n) {
+    bool seen[256] = {};
+    double alphabet = 0, sum = 0;
+    std::vector<std::string> heads;
+    for (size_t k = 0; k < n; ++k) {
+      heads.emplace_back(reinterpret_cast<const char*>(strings[k].p), std::min(strings[k].len, most));
+      for (uint32_t j = 0; j < strings[k].len; ++j) seen[strings[k].p[j]] = true;
+    }
+    for (bool x : seen) alphabet += x ? 1 : 0;
+    std::sort(heads.begin(), heads.end());
+    heads.erase(std::unique(heads.begin(), heads.end()), heads.end());
+    for (const std::string& h : heads) sum += std::pow(alphabet, -(double)h.size());
+    return sum;
+  };
+  return std::max(share(strings.size()), t.n_literals >= kOwnAlphabet ? share(t.n_literals) : 0.0) > 1.0 / 80;
+}
+
+double filter_ms_per_gib(const LiteralPlan& plan) {
+  if (plan.n_strings == 0) return 0;
+  if (plan.gram_kernel) return plan.period == 4 ? (plan.gram_len == 16 ? 0.25 : 0.18) : plan.period == 2 ? 0.27 : 0.55;
+  return plan.period == 4 ? 0.9 : plan.period == 2 ? 1.5 : 2.6;
+}
+
+double literals_ms_per_gib(const ws_pattern_tables& t) {
+  std::vector<FilterString> strings;
+  for (uint32_t li = 0; li < t.n_literals; ++li)
+    strings.push_back({t.packed_bytes + t.offsets[2 * li], t.offsets[2 * li + 1]});
+  const Layout l = choose_layout(strings, strings.size());
+  LiteralPlan plan;
+  plan.n_strings = t.n_literals;
+  plan.gram_kernel = l.gram_kernel;
+  plan.period = l.period;
+  plan.gram_len = l.gram_len;
+  return filter_ms_per_gib(plan);
 }
 
 void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan, const std::vector<std::string>& prefixes) {
@@ -274,7 +317,7 @@ void plan_literals(const ws_pattern_tables& given, LiteralPlan& plan, const std:
   for (const std::string& x : pre) strings.push_back({reinterpret_cast<const uint8_t*>(x.data()), (uint32_t)x.size()});
   plan.max_len = 0;
   for (const FilterString& f : strings) plan.max_len = std::max(plan.max_len, f.len);
-  const Layout layout = choose_layout(strings);
+  const Layout layout = choose_layout(strings, t.n_literals);
   plan.has_long = layout.has_long;
   plan.has_short = layout.has_short;
   plan.period = layout.period;
@@ -512,6 +555,6 @@ extern "C" void ws_testing_literal_layout(const ws_ir* ir, unsigned* out) {
   std::vector<FilterString> strings;
   for (size_t k = 0; k < ir->d.literal_pattern_ids.size(); ++k)
     strings.push_back({ir->d.packed_bytes.data() + ir->d.offsets[2 * k], ir->d.offsets[2 * k + 1]});
-  const Layout l = choose_layout(strings);
+  const Layout l = choose_layout(strings, strings.size());
   out[0] = l.period, out[1] = l.gram_len, out[2] = l.gram_kernel ? 1 : 0;
 }

@@ -243,8 +243,9 @@ uint32_t enqueue_scan(ws_matcher* m, Scratch& s, cudaStream_t st, const uint8_t*
 uint32_t enqueue_scan(ws_matcher* m, RegexPlan& rx, const LiteralPlan& lit, Scratch& s, cudaStream_t st,
                       const uint8_t* d_data, uint64_t len, ws_match* d_out, uint64_t cap, unsigned long long* d_counter,
                       const ScanExtras& x);
-// Whether the matcher's scans by these plans look for the regexes' prefixes.
-bool scans_prefixes(const ws_matcher* m, const RegexPlan& rx, const LiteralPlan& lit);
+// Whether the matcher's scans of `len` bytes by these plans look for the regexes'
+// prefixes.
+bool scans_prefixes(const ws_matcher* m, const RegexPlan& rx, const LiteralPlan& lit, uint64_t len);
 // Waits for the last profiled scan and reads its phase times (ms[8], the
 // layout of ws_matcher_info.last_kernel_ms).
 void read_phases(ws_matcher* m, double* ms);

@@ -186,6 +186,13 @@ void plan_filter(const ws_pattern_tables& t, const RegexPlan& P, LiteralPlan& pl
     entry.insert(entry.end(), {e.w0, e.w1, e.mask, e.r});
   }
   for (size_t k = 1; k < range.size(); ++k) range[k] += range[k - 1];
+  // A pass of the compacting kernels takes longer than a walk of one group, 0.55
+  // ms per GiB (a group with assertions 6): there the filter serves inputs up to
+  // the size where that eats the 0.15 ms that a small walk and its reverse walks
+  // take at least.
+  const double extra = filter_ms_per_gib(plan) - literals_ms_per_gib(t) -
+                       (0.55 * (P.n_spec - P.n_walk) + 6.0 * (P.n_groups - P.n_ctx_walk));
+  plan.prefix_most = plan.gram_kernel || extra <= 0 ? UINT64_MAX : (uint64_t)(0.15 / extra * (1ull << 30));
   plan.prefix_shift = 32 - bits;
   plan.n_prefixes = (uint32_t)es.size();
   plan.d_prefix_range.upload(range.data(), range.size() * 4);

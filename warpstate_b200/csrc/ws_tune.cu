@@ -47,7 +47,7 @@ double time_scan(ws_matcher* m, RegexPlan& P, const LiteralPlan& lit, const uint
   check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
   check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
   const bool whole = m->cfg.regex_mode != WS_REGEX_SPECULATIVE ||
-                     (scans_prefixes(m, P, lit) && P.n_walk == 0 && P.n_ctx_walk == P.n_spec);
+                     (scans_prefixes(m, P, lit, len) && P.n_walk == 0 && P.n_ctx_walk == P.n_spec);
   ScanExtras x;
   x.literals = false;
   Scratch s;  // (of its own: a pooled one would keep buffers of this size)
