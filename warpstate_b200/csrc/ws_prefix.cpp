@@ -112,14 +112,15 @@ void drop_shared(RegexPlan& P) {
 // the literals allow too: 7 bytes for every fourth, 5 for every second.  Longer
 // prefixes are more strings (a class in the prefix multiplies them): at most
 // 4,096 at 7 bytes and 16,384 at 5, beyond which the crowded filter costs more
-// than the lookups it saves.  A set whose 4-byte grams crowd their alphabet
-// takes 20 bytes (16-byte grams), and there one short string would choose the
-// layout of all: 4-byte grams, nearly all of which a nucleotide input passes.  So
-// a regex is covered there only if each of its strings has the 19 bytes that
-// 16-byte grams at every fourth position need; the others are walked (20,000
-// k-mers and 100 motifs over 512 MiB, us a scan: with one motif more of 8 bases
-// 19,600 -> 1,560, of 12 bases 1,810 -> 950).  Where no length is possible, every
-// regex is walked.
+// than the lookups it saves.  A set whose strings would fill the survivor list on
+// an input over their alphabet, or whose literals would lose their long grams
+// (filter_crowded), takes 20 bytes (16-byte grams), and there one short string
+// would choose the layout of all: 4-byte grams, nearly all of which a nucleotide
+// input passes.  So a regex is covered there only if each of its strings has the
+// 19 bytes that 16-byte grams at every fourth position need; the others are walked
+// (20,000 k-mers and 100 motifs over 512 MiB, us a scan: with one motif more of 8
+// bases 19,600 -> 1,190, of 12 bases 1,810 -> 640).  Where no length is possible,
+// every regex is walked.
 void choose_prefixes(const ws_pattern_tables& t, RegexPlan& P) {
   P.prefix_len = -1;
   drop_shared(P);
