@@ -2104,8 +2104,9 @@ uint32_t regex_finish(RegexPlan& P, RegexScan& rs, const RegexLaunch& l, cudaStr
   launch_pdl(k_scatter_kernel, hg, 256, osmem, st, p, P.n_regex);
   launches += 1;
   if (rs.prefixes && t.n_walk == 0 && t.n_ctx_walk == P.n_spec) {
-    // a block per regex; at least two per SM, for long lists
-    const uint32_t blocks = std::min<uint32_t>(std::max<uint32_t>(P.n_regex, 2 * sm_count), 4096);
+    // a block per regex; for long lists one per 16 KiB, at most two per SM, if that is more
+    const uint32_t shared = (uint32_t)std::min<uint64_t>(l.len >> 14, 2 * (uint64_t)sm_count);
+    const uint32_t blocks = std::min<uint32_t>(std::max<uint32_t>(P.n_regex, shared), 4096);
     launch_pdl(k_resolve_kernel, blocks, kChainThreads, 0, st, t, p, P.n_regex, l.need);
     launches += 1;
   } else {
